@@ -1,11 +1,12 @@
 // explicit_s.cuh — the explicit reduced camera system S and its banded tiled FP64 Cholesky factor.
 //
 // S = U - W Vhat^-1 W^T over the free camera parameters (schur/assembly.rs:832-1069 assembles the same
-// matrix into faer's sparse pattern, sparse/direct_assembly.rs:371-687). Here it is built by block
-// rows: one CTA per parameter block X computes every block S_XY of its row (all co-visible blocks Y,
-// both triangles), walking X's entities in a fixed order and the entities of each entity's point, so
-// the row is the same bits run to run and needs no atomics. The rows serve as a block-sparse (BSR)
-// operator directly (the PCG product and the model reduction) and are scattered into a banded tiled
+// matrix into faer's sparse pattern, sparse/direct_assembly.rs:371-687). It is built from camera
+// pairs (pair_rows.cuh), or, where their lists do not fit the caller's workspace budget, by block rows:
+// one CTA per parameter block X computes every block S_XY of its row (all co-visible blocks Y, both
+// triangles), walking X's entities in a fixed order and the entities of each entity's point, so the
+// row is the same bits run to run, needs no atomics and no storage beyond the rows. The rows serve as
+// a block-sparse (BSR) operator directly (the PCG product and the model reduction) and are scattered into a banded tiled
 // matrix for the factorization.
 //
 // Factorization. The parameter blocks are permuted so that each camera's pose block is followed by

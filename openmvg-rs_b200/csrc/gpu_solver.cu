@@ -961,6 +961,7 @@ __global__ void k_pcg_direction(int n, const double* __restrict__ rr_part, const
 #include "mv_tiles.cuh"
 #include "asm_tiles.cuh"
 #include "explicit_s.cuh"
+#include "pair_rows.cuh"
 #include "two_view.cuh"
 namespace omvgba {
 
@@ -2250,6 +2251,17 @@ struct Solver {
   DBuf<double> d_rows, d_tiles, d_winv, d_ztiles, d_perm_vec, d_marg_out, d_power;
   bool rows_valid = false;  // the rows hold S of the current assembly
   bool rows_attr = false;   // k_block_rows may take kRowSmemDoubles of dynamic shared memory
+  // camera pairs of the explicit S (pair_rows.cuh), built at the first build of the rows
+  enum PairState { kPairsUnknown, kPairsReady, kPairsUnusable } pair_state = kPairsUnknown;
+  CamPairs cam_pairs{};
+  uint32_t heavy_ctas = 0;
+  DBuf<uint32_t> d_pr_point, d_pr_cam_begin, d_pr_cam_obs, d_pr_adj_begin, d_pr_adj, d_pr_up_begin, d_pr_item_begin,
+      d_pr_item_pair, d_pr_cont_begin, d_pr_heavy;
+  DBuf<int> d_pr_unit;
+  DBuf<uint64_t> d_pr_list_begin;
+  DBuf<uint2> d_pr_entries, d_pr_cont;
+  DBuf<double> d_pr_operands, d_pr_part;
+  bool pairs_attr = false;  // k_pair_operands may stage a tile of the widest cameras
   bool asm_attr = false;    // k_block_tiles stages kAsmComp (TILE + 1) doubles in dynamic shared memory
   DBuf<double> d_asm_rec;   // per (block, segment) assembly records, kAsmRecordScale per partial element
   // PCG vectors
@@ -2703,7 +2715,228 @@ struct Solver {
     OMVGBA_LAUNCH(k_block_records, nb, 128, 0, st, mt, bt.blk_edge, d_asm_rec.p, d_blk_out.p);
   }
 
+  // The camera-pair tables, once per solver; false when the pairs do not serve this problem: more
+  // cameras than a neighbour bitmap holds, operands and lists past kPairMaxBytes, or past what the
+  // caller's workspace budget leaves. Those build by block rows (k_block_rows), which needs no storage
+  // of its own.
+  static constexpr uint64_t kPairMaxBytes = uint64_t(48) << 30;
+  static constexpr int kPairMaxCameras = 8 * 48 * 1024;
+  bool ensure_pairs() {
+    if (pair_state != kPairsUnknown) return pair_state == kPairsReady;
+    pair_state = kPairsUnusable;
+    int widest = 0;
+    for (int c = 0; c < n.ncam; ++c)
+      widest = std::max(widest, L.pose_dim[c] + (n.self_cal ? L.intr_dim[n.cam_group[c]] : 0));
+    if (N == 0 || nb == 0 || widest == 0 || n.ncam > kPairMaxCameras) return false;
+    const int ncam = n.ncam, gw = 3 * widest;
+    uint64_t bytes = 2 * sizeof(double) * (uint64_t)N * gw + 2 * sizeof(uint32_t) * (uint64_t)N;
+    auto fits = [&](uint64_t b) {
+      return b <= kPairMaxBytes && (!opt.workspace_budget || workspace_bytes + b <= opt.workspace_budget);
+    };
+    if (!fits(bytes)) return false;
+    CamPairs t{};
+    t.ncam = ncam;
+    t.gw = gw;
+    t.pt_off = d_pt_off.p;
+    t.obs_cam = d_obs_cam.p;
+    t.fixed_points = d_fixed_points.p;
+    // cameras' observations
+    d_pr_point.alloc(N, st);
+    OMVGBA_LAUNCH(k_pair_obs_point, grid_for(P, 256), 256, 0, st, P, d_pt_off.p, d_pr_point.p);
+    t.obs_point = d_pr_point.p;
+    d_pr_unit.alloc(ncam, st);
+    OMVGBA_LAUNCH(k_pair_units, grid_for(ncam, 256), 256, 0, st, ncam, d_pose_dim.p, d_cam_group.p, d_intr_dim.p,
+                  n.self_cal ? 1 : 0, d_pr_unit.p);
+    t.unit_dim = d_pr_unit.p;
+    const int nchunks = (int)std::min<size_t>(512, ((size_t)N + 1023) / 1024);
+    const uint32_t per = (uint32_t)(((size_t)N + nchunks - 1) / nchunks);
+    DBuf<uint32_t> counts, total, full, upper;
+    counts.alloc((size_t)nchunks * ncam, st);
+    counts.zero();
+    total.alloc(ncam, st);
+    d_pr_cam_begin.alloc(ncam + 1, st);
+    d_pr_cam_obs.alloc(N, st);
+    OMVGBA_LAUNCH(k_pair_cam_sort, nchunks, 32, 0, st, (uint32_t)N, per, ncam, d_obs_cam.p, counts.p,
+                  (const uint32_t*)nullptr, (uint32_t*)nullptr);
+    OMVGBA_LAUNCH(k_pair_cam_prefix, grid_for(ncam, 128), 128, 0, st, ncam, nchunks, counts.p, total.p);
+    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, total.p, (size_t)ncam, d_pr_cam_begin.p);
+    OMVGBA_LAUNCH(k_pair_cam_sort, nchunks, 32, 0, st, (uint32_t)N, per, ncam, d_obs_cam.p, counts.p,
+                  (const uint32_t*)d_pr_cam_begin.p, d_pr_cam_obs.p);
+    t.cam_begin = d_pr_cam_begin.p;
+    t.cam_obs = d_pr_cam_obs.p;
+    // neighbours
+    const size_t bits = sizeof(uint32_t) * (size_t)((ncam + 31) / 32);
+    full.alloc(ncam, st);
+    upper.alloc(ncam, st);
+    d_pr_adj_begin.alloc(ncam + 1, st);
+    d_pr_up_begin.alloc(ncam + 1, st);
+    OMVGBA_LAUNCH(k_pair_neighbours, ncam, 256, bits, st, t, full.p, upper.p, (uint32_t*)nullptr);
+    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, full.p, (size_t)ncam, d_pr_adj_begin.p);
+    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, upper.p, (size_t)ncam, d_pr_up_begin.p);
+    check_launch();
+    uint32_t nadj = 0;
+    CUDA_OK(copy_async(&nadj, d_pr_adj_begin.p + ncam, sizeof(nadj), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(copy_async(&t.npairs, d_pr_up_begin.p + ncam, sizeof(t.npairs), cudaMemcpyDeviceToHost, st));
+    sync();
+    t.adj_begin = d_pr_adj_begin.p;
+    t.up_begin = d_pr_up_begin.p;
+    d_pr_adj.alloc(std::max<uint32_t>(nadj, 1), st);
+    OMVGBA_LAUNCH(k_pair_neighbours, ncam, 256, bits, st, t, (uint32_t*)nullptr, (uint32_t*)nullptr, d_pr_adj.p);
+    t.adj = d_pr_adj.p;
+    // lists: a warp per (camera, segment of about 256 observations)
+    t.segs = (int)std::min<size_t>(256, std::max<size_t>(1, (size_t)N / ncam / 256));
+    while (t.segs > 1 && (uint64_t)t.npairs * t.segs > (uint64_t(1) << 26)) t.segs /= 2;
+    const size_t cells = (size_t)t.npairs * t.segs;
+    DBuf<uint32_t> cell_count;
+    DBuf<uint64_t> cursor;
+    cell_count.alloc(std::max<size_t>(cells, 1), st);
+    cell_count.zero();
+    cursor.alloc(cells + 1, st);
+    d_pr_list_begin.alloc(cells + 1, st);
+    OMVGBA_LAUNCH(k_pair_lists<uint32_t>, dim3(ncam, t.segs), 32, 0, st, t, cell_count.p, (uint2*)nullptr);
+    OMVGBA_LAUNCH(k_pair_scan<uint64_t>, 1, 1024, 0, st, cell_count.p, cells, d_pr_list_begin.p);
+    t.list_begin = d_pr_list_begin.p;
+    check_launch();
+    uint64_t entries = 0;
+    CUDA_OK(copy_async(&entries, d_pr_list_begin.p + cells, sizeof(entries), cudaMemcpyDeviceToHost, st));
+    sync();
+    // items of at most 256 entries, fewer when that would leave less than two items per resident warp slot
+    // of the chip's SMs
+    t.chunk = (uint32_t)std::min<uint64_t>(256, std::max<uint64_t>(32, entries / (148 * 32) / 32 * 32));
+    bytes += sizeof(uint2) * entries + sizeof(double) * kPairPart * (entries / t.chunk + t.npairs) +
+             sizeof(uint64_t) * cells + sizeof(uint2) * S.nbr.size();
+    if (!fits(bytes) || t.npairs >= (1u << 31)) {
+      for (DBuf<uint32_t>* d : {&d_pr_point, &d_pr_cam_begin, &d_pr_cam_obs, &d_pr_adj_begin, &d_pr_adj, &d_pr_up_begin})
+        d->release();
+      d_pr_list_begin.release();
+      d_pr_unit.release();
+      return false;
+    }
+    CUDA_OK(cudaMemcpyAsync(cursor.p, d_pr_list_begin.p, sizeof(uint64_t) * (cells + 1), cudaMemcpyDeviceToDevice, st));
+    d_pr_entries.alloc(std::max<uint64_t>(entries, 1), st);
+    OMVGBA_LAUNCH(k_pair_lists<uint64_t>, dim3(ncam, t.segs), 32, 0, st, t, cursor.p, d_pr_entries.p);
+    t.entries = d_pr_entries.p;
+    DBuf<uint32_t> item_count, cont_count;
+    item_count.alloc(std::max<uint32_t>(t.npairs, 1), st);
+    d_pr_item_begin.alloc(t.npairs + 1, st);
+    if (t.npairs > 0)
+      OMVGBA_LAUNCH(k_pair_item_count, grid_for(t.npairs, 256), 256, 0, st, t, item_count.p);
+    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, item_count.p, (size_t)t.npairs, d_pr_item_begin.p);
+    t.item_begin = d_pr_item_begin.p;
+    // contributions of the pairs to the blocks of S
+    std::vector<uint32_t> bc_begin(nb + 1, 0), bc_cams;
+    std::vector<int> blk_pose(nb, -1), blk_group(nb, -1);
+    for (int c = 0; c < ncam; ++c)
+      if (S.cam_block[c] >= 0) blk_pose[S.cam_block[c]] = c;
+    for (size_t g = 0; g < S.grp_block.size(); ++g)
+      if (S.grp_block[g] >= 0) blk_group[S.grp_block[g]] = (int)g;
+    if (n.self_cal)
+      for (int c = 0; c < ncam; ++c)
+        if (const int b = S.grp_block[n.cam_group[c]]; b >= 0) ++bc_begin[b + 1];
+    for (int b = 0; b < nb; ++b) bc_begin[b + 1] = bc_begin[b] + (blk_pose[b] >= 0 ? 1 : bc_begin[b + 1]);
+    bc_cams.resize(std::max<uint32_t>(bc_begin[nb], 1));
+    std::vector<uint32_t> at(bc_begin.begin(), bc_begin.end() - 1);
+    for (int c = 0; c < ncam; ++c) {
+      if (S.cam_block[c] >= 0) bc_cams[at[S.cam_block[c]]++] = (uint32_t)c;
+      if (n.self_cal)
+        if (const int b = S.grp_block[n.cam_group[c]]; b >= 0) bc_cams[at[b]++] = (uint32_t)c;
+    }
+    DBuf<uint32_t> d_bc_begin, d_bc_cams, heavy_n;
+    DBuf<int> d_blk_pose, d_blk_group;
+    d_bc_begin.upload(bc_begin.data(), bc_begin.size(), st);
+    d_bc_cams.upload(bc_cams.data(), bc_cams.size(), st);
+    d_blk_pose.upload(blk_pose.data(), blk_pose.size(), st);
+    d_blk_group.upload(blk_group.data(), blk_group.size(), st);
+    const BlockCams bc{d_bc_begin.p, d_bc_cams.p, d_blk_pose.p, d_blk_group.p, d_cam_group.p, d_pose_dim.p};
+    const uint32_t slots = (uint32_t)S.nbr.size();
+    cont_count.alloc(std::max<uint32_t>(slots, 1), st);
+    d_pr_cont_begin.alloc(slots + 1, st);
+    d_pr_heavy.alloc(slots + 1, st);  // the number of heavy blocks, then the blocks
+    CUDA_OK(cudaMemsetAsync(d_pr_heavy.p, 0, sizeof(uint32_t), st));
+    OMVGBA_LAUNCH(k_pair_slots, grid_for(slots, 8), 256, 0, st, t, bc, slots, d_nbr.p, d_nbr_row.p, cont_count.p,
+                  (const uint32_t*)nullptr, (uint2*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr);
+    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, cont_count.p, (size_t)slots, d_pr_cont_begin.p);
+    check_launch();
+    uint32_t nitems = 0, ncont = 0;
+    CUDA_OK(copy_async(&nitems, d_pr_item_begin.p + t.npairs, sizeof(nitems), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(copy_async(&ncont, d_pr_cont_begin.p + slots, sizeof(ncont), cudaMemcpyDeviceToHost, st));
+    sync();
+    t.nitems = nitems;
+    d_pr_item_pair.alloc(std::max<uint32_t>(nitems, 1), st);
+    d_pr_cont.alloc(std::max<uint32_t>(ncont, 1), st);
+    if (t.npairs > 0) OMVGBA_LAUNCH(k_pair_item_fill, grid_for(t.npairs, 256), 256, 0, st, t, d_pr_item_pair.p);
+    t.item_pair = d_pr_item_pair.p;
+    OMVGBA_LAUNCH(k_pair_slots, grid_for(slots, 8), 256, 0, st, t, bc, slots, d_nbr.p, d_nbr_row.p,
+                  (uint32_t*)nullptr, (const uint32_t*)d_pr_cont_begin.p, d_pr_cont.p, d_pr_heavy.p, d_pr_heavy.p + 1);
+    check_launch();
+    uint32_t heavy = 0;
+    CUDA_OK(copy_async(&heavy, d_pr_heavy.p, sizeof(heavy), cudaMemcpyDeviceToHost, st));
+    d_pr_operands.alloc((size_t)2 * N * gw, st);
+    d_pr_part.alloc((size_t)kPairPart * std::max<uint32_t>(nitems, 1), st);
+    sync();
+    heavy_ctas = heavy;
+    // the tables the build does not read again
+    d_pr_point.release();
+    d_pr_cam_begin.release();
+    d_pr_cam_obs.release();
+    cam_pairs = t;
+    pair_state = kPairsReady;
+    return true;
+  }
+
+  // S of the current linearization. The camera-side records (camera_sums) must be those of the same
+  // linearization.
   void build_rows() {
+    const bool timing = std::getenv("OMVGBA_PHASE_TIMES") != nullptr;
+    if (timing) sync();
+    const double t0 = now();
+    if (ensure_pairs())
+      build_rows_by_pairs();
+    else
+      build_rows_by_block();
+    check_launch();
+    if (timing) {
+      sync();
+      std::fprintf(stderr, "[omvgba] block rows %.4fs (%d blocks, %zu entries)\n", now() - t0, nb, S.nbr.size());
+    }
+    rows_valid = true;
+  }
+
+  void build_rows_by_pairs() {
+    const CamPairs& t = cam_pairs;
+    const TileSetDev& ts = mixed ? dT32 : dT64;
+    const MvTiles mt = ts.view(d_blk_dim.p, d_blk_off.p, nb);
+    double *w_op = d_pr_operands.p, *e_op = w_op + (size_t)N * t.gw;
+    const size_t smem = sizeof(double) * t.gw * (mixed ? mv_tile_obs<float>() : mv_tile_obs<T>());
+    if (!pairs_attr) {
+      CUDA_OK(cudaFuncSetAttribute(k_pair_operands<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(sizeof(double) * 3 * kPairDim * mv_tile_obs<float>())));
+      CUDA_OK(cudaFuncSetAttribute(k_pair_operands<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(sizeof(double) * 3 * kPairDim * mv_tile_obs<T>())));
+      pairs_attr = true;
+    }
+    if (mixed)
+      OMVGBA_LAUNCH(k_pair_operands<float>, mt.ntiles, mv_tile_obs<float>(), smem, st, mt, lin32(), t.gw, d_pt_off.p, w_op,
+                    e_op);
+    else
+      OMVGBA_LAUNCH(k_pair_operands<T>, mt.ntiles, mv_tile_obs<T>(), smem, st, mt, lin(), t.gw, d_pt_off.p, w_op,
+                    e_op);
+    if (t.nitems > 0) {
+      if (t.gw == 3 * kPairDim)
+        OMVGBA_LAUNCH(k_pair_products<true>, grid_for(t.nitems, 8), 256, 0, st, t, w_op, e_op, d_pr_part.p);
+      else
+        OMVGBA_LAUNCH(k_pair_products<false>, grid_for(t.nitems, 8), 256, 0, st, t, w_op, e_op, d_pr_part.p);
+    }
+    const RowTables rt = row_tables();
+    OMVGBA_LAUNCH(k_pair_gather, grid_for(rt.entries, 8), 256, 0, st, t, rt, d_pr_cont_begin.p, d_pr_cont.p,
+                  d_pr_part.p, d_blk_out.p, d_blk_edge.p, d_rows.p);
+    if (heavy_ctas > 0)
+      OMVGBA_LAUNCH(k_pair_gather_heavy, std::min<uint32_t>(heavy_ctas, 4096), 36 * kPairShares, 0, st, t, rt,
+                    d_pr_cont_begin.p, d_pr_cont.p, d_pr_part.p, d_blk_out.p, d_blk_edge.p, d_pr_heavy.p,
+                    d_pr_heavy.p + 1, d_rows.p);
+  }
+
+  void build_rows_by_block() {
     const int row_smem = (int)std::min<uint64_t>(S.max_row, (uint64_t)kRowSmemDoubles);
     const size_t smem = (size_t)row_smem * sizeof(double);
     if (!rows_attr) {
@@ -2713,19 +2946,10 @@ struct Solver {
                                    kRowSmemDoubles * (int)sizeof(double)));
       rows_attr = true;
     }
-    const bool timing = std::getenv("OMVGBA_PHASE_TIMES") != nullptr;
-    if (timing) sync();
-    const double t0 = now();
     if (mixed)
       OMVGBA_LAUNCH(k_block_rows<float>, nb, kRowThreads, smem, st, row_tables(), lin32(), row_smem, d_rows.p);
     else
       OMVGBA_LAUNCH(k_block_rows<T>, nb, kRowThreads, smem, st, row_tables(), lin(), row_smem, d_rows.p);
-    check_launch();
-    if (timing) {
-      sync();
-      std::fprintf(stderr, "[omvgba] block rows %.4fs (%d blocks, %zu entries)\n", now() - t0, nb, S.nbr.size());
-    }
-    rows_valid = true;
   }
 
   // y = (S + lambda diag) x from the rows

@@ -1,0 +1,112 @@
+"""The explicit reduced camera system built from camera pairs (csrc/pair_rows.cuh) against the
+matrix-free product of the same linearization, where its pair lists, items and blocks can go wrong:
+cameras that see a point twice, pose masks and the S^2 chart (pose dimensions 2 to 6), fixed poses with
+free intrinsics, one shared intrinsic group (a block that collects every pair), a group per camera (the
+9-parameter products), fixed points, angular residuals, and few cameras with long lists.
+
+Both products sum the same terms in FP64 in different orders, so they agree to rounding of the largest
+entries: 1e-9 of the product's largest value, the tolerance of the operator parity tests."""
+import numpy as np
+import pytest
+
+from openmvg_ba_cuda import CameraIntrinsics, Gauge, RobustLoss, SolveConfig, abi, synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+def _ring(**kw):
+    return synthetic.ring_problem(seed=6, **kw)
+
+
+def _seen_twice():
+    p = _ring(points=300)
+    keep = np.arange(0, p.observation_count, 3)  # a third of the observations once more, moved by a pixel
+    p.observation_pose = np.concatenate([p.observation_pose, p.observation_pose[keep]])
+    p.observation_intrinsic = np.concatenate([p.observation_intrinsic, p.observation_intrinsic[keep]])
+    p.observation_point = np.concatenate([p.observation_point, p.observation_point[keep]])
+    p.observation_pixel = np.vstack([p.observation_pixel, p.observation_pixel[keep] + 1.0])
+    return p
+
+
+def _masks():
+    return _ring(points=400, pose_variables=np.array([0, 0] + [1, 2, 3] * 6, dtype=np.uint32))
+
+
+def _baseline():
+    p = _ring(points=400)
+    p.pose_variables[0] = 0
+    p.gauge = Gauge.fixed_baseline(0, 3, float(np.linalg.norm(p.centers[3] - p.centers[0])))
+    return p
+
+
+def _shared_group():
+    return _ring(self_calibrating=True, radius=3.0)
+
+
+def _two_groups_fixed_pose():
+    p = _ring(points=500, self_calibrating=True, radius=3.0)
+    second = CameraIntrinsics(model=abi.CAMERA_BROWN_CONRADY, fx=498.0, fy=498.0, cx=320.0, cy=240.0,
+                              radial_kind=abi.RADIAL_K1K2, k1=-0.1, k2=0.0, variables=abi.INTRINSIC_FOCAL)
+    p.intrinsics = p.intrinsics + [second]
+    p.observation_intrinsic = (p.observation_pose % 2).astype(np.uint32)
+    p.pose_variables[[0, 5]] = 0
+    return p
+
+
+def _group_per_camera():
+    p = synthetic.plane_problem(seed=12, cameras=37, points=3001, mean_track=6.5, extent=27.0)
+    # without damping a point needs parallax: keep those with three views
+    keep = (np.bincount(p.observation_point, minlength=len(p.points)) >= 3)[p.observation_point]
+    points, index = np.unique(p.observation_point[keep], return_inverse=True)
+    p.points, p.point_fixed, p.observation_point = p.points[points], p.point_fixed[points], index.astype(np.uint32)
+    p.observation_pose, p.observation_intrinsic = p.observation_pose[keep], p.observation_intrinsic[keep]
+    p.observation_pixel = p.observation_pixel[keep]
+    return p
+
+
+def _fixed_points():
+    p = _ring(points=400)
+    p.point_fixed[::4] = 1
+    return p
+
+
+def _few_cameras():
+    return _ring(cameras=8, points=6001)
+
+
+CASES = {f.__name__[1:]: f for f in (_seen_twice, _masks, _baseline, _shared_group, _two_groups_fixed_pose,
+                                     _group_per_camera, _fixed_points, _few_cameras)}
+
+
+@pytest.mark.parametrize("case", sorted(CASES))
+@pytest.mark.parametrize("damping", [0.0, 1e-2])
+def test_pair_rows_equal_the_matrix_free_product(adjuster, case, damping):
+    p = CASES[case]()
+    p.robust_loss = RobustLoss.huber(1.0)
+    d = adjuster.debug_schur_product(p, None)
+    rng = np.random.default_rng(1)
+    for _ in range(2):
+        x = rng.standard_normal(d)
+        free, explicit = adjuster.debug_schur_product(p, x, damping)
+        assert np.max(np.abs(free - explicit)) <= 1e-9 * np.max(np.abs(explicit))
+
+
+def test_a_budget_without_room_for_the_pairs_builds_by_block_rows(adjuster):
+    """The two builds of S take the same steps: a budget that leaves no room for the pair lists uses
+    k_block_rows, and the solves agree to rounding."""
+    p = _ring(points=600)
+    cfg = SolveConfig(linear_solver=abi.SOLVER_DIRECT, max_iterations=6)
+    free = adjuster.solve(p, cfg)
+    budget = 1 << 20  # grow until the solve is accepted: the first accepted budget has no slack for the pairs
+    while True:
+        try:
+            tight = adjuster.solve(p, cfg.with_(workspace_budget_bytes=budget))
+            break
+        except Exception as e:
+            assert "budget" in str(e)
+            budget += 1 << 16
+    assert tight.report["iteration_count"] == free.report["iteration_count"]
+    rel = abs(tight.report["final_objective"] - free.report["final_objective"]) / free.report["final_objective"]
+    assert rel <= 1e-9
+    assert np.max(np.abs(tight.points - free.points)) <= 1e-7
+    assert np.max(np.abs(tight.centers - free.centers)) <= 1e-7
