@@ -24,6 +24,8 @@
 // covariances (sparse/covariance.rs:564-587) from the selected inverse of S inside the band.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include <cstdint>
 
 namespace omvgba {
@@ -400,331 +402,366 @@ __global__ void k_tiles_pad(TileBand tb) {
   tb.t[tile_at(tb, i, i) + (size_t)(r % kCT) * kCT + (r % kCT)] = 1.0;
 }
 
-// Operands of the tile products are staged in shared memory with a padded row of kTS doubles (16-byte
-// aligned rows; transposed stores hit 8 banks per warp instead of one).
-constexpr int kTS = 66;
+// Tiles in shared memory keep their column-major order with a column stride of kTS doubles: 4 modulo 16,
+// so that the FP64 tensor fragments below read 16 different 8-byte banks per half warp both along a
+// tile's columns and along its rows. Every operand is therefore staged by plain 16-byte asynchronous
+// copies, transposed or not.
+constexpr int kTS = 68;
 constexpr size_t kStagedTile = sizeof(double) * kCT * kTS;
 
-// acc (4 x 4 per thread, 16 x 16 threads) += A B for 64 x 64 tiles staged as Ta[q * kTS + r] = A(r, q)
-// and Tb[q * kTS + c] = B(q, c); the sum over q runs in order.
-__device__ __forceinline__ void tile_mma_acc(const double* Ta, const double* Tb, double acc[4][4]) {
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+// Copies the column-major tile g into T (256 threads); complete after stage_wait() and a barrier.
+__device__ __forceinline__ void stage_tile(const double* __restrict__ g, double* T) {
+#pragma unroll
+  for (int i = 0; i < kCTT / 2 / 256; ++i) {
+    const int w = threadIdx.x + 256 * i, c = w >> 5, r = (w & 31) * 2;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(T + c * kTS + r);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(g + 2 * (size_t)w) : "memory");
+  }
+}
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// A 64 x 64 product on the FP64 tensor pipe (m8n8k4), 8 warps: warp w owns rows 16 (w / 2) .. + 15 and
+// columns 32 (w % 2) .. + 31 of the result, acc[i][j][e] being element (8 i + g, 8 j + 2 t + e) of
+// that part for lane 4 g + t. The sum over the tile's 64 columns runs in order, four at a time.
+// Against the 4 x 4-outputs-per-thread loop on the FP64 cores and the transposing copies it replaced
+// (500-camera survey, 14 tiles a column, per launch): trsm 15.0 -> 6.2 us, update 17.4 -> 7.0 us,
+// Takahashi partial sums 41.6 -> 16.0 us, off-diagonal tiles 34.3 -> 21.2 us.
+struct TileAcc {
+  double v[2][4][2];
+};
+__device__ __forceinline__ void zero_acc(TileAcc& acc) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc.v[i][j][0] = acc.v[i][j][1] = 0.0;
+}
+// acc += op(Ta) op(Tb), op the transpose when AT / BT is set.
+template <bool AT, bool BT>
+__device__ __forceinline__ void tile_mma_acc(const double* Ta, const double* Tb, TileAcc& acc) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int r0 = 16 * (w >> 1) + g, c0 = 32 * (w & 1) + g;
 #pragma unroll 4
-  for (int q = 0; q < kCT; ++q) {
-    const double2 a01 = *reinterpret_cast<const double2*>(Ta + q * kTS + 4 * ty);
-    const double2 a23 = *reinterpret_cast<const double2*>(Ta + q * kTS + 4 * ty + 2);
-    const double2 b01 = *reinterpret_cast<const double2*>(Tb + q * kTS + 4 * tx);
-    const double2 b23 = *reinterpret_cast<const double2*>(Tb + q * kTS + 4 * tx + 2);
-    const double av[4] = {a01.x, a01.y, a23.x, a23.y}, bv[4] = {b01.x, b01.y, b23.x, b23.y};
+  for (int k0 = 0; k0 < kCT; k0 += 4) {
+    const int k = k0 + t;
+    double a[2], b[4];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int i = 0; i < 2; ++i) a[i] = AT ? Ta[(r0 + 8 * i) * kTS + k] : Ta[k * kTS + r0 + 8 * i];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] += av[a] * bv[b];
+    for (int j = 0; j < 4; ++j) b[j] = BT ? Tb[k * kTS + c0 + 8 * j] : Tb[(c0 + 8 * j) * kTS + k];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dmma_m8n8k4(a[i], b[j], acc.v[i][j][0], acc.v[i][j][1]);
   }
 }
-
-// Stage the column-major tile g (element (r, c) at g[c * 64 + r]) as the operand M = g (flip false)
-// or g^T (flip true), in the A layout (T[q * kTS + r] = M(r, q)) or the B layout (T[q * kTS + c] =
-// M(q, c)). Global reads run along g's storage (coalesced).
-__device__ __forceinline__ void stage_tile(const double* __restrict__ g, double* T, bool as_b, bool flip) {
-  const bool direct = as_b == flip;  // A of g and B of g^T keep g's column-major order
-  for (int w = threadIdx.x; w < kCTT; w += blockDim.x) {
-    const int c = w / kCT, r = w - c * kCT;  // g(r, c)
-    const double v = g[w];
-    if (direct)
-      T[c * kTS + r] = v;
-    else
-      T[r * kTS + c] = v;
-  }
+// f(row, column, value) over this thread's elements of the result.
+template <typename F>
+__device__ __forceinline__ void acc_each(const TileAcc& acc, F f) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int r0 = 16 * (w >> 1) + g, c0 = 32 * (w & 1) + 2 * t;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) f(r0 + 8 * i, c0 + 8 * j + e, acc.v[i][j][e]);
+}
+__device__ __forceinline__ void acc_store(const TileAcc& acc, double* g) {
+  acc_each(acc, [&](int r, int c, double v) { g[(size_t)c * kCT + r] = v; });
 }
 
-__device__ __forceinline__ void zero_acc(double acc[4][4]) {
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
+// C (8 x 8, column-major at stride kTS) += sign * A B for one warp, A and B read through the lambdas
+// a(row, k) and b(k, column), k < depth.
+template <typename FA, typename FB>
+__device__ __forceinline__ void mma8(int depth, FA a, FB b, double& c0, double& c1) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  for (int k0 = 0; k0 < depth; k0 += 4) dmma_m8n8k4(a(g, k0 + t), b(k0 + t, g), c0, c1);
 }
 
-// acc (output tile element (4 ty + a, 4 tx + b)) into a staged A operand: T[c * kTS + r] = scale acc(r, c)
-__device__ __forceinline__ void acc_to_a(const double acc[4][4], double scale, double* T) {
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) T[(4 * tx + b) * kTS + 4 * ty + a] = scale * acc[a][b];
-}
-
-__device__ __forceinline__ void acc_store(const double acc[4][4], double* g) {
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-#pragma unroll
-  for (int b = 0; b < 4; ++b)
-#pragma unroll
-    for (int a = 0; a < 4; ++a) g[(size_t)(4 * tx + b) * kCT + 4 * ty + a] = acc[a][b];
-}
-
-// POTRF of diagonal tile k and the inverse W_k = L_kk^-1 of its factor, both right-looking with the
-// tile in registers: thread (ty, tx) of 16 x 16 holds elements (4 ty + a, 4 tx + b). Step j of the
-// factorization publishes column j (its owners write it to shared memory, one barrier), and every
-// thread scales it by 1 / sqrt(pivot) and updates its elements right of the column; step j of the
-// inverse publishes the finished row j of W and every thread updates its rows below. The published
-// buffers alternate, so each step takes one barrier. status[0] = 0 when a pivot is not finite and
-// positive; later launches of the factorization then return at once.
+// POTRF of diagonal tile k and the inverse W_k = L_kk^-1 of its factor, one CTA of 8 warps, blocked by
+// 8 columns. A panel (all rows, 8 columns) is factored by warp 0 in registers, two rows per lane: a
+// step is one reciprocal root, one scaling and the shuffles that hand the pivot row's entries to the
+// columns right of it, with no barrier; then every warp subtracts the panel's rank-8 product from
+// its 8 x 8 blocks of the trailing triangle on the FP64 tensor pipe. The inverse of the factor starts
+// from the 8 x 8 diagonal blocks (a warp each) and doubles the block size three times with
+// W_21 = -W_22 (L_21 W_11), the products on the tensor pipe, their middle factor in the unused upper
+// triangle. Bound: the 64 dependent pivot steps. A right-looking factor with one barrier per column and
+// a second sweep of 64 barriers for the inverse took 64 us per tile; this takes 23.5.
+// status[0] = 0 when a pivot is not finite and positive; later launches of the factorization then
+// return at once.
+constexpr size_t kPotrfSmem = 2 * kStagedTile;
 __global__ void __launch_bounds__(256) k_tile_potrf(TileBand tb, int k, int* status) {
-  __shared__ double Ls[kCT * (kCT + 1)];  // the tile in, then L (column-major, padded)
-  __shared__ double pub[2][kCT];
-  __shared__ double piv[2][3];  // pivot, its square root and the root's reciprocal
+  extern __shared__ __align__(16) double sh[];
   __shared__ double rdiag[kCT];
+  __shared__ int s_bad;
   if (status[0] == 0) return;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  double* g = tb.t + tile_at(tb, k, k);
-  for (int w = tid; w < kCTT; w += blockDim.x) {
-    const int c = w / kCT, r = w - c * kCT;
-    Ls[c * (kCT + 1) + r] = g[w];
-  }
+  double* A = sh;               // the tile, then L; the strict upper triangle is scratch
+  double* W = sh + kCT * kTS;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+  double* gt = tb.t + tile_at(tb, k, k);
+  stage_tile(gt, A);
+  for (int i = tid; i < kCT * kTS; i += 256) W[i] = 0.0;
+  if (tid == 0) s_bad = 0;
+  stage_wait();
   __syncthreads();
-  double a[4][4];
+  for (int j0 = 0; j0 < kCT; j0 += 8) {
+    if (w == 0) {
+      double lo[8], hi[8];  // rows lane and lane + 32 of the panel
 #pragma unroll
-  for (int ai = 0; ai < 4; ++ai)
+      for (int c = 0; c < 8; ++c) {
+        lo[c] = A[(j0 + c) * kTS + lane];
+        hi[c] = A[(j0 + c) * kTS + lane + 32];
+      }
+      const bool upper_half = j0 >= 32;  // the panel's diagonal rows lie in hi
+      bool bad = false;
 #pragma unroll
-    for (int bi = 0; bi < 4; ++bi) a[ai][bi] = Ls[(4 * tx + bi) * (kCT + 1) + 4 * ty + ai];
-  for (int j = 0; j < kCT; ++j) {
-    double* cj = pub[j & 1];
-    if (tx == (j >> 2)) {  // static register indices: the column is picked by selects
-      const int bj = j & 3;
+      for (int c = 0; c < 8; ++c) {
+        const int pl = (j0 + c) & 31;
+        const double d = __shfl_sync(0xffffffffu, upper_half ? hi[c] : lo[c], pl);
+        bad = bad || !(isfinite(d) && d > 0.0);
+        const double rs = rsqrt(d);
+        lo[c] *= rs;
+        hi[c] *= rs;
+        if (lane == pl) {
+          const double sd = sqrt(d);
+          if (upper_half)
+            hi[c] = sd;
+          else
+            lo[c] = sd;
+          rdiag[j0 + c] = 1.0 / sd;
+        }
 #pragma unroll
-      for (int ai = 0; ai < 4; ++ai) {
-        const double v = bj == 0 ? a[ai][0] : (bj == 1 ? a[ai][1] : (bj == 2 ? a[ai][2] : a[ai][3]));
-        cj[4 * ty + ai] = v;
-        if (4 * ty + ai == j) {  // the diagonal's owner takes the root once for every thread
-          const double r = sqrt(v);
-          piv[j & 1][0] = v;
-          piv[j & 1][1] = r;
-          piv[j & 1][2] = 1.0 / r;
+        for (int c2 = c + 1; c2 < 8; ++c2) {
+          const double l = __shfl_sync(0xffffffffu, upper_half ? hi[c] : lo[c], (j0 + c2) & 31);
+          lo[c2] -= lo[c] * l;
+          hi[c2] -= hi[c] * l;
         }
       }
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {  // rows above the panel's diagonal are scratch
+        if (lane >= j0 + c) A[(j0 + c) * kTS + lane] = lo[c];
+        if (lane + 32 >= j0 + c) A[(j0 + c) * kTS + lane + 32] = hi[c];
+      }
+      if (bad && lane == 0) s_bad = 1;
     }
     __syncthreads();
-    const double d = piv[j & 1][0];  // the same value in every thread: all leave together
-    if (!(isfinite(d) && d > 0.0)) {
+    if (s_bad) {
       if (tid == 0) status[0] = 0;
       return;
     }
-    const double sd = piv[j & 1][1], rs = piv[j & 1][2];
-    // branch-free update: the multipliers of columns at or left of j are zero, so those columns keep
-    // their values; elements above the diagonal take values that are never read (zeroed on output)
-    double li[4], lc[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      li[q] = cj[4 * ty + q] * rs;
-      lc[q] = 4 * tx + q > j ? cj[4 * tx + q] * rs : 0.0;
-    }
-#pragma unroll
-    for (int ai = 0; ai < 4; ++ai)
-#pragma unroll
-      for (int bi = 0; bi < 4; ++bi) a[ai][bi] -= li[ai] * lc[bi];
-    if (tx == (j >> 2)) {  // column j becomes the factor's column
-#pragma unroll
-      for (int bi = 0; bi < 4; ++bi)
-        if (4 * tx + bi == j) {
-#pragma unroll
-          for (int ai = 0; ai < 4; ++ai) {
-            const int i = 4 * ty + ai;
-            if (i >= j) a[ai][bi] = i == j ? sd : li[ai];
-          }
-        }
-    }
-  }
-  __syncthreads();  // every thread has read the last published column before Ls is rewritten
-#pragma unroll
-  for (int ai = 0; ai < 4; ++ai)
-#pragma unroll
-    for (int bi = 0; bi < 4; ++bi) {
-      const int i = 4 * ty + ai, c = 4 * tx + bi;
-      Ls[c * (kCT + 1) + i] = i >= c ? a[ai][bi] : 0.0;
-    }
-  __syncthreads();
-  for (int w = tid; w < kCTT; w += blockDim.x) {
-    const int c = w / kCT, r = w - c * kCT;
-    g[w] = Ls[c * (kCT + 1) + r];
-  }
-  if (tid < kCT) rdiag[tid] = 1.0 / Ls[tid * (kCT + 1) + tid];
-  // W = L^-1: row j of W is final once rows above it have been eliminated; it is published and the
-  // rows below subtract L(i, j) times it
-#pragma unroll
-  for (int ai = 0; ai < 4; ++ai)
-#pragma unroll
-    for (int bi = 0; bi < 4; ++bi) a[ai][bi] = (4 * ty + ai == 4 * tx + bi) ? 1.0 : 0.0;
-  __syncthreads();
-  for (int j = 0; j < kCT; ++j) {
-    double* xj = pub[j & 1];
-    if (ty == (j >> 2)) {
-      const int aj = j & 3;
-      const double rd = rdiag[j];
-#pragma unroll
-      for (int ai = 0; ai < 4; ++ai)
-        if (ai == aj) {
-#pragma unroll
-          for (int bi = 0; bi < 4; ++bi) {
-            const double v = 4 * tx + bi <= j ? a[ai][bi] * rd : 0.0;
-            a[ai][bi] = v;
-            xj[4 * tx + bi] = v;
-          }
-        }
+    // trailing blocks (bi >= bj > j0 / 8), column by column of blocks
+    const int p = j0 >> 3, m = 7 - p;
+    for (int q = w; q < m * (m + 1) / 2; q += 8) {
+      int col = 0, at = q;
+      while (at >= m - col) at -= m - col++;
+      const int bj = p + 1 + col, bi = bj + at;
+      double* C = A + (8 * bj + 2 * t) * kTS + 8 * bi + g;
+      double c0 = C[0], c1 = C[kTS];
+      mma8(8, [&](int r, int kk) { return -A[(j0 + kk) * kTS + 8 * bi + r]; },
+           [&](int kk, int c) { return A[(j0 + kk) * kTS + 8 * bj + c]; }, c0, c1);
+      C[0] = c0;
+      C[kTS] = c1;
     }
     __syncthreads();
-    // branch-free: the published row is zero right of column j and the multipliers are zero at or
-    // above row j, so only the rows below j change, in the columns up to j
+  }
+  // the factor out (zero above the diagonal)
+  for (int i = tid; i < kCTT; i += 256) {
+    const int c = i >> 6, r = i & 63;
+    gt[i] = r >= c ? A[c * kTS + r] : 0.0;
+  }
+  // W: diagonal blocks, warp w block w, lane c its column c
+  if (lane < 8) {
+    double x[8];
 #pragma unroll
-    for (int ai = 0; ai < 4; ++ai) {
-      const int i = 4 * ty + ai;
-      const double lij = i > j ? Ls[j * (kCT + 1) + i] : 0.0;
+    for (int i = 0; i < 8; ++i) {
+      double v = i == lane ? 1.0 : 0.0;
 #pragma unroll
-      for (int bi = 0; bi < 4; ++bi) a[ai][bi] -= lij * xj[4 * tx + bi];
+      for (int q = 0; q < i; ++q) v -= A[(8 * w + q) * kTS + 8 * w + i] * x[q];
+      x[i] = i >= lane ? v * rdiag[8 * w + i] : 0.0;
+      W[(8 * w + lane) * kTS + 8 * w + i] = x[i];
     }
   }
-  __syncthreads();  // Ls is reused to stage W for coalesced stores
-#pragma unroll
-  for (int ai = 0; ai < 4; ++ai)
-#pragma unroll
-    for (int bi = 0; bi < 4; ++bi) {
-      const int i = 4 * ty + ai, c = 4 * tx + bi;
-      Ls[c * (kCT + 1) + i] = i >= c ? a[ai][bi] : 0.0;
+  __syncthreads();  // the factor has been read out: the upper triangle is scratch from here on
+  for (int h = 8; h < kCT; h *= 2) {
+    const int nbk = h / 8, per = nbk * nbk, pairs = kCT / (2 * h);
+    // T = L_21 W_11 (h x h) of every pair, into rows [b, b + h), columns [b + h, b + 2 h)
+    for (int q = w; q < pairs * per; q += 8) {
+      const int b = 2 * h * (q / per), bi = (q % per) % nbk, bj = (q % per) / nbk;
+      double c0 = 0.0, c1 = 0.0;
+      mma8(h, [&](int r, int kk) { return A[(b + kk) * kTS + b + h + 8 * bi + r]; },
+           [&](int kk, int c) { return W[(b + 8 * bj + c) * kTS + b + kk]; }, c0, c1);
+      double* T = A + (b + h + 8 * bj + 2 * t) * kTS + b + 8 * bi + g;
+      T[0] = c0;
+      T[kTS] = c1;
     }
-  __syncthreads();
+    __syncthreads();
+    for (int q = w; q < pairs * per; q += 8) {
+      const int b = 2 * h * (q / per), bi = (q % per) % nbk, bj = (q % per) / nbk;
+      double c0 = 0.0, c1 = 0.0;
+      mma8(h, [&](int r, int kk) { return -W[(b + h + kk) * kTS + b + h + 8 * bi + r]; },
+           [&](int kk, int c) { return A[(b + h + 8 * bj + c) * kTS + b + kk]; }, c0, c1);
+      double* O = W + (b + 8 * bj + 2 * t) * kTS + b + h + 8 * bi + g;
+      O[0] = c0;
+      O[kTS] = c1;
+    }
+    __syncthreads();
+  }
   double* wk = tb.w + (size_t)k * kCTT;
-  for (int w = tid; w < kCTT; w += blockDim.x) {
-    const int c = w / kCT, r = w - c * kCT;
-    wk[w] = Ls[c * (kCT + 1) + r];
-  }
+  for (int i = tid; i < kCTT; i += 256) wk[i] = W[(i >> 6) * kTS + (i & 63)];
 }
 
 // TRSM as a product: the tiles below diagonal tile k, L_ik = A_ik W_k^T (CTA per tile). Dynamic shared
 // memory: two staged operands.
 constexpr size_t kTrsmSmem = 2 * kStagedTile;
 __global__ void __launch_bounds__(256) k_tile_trsm(TileBand tb, int k, const int* status) {
-  extern __shared__ double shm[];
+  extern __shared__ __align__(16) double shm[];
   if (status[0] == 0) return;
   double* Ta = shm;
   double* Tb = shm + kCT * kTS;
   const int i = k + 1 + blockIdx.x;
   double* bi = tb.t + tile_at(tb, i, k);
-  stage_tile(bi, Ta, false, false);                       // A_ik
-  stage_tile(tb.w + (size_t)k * kCTT, Tb, true, true);    // W_k^T
+  stage_tile(bi, Ta);                        // A_ik
+  stage_tile(tb.w + (size_t)k * kCTT, Tb);   // W_k
+  stage_wait();
   __syncthreads();
-  double acc[4][4];
+  TileAcc acc;
   zero_acc(acc);
-  tile_mma_acc(Ta, Tb, acc);
+  tile_mma_acc<false, true>(Ta, Tb, acc);
   acc_store(acc, bi);
 }
 
 // Trailing update of step k: A_ij -= L_ik L_jk^T for k < j <= i <= min(k + bwt, nt - 1), one CTA per
-// tile, 16 x 16 threads with 4 x 4 outputs each; the sum over the tile's 64 columns runs in order.
+// tile; the sum over the tile's 64 columns runs in order.
 constexpr size_t kUpdateSmem = 2 * kStagedTile;
 __global__ void __launch_bounds__(256) k_tile_update(TileBand tb, int k, const int* status) {
-  extern __shared__ double sh[];
+  extern __shared__ __align__(16) double sh[];
   if (status[0] == 0) return;
   double* Ta = sh;
   double* Tb = sh + kCT * kTS;
   int idx = blockIdx.x;
-  int ii = 0;
+  int ii = (int)((sqrtf(8.0f * (float)idx + 1.0f) - 1.0f) * 0.5f);
   while ((ii + 1) * (ii + 2) / 2 <= idx) ++ii;
+  while (ii * (ii + 1) / 2 > idx) --ii;
   const int jj = idx - ii * (ii + 1) / 2;
   const int i = k + 1 + ii, j = k + 1 + jj;
-  stage_tile(tb.t + tile_at(tb, i, k), Ta, false, false);  // L_ik
-  stage_tile(tb.t + tile_at(tb, j, k), Tb, true, true);    // L_jk^T
-  __syncthreads();
-  double acc[4][4];
-  zero_acc(acc);
-  tile_mma_acc(Ta, Tb, acc);
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  stage_tile(tb.t + tile_at(tb, i, k), Ta);  // L_ik
+  stage_tile(tb.t + tile_at(tb, j, k), Tb);  // L_jk
   double* cij = tb.t + tile_at(tb, i, j);
+  TileAcc acc, old;
+  zero_acc(acc);
+  {  // the tile's own values, requested with the operands
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const double* c = cij + (size_t)(32 * (w & 1) + 2 * t) * kCT + 16 * (w >> 1) + g;
 #pragma unroll
-  for (int b = 0; b < 4; ++b)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-    for (int a = 0; a < 4; ++a) cij[(size_t)(4 * tx + b) * kCT + 4 * ty + a] -= acc[a][b];
+      for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) old.v[a][b][e] = c[(8 * b + e) * kCT + 8 * a];
+  }
+  stage_wait();
+  __syncthreads();
+  tile_mma_acc<false, true>(Ta, Tb, acc);
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) acc.v[a][b][e] = old.v[a][b][e] - acc.v[a][b][e];
+  acc_store(acc, cij);
 }
 
-// Forward (L y = b) and backward (L^T x = y) substitution with the banded tiled factor, one CTA of
-// 256 threads, in place on the permuted vector v (n entries; the padding is not touched). Four
-// threads per row of a tile sum the band's products in quarters, combined in a fixed order; the
-// triangle inside a tile is solved by one warp with a fixed shuffle tree per row.
-__device__ void tile_forward_rows(const TileBand& tb, double* v, int i, int j_lo, double* part, double* yt) {
-  const int tid = threadIdx.x, r = tid & (kCT - 1), qtr = tid >> 6;  // 256 threads: 4 quarters
+// Forward (L y = b) and backward (L^T x = y) substitution with the banded tiled factor, in place on the
+// permuted vector v (n entries; the padding is not touched), one cluster of up to kSolveCtas CTAs.
+// Right-looking: CTA i mod size owns rows of tile i. In step k the owner of tile k multiplies its
+// finished part by the inverse of the diagonal tile (W_k, from the factorization), hands the 64
+// results to every CTA's shared memory, and after one cluster barrier each CTA subtracts the products
+// of its own tiles of the column (forward) or row (backward). Each entry of v is only ever touched
+// by its owner, in step order. Bound: 2 nt steps of one L2 latency, one cluster barrier and one more
+// L2 latency. One CTA that walked each row of the band with an in-tile triangular solve by one warp took
+// 12.8 ms for 71 tiles in a band of 14; this takes 0.79 ms (two tiles: 184 us before).
+constexpr int kSolveCtas = 8;
+// y[0..64) = M u (or M^T u) for the column-major 64 x 64 tile M; 256 threads, u in shared memory.
+__device__ __forceinline__ void tile_times(const double* __restrict__ M, const double* u, double* part, double* y) {
+  const int r = threadIdx.x & (kCT - 1), qtr = threadIdx.x >> 6;
+  double m[16];
+#pragma unroll
+  for (int c = 0; c < 16; ++c) m[c] = M[(size_t)(16 * qtr + c) * kCT + r];
   double s = 0.0;
-  const int j_first = max(j_lo, i - tb.bwt);
-  for (int j = j_first; j < i; ++j) {
-    const double* L = tb.t + tile_at(tb, i, j);
-    for (int c = qtr; c < kCT; c += 4) s += L[(size_t)c * kCT + r] * v[j * kCT + c];
-  }
+#pragma unroll
+  for (int c = 0; c < 16; ++c) s += m[c] * u[16 * qtr + c];
   part[qtr * kCT + r] = s;
   __syncthreads();
-  if (tid < kCT) {
-    const int rr = tid;
-    const int P = i * kCT + rr;
-    const double b = P < tb.n ? v[P] : 0.0;
-    yt[rr] = b - (((part[rr] + part[kCT + rr]) + part[2 * kCT + rr]) + part[3 * kCT + rr]);
-  }
+  if (threadIdx.x < kCT) y[r] = ((part[r] + part[kCT + r]) + part[2 * kCT + r]) + part[3 * kCT + r];
   __syncthreads();
-  if (tid < 32) {  // in-tile forward solve, one warp
-    const double* L = tb.t + tile_at(tb, i, i);
-    for (int rr = 0; rr < kCT; ++rr) {
-      double d = 0.0;
-      for (int c = tid; c < rr; c += 32) d += L[(size_t)c * kCT + rr] * yt[c];
-      d = warp_sum(d);
-      if (tid == 0) yt[rr] = (yt[rr] - d) / L[(size_t)rr * kCT + rr];
-      __syncwarp();
-    }
+}
+__device__ __forceinline__ void tile_times_t(const double* __restrict__ M, const double* u, double* y) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double m0[8], m1[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    m0[c] = M[(size_t)(8 * w + c) * kCT + lane];
+    m1[c] = M[(size_t)(8 * w + c) * kCT + lane + 32];
   }
-  __syncthreads();
-  if (tid < kCT) {
-    const int P = i * kCT + tid;
-    if (P < tb.n) v[P] = yt[tid];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const double s = warp_sum(m0[c] * u[lane] + m1[c] * u[lane + 32]);
+    if (lane == 0) y[8 * w + c] = s;
   }
   __syncthreads();
 }
-
 __global__ void __launch_bounds__(256) k_tile_solve(TileBand tb, double* v, const int* status) {
-  __shared__ double part[4 * kCT];
-  __shared__ double yt[kCT];
-  if (status[0] == 0) return;
-  const int tid = threadIdx.x, r = tid & (kCT - 1), qtr = tid >> 6;
-  for (int i = 0; i < tb.nt; ++i) tile_forward_rows(tb, v, i, 0, part, yt);
-  for (int i = tb.nt - 1; i >= 0; --i) {
-    // x_i = L_ii^-T (y_i - sum_{j > i} L_ji^T x_j)
-    double s = 0.0;
-    const int j_last = min(tb.nt - 1, i + tb.bwt);
-    for (int j = i + 1; j <= j_last; ++j) {
-      const double* L = tb.t + tile_at(tb, j, i);
-      for (int c = qtr; c < kCT; c += 4) {
-        const int Q = j * kCT + c;
-        if (Q < tb.n) s += L[(size_t)r * kCT + c] * v[Q];
-      }
-    }
-    part[qtr * kCT + r] = s;
+  namespace cg = cooperative_groups;
+  __shared__ double part[4 * kCT], u[kCT], y[kCT];
+  __shared__ double step[2][kCT];  // the finished part of the step, from its owner
+  if (status[0] == 0) return;      // the same value in every CTA of the cluster
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), size = (int)cluster.num_blocks(), tid = threadIdx.x;
+  auto load = [&](int tile) {
+    if (tid < kCT) u[tid] = tile * kCT + tid < tb.n ? v[tile * kCT + tid] : 0.0;
     __syncthreads();
-    if (tid < kCT) {
-      const int P = i * kCT + tid;
-      const double b = P < tb.n ? v[P] : 0.0;
-      yt[tid] = b - (((part[tid] + part[kCT + tid]) + part[2 * kCT + tid]) + part[3 * kCT + tid]);
+  };
+  auto publish = [&](int tile, int buf) {  // y: store it and hand it to every CTA
+    if (tid < kCT && tile * kCT + tid < tb.n) v[tile * kCT + tid] = y[tid];
+    for (int i = tid; i < size * kCT; i += 256) {
+      double* dst = cluster.map_shared_rank(&step[buf][0], i / kCT);
+      dst[i % kCT] = y[i % kCT];
     }
+  };
+  auto subtract = [&](int tile) {
+    if (tid < kCT && tile * kCT + tid < tb.n) v[tile * kCT + tid] -= y[tid];
     __syncthreads();
-    if (tid < 32) {  // in-tile backward solve with L_ii^T
-      const double* L = tb.t + tile_at(tb, i, i);
-      for (int rr = kCT - 1; rr >= 0; --rr) {
-        double d = 0.0;
-        for (int c = rr + 1 + tid; c < kCT; c += 32) d += L[(size_t)rr * kCT + c] * yt[c];
-        d = warp_sum(d);
-        if (tid == 0) yt[rr] = (yt[rr] - d) / L[(size_t)rr * kCT + rr];
-        __syncwarp();
-      }
+  };
+  cluster.sync();  // every CTA runs before any of them is written to
+  for (int k = 0; k < tb.nt; ++k) {
+    const int buf = k & 1;
+    if (k % size == rank) {
+      load(k);
+      tile_times(tb.w + (size_t)k * kCTT, u, part, y);
+      publish(k, buf);
     }
-    __syncthreads();
-    if (tid < kCT) {
-      const int P = i * kCT + tid;
-      if (P < tb.n) v[P] = yt[tid];
+    cluster.sync();
+    const int last = min(tb.nt - 1, k + tb.bwt);
+    for (int i = k + 1 + (rank - (k + 1) % size + size) % size; i <= last; i += size) {
+      tile_times(tb.t + tile_at(tb, i, k), step[buf], part, y);
+      subtract(i);
     }
-    __syncthreads();
   }
+  for (int k = tb.nt - 1; k >= 0; --k) {
+    const int buf = (tb.nt + tb.nt - 1 - k) & 1;  // alternates on from the forward sweep's last step
+    if (k % size == rank) {
+      load(k);
+      tile_times_t(tb.w + (size_t)k * kCTT, u, y);
+      publish(k, buf);
+    }
+    cluster.sync();
+    const int first = max(0, k - tb.bwt);
+    for (int j = first + (rank - first % size + size) % size; j < k; j += size) {
+      tile_times_t(tb.t + tile_at(tb, k, j), step[buf], y);
+      subtract(j);
+    }
+  }
+  cluster.sync();  // no CTA leaves while another may still write to it
 }
 
 // Gather / scatter between the original and the permuted parameter order.
@@ -753,41 +790,34 @@ __global__ void k_perm_scatter(int n, const int* __restrict__ perm_to_orig, cons
 //                       chunks of kTakahashiChunk consecutive k in order
 //  k_takahashi_offdiag  CTA b: Z_ij = -(sum_s part(b, s)) W_j, and its share of the diagonal sum,
 //                       q(b) = Z_ij^T L_ij
-//  k_takahashi_diag     one CTA: Z_jj = (W_j^T - sum_b q(b)) W_j
+//  k_takahashi_diag     CTA r: rows 8 r .. 8 r + 7 of Z_jj = (W_j^T - sum_b q(b)) W_j
 // Every sum runs in a fixed order, so Z does not depend on scheduling. Dynamic shared memory:
 // kTakahashiSmem (two staged operands).
 constexpr size_t kTakahashiSmem = 2 * kStagedTile;
 constexpr int kTakahashiChunk = 4;
-
-// acc (output tile element (4 ty + a, 4 tx + b)) transposed into a staged A operand: A(c, r) = acc(r, c)
-__device__ __forceinline__ void acc_to_at(const double acc[4][4], double* T) {
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) T[(4 * ty + a) * kTS + 4 * tx + b] = acc[a][b];
-}
+constexpr int kTakahashiDiagCtas = 8;
 
 __global__ void __launch_bounds__(256) k_takahashi_partial(TileBand L, TileBand Z, int j, double* part,
                                                            const int* status) {
-  extern __shared__ double sh[];
+  extern __shared__ __align__(16) double sh[];
   if (status[0] == 0) return;
   double* Ta = sh;
   double* Tb = sh + kCT * kTS;
   const int i = j + 1 + blockIdx.x;
   const int kmax = min(L.nt - 1, j + L.bwt);
   const int k0 = j + 1 + kTakahashiChunk * blockIdx.y, k1 = min(kmax, k0 + kTakahashiChunk - 1);
-  double acc[4][4];
+  TileAcc acc;
   zero_acc(acc);
   for (int k = k0; k <= k1; ++k) {
     __syncthreads();
-    if (i >= k)
-      stage_tile(Z.t + tile_at(Z, i, k), Ta, false, false);  // Z_ik
-    else
-      stage_tile(Z.t + tile_at(Z, k, i), Ta, false, true);   // Z_ki^T
-    stage_tile(L.t + tile_at(L, k, j), Tb, true, false);     // L_kj
+    stage_tile(Z.t + (i >= k ? tile_at(Z, i, k) : tile_at(Z, k, i)), Ta);  // Z_ik, or Z_ki for its transpose
+    stage_tile(L.t + tile_at(L, k, j), Tb);
+    stage_wait();
     __syncthreads();
-    tile_mma_acc(Ta, Tb, acc);
+    if (i >= k)
+      tile_mma_acc<false, false>(Ta, Tb, acc);
+    else
+      tile_mma_acc<true, false>(Ta, Tb, acc);
   }
   acc_store(acc, part + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * kCTT);
 }
@@ -795,57 +825,62 @@ __global__ void __launch_bounds__(256) k_takahashi_partial(TileBand L, TileBand 
 __global__ void __launch_bounds__(256) k_takahashi_offdiag(TileBand L, TileBand Z, int j, int nsplit,
                                                            const double* __restrict__ part, double* q,
                                                            const int* status) {
-  extern __shared__ double sh[];
+  extern __shared__ __align__(16) double sh[];
   if (status[0] == 0) return;
   double* Ta = sh;
   double* Tb = sh + kCT * kTS;
   const int i = j + 1 + blockIdx.x;
-  // -(sum of the partial tiles, in order) into the A operand, read along the tiles' storage
+  stage_tile(L.w + (size_t)j * kCTT, Tb);  // W_j
+  // -(sum of the partial tiles, in order) into the A operand
   const double* pb = part + (size_t)blockIdx.x * nsplit * kCTT;
-  for (int w = threadIdx.x; w < kCTT; w += blockDim.x) {
+#pragma unroll 4
+  for (int w = threadIdx.x; w < kCTT; w += 256) {
     double v = 0.0;
     for (int s = 0; s < nsplit; ++s) v += pb[(size_t)s * kCTT + w];
-    Ta[(w / kCT) * kTS + (w % kCT)] = -v;
+    Ta[(w >> 6) * kTS + (w & 63)] = -v;
   }
-  stage_tile(L.w + (size_t)j * kCTT, Tb, true, false);  // W_j
+  stage_wait();
   __syncthreads();
-  double acc[4][4];
+  TileAcc acc;
   zero_acc(acc);
-  tile_mma_acc(Ta, Tb, acc);
+  tile_mma_acc<false, false>(Ta, Tb, acc);
   acc_store(acc, Z.t + tile_at(Z, i, j));
   __syncthreads();
-  acc_to_at(acc, Ta);                                    // Z_ij^T
-  stage_tile(L.t + tile_at(L, i, j), Tb, true, false);  // L_ij
+  stage_tile(L.t + tile_at(L, i, j), Tb);  // L_ij
+  acc_each(acc, [&](int r, int c, double v) { Ta[c * kTS + r] = v; });
+  stage_wait();
   __syncthreads();
   zero_acc(acc);
-  tile_mma_acc(Ta, Tb, acc);
+  tile_mma_acc<true, false>(Ta, Tb, acc);  // Z_ij^T L_ij
   acc_store(acc, q + (size_t)blockIdx.x * kCTT);
 }
 
+// The diagonal tile's sum over the column's m shares reads m tiles: split by rows over eight CTAs (at
+// m = 14 one CTA took 45.5 us, the eight take 9.1).
 __global__ void __launch_bounds__(256) k_takahashi_diag(TileBand L, TileBand Z, int j, int m,
                                                         const double* __restrict__ q, const int* status) {
-  extern __shared__ double sh[];
+  extern __shared__ __align__(16) double sh[];
   if (status[0] == 0) return;
-  double* Ta = sh;
-  double* Tb = sh + kCT * kTS;
-  // -(sum of the tiles' shares, in order) into the A operand, read along the tiles' storage
-  for (int w = threadIdx.x; w < kCTT; w += blockDim.x) {
-    double v = 0.0;
-    for (int b = 0; b < m; ++b) v += q[(size_t)b * kCTT + w];
-    Ta[(w / kCT) * kTS + (w % kCT)] = -v;
-  }
+  double* Ta = sh;             // 8 rows x 64: element (r, c) at c * 12 + r
+  double* Tb = sh + kCT * 12;
+  const int r0 = 8 * blockIdx.x, tid = threadIdx.x;
   const double* wj = L.w + (size_t)j * kCTT;
-  __syncthreads();
-  for (int w = threadIdx.x; w < kCTT; w += blockDim.x) {  // + W_j^T: A(r, q) += W(q, r)
-    const int c = w / kCT, r = w - c * kCT;                // W(r, c) at wj[w]
-    Ta[r * kTS + c] += wj[w];                              // A element (c, r) of the operand
+  stage_tile(wj, Tb);
+  for (int w = tid; w < 8 * kCT; w += 256) {
+    const int c = w >> 3, r = w & 7;
+    double v = 0.0;
+    for (int b = 0; b < m; ++b) v += q[(size_t)b * kCTT + c * kCT + r0 + r];
+    Ta[c * 12 + r] = wj[(size_t)(r0 + r) * kCT + c] - v;  // W_j^T(r, c) = W_j(c, r)
   }
-  double acc[4][4];
-  stage_tile(wj, Tb, true, false);  // W_j
+  stage_wait();
   __syncthreads();
-  zero_acc(acc);
-  tile_mma_acc(Ta, Tb, acc);
-  acc_store(acc, Z.t + tile_at(Z, j, j));
+  const int lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+  double c0 = 0.0, c1 = 0.0;
+  mma8(kCT, [&](int r, int kk) { return Ta[kk * 12 + r]; },
+       [&](int kk, int c) { return Tb[(8 * w + c) * kTS + kk]; }, c0, c1);
+  double* out = Z.t + tile_at(Z, j, j) + (size_t)(8 * w + 2 * t) * kCT + r0 + g;
+  out[0] = c0;
+  out[kCT] = c1;
 }
 
 // (S^-1)_gg of each free group from Z: 9 values per group (row-major), thread per group.

@@ -2122,6 +2122,12 @@ ExecutionPlan execution_plan(const NativeProblem& n, const LmOptions& opt) {
   return plan;
 }
 
+static void tile_factor_attributes() {
+  CUDA_OK(cudaFuncSetAttribute(k_tile_potrf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPotrfSmem));
+  CUDA_OK(cudaFuncSetAttribute(k_tile_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
+  CUDA_OK(cudaFuncSetAttribute(k_tile_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpdateSmem));
+}
+
 // Positive-definiteness certificate of a symmetric matrix from its lower-triangle entries: the entries
 // are scattered into the banded tile layout of the explicit reduced camera system (bandwidth from the
 // entries themselves) and factored by the same tiled Cholesky kernels; the status word says whether
@@ -2146,8 +2152,7 @@ bool device_certify_positive_definite(Context* ctx, int n, const std::vector<int
   d_rows.upload(rows.data(), rows.size(), st);
   d_cols.upload(cols.data(), cols.size(), st);
   vals.upload(values.data(), values.size(), st);
-  CUDA_OK(cudaFuncSetAttribute(k_tile_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
-  CUDA_OK(cudaFuncSetAttribute(k_tile_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpdateSmem));
+  tile_factor_attributes();
   CUDA_OK(cudaMemsetAsync(tiles.p, 0, sizeof(double) * count, st));
   OMVGBA_LAUNCH(k_set_int, 1, 1, 0, st, status.p, 1);
   TileBand tb{n, nt, bwt, tiles.p, winv.p};
@@ -2156,7 +2161,7 @@ bool device_certify_positive_definite(Context* ctx, int n, const std::vector<int
                   d_cols.p, vals.p, tb);
   OMVGBA_LAUNCH(k_tiles_pad, 1, kCT, 0, st, tb);
   for (int k = 0; k < nt; ++k) {
-    OMVGBA_LAUNCH(k_tile_potrf, 1, 256, 0, st, tb, k, status.p);
+    OMVGBA_LAUNCH(k_tile_potrf, 1, 256, kPotrfSmem, st, tb, k, status.p);
     const int m = std::min(bwt, nt - 1 - k);
     if (m > 0) {
       OMVGBA_LAUNCH(k_tile_trsm, m, 256, kTrsmSmem, st, tb, k, status.p);
@@ -2678,7 +2683,22 @@ struct Solver {
   bool direct_step(double lambda) {
     if (!factor_band(lambda, nullptr, 0.0)) return false;
     OMVGBA_LAUNCH(k_perm_gather, grid_for(D, 256), 256, 0, st, D, d_perm_to_orig.p, d_gred.p, -1.0, d_perm_vec.p);
-    OMVGBA_LAUNCH(k_tile_solve, 1, 256, 0, st, tile_band(), d_perm_vec.p, d_status.p);
+    {  // one cluster: a CTA per tile of the band, up to kSolveCtas
+      int ctas = 1;
+      while (ctas < kSolveCtas && ctas < S.bwt) ctas *= 2;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(ctas);
+      cfg.blockDim = dim3(256);
+      cfg.stream = st;
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = ctas;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      (void)cudaLaunchKernelEx(&cfg, k_tile_solve, tile_band(), d_perm_vec.p, (const int*)d_status.p);
+      ++tl_telemetry.launches;
+    }
     OMVGBA_LAUNCH(k_perm_scatter, grid_for(D, 256), 256, 0, st, D, d_perm_to_orig.p, d_perm_vec.p, d_step.p);
     check_launch();
     return true;
@@ -2999,9 +3019,7 @@ struct Solver {
       throw SolveFailure{3, "the banded factor of the reduced camera system exceeds 16 GiB"};
     if (d_tiles.n != count) d_tiles.alloc(count, st);
     if (d_winv.n != (size_t)S.nt * kCTT) d_winv.alloc((size_t)S.nt * kCTT, st);
-    // per device and cheap: set on every factorization
-    CUDA_OK(cudaFuncSetAttribute(k_tile_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
-    CUDA_OK(cudaFuncSetAttribute(k_tile_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpdateSmem));
+    tile_factor_attributes();  // per device and cheap: set on every factorization
     CUDA_OK(cudaMemsetAsync(d_tiles.p, 0, sizeof(double) * count, st));
     OMVGBA_LAUNCH(k_set_int, 1, 1, 0, st, d_status.p, 1);
     const TileBand tb = tile_band();
@@ -3010,7 +3028,7 @@ struct Solver {
     OMVGBA_LAUNCH(k_tiles_pad, 1, kCT, 0, st, tb);
     run_as_graph([&] {
       for (int k = 0; k < S.nt; ++k) {
-        OMVGBA_LAUNCH(k_tile_potrf, 1, 256, 0, st, tb, k, d_status.p);
+        OMVGBA_LAUNCH(k_tile_potrf, 1, 256, kPotrfSmem, st, tb, k, d_status.p);
         const int m = std::min(S.bwt, S.nt - 1 - k);
         if (m > 0) {
           OMVGBA_LAUNCH(k_tile_trsm, m, 256, kTrsmSmem, st, tb, k, d_status.p);
@@ -3107,7 +3125,7 @@ struct Solver {
           OMVGBA_LAUNCH(k_takahashi_offdiag, m, 256, kTakahashiSmem, st, tl, tz, j, nsplit, d_zpart.p, d_zq.p,
                         d_status.p);
         }
-        OMVGBA_LAUNCH(k_takahashi_diag, 1, 256, kTakahashiSmem, st, tl, tz, j, m, d_zq.p, d_status.p);
+        OMVGBA_LAUNCH(k_takahashi_diag, kTakahashiDiagCtas, 256, kTakahashiSmem, st, tl, tz, j, m, d_zq.p, d_status.p);
       }
     });
     DBuf<int> d_pos, d_dims;
