@@ -272,62 +272,88 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_block_rows(RowTables rt, Lin
     for (uint32_t k = tid; k < rlen; k += kRowThreads) rows[r0 + k] = row_sh[k];
 }
 
-// y = (S + lambda diag) x from the block rows: one warp per block row, lanes over the row's entries
-// in a fixed assignment, then a fixed shuffle tree. With scale non-null the operator is the Jacobi-
-// equilibrated D S D (D = diag(scale)) and lambda must be 0. With xy non-null, xy[CTA] = sum of
-// x_b . y_b over the CTA's blocks in block order.
-__global__ void __launch_bounds__(256) k_rows_matvec(RowTables rt, const double* __restrict__ rows,
-                                                     const double* __restrict__ diag, double lambda,
-                                                     const double* __restrict__ scale,
-                                                     const double* __restrict__ x, double* __restrict__ y,
-                                                     double* __restrict__ xy, const PcgCtl* ctl) {
-  __shared__ double s_dot[8];
+// acc[m] += row m of block row X of S times x, a block per lane, over the row's blocks from `first` in
+// steps of `stride`; xs gives x by parameter.
+template <typename FX>
+__device__ __forceinline__ void row_times(const RowTables& rt, const double* __restrict__ rows, int X, int dX,
+                                          uint32_t first, uint32_t stride, FX xs, double acc[6]) {
+  const uint32_t n1 = rt.nbr_begin[X + 1];
+  for (uint32_t q = rt.nbr_begin[X] + first; q < n1; q += stride) {
+    const int Y = rt.nbr[q], dY = rt.blk_dim[Y], oY = rt.blk_off[Y];
+    const double* S = rows + rt.slot_off[q];
+    double xv[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) xv[c] = c < dY ? xs(oY + c) : 0.0;
+#pragma unroll
+    for (int m = 0; m < 6; ++m)
+      if (m < dX) {
+        double s = 0.0;
+#pragma unroll
+        for (int c = 0; c < 6; ++c)
+          if (c < dY) s += S[m * dY + c] * xv[c];
+        acc[m] += s;
+      }
+  }
+}
+
+// y = (S + lambda diag) x from the block rows: SPLIT warps per block row, the row's blocks dealt over
+// their lanes in a fixed assignment, then a fixed shuffle tree and the warps in order. With xy non-null,
+// xy[CTA] = sum of x_b . y_b over the CTA's blocks in block order.
+// Bound: L2 where S fits it (500 cameras: 30 MB), HBM above, latency below. SPLIT: while one warp per row
+// leaves an SM fewer than eight warps (row_split) its loads do not cover the latency; measured on block
+// rows of 61 cameras (one / two / four warps, back to back): 120 cameras 12.3 / 8.3 / 6.2 us, 500 12.4 /
+// 10.3 / 10.3 us, 1,000 14.4 / 14.7 / 16.1 us, 3,000 37.9 / 39.1 / 43.2 us.
+constexpr int kRowProductWarps = 8;
+inline int row_split(int nblocks) { return nblocks <= 592 ? 4 : (nblocks <= 1184 ? 2 : 1); }
+template <int SPLIT>
+__global__ void __launch_bounds__(32 * kRowProductWarps) k_rows_matvec(RowTables rt, const double* __restrict__ rows,
+                                                                       const double* __restrict__ diag, double lambda,
+                                                                       const double* __restrict__ x,
+                                                                       double* __restrict__ y, double* __restrict__ xy,
+                                                                       const PcgCtl* ctl) {
+  constexpr int ROWS = kRowProductWarps / SPLIT;
+  __shared__ double s_part[kRowProductWarps][6];
+  __shared__ double s_dot[ROWS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int X = blockIdx.x * 8 + warp;
+  const int X = blockIdx.x * ROWS + warp / SPLIT;
   const bool have = X < rt.nblocks;
   pdl_trigger();
   pdl_wait();
   if (pcg_stopped(ctl)) return;
-  double dot = 0.0;
+  const int dX = have ? rt.blk_dim[X] : 0;
   if (have) {
-    const int dX = rt.blk_dim[X], oX = rt.blk_off[X];
-    const uint32_t n0 = rt.nbr_begin[X], n1 = rt.nbr_begin[X + 1];
     double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (uint32_t q = n0 + lane; q < n1; q += 32) {
-      const int Y = rt.nbr[q];
-      const int dY = rt.blk_dim[Y], oY = rt.blk_off[Y];
-      const double* S = rows + rt.slot_off[q];
-      double xv[6];
+    row_times(rt, rows, X, dX, 32u * (warp % SPLIT) + lane, 32u * SPLIT, [&](int i) { return x[i]; }, acc);
 #pragma unroll
-      for (int c = 0; c < 6; ++c) xv[c] = c < dY ? x[oY + c] * (scale ? scale[oY + c] : 1.0) : 0.0;
-#pragma unroll
-      for (int m = 0; m < 6; ++m)
-        if (m < dX) {
-          double s = 0.0;
-#pragma unroll
-          for (int c = 0; c < 6; ++c)
-            if (c < dY) s += S[m * dY + c] * xv[c];
-          acc[m] += s;
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < 6; ++m) acc[m] = warp_sum(acc[m]);
-    if (lane == 0) {
-      for (int m = 0; m < dX; ++m) {
-        double v = acc[m];
-        if (scale) v *= scale[oX + m];
-        v += lambda * diag[oX + m] * x[oX + m];
-        y[oX + m] = v;
-        dot += x[oX + m] * v;
-      }
+    for (int m = 0; m < 6; ++m) {
+      acc[m] = warp_sum(acc[m]);
+      if (lane == 0) s_part[warp][m] = acc[m];
     }
   }
+  if (SPLIT > 1)
+    __syncthreads();
+  else
+    __syncwarp();
+  if (warp % SPLIT == 0) {
+    double dot = 0.0;
+    if (lane < dX) {
+      const int o = rt.blk_off[X] + lane;
+      double v = 0.0;
+#pragma unroll
+      for (int s = 0; s < SPLIT; ++s) v += s_part[warp + s][lane];
+      const double xv = x[o];
+      v += lambda * diag[o] * xv;
+      y[o] = v;
+      dot = xv * v;
+    }
+    dot = warp_sum(dot);
+    if (lane == 0) s_dot[warp / SPLIT] = dot;
+  }
   if (xy) {
-    if (lane == 0) s_dot[warp] = dot;
     __syncthreads();
     if (threadIdx.x == 0) {
       double t = 0.0;
-      for (int w = 0; w < 8; ++w) t += s_dot[w];
+      for (int w = 0; w < ROWS; ++w) t += s_dot[w];
       xy[blockIdx.x] = t;
     }
   }
@@ -906,43 +932,66 @@ __global__ void k_z_marginals(TileBand Z, int ngroups, const int* __restrict__ p
 }
 
 // Largest |eigenvalue| of the equilibrated D S D by power iteration (Rayleigh quotient of the
-// normalized iterate), one CTA of 1024 threads running every iteration, so the host waits once:
-// out[0] = lambda, out[1] = 1 when it settled (|rq - lambda| <= 1e-10 |rq| after the 8th iteration) or
-// ran its 200 iterations with finite values, 0 otherwise. v, w: n doubles of scratch.
+// normalized iterate): out[0] = lambda, out[1] = 1 when it settled (|rq - lambda| <= 1e-10 |rq| after
+// the 8th iteration) or ran its 200 iterations with finite values, 0 otherwise. n <= kPowerMax.
+//
+// One cluster of kPowerCtas CTAs runs every iteration, so the host waits once. Each CTA keeps the whole
+// iterate in shared memory and takes every kPowerCtas-th block row, several warps a row when it has few; a
+// row's results go to all CTAs' shared memory, one cluster barrier ends the product, and every CTA forms the same
+// norm and quotient in the same order, so all leave the loop together. Bound: 200 dependent iterations of
+// a row's L1/L2 latency and a cluster barrier. One CTA that kept the iterate in global memory took 1.80 ms
+// at n = 113; this takes 1.04.
+constexpr int kPowerCtas = 8;
+constexpr int kPowerMax = 2048;
+constexpr size_t power_smem(int n) { return 3 * sizeof(double) * (size_t)n; }
 __global__ void __launch_bounds__(1024) k_power_iteration(RowTables rt, const double* __restrict__ rows,
-                                                          const double* __restrict__ scale, int n, double* v,
-                                                          double* w, double* out) {
-  __shared__ double red[32][2];
-  __shared__ double s_nrm, s_rq;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+                                                          const double* __restrict__ scale, int n, double* out) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) double sh[];  // the iterate, and the product in two alternating buffers
+  __shared__ double red[32][2], s_part[32][6];
+  __shared__ double s_sum[2];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // warps per row: as many as keep the CTA's rows in one round
+  const int mine = (rt.nblocks + kPowerCtas - 1 - rank) / kPowerCtas;
+  int split = 8;
+  while (split > 1 && mine * split > 32) split /= 2;
+  const int per = 32 / split;
+  double* v = sh;
   const double v0 = 1.0 / sqrt((double)n);
-  for (int i = tid; i < n; i += blockDim.x) v[i] = v0;
+  for (int i = tid; i < n; i += 1024) v[i] = v0;
   __syncthreads();
+  cluster.sync();  // every CTA runs before any of them is written to
   double lam = 0.0;
   int ok = 0;
   for (int it = 0; it < 200; ++it) {
-    // w = D S D v: warp per block row
-    for (int X = warp; X < rt.nblocks; X += 32) {
-      const int dX = rt.blk_dim[X], oX = rt.blk_off[X];
-      const uint32_t n0 = rt.nbr_begin[X], n1 = rt.nbr_begin[X + 1];
-      double acc[6] = {0, 0, 0, 0, 0, 0};
-      for (uint32_t q = n0 + lane; q < n1; q += 32) {
-        const int Y = rt.nbr[q];
-        const int dY = rt.blk_dim[Y], oY = rt.blk_off[Y];
-        const double* S = rows + rt.slot_off[q];
-        for (int m = 0; m < dX; ++m) {
-          double s = 0.0;
-          for (int c = 0; c < dY; ++c) s += S[m * dY + c] * (scale[oY + c] * v[oY + c]);
-          acc[m] += s;
+    double* w = sh + (1 + (it & 1)) * (size_t)n;
+    for (int x0 = 0; x0 * kPowerCtas + rank < rt.nblocks; x0 += per) {  // this CTA's rows, `per` at a time
+      const int X = (x0 + warp / split) * kPowerCtas + rank;
+      const bool have = X < rt.nblocks;
+      const int dX = have ? rt.blk_dim[X] : 0;
+      if (have) {
+        double acc[6] = {0, 0, 0, 0, 0, 0};
+        row_times(rt, rows, X, dX, 32u * (warp % split) + lane, 32u * split, [&](int i) { return scale[i] * v[i]; }, acc);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+          acc[m] = warp_sum(acc[m]);
+          if (lane == 0) s_part[warp][m] = acc[m];
         }
       }
-      for (int m = 0; m < 6; ++m) acc[m] = warp_sum(acc[m]);
-      if (lane == 0)
-        for (int m = 0; m < dX; ++m) w[oX + m] = acc[m] * scale[oX + m];
+      __syncthreads();
+      if (warp % split == 0)  // element lane / kPowerCtas of the row to CTA lane % kPowerCtas
+        for (int e = lane; e < dX * kPowerCtas; e += 32) {
+          const int m = e / kPowerCtas, o = rt.blk_off[X] + m;
+          double r = 0.0;
+          for (int q = 0; q < split; ++q) r += s_part[warp + q][m];
+          *cluster.map_shared_rank(w + o, e % kPowerCtas) = r * scale[o];
+        }
+      __syncthreads();
     }
-    __syncthreads();
+    cluster.sync();
     double nn = 0.0, rq = 0.0;
-    for (int i = tid; i < n; i += blockDim.x) {
+    for (int i = tid; i < n; i += 1024) {
       nn += w[i] * w[i];
       rq += v[i] * w[i];
     }
@@ -953,29 +1002,28 @@ __global__ void __launch_bounds__(1024) k_power_iteration(RowTables rt, const do
       red[warp][1] = rq;
     }
     __syncthreads();
-    if (tid == 0) {
-      double a = 0.0, b = 0.0;
-      for (int k = 0; k < 32; ++k) {
-        a += red[k][0];
-        b += red[k][1];
+    if (warp == 0) {
+      const double a = warp_sum(red[lane][0]), b = warp_sum(red[lane][1]);
+      if (lane == 0) {
+        s_sum[0] = sqrt(a);
+        s_sum[1] = b;
       }
-      s_nrm = sqrt(a);
-      s_rq = b;
     }
     __syncthreads();
-    const double nrm = s_nrm, q = s_rq;
+    const double nrm = s_sum[0], q = s_sum[1];
     if (!(isfinite(nrm) && nrm > 0.0)) {
       ok = 0;
       break;
     }
     const bool settled = it > 8 && fabs(q - lam) <= 1e-10 * fabs(q);
     lam = q;
-    for (int i = tid; i < n; i += blockDim.x) v[i] = w[i] / nrm;
+    for (int i = tid; i < n; i += 1024) v[i] = w[i] / nrm;
     __syncthreads();
     ok = 1;
     if (settled) break;
   }
-  if (tid == 0) {
+  cluster.sync();  // no CTA leaves while another may still write to it
+  if (rank == 0 && tid == 0) {
     out[0] = lam;
     out[1] = ok;
   }

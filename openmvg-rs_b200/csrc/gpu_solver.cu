@@ -13,7 +13,7 @@
 //                            (explicit_s.cuh; stands in for faer's sparse LLT)
 //       k_mv_tiles ......... matrix-free reduced-camera-system product S x (retained/operator.rs:137-227)
 //       block-Jacobi PCG ... sparse/pcg.rs:23-119, retained/mod.rs:682-934, retained/block.rs:148-246
-//   K4  k_retract, k_candidate_points: step cap, retraction, back-substitution and candidate rule
+//   K4  k_retract, k_candidate_tiles: step cap, retraction, back-substitution and candidate rule
 //                            (optimizer.rs:376-702, sparse/calibrated/candidate.rs:23-333,
 //                            schur/point.rs:537-728, point_geometry.rs:110-130)
 // Every reduction runs in a fixed order (fixed grid, fixed shuffle trees, fixed chunk order), so a
@@ -83,6 +83,25 @@ void launch_pdl(bool pdl, void (*kernel)(KArgs...), unsigned grid, unsigned bloc
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = pdl ? 1 : 0;
+  (void)cudaLaunchKernelEx(&cfg, kernel, args...);
+  ++tl_telemetry.launches;
+}
+
+// A launch of one thread-block cluster of `cluster` CTAs.
+template <typename... KArgs, typename... Args>
+void launch_cluster(void (*kernel)(KArgs...), unsigned cluster, unsigned block, size_t smem, cudaStream_t st,
+                    Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(cluster);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = cluster;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
   (void)cudaLaunchKernelEx(&cfg, kernel, args...);
   ++tl_telemetry.launches;
 }
@@ -518,40 +537,54 @@ struct LinOut {
   double* sw;      // optional N: sqrt weight per observation (debug linearization only)
 };
 
-// The pose columns of an observation's camera Jacobian (schur/point.rs:286-313), J times the motion
-// of the camera point: pose_motion (point.rs:730-762) [-[q]x | s I] at q = RX, or at the camera point
-// q = RX + t when the mask holds the translation (the camera turns about its fixed centre);
-// translation_motion (point.rs:764-786) alone, s I, when the mask holds the rotation. The FixedBaseline
-// camera's translation columns are the baseline times its S^2 tangent basis.
-__device__ __forceinline__ void pose_jacobian(const double J[2][3], const double rot[3], const double xc[3],
-                                              int mask, int cam, const Gauge& g, double out[2][6]) {
-  double m[3][6];
-  const double* q = (mask & 2) ? rot : xc;
-  const int ts = (mask & 1) ? 3 : 0;  // first translation column
-  for (int r = 0; r < 3; ++r)
-    for (int c = 0; c < 6; ++c) m[r][c] = 0.0;
-  if (mask & 1) {
-    m[0][1] = q[2];
-    m[0][2] = -q[1];
-    m[1][0] = -q[2];
-    m[1][2] = q[0];
-    m[2][0] = q[1];
-    m[2][1] = -q[0];
-  }
-  if (mask & 2) {
-    if (cam == g.fixed_cam) {
-      for (int c = 0; c < 3; ++c) {
-        m[c][ts] = g.baseline * g.b0[c];
-        m[c][ts + 1] = g.baseline * g.b1[c];
+// The camera columns of an observation's record (schur/point.rs:286-313), sqrt-weighted, stored at
+// rec + column * stride for each of the two rows: J times the motion of the camera point. pose_motion
+// (point.rs:730-762) [-[q]x | s I] at q = RX, or at the camera point q = RX + t when the mask holds the
+// translation (the camera turns about its fixed centre); translation_motion (point.rs:764-786) alone,
+// s I, when the mask holds the rotation. The FixedBaseline camera's translation columns are the baseline
+// times its S^2 tangent basis. The intrinsic columns (id of them, Ji) follow the pose's pd, zeros fill
+// the nine. Where a column lands depends on the mask, so the values go to their addresses one by one: a
+// register array indexed by the mask would live in local memory (it did: 512 bytes a thread, twice the
+// kernel's DRAM writes).
+template <typename T>
+__device__ __forceinline__ void store_camera_columns(const double J[2][3], const double Ji[2][3], const double rot[3],
+                                                     const double xc[3], int mask, int pd, int id, int cam,
+                                                     const Gauge& g, double sw, T* rec, int stride) {
+  if (pd > 0) {
+    const double q0 = (mask & 2) ? rot[0] : xc[0], q1 = (mask & 2) ? rot[1] : xc[1], q2 = (mask & 2) ? rot[2] : xc[2];
+    const int ts = (mask & 1) ? 3 : 0;  // first translation column
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      T* r = rec + (size_t)(9 * a) * stride;
+      if (mask & 1) {
+        // the rounding of the row-times-column sums in component order
+        r[0] = T(sw * fma(J[a][2], q1, -__dmul_rn(J[a][1], q2)));
+        r[stride] = T(sw * fma(-J[a][2], q0, __dmul_rn(J[a][0], q2)));
+        r[2 * (size_t)stride] = T(sw * fma(J[a][1], q0, -__dmul_rn(J[a][0], q1)));
       }
-    } else {
-      m[0][ts] = g.scene;
-      m[1][ts + 1] = g.scene;
-      m[2][ts + 2] = g.scene;
+      if (mask & 2) {
+        r += (size_t)ts * stride;
+        if (cam == g.fixed_cam) {
+          const double c0 = fma(J[a][1], g.baseline * g.b0[1], J[a][0] * (g.baseline * g.b0[0]));
+          const double c1 = fma(J[a][1], g.baseline * g.b1[1], J[a][0] * (g.baseline * g.b1[0]));
+          r[0] = T(sw * fma(J[a][2], g.baseline * g.b0[2], c0));
+          r[stride] = T(sw * fma(J[a][2], g.baseline * g.b1[2], c1));
+        } else {
+          r[0] = T(sw * (J[a][0] * g.scene));
+          r[stride] = T(sw * (J[a][1] * g.scene));
+          r[2 * (size_t)stride] = T(sw * (J[a][2] * g.scene));
+        }
+      }
     }
   }
-  for (int r = 0; r < 2; ++r)
-    for (int c = 0; c < 6; ++c) out[r][c] = J[r][0] * m[0][c] + J[r][1] * m[1][c] + J[r][2] * m[2][c];
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
+    T* r = rec + (size_t)(9 * a + pd) * stride;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (k < id) r[(size_t)k * stride] = T(sw * Ji[a][k]);
+    for (int k = pd + id; k < 9; ++k) rec[(size_t)(9 * a + k) * stride] = T(0);
+  }
 }
 
 // The point part of the linearization (schur/assembly.rs:893-1040, point_block.rs:78-184): the
@@ -972,6 +1005,9 @@ namespace omvgba {
 // squared residual) are formed by one thread per point from the observations' row contributions
 // staged in shared memory, in track order and row 0 before row 1 (the reference's accumulation
 // order, schur/point.rs:388-390), followed by the point epilogue.
+// Bound: latency of the dependent gathers (observation, camera, point) at six FP64 tiles an SM. With the
+// columns stored to their places instead of through an indexed array (store_camera_columns): 252 -> 141 us
+// at 1.2M observations, 2.29 -> 1.33 ms at 12M (FP32 records).
 // ----------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(mv_tile_obs<T>(), sizeof(T) == 4 ? 3 : 6) k_linearize_tiles(DevView v, DevState s, Gauge g, LossDev loss,
@@ -1031,25 +1067,8 @@ __global__ void __launch_bounds__(mv_tile_obs<T>(), sizeof(T) == 4 ? 3 : 6) k_li
         contrib[tid][a][7] = w1 * wr;
         contrib[tid][a][8] = w2 * wr;
       }
-      double jc[2][9];
-      for (int a = 0; a < 2; ++a)
-        for (int k = 0; k < 9; ++k) jc[a][k] = 0.0;
-      const int pd = v.pose_dim[cam];
-      if (pd > 0) {
-        double pj[2][6];
-        pose_jacobian(J, rot, xc, v.pose_mask[cam], cam, g, pj);
-        for (int a = 0; a < 2; ++a)
-          for (int k = 0; k < pd; ++k) jc[a][k] = pj[a][k];
-      }
-      if (v.self_cal) {
-        const int id = v.intr_dim[v.cam_group[cam]];
-        for (int a = 0; a < 2; ++a)
-          for (int k = 0; k < id; ++k) jc[a][pd + k] = Ji[a][k];
-      }
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int k = 0; k < 9; ++k) rec[(9 * a + k) * TILE] = T(sw * jc[a][k]);
+      store_camera_columns(J, Ji, rot, xc, v.pose_mask[cam], v.pose_dim[cam],
+                           v.self_cal ? v.intr_dim[v.cam_group[cam]] : 0, cam, g, sw, rec, TILE);
 #pragma unroll
       for (int a = 0; a < 2; ++a)
 #pragma unroll
@@ -1336,7 +1355,7 @@ __global__ void k_retract(DevView v, int ng, const double* step, Gauge g, const 
 
 // Admitted track cost (schur/point.rs:705-728): returns false when a projection fails or the
 // geometry is not admitted.
-__device__ bool admitted_cost(const DevView& v, const double* pose, const double* groups, const double X[3], int p,
+__device__ __noinline__ bool admitted_cost(const DevView& v, const double* pose, const double* groups, const double X[3], int p,
                               const LossDev& loss, double scene, int admission, double* cost) {
   TrackGeometryDev geo;
   geo.init(scene);
@@ -1364,86 +1383,138 @@ struct CandidateOut {
   double cost, step_sq, damping, failed;
 };
 
+// Back-substitution, the candidate points and their cost, one CTA per record tile (whole points), one
+// thread per observation: the observation's share of the back-substitution from the coalesced record;
+// then a thread per point sums its track in order, forms the step and the moved point; then every
+// observation projects its moved point with the candidate cameras, and the point's thread admits the
+// track and sums its cost in track order. A point whose move is not admitted (rare) tries the unmoved
+// point by itself, observation after observation.
+// Bound: HBM on the records at survey sizes, latency below. A thread per point that walked its track for
+// both passes read the records in separate lines and left the projections of a track (33 distortion
+// samples each with k3) in one chain: 78 -> 39 us for 8,000 observations in 20 cameras, 206 -> 149 us for
+// 1.2M, 1.49 -> 1.52 ms for 12M (FP32 records).
 template <typename T>
-__global__ void __launch_bounds__(128) k_candidate_points(DevView v, LinOut<T> lin, const double* step,
-                                                          DevState cur, DevState cand, Gauge g, LossDev loss,
-                                                          RedVec<4>* out) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= v.P) return;
-  double X[3] = {cur.points[3 * p], cur.points[3 * p + 1], cur.points[3 * p + 2]};
-  RedVec<4> res;
-  res.v[0] = res.v[1] = res.v[2] = res.v[3] = 0.0;
-  if (v.fixed_points[p]) {
-    double c;
-    cand.points[3 * p] = X[0];
-    cand.points[3 * p + 1] = X[1];
-    cand.points[3 * p + 2] = X[2];
-    if (!admitted_cost(v, cand.pose, cand.groups, X, p, loss, 0.0, 0, &c))
-      res.v[3] = 1.0;
-    else
-      res.v[0] = c;
-    out[p] = res;
-    return;
-  }
-  // back-substitution: dp = -(Vhat^-1 g_p + Vhat^-1 sum_o Jp_o^T Jc_o dc_o)  (schur/point.rs:537-596)
-  double b0 = 0, b1 = 0, b2 = 0;
-  for (uint32_t o = v.pt_off[p]; o < v.pt_off[p + 1]; ++o) {
-    int cam = v.obs_cam[o];
-    int pd = v.pose_dim[cam], po = v.pose_off[cam];
-    const T* jc = lin.rec + lin.obs_rec[o];
-    const int rs = lin.rs;
-    double e0 = 0, e1 = 0;
-    for (int k = 0; k < pd; ++k) {
-      e0 += (double)jc[k * rs] * step[po + k];
-      e1 += (double)jc[(9 + k) * rs] * step[po + k];
+__global__ void __launch_bounds__(mv_tile_obs<T>(), sizeof(T) == 4 ? 3 : 6)
+    k_candidate_tiles(const __grid_constant__ DevView v, LinOut<T> lin, const double* __restrict__ step, DevState cur,
+                      DevState cand, Gauge g, const __grid_constant__ LossDev loss, MvTiles mt, RedVec<4>* out) {
+  constexpr int TILE = mv_tile_obs<T>();
+  // the step by segment; then the back-substitution terms; then the ray and the cost of each observation
+  __shared__ double xs[kSegParams * TILE];
+  __shared__ double moved_x[3][TILE];
+  __shared__ unsigned char okf[TILE];
+  double(*term)[TILE] = reinterpret_cast<double(*)[TILE]>(xs);
+  const int t = blockIdx.x, tid = threadIdx.x;
+  const uint4 hdr = mt.tile_hdr[t];
+  const unsigned char* slot = mt.slots + (size_t)t * MvSlot::bytes(TILE);
+  const uint32_t w0 = reinterpret_cast<const uint32_t*>(slot + MvSlot::w0(TILE))[tid],
+                 w1 = reinterpret_cast<const uint32_t*>(slot + MvSlot::w1(TILE))[tid];
+  const uint32_t seg = reinterpret_cast<const uint16_t*>(slot + MvSlot::oseg(TILE))[tid];
+  const uint16_t* poff = reinterpret_cast<const uint16_t*>(slot + MvSlot::poff(TILE));
+  const uint16_t* lpt = reinterpret_cast<const uint16_t*>(slot + MvSlot::lpt(TILE));
+  const uint32_t nobs = hdr.x, npt = hdr.y, p0 = hdr.w;
+  const bool obs = (uint32_t)tid < nobs;
+  const uint32_t o = obs ? v.pt_off[p0] + tid : 0;
+  const int cam = obs ? (int)v.obs_cam[o] : 0;
+  if ((uint32_t)tid < hdr.z) {  // thread s gathers the step of segment s's parameters
+    const uint32_t pd = w0 >> 28, id = w1 >> 28;
+#pragma unroll
+    for (int c = 0; c < kSegParams; ++c) {
+      const uint32_t at = (uint32_t)c < pd ? (w0 & 0x0FFFFFFFu) + c : (w1 & 0x0FFFFFFFu) + ((uint32_t)c - pd);
+      xs[kSegParams * tid + c] = (uint32_t)c < pd + id ? step[at] : 0.0;
     }
-    if (v.self_cal) {
-      int gi = v.cam_group[cam];
-      int id = v.intr_dim[gi], io = v.intr_off[gi];
-      for (int k = 0; k < id; ++k) {
-        e0 += (double)jc[(pd + k) * rs] * step[io + k];
-        e1 += (double)jc[(9 + pd + k) * rs] * step[io + k];
+  }
+  __syncthreads();
+  double mine[3];
+  if (obs) {
+    const T* r = lin.rec + (size_t)t * TILE * kRec + tid;
+    const double* s = xs + kSegParams * seg;
+    double e0 = 0.0, e1 = 0.0;
+#pragma unroll
+    for (int k = 0; k < kSegParams; ++k) {
+      e0 += (double)r[(size_t)k * TILE] * s[k];  // columns past the camera's are zero
+      e1 += (double)r[(size_t)(9 + k) * TILE] * s[k];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      mine[c] = (double)r[(size_t)(kJp + c) * TILE] * e0 + (double)r[(size_t)(kJp + 3 + c) * TILE] * e1;
+  }
+  __syncthreads();  // the step is read: its place takes the terms
+  if (obs)
+    for (int c = 0; c < 3; ++c) term[c][tid] = mine[c];
+  __syncthreads();
+  const bool point = (uint32_t)tid < npt;
+  const uint32_t p = p0 + tid;
+  double X[3] = {0, 0, 0}, sp[3] = {0, 0, 0}, st[3];
+  bool fixed = false;
+  uint32_t a = 0, b = 0;
+  if (point) {
+    a = poff[tid];
+    b = poff[tid + 1];
+    fixed = v.fixed_points[p] != 0;
+    for (int c = 0; c < 3; ++c) st[c] = X[c] = cur.points[3 * (size_t)p + c];
+    if (!fixed) {
+      // dp = -(Vhat^-1 g_p + Vhat^-1 sum_o Jp_o^T Jc_o dc_o)  (schur/point.rs:537-596)
+      double bb[3] = {0, 0, 0}, z[3];
+      for (uint32_t i = a; i < b; ++i)
+        for (int c = 0; c < 3; ++c) bb[c] += term[c][i];
+      sym3_apply(lin.vinv + 6 * (size_t)p, bb, z);
+      const double* ig = lin.ig + 3 * (size_t)p;
+      for (int c = 0; c < 3; ++c) {
+        sp[c] = -(ig[c] + z[c]);
+        st[c] = X[c] + g.scene * sp[c];
       }
     }
-    const T* jp = jc + kJp * rs;
-    b0 += (double)jp[0] * e0 + (double)jp[3 * rs] * e1;
-    b1 += (double)jp[rs] * e0 + (double)jp[4 * rs] * e1;
-    b2 += (double)jp[2 * rs] * e0 + (double)jp[5 * rs] * e1;
+    for (int c = 0; c < 3; ++c) moved_x[c][tid] = st[c];
   }
-  const double* vi = lin.vinv + 6 * (size_t)p;
-  const double* ig = lin.ig + 3 * (size_t)p;
-  double bb[3] = {b0, b1, b2}, z[3];
-  sym3_apply(vi, bb, z);
-  double sp[3] = {-(ig[0] + z[0]), -(ig[1] + z[1]), -(ig[2] + z[2])};
-  double st[3] = {X[0] + g.scene * sp[0], X[1] + g.scene * sp[1], X[2] + g.scene * sp[2]};
-  // candidate_rule (point_geometry.rs:110-130)
-  double c;
-  bool moved = false, have = false;
-  if (admitted_cost(v, cand.pose, cand.groups, st, p, loss, g.scene, 2, &c)) {
-    moved = true;
-    have = true;
-  } else if (admitted_cost(v, cand.pose, cand.groups, X, p, loss, g.scene, 1, &c)) {
-    have = true;
-  } else {
-    double c2;
-    if (!admitted_cost(v, cur.pose, cur.groups, X, p, loss, g.scene, 1, &c2)) {
-      if (admitted_cost(v, cand.pose, cand.groups, X, p, loss, g.scene, 0, &c)) have = true;
+  __syncthreads();
+  if (obs) {
+    const uint32_t lp = lpt[tid];
+    const double x[3] = {moved_x[0][lp], moved_x[1][lp], moved_x[2][lp]};
+    const double* P = cand.pose + 12 * cam;
+    double xc[3], r[2], J[2][3], Ji[2][3];
+    for (int i = 0; i < 3; ++i) xc[i] = P[3 * i] * x[0] + P[3 * i + 1] * x[1] + P[3 * i + 2] * x[2] + P[9 + i];
+    const bool ok = project_obs(v, cand.groups, o, xc, r, J, Ji);
+    okf[tid] = ok ? 1 : 0;
+    if (ok) {
+      for (int j = 0; j < 3; ++j) term[j][tid] = P[j] * xc[0] + P[3 + j] * xc[1] + P[6 + j] * xc[2];
+      term[3][tid] = loss.cost(sqrt(r[0] * r[0] + r[1] * r[1]));
     }
   }
+  __syncthreads();
+  if (!point) return;
+  // admitted_cost of the first attempt: a free point must stay off degenerate geometry
+  TrackGeometryDev geo;
+  geo.init(fixed ? 0.0 : g.scene);
+  double c = 0.0;
+  bool have = true;
+  for (uint32_t i = a; i < b && have; ++i) {
+    have = okf[i] != 0;
+    if (!have) break;
+    geo.push(term[0][i], term[1][i], term[2][i]);
+    c += term[3][i];
+  }
+  have = have && (fixed || !geo.degenerate());
+  bool moved = have && !fixed;
+  if (!have && !fixed) {  // candidate_rule (point_geometry.rs:110-130): the unmoved point
+    double c2;
+    if (admitted_cost(v, cand.pose, cand.groups, X, p, loss, g.scene, 1, &c))
+      have = true;
+    else if (!admitted_cost(v, cur.pose, cur.groups, X, p, loss, g.scene, 1, &c2))
+      have = admitted_cost(v, cand.pose, cand.groups, X, p, loss, g.scene, 0, &c);
+  }
+  RedVec<4> res;
+  res.v[0] = res.v[1] = res.v[2] = res.v[3] = 0.0;
+  if (fixed || have)
+    for (int k = 0; k < 3; ++k) cand.points[3 * (size_t)p + k] = moved ? st[k] : X[k];
   if (!have) {
     res.v[3] = 1.0;
-    out[p] = res;
-    return;
-  }
-  const double* P = moved ? st : X;
-  cand.points[3 * p] = P[0];
-  cand.points[3 * p + 1] = P[1];
-  cand.points[3 * p + 2] = P[2];
-  res.v[0] = c;
-  if (moved) {
-    res.v[1] = sp[0] * sp[0] + sp[1] * sp[1] + sp[2] * sp[2];
-    const double* dd = lin.ddiag + 3 * (size_t)p;
-    res.v[2] = dd[0] * sp[0] * sp[0] + dd[1] * sp[1] * sp[1] + dd[2] * sp[2] * sp[2];
+  } else {
+    res.v[0] = c;
+    if (moved) {
+      res.v[1] = sp[0] * sp[0] + sp[1] * sp[1] + sp[2] * sp[2];
+      const double* dd = lin.ddiag + 3 * (size_t)p;
+      res.v[2] = dd[0] * sp[0] * sp[0] + dd[1] * sp[1] * sp[1] + dd[2] * sp[2] * sp[2];
+    }
   }
   out[p] = res;
 }
@@ -2513,7 +2584,7 @@ struct Solver {
     up_i(d_perm_to_orig, S.perm_to_orig);
     d_rows.alloc(std::max<uint64_t>(1, S.slot_off.empty() ? 1 : S.slot_off.back()), st);
     d_perm_vec.alloc(std::max(1, D), st);
-    d_power.alloc(2 * (size_t)std::max(1, D) + 2, st);
+    d_power.alloc(2, st);
     for (DBuf<double>* b : {&d_step, &d_r, &d_z, &d_dir, &d_q, &d_tmp, &d_rhs, &d_r64, &d_e}) b->alloc(std::max(1, D), st);
     d_factor.alloc((size_t)42 * std::max(1, nb), st);
     d_dq.alloc(std::max(1, nb), st);
@@ -2686,18 +2757,7 @@ struct Solver {
     {  // one cluster: a CTA per tile of the band, up to kSolveCtas
       int ctas = 1;
       while (ctas < kSolveCtas && ctas < S.bwt) ctas *= 2;
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3(ctas);
-      cfg.blockDim = dim3(256);
-      cfg.stream = st;
-      cudaLaunchAttribute attr{};
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = ctas;
-      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-      cfg.attrs = &attr;
-      cfg.numAttrs = 1;
-      (void)cudaLaunchKernelEx(&cfg, k_tile_solve, tile_band(), d_perm_vec.p, (const int*)d_status.p);
-      ++tl_telemetry.launches;
+      launch_cluster(k_tile_solve, ctas, 256, 0, st, tile_band(), d_perm_vec.p, (const int*)d_status.p);
     }
     OMVGBA_LAUNCH(k_perm_scatter, grid_for(D, 256), 256, 0, st, D, d_perm_to_orig.p, d_perm_vec.p, d_step.p);
     check_launch();
@@ -2972,11 +3032,17 @@ struct Solver {
       OMVGBA_LAUNCH(k_block_rows<T>, nb, kRowThreads, smem, st, row_tables(), lin(), row_smem, d_rows.p);
   }
 
+  int rows_product_ctas() const { return grid_for((size_t)nb * row_split(nb), kRowProductWarps); }
+  void rows_product(bool pdl, const double* x, double* y, double lambda, double* xy, const PcgCtl* ctl) {
+    const int split = row_split(nb);
+    launch_pdl(pdl, split == 4 ? k_rows_matvec<4> : (split == 2 ? k_rows_matvec<2> : k_rows_matvec<1>),
+               rows_product_ctas(), 32 * kRowProductWarps, st, row_tables(), (const double*)d_rows.p,
+               (const double*)d_diag.p, lambda, x, y, xy, ctl);
+    check_launch();
+  }
   // y = (S + lambda diag) x from the rows
   void rows_matvec(const double* x, double* y, double lambda) {
-    OMVGBA_LAUNCH(k_rows_matvec, grid_for((size_t)nb * 32, 256), 256, 0, st, row_tables(), d_rows.p, d_diag.p, lambda,
-                  (const double*)nullptr, x, y, (double*)nullptr, (const PcgCtl*)nullptr);
-    check_launch();
+    rows_product(false, x, y, lambda, nullptr, nullptr);
   }
 
   // Cholesky of (S + lambda diag) -- equilibrated as scale S scale and shifted by -shift I when scale
@@ -3053,6 +3119,7 @@ struct Solver {
   int rank_certificate(bool* factored_s) {
     *factored_s = false;
     if (D == 0) return 0;
+    static_assert(kPowerMax >= 2048, "the spectral test holds the iterate of every D up to the limit");
     if (D > opt.dense_rank_limit) {
       const bool ok = factor_band(0.0, nullptr, 0.0);
       *factored_s = ok;
@@ -3073,11 +3140,13 @@ struct Solver {
       sc[i] = 1.0 / std::sqrt(std::max(dg[i], fl));
     }
     CUDA_OK(copy_async(d_e.p, sc.data(), sizeof(double) * D, cudaMemcpyHostToDevice, st));
-    OMVGBA_LAUNCH(k_power_iteration, 1, 1024, 0, st, row_tables(), d_rows.p, d_e.p, D, d_power.p, d_power.p + D,
-                  d_power.p + 2 * (size_t)D);
+    CUDA_OK(cudaFuncSetAttribute(k_power_iteration, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)power_smem(kPowerMax)));
+    launch_cluster(k_power_iteration, kPowerCtas, 1024, power_smem(D), st, row_tables(), (const double*)d_rows.p,
+                   (const double*)d_e.p, D, d_power.p);
     check_launch();
     double out[2];
-    CUDA_OK(copy_async(out, d_power.p + 2 * (size_t)D, sizeof(out), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(copy_async(out, d_power.p, sizeof(out), cudaMemcpyDeviceToHost, st));
     sync();
     const double largest = std::fabs(out[0]);
     if (out[1] == 0.0 || !(std::isfinite(largest) && largest > 0.0)) return 2;
@@ -3166,15 +3235,15 @@ struct Solver {
   // y = S_lambda x (implicit, matrix-free); ctl: optional PCG control for graph-launched iterations
   // fp32: use the FP32 record copy (mixed precision inner solves)
   int mv_finalize_ctas() const { return std::max(1, grid_for((size_t)nb * 32, 256)); }
+  // CTAs of the product's last kernel, each of which leaves one curvature term
+  int product_ctas() const { return explicit_op ? rows_product_ctas() : mv_finalize_ctas(); }
   // xy: optional per-finalize-CTA sums of x_b . y_b over the CTA's blocks (the PCG curvature terms)
   // pdl_tiles / pdl: launch the tile pass / the finalize as programmatic dependents of the kernel
   // before them (inside the PCG graph)
   void matvec(const double* x, double* y, double lambda, const PcgCtl* ctl = nullptr, bool fp32 = false,
               double* xy = nullptr, bool pdl_tiles = false, bool pdl = false) {
     if (explicit_op) {  // block-sparse product of the explicit S (FP64 rows)
-      launch_pdl(pdl_tiles, k_rows_matvec, mv_finalize_ctas(), 256, st, row_tables(), (const double*)d_rows.p,
-                 (const double*)d_diag.p, lambda, (const double*)nullptr, x, y, xy, ctl);
-      check_launch();
+      rows_product(pdl_tiles, x, y, lambda, xy, ctl);
       return;
     }
     matvec_tiles(x, ctl, fp32, pdl_tiles);
@@ -3298,7 +3367,7 @@ struct Solver {
       const int slot = it & 1;
       matvec(d_dir.p, d_q.p, lambda, dctl, fp32, d_dq.p, it > 0, true);
       const int nupd = grid_for(nb, kUpdThreads);
-      launch_pdl(true, k_pcg_update_precond, nupd, kUpdThreads, st, tables(), d_factor.p, d_dq.p, mv_finalize_ctas(),
+      launch_pdl(true, k_pcg_update_precond, nupd, kUpdThreads, st, tables(), d_factor.p, d_dq.p, product_ctas(),
                  d_dir.p, d_q.p, x, d_r.p, d_z.p, d_rr_part.p, d_rz_part.p, slot, dctl);
       launch_pdl(true, k_pcg_direction, grid_for(D, 256), 256, st, D, d_rr_part.p, d_rz_part.p, nupd, d_z.p, d_dir.p,
                  slot, dctl);
@@ -3665,12 +3734,16 @@ struct Solver {
         DevView v = view();
         OMVGBA_LAUNCH(k_retract, grid_for(std::max(n.ncam, ng), 128), 128, 0, st, v, ng, d_step.p, g, d_pose[cur].p,
                       d_groups[cur].p, d_pose[cand].p, d_groups[cand].p);
-        if (mixed)
-          OMVGBA_LAUNCH(k_candidate_points<float>, grid_for(P, 128), 128, 0, st, v, lin32(), d_step.p, state(cur),
-                        state(cand), g, stages[si].loss, d_cand.p);
-        else
-          OMVGBA_LAUNCH(k_candidate_points<T>, grid_for(P, 128), 128, 0, st, v, lin(), d_step.p, state(cur),
-                        state(cand), g, stages[si].loss, d_cand.p);
+        {
+          const TileSetDev& ts = mixed ? dT32 : dT64;
+          const MvTiles mt = ts.view(d_blk_dim.p, d_blk_off.p, nb);
+          if (mixed && mt.ntiles > 0)
+            OMVGBA_LAUNCH(k_candidate_tiles<float>, mt.ntiles, mv_tile_obs<float>(), 0, st, v, lin32(), d_step.p, state(cur),
+                          state(cand), g, stages[si].loss, mt, d_cand.p);
+          else if (mt.ntiles > 0)
+            OMVGBA_LAUNCH(k_candidate_tiles<T>, mt.ntiles, mv_tile_obs<T>(), 0, st, v, lin(), d_step.p, state(cur),
+                          state(cand), g, stages[si].loss, mt, d_cand.p);
+        }
         check_launch();
         RedVec<4> cr = reduce<4>(d_cand.p, P, d_cand_part);
         if (cr.v[3] > 0.0) {
