@@ -298,7 +298,8 @@ __device__ __forceinline__ void row_times(const RowTables& rt, const double* __r
 
 // y = (S + lambda diag) x from the block rows: SPLIT warps per block row, the row's blocks dealt over
 // their lanes in a fixed assignment, then a fixed shuffle tree and the warps in order. With xy non-null,
-// xy[CTA] = sum of x_b . y_b over the CTA's blocks in block order.
+// xy[CTA] = sum of x_b . y_b over the CTA's blocks in block order. With ctl the damping is the control
+// block's.
 // Bound: L2 where S fits it (500 cameras: 30 MB), HBM above, latency below. SPLIT: while one warp per row
 // leaves an SM fewer than eight warps (row_split) its loads do not cover the latency; measured on block
 // rows of 61 cameras (one / two / four warps, back to back): 120 cameras 12.3 / 8.3 / 6.2 us, 500 12.4 /
@@ -320,6 +321,7 @@ __global__ void __launch_bounds__(32 * kRowProductWarps) k_rows_matvec(RowTables
   pdl_trigger();
   pdl_wait();
   if (pcg_stopped(ctl)) return;
+  if (ctl) lambda = ctl->lambda;
   const int dX = have ? rt.blk_dim[X] : 0;
   if (have) {
     double acc[6] = {0, 0, 0, 0, 0, 0};

@@ -132,6 +132,33 @@ struct PinnedStage {
 };
 thread_local PinnedStage tl_pinned;
 thread_local PinnedStage tl_poll;  // the PCG loop's status mirrors (read while the next batch runs)
+thread_local PinnedStage tl_read;  // the results of a group of kernels (Readback)
+
+// Several device results read with one wait: room for `bytes` in the calling thread's pinned buffer (in
+// pageable memory when there is none), copies queued on the stream, then wait() before the host reads.
+// One Readback per thread is in use at a time.
+struct Readback {
+  cudaStream_t st;
+  unsigned char* base;
+  size_t used = 0;
+  std::vector<unsigned char> pageable;
+  Readback(cudaStream_t stream, size_t bytes) : st(stream), base(static_cast<unsigned char*>(tl_read.get(bytes))) {
+    if (!base) {
+      pageable.resize(bytes);
+      base = pageable.data();
+    }
+  }
+  static size_t room(size_t bytes) { return (bytes + 15) & ~size_t(15); }
+  template <typename V>
+  const V* add(const V* device, size_t count) {
+    V* host = reinterpret_cast<V*>(base + used);
+    used += room(sizeof(V) * count);
+    if (count) CUDA_OK(cudaMemcpyAsync(host, device, sizeof(V) * count, cudaMemcpyDeviceToHost, st));
+    tl_telemetry.d2h += sizeof(V) * count;
+    return host;
+  }
+  void wait() { CUDA_OK(cudaStreamSynchronize(st)); }
+};
 constexpr size_t kStagedCopyMax = 1u << 20;
 
 // Large host->device copies from pageable memory: the source is copied by several host threads into
@@ -794,7 +821,8 @@ enum PcgStatus : int { kRunning = 0, kCheckResidual = 1, kRejected = 2, kExhaust
 struct PcgCtl {
   // rho_slot: r.z of the current residual, in one of two slots: an iteration reads slot p and its
   // direction kernel writes slot p ^ 1, so no CTA reads a value another CTA of the same kernel writes.
-  double n0, rho_slot[2], alpha, beta, curv, rr, rz, ratio, tol;
+  // lambda: the damping of the product, here so that one captured iteration serves every damping.
+  double n0, rho_slot[2], alpha, beta, curv, rr, rz, ratio, tol, lambda;
   int status, terms, max_it, pad;
 };
 
@@ -1229,29 +1257,33 @@ __global__ void k_residual_update(int n, const double* g, const double* q, doubl
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) r[i] = -g[i] - q[i];
 }
-__global__ void k_scale(int n, double s, double* x) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) x[i] *= s;
-}
 
 // ----------------------------------------------------------------------------------------------
 // K4: step cap, retraction, candidate points
 // ----------------------------------------------------------------------------------------------
-// Per camera: max of the rotation-part norm and the rest (limit_camera_step, optimizer.rs:677-702)
-__global__ void k_step_block_norm(int ncam, const int* pose_off, const int* pose_dim, const double* step,
-                                  double* out) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncam) return;
-  int d = pose_dim[c], o = pose_off[c];
-  if (d == 0) {
-    out[c] = 0.0;
-    return;
+// limit_camera_step (optimizer.rs:677-702): the largest over the cameras of the norms of a pose step's
+// first three coordinates and of the rest; when it is above 0.5 the whole step is scaled down to it.
+// One CTA, so that the step is capped without a trip to the host.
+__global__ void __launch_bounds__(1024) k_step_cap(int ncam, const int* __restrict__ pose_off,
+                                                   const int* __restrict__ pose_dim, int n, double* step) {
+  __shared__ double sh[32];
+  double mx = 0.0;
+  for (int c = threadIdx.x; c < ncam; c += blockDim.x) {
+    const int d = pose_dim[c], o = pose_off[c];
+    const int fd = d < 3 ? d : 3;
+    double s1 = 0.0, s2 = 0.0;
+    for (int k = 0; k < fd; ++k) s1 += step[o + k] * step[o + k];
+    for (int k = fd; k < d; ++k) s2 += step[o + k] * step[o + k];
+    mx = fmax(mx, fmax(sqrt(s1), sqrt(s2)));
   }
-  int fd = d < 3 ? d : 3;
-  double s1 = 0.0, s2 = 0.0;
-  for (int k = 0; k < fd; ++k) s1 += step[o + k] * step[o + k];
-  for (int k = fd; k < d; ++k) s2 += step[o + k] * step[o + k];
-  out[c] = fmax(sqrt(s1), sqrt(s2));
+  mx = warp_max(mx);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = mx;
+  __syncthreads();  // every norm has been taken before any coordinate is scaled
+  mx = sh[0];
+  for (int w = 1; w < 32; ++w) mx = fmax(mx, sh[w]);
+  if (!(mx > 0.5)) return;
+  const double s = 0.5 / mx;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) step[i] *= s;
 }
 
 __host__ __device__ __forceinline__ void exp_so3_dev(const double w[3], double R[9]) {
@@ -2324,7 +2356,7 @@ struct Solver {
   DBuf<uint32_t> d_blk_ent, d_nbr_begin;
   DBuf<int> d_ent_block, d_nbr, d_nbr_row, d_perm_off, d_perm_to_orig;
   DBuf<uint64_t> d_slot_off;
-  DBuf<double> d_rows, d_tiles, d_winv, d_ztiles, d_perm_vec, d_marg_out, d_power;
+  DBuf<double> d_rows, d_tiles, d_winv, d_ztiles, d_zpart, d_zq, d_perm_vec, d_marg_out, d_power;
   bool rows_valid = false;  // the rows hold S of the current assembly
   bool rows_attr = false;   // k_block_rows may take kRowSmemDoubles of dynamic shared memory
   // camera pairs of the explicit S (pair_rows.cuh), built at the first build of the rows
@@ -2345,7 +2377,7 @@ struct Solver {
   DBuf<int> d_fail;
 
 
-  DBuf<double> d_scalars, d_cam_norm, d_ctl;
+  DBuf<double> d_scalars, d_ctl;
   DBuf<RedVec<4>> d_cand, d_cand_part;
   DBuf<RedVec<3>> d_met, d_met_part;
   DBuf<RedVec<1>> d_one, d_one_part;
@@ -2602,7 +2634,6 @@ struct Solver {
     }
     d_scalars.alloc(16, st);
     d_ctl.alloc((sizeof(PcgCtl) + sizeof(double) - 1) / sizeof(double), st);
-    d_cam_norm.alloc(std::max(1, n.ncam), st);
     d_cand.alloc(P, st);
     d_cand_part.alloc(red_blocks, st);
     d_met.alloc(P, st);
@@ -2694,31 +2725,21 @@ struct Solver {
     BlockTables bt = tables();
     if (bt.nchunks > 0) {
       camera_sums();
-      CUDA_OK(cudaMemsetAsync(d_gfull.p, 0, sizeof(double) * std::max(1, D), st));
-      CUDA_OK(cudaMemsetAsync(d_gred.p, 0, sizeof(double) * std::max(1, D), st));
-      CUDA_OK(cudaMemsetAsync(d_diag.p, 0, sizeof(double) * std::max(1, D), st));
       OMVGBA_LAUNCH(k_block_vectors, grid_for(nb, 64), 64, 0, st, bt, d_blk_out.p, d_gfull.p, d_gred.p, d_diag.p, d_clamp.p,
                                                      d_diag_minmax.p);
       check_launch();
     }
     rows_valid = false;
     if (build_rows && D > 0) this->build_rows();
-    PointSummary ps;
-    CUDA_OK(copy_async(&ps, d_summary_part.p, sizeof(ps), cudaMemcpyDeviceToHost, st));
-    std::vector<double> mm(2 * std::max(nb, 1));
-    std::vector<int> cl(std::max(nb, 1));
-    std::vector<double> gvals(std::max(D, 1)), dvals(std::max(D, 1));
-    if (nb > 0) {
-      CUDA_OK(copy_async(mm.data(), d_diag_minmax.p, sizeof(double) * 2 * nb, cudaMemcpyDeviceToHost, st));
-      CUDA_OK(copy_async(cl.data(), d_clamp.p, sizeof(int) * nb, cudaMemcpyDeviceToHost, st));
-    }
-    if (D > 0) {
-      CUDA_OK(copy_async(gvals.data(), d_gfull.p, sizeof(double) * D, cudaMemcpyDeviceToHost, st));
-      CUDA_OK(copy_async(dvals.data(), d_diag.p, sizeof(double) * D, cudaMemcpyDeviceToHost, st));
-    }
-    std::vector<double> gr(std::max(D, 1));
-    if (D > 0) CUDA_OK(copy_async(gr.data(), d_gred.p, sizeof(double) * D, cudaMemcpyDeviceToHost, st));
-    sync();
+    // every result of the assembly with one wait
+    Readback rb(st, Readback::room(sizeof(PointSummary)) + Readback::room(sizeof(double) * 2 * nb) +
+                        Readback::room(sizeof(int) * nb) + 3 * Readback::room(sizeof(double) * D));
+    const PointSummary* psp = rb.add(d_summary_part.p, 1);
+    const double* mm = rb.add(d_diag_minmax.p, 2 * (size_t)nb);
+    const int* cl = rb.add(d_clamp.p, nb);
+    const double *gvals = rb.add(d_gfull.p, D), *dvals = rb.add(d_diag.p, D), *gr = rb.add(d_gred.p, D);
+    rb.wait();
+    const PointSummary ps = *psp;
     Assembly a;
     a.valid = ps.invalid == 0.0;
     a.cost = ps.cost;
@@ -2751,8 +2772,9 @@ struct Solver {
   }
 
   // ---- camera step ----
-  bool direct_step(double lambda) {
-    if (!factor_band(lambda, nullptr, 0.0)) return false;
+  // Whether the factorization succeeded is in d_status when the stream gets there.
+  void direct_step(double lambda) {
+    factor_band(lambda, nullptr, 0.0, false);
     OMVGBA_LAUNCH(k_perm_gather, grid_for(D, 256), 256, 0, st, D, d_perm_to_orig.p, d_gred.p, -1.0, d_perm_vec.p);
     {  // one cluster: a CTA per tile of the band, up to kSolveCtas
       int ctas = 1;
@@ -2761,7 +2783,6 @@ struct Solver {
     }
     OMVGBA_LAUNCH(k_perm_scatter, grid_for(D, 256), 256, 0, st, D, d_perm_to_orig.p, d_perm_vec.p, d_step.p);
     check_launch();
-    return true;
   }
 
   // S of the current linearization (no damping) by block rows, from the FP64 or FP32 records.
@@ -3077,7 +3098,9 @@ struct Solver {
     CUDA_OK(se);
   }
 
-  bool factor_band(double lambda, const double* scale, double shift) {
+  // With check false the status stays on the device: the kernels after a failed factorization return at
+  // once, and the caller reads d_status with its next results.
+  bool factor_band(double lambda, const double* scale, double shift, bool check = true) {
     if (D == 0) return true;
     const double t_factor = now();
     const size_t count = (size_t)S.nt * (S.bwt + 1) * kCTT;
@@ -3103,6 +3126,7 @@ struct Solver {
       }
     });
     check_launch();
+    if (!check) return true;
     int ok = 0;
     CUDA_OK(copy_async(&ok, d_status.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     sync();
@@ -3173,7 +3197,7 @@ struct Solver {
     if (!factored_s && !factor_band(0.0, nullptr, 0.0)) return false;
     // selected inverse of S inside the band (Takahashi recurrence), last tile column first
     const size_t count = (size_t)S.nt * (S.bwt + 1) * kCTT;
-    d_ztiles.alloc(count, st);
+    if (d_ztiles.n != count) d_ztiles.alloc(count, st);
     CUDA_OK(cudaFuncSetAttribute(k_takahashi_partial, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakahashiSmem));
     CUDA_OK(cudaFuncSetAttribute(k_takahashi_offdiag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakahashiSmem));
     CUDA_OK(cudaFuncSetAttribute(k_takahashi_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakahashiSmem));
@@ -3181,9 +3205,9 @@ struct Solver {
     const TileBand tz{D, S.nt, S.bwt, d_ztiles.p, nullptr};
     // scratch: the split partial sums of one column and the diagonal shares of its tiles
     const int max_split = (S.bwt + kTakahashiChunk - 1) / kTakahashiChunk;
-    DBuf<double> d_zpart, d_zq;
-    d_zpart.alloc((size_t)std::max(S.bwt, 1) * std::max(max_split, 1) * kCTT, st);
-    d_zq.alloc((size_t)std::max(S.bwt, 1) * kCTT, st);
+    const size_t npart = (size_t)std::max(S.bwt, 1) * std::max(max_split, 1) * kCTT;
+    if (d_zpart.n != npart) d_zpart.alloc(npart, st);
+    if (d_zq.n != (size_t)std::max(S.bwt, 1) * kCTT) d_zq.alloc((size_t)std::max(S.bwt, 1) * kCTT, st);
     run_as_graph([&] {
       for (int j = S.nt - 1; j >= 0; --j) {
         const int m = std::min(S.bwt, S.nt - 1 - j);
@@ -3210,7 +3234,6 @@ struct Solver {
     CUDA_OK(copy_async(m.data(), d_marg_out.p, sizeof(double) * m.size(), cudaMemcpyDeviceToHost, st));
     CUDA_OK(copy_async(&ok, d_status.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     sync();
-    d_ztiles.release();
     if (!ok) return false;
     for (int i = 0; i < total; ++i)
       for (int k = 0; k < 9; ++k) out[9 * (size_t)gid[i] + k] = m[9 * (size_t)i + k];
@@ -3218,6 +3241,12 @@ struct Solver {
   }
 
   void dots(std::initializer_list<std::pair<const double*, const double*>> pairs, double* out) {
+    queue_dots(pairs);
+    CUDA_OK(copy_async(out, d_scalars.p, sizeof(double) * pairs.size(), cudaMemcpyDeviceToHost, st));
+    sync();
+  }
+  // into d_scalars, from element `at`
+  void queue_dots(std::initializer_list<std::pair<const double*, const double*>> pairs, int at = 0) {
     DotArgs a{};
     int k = 0;
     for (auto& pr : pairs) {
@@ -3226,10 +3255,8 @@ struct Solver {
       ++k;
     }
     a.count = k;
-    OMVGBA_LAUNCH(k_dots, 1, 1024, 0, st, a, D, d_scalars.p);
+    OMVGBA_LAUNCH(k_dots, 1, 1024, 0, st, a, D, d_scalars.p + at);
     check_launch();
-    CUDA_OK(copy_async(out, d_scalars.p, sizeof(double) * k, cudaMemcpyDeviceToHost, st));
-    sync();
   }
 
   // y = S_lambda x (implicit, matrix-free); ctl: optional PCG control for graph-launched iterations
@@ -3310,6 +3337,54 @@ struct Solver {
   // b - S x (the reference's rule); without it the recursive residual decides (inner solves of the
   // mixed-precision refinement, whose outer loop checks the FP64 residual). fp32: FP32 products.
   static constexpr int kPoll = 8;
+  // One poll batch (kPoll iterations, an even count) as an instantiated graph, kept with the solver: it
+  // depends on the solution vector, the products' precision and the operator, which take a handful of
+  // values in a solve, and on nothing else (the damping is in the control block; every buffer lives as
+  // long as the solver). Capturing and instantiating it for every run cost 0.17-0.4 ms each.
+  struct PcgGraph {
+    const double* x;
+    bool fp32, explicit_op;
+    cudaGraphExec_t exec;
+    uint64_t kernels;
+  };
+  std::vector<PcgGraph> pcg_graphs;
+  const PcgGraph& pcg_graph(double* x, bool fp32) {
+    for (const PcgGraph& g : pcg_graphs)
+      if (g.x == x && g.fp32 == fp32 && g.explicit_op == explicit_op) return g;
+    PcgCtl* dctl = reinterpret_cast<PcgCtl*>(d_ctl.p);
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    const uint64_t launches_before = tl_telemetry.launches;
+    CUDA_OK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    // even iterations read rho slot 0, odd ones slot 1 (every kernel after the graph's first is a
+    // programmatic dependent of the one before it)
+    static_assert(kPoll % 2 == 0, "the rho slots alternate");
+    for (int it = 0; it < kPoll; ++it) {
+      const int slot = it & 1;
+      matvec(d_dir.p, d_q.p, 0.0, dctl, fp32, d_dq.p, it > 0, true);
+      const int nupd = grid_for(nb, kUpdThreads);
+      launch_pdl(true, k_pcg_update_precond, nupd, kUpdThreads, st, tables(), d_factor.p, d_dq.p, product_ctas(),
+                 d_dir.p, d_q.p, x, d_r.p, d_z.p, d_rr_part.p, d_rz_part.p, slot, dctl);
+      launch_pdl(true, k_pcg_direction, grid_for(D, 256), 256, st, D, d_rr_part.p, d_rz_part.p, nupd, d_z.p, d_dir.p,
+                 slot, dctl);
+    }
+    const cudaError_t ce = cudaStreamEndCapture(st, &graph);
+    const uint64_t kernels = tl_telemetry.launches - launches_before;  // counted at capture
+    tl_telemetry.launches = launches_before;
+    if (ce != cudaSuccess) {
+      if (graph) cudaGraphDestroy(graph);
+      CUDA_OK(ce);
+    }
+    const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
+    cudaGraphDestroy(graph);
+    CUDA_OK(ie);
+    pcg_graphs.push_back({x, fp32, explicit_op, exec, kernels});
+    return pcg_graphs.back();
+  }
+  ~Solver() {
+    for (PcgGraph& g : pcg_graphs) cudaGraphExecDestroy(g.exec);
+  }
+
   PcgResult pcg_run(const double* b, double* x, double lambda, uint64_t max_it, double tol, bool fp32, bool confirm) {
     double t_start = now();
     int launches = 0, restarts = 0;
@@ -3332,7 +3407,12 @@ struct Solver {
     CUDA_OK(cudaMemsetAsync(x, 0, sizeof(double) * D, st));
     CUDA_OK(copy_async(d_r.p, b, sizeof(double) * D, cudaMemcpyDeviceToDevice, st));
     double h[4];
-    dots({{d_r.p, d_r.p}}, h);
+    queue_dots({{d_r.p, d_r.p}});
+    precond(d_r.p, d_z.p);
+    CUDA_OK(copy_async(d_dir.p, d_z.p, sizeof(double) * D, cudaMemcpyDeviceToDevice, st));
+    queue_dots({{d_r.p, d_z.p}}, 1);
+    CUDA_OK(copy_async(h, d_scalars.p, sizeof(double) * 2, cudaMemcpyDeviceToHost, st));
+    sync();
     double n0 = std::sqrt(h[0]);
     if (!std::isfinite(n0)) return res;
     if (n0 == 0.0) {
@@ -3340,10 +3420,7 @@ struct Solver {
       res.rel = 0.0;
       return res;
     }
-    precond(d_r.p, d_z.p);
-    CUDA_OK(copy_async(d_dir.p, d_z.p, sizeof(double) * D, cudaMemcpyDeviceToDevice, st));
-    dots({{d_r.p, d_z.p}}, h);
-    double rho = h[0];
+    double rho = h[1];
     if (!(std::isfinite(rho) && rho > 0.0)) return res;
     if (max_it == 0) return res;
     PcgCtl ctl{};
@@ -3353,38 +3430,13 @@ struct Solver {
     ctl.status = kRunning;
     ctl.terms = 0;
     ctl.max_it = (int)std::min<uint64_t>(max_it, (uint64_t)INT32_MAX);
+    ctl.lambda = lambda;
     PcgCtl* dctl = reinterpret_cast<PcgCtl*>(d_ctl.p);
     CUDA_OK(copy_async(dctl, &ctl, sizeof(ctl), cudaMemcpyHostToDevice, st));
-    cudaGraph_t graph;
-    cudaGraphExec_t exec;
-    const uint64_t launches_before = tl_telemetry.launches;
-    CUDA_OK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    // one poll batch (kPoll iterations, an even count) per graph: even iterations read rho slot 0,
-    // odd ones slot 1 (every kernel after the graph's first is a programmatic dependent of the one
-    // before it)
-    static_assert(kPoll % 2 == 0, "the rho slots alternate");
-    for (int it = 0; it < kPoll; ++it) {
-      const int slot = it & 1;
-      matvec(d_dir.p, d_q.p, lambda, dctl, fp32, d_dq.p, it > 0, true);
-      const int nupd = grid_for(nb, kUpdThreads);
-      launch_pdl(true, k_pcg_update_precond, nupd, kUpdThreads, st, tables(), d_factor.p, d_dq.p, product_ctas(),
-                 d_dir.p, d_q.p, x, d_r.p, d_z.p, d_rr_part.p, d_rz_part.p, slot, dctl);
-      launch_pdl(true, k_pcg_direction, grid_for(D, 256), 256, st, D, d_rr_part.p, d_rz_part.p, nupd, d_z.p, d_dir.p,
-                 slot, dctl);
-    }
-    CUDA_OK(cudaStreamEndCapture(st, &graph));
-    const uint64_t kernels_per_graph = tl_telemetry.launches - launches_before;  // counted at capture
-    tl_telemetry.launches = launches_before;
-    CUDA_OK(cudaGraphInstantiate(&exec, graph, 0));
+    const PcgGraph& pg = pcg_graph(x, fp32);
+    cudaGraphExec_t exec = pg.exec;
+    const uint64_t kernels_per_graph = pg.kernels;
     t_ready = now();
-    struct GraphGuard {
-      cudaGraph_t g;
-      cudaGraphExec_t e;
-      ~GraphGuard() {
-        cudaGraphExecDestroy(e);
-        cudaGraphDestroy(g);
-      }
-    } guard{graph, exec};
     auto recompute = [&]() {
       matvec(x, d_q.p, lambda, nullptr, fp32);
       OMVGBA_LAUNCH(k_sub, grid_for(D, 256), 256, 0, st, D, b, d_q.p, d_r.p);
@@ -3691,7 +3743,7 @@ struct Solver {
         double rel_res = 0.0;
         bool solved = true;
         if (direct) {
-          solved = D == 0 || direct_step(lambda);
+          if (D > 0) direct_step(lambda);  // its status comes with the candidate's results
         } else {
           solved = factor_preconditioner(lambda);
           if (solved) {
@@ -3718,18 +3770,8 @@ struct Solver {
         }
         // step cap (calibrated only)
         if (!n.self_cal && D > 0) {
-          OMVGBA_LAUNCH(k_step_block_norm, grid_for(n.ncam, 128), 128, 0, st, n.ncam, d_pose_off.p, d_pose_dim.p, d_step.p,
-                                                                   d_cam_norm.p);
+          OMVGBA_LAUNCH(k_step_cap, 1, 1024, 0, st, n.ncam, d_pose_off.p, d_pose_dim.p, D, d_step.p);
           check_launch();
-          std::vector<double> norms(n.ncam);
-          CUDA_OK(copy_async(norms.data(), d_cam_norm.p, sizeof(double) * n.ncam, cudaMemcpyDeviceToHost, st));
-          sync();
-          double largest = 0.0;
-          for (double x : norms) largest = std::max(largest, x);
-          if (largest > 0.5) {
-            OMVGBA_LAUNCH(k_scale, grid_for(D, 256), 256, 0, st, D, 0.5 / largest, d_step.p);
-            check_launch();
-          }
         }
         DevView v = view();
         OMVGBA_LAUNCH(k_retract, grid_for(std::max(n.ncam, ng), 128), 128, 0, st, v, ng, d_step.p, g, d_pose[cur].p,
@@ -3745,7 +3787,44 @@ struct Solver {
                           state(cand), g, stages[si].loss, mt, d_cand.p);
         }
         check_launch();
-        RedVec<4> cr = reduce<4>(d_cand.p, P, d_cand_part);
+        // the candidate's sums and the model reduction (camera_step.rs:44-81, optimizer.rs:590-618,
+        // retained/mod.rs:742-800): everything queued, then one wait
+        OMVGBA_LAUNCH(k_reduce_vec<4>, red_blocks, kReduceThreads, 0, st, d_cand.p, P, d_cand_part.p);
+        OMVGBA_LAUNCH(k_reduce_vec<4>, 1, kReduceThreads, 0, st, d_cand_part.p, red_blocks, d_cand_part.p);
+        check_launch();
+        if (D > 0) {
+          if (!iterative_step)
+            rows_matvec(d_step.p, d_q.p, lambda);
+          else
+            matvec(d_step.p, d_q.p, lambda);
+          queue_dots({{d_gred.p, d_step.p}, {d_step.p, d_q.p}});
+        }
+        double h[4] = {0, 0, 0, 0};
+        double cd[1] = {0.0};
+        RedVec<4> cr;
+        {
+          Readback rb(st, Readback::room(sizeof(cr)) + Readback::room(sizeof(double) * 2) + Readback::room(sizeof(int)) +
+                              2 * Readback::room(sizeof(double) * D));
+          const RedVec<4>* crp = rb.add(d_cand_part.p, 1);
+          const double* dp = rb.add(d_scalars.p, 2);
+          const int* okp = rb.add(d_status.p, 1);
+          const double *hs = rb.add(d_step.p, D), *hd = rb.add(d_diag.p, D);
+          rb.wait();
+          cr = *crp;
+          if (direct && D > 0) solved = *okp != 0;
+          if (D > 0) {
+            h[0] = dp[0];
+            h[1] = dp[1];
+            // camera damping norm: sum diag * step^2
+            for (int i = 0; i < D; ++i) cd[0] += hd[i] * hs[i] * hs[i];
+            for (int i = 0; i < D; ++i) h[2] += hs[i] * hs[i];
+          }
+        }
+        if (!solved) {
+          rej[1]++;
+          increase();
+          continue;
+        }
         if (cr.v[3] > 0.0) {
           rej[2]++;
           increase();
@@ -3754,36 +3833,12 @@ struct Solver {
         }
         double point_rms =
             std::sqrt(cr.v[1] / double(n.self_cal ? std::max(P, 1) : std::max<size_t>(free_points, 1)));
-        // model reduction (camera_step.rs:44-81, optimizer.rs:590-618, retained/mod.rs:742-800)
         double damped;
-        if (!iterative_step) {
-          if (D > 0)
-            rows_matvec(d_step.p, d_q.p, lambda);
-          else
-            CUDA_OK(cudaMemsetAsync(d_q.p, 0, sizeof(double), st));
-        } else {
-          matvec(d_step.p, d_q.p, lambda);
-        }
-        double h[4] = {0, 0, 0, 0};
-        if (D > 0) dots({{d_gred.p, d_step.p}, {d_step.p, d_q.p}}, h);
         if (!iterative_step) {
           damped = a.point_red - h[0] - 0.5 * h[1];
         } else {
           damped = a.point_red + (-h[0] - 0.5 * h[1]);
           if (!(std::isfinite(damped) && damped > 0.0)) damped = NAN;
-        }
-        // camera damping norm: sum diag * step^2
-        CUDA_OK(copy_async(d_tmp.p, d_step.p, sizeof(double) * std::max(D, 1), cudaMemcpyDeviceToDevice, st));
-        double cd[1] = {0.0};
-        if (D > 0) {
-          std::vector<double> hs(D), hd(D);
-          CUDA_OK(copy_async(hs.data(), d_step.p, sizeof(double) * D, cudaMemcpyDeviceToHost, st));
-          CUDA_OK(copy_async(hd.data(), d_diag.p, sizeof(double) * D, cudaMemcpyDeviceToHost, st));
-          sync();
-          for (int i = 0; i < D; ++i) cd[0] += hd[i] * hs[i] * hs[i];
-          double ss = 0.0;
-          for (int i = 0; i < D; ++i) ss += hs[i] * hs[i];
-          h[2] = ss;
         }
         double predicted = damped + 0.5 * lambda * (cd[0] + cr.v[2]);
         t_candidate += now() - t2;

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(mv_tile_obs<R>(), sizeof(T) == sizeof(R) ? 4 :
 // block; lane l sums segments l, l + 32, ... of the block's contiguous region in order, then a
 // fixed shuffle tree. A block no observation touches has an empty region: y_b = lambda diag_b x_b.
 // With xy non-null, xy[CTA] = sum over the CTA's blocks, in block order, of x_b . y_b (the PCG
-// curvature terms).
+// curvature terms). With ctl the damping is the control block's.
 __global__ void __launch_bounds__(256) k_mv_tiles_finalize(MvTiles mt, const double* __restrict__ partial,
                                                            const double* __restrict__ diag, double lambda,
                                                            const double* __restrict__ x, double* __restrict__ y,
@@ -279,6 +279,7 @@ __global__ void __launch_bounds__(256) k_mv_tiles_finalize(MvTiles mt, const dou
   pdl_trigger();
   pdl_wait();
   if (pcg_stopped(ctl)) return;
+  if (ctl) lambda = ctl->lambda;
   double dot = 0.0;
   if (have) {
     double xv[6];
