@@ -130,19 +130,50 @@ struct PinnedStage {
     return p;
   }
 };
-thread_local PinnedStage tl_pinned;
-thread_local PinnedStage tl_poll;  // the PCG loop's status mirrors (read while the next batch runs)
-thread_local PinnedStage tl_read;  // the results of a group of kernels (Readback)
+constexpr size_t kStagedCopyMax = 1u << 20;
+constexpr size_t kStagedRoom = 4u << 20;
 
-// Several device results read with one wait: room for `bytes` in the calling thread's pinned buffer (in
+// Pinned host memory of one solver at a time: the staged copies' room, the PCG loop's status mirrors
+// (read while the next batch runs) and the results of a group of kernels (Readback). It belongs to a
+// context, so that it is pinned once and not for every solve or worker thread.
+// Staged host->device copies take successive places in the room; the stream is waited for only when the
+// room is used up (or belongs to another stream), so a set-up's many small tables queue up behind each
+// other. A device->host copy waits anyway and starts the room over.
+struct HostStage {
+  PinnedStage room, poll, read;
+  size_t at = 0;
+  cudaStream_t st = nullptr;
+  cudaError_t settle() {
+    const cudaError_t e = at > 0 ? cudaStreamSynchronize(st) : cudaSuccess;
+    at = 0;
+    return e;
+  }
+  // A place for `bytes` (at most kStagedCopyMax), nullptr when no pinned memory is to be had.
+  void* place(size_t bytes, cudaStream_t stream) {
+    if (at + bytes > kStagedRoom || stream != st)
+      if (settle() != cudaSuccess) return nullptr;
+    unsigned char* base = static_cast<unsigned char*>(room.get(kStagedRoom));
+    if (!base) return nullptr;
+    st = stream;
+    void* p = base + at;
+    at += (bytes + 255) & ~size_t(255);
+    return p;
+  }
+};
+thread_local HostStage tl_own_stage;           // callers without a context
+thread_local HostStage* tl_stage = nullptr;    // the stage of the context in use (ContextScope)
+thread_local cudaMemPool_t tl_pool = nullptr;  // its device memory pool
+inline HostStage& host_stage() { return tl_stage ? *tl_stage : tl_own_stage; }
+
+// Several device results read with one wait: room for `bytes` in the context's pinned buffer (in
 // pageable memory when there is none), copies queued on the stream, then wait() before the host reads.
-// One Readback per thread is in use at a time.
+// One Readback is in use at a time.
 struct Readback {
   cudaStream_t st;
   unsigned char* base;
   size_t used = 0;
   std::vector<unsigned char> pageable;
-  Readback(cudaStream_t stream, size_t bytes) : st(stream), base(static_cast<unsigned char*>(tl_read.get(bytes))) {
+  Readback(cudaStream_t stream, size_t bytes) : st(stream), base(static_cast<unsigned char*>(host_stage().read.get(bytes))) {
     if (!base) {
       pageable.resize(bytes);
       base = pageable.data();
@@ -159,13 +190,12 @@ struct Readback {
   }
   void wait() { CUDA_OK(cudaStreamSynchronize(st)); }
 };
-constexpr size_t kStagedCopyMax = 1u << 20;
-
 // Large host->device copies from pageable memory: the source is copied by several host threads into
 // one of two pinned chunks while the other chunk's DMA runs (an event per chunk guards its reuse).
 // Returns when every chunk has reached the device, as a pageable copy would.
 constexpr size_t kPipelinedCopyMin = 32u << 20;
 constexpr size_t kPipelineChunk = 16u << 20;
+constexpr size_t kBulkCopyMin = 4u << 20;  // of the copies whose caller waits for each (copy_to_device)
 struct PinnedRing {
   void* p[2] = {nullptr, nullptr};
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -232,22 +262,61 @@ inline cudaError_t upload_pipelined(void* dst, const void* src, size_t bytes, cu
   return e != cudaSuccess ? e : w;
 }
 
+// The same in the other direction: each chunk's DMA runs while the host threads copy the one before it out.
+inline cudaError_t download_pipelined(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  if (!tl_ring.ensure()) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(st);
+  }
+  const size_t chunks = (bytes + kPipelineChunk - 1) / kPipelineChunk;
+  cudaError_t e = cudaSuccess;
+  for (size_t i = 0; i <= chunks && e == cudaSuccess; ++i) {
+    if (i < chunks) {
+      const size_t off = i * kPipelineChunk;
+      e = cudaMemcpyAsync(tl_ring.p[i & 1], static_cast<const char*>(src) + off, std::min(kPipelineChunk, bytes - off),
+                          cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess) e = cudaEventRecord(tl_ring.ev[i & 1], st);
+    }
+    if (i > 0 && e == cudaSuccess) {
+      const size_t off = (i - 1) * kPipelineChunk;
+      e = cudaEventSynchronize(tl_ring.ev[(i - 1) & 1]);
+      if (e == cudaSuccess)
+        parallel_memcpy(static_cast<char*>(dst) + off, tl_ring.p[(i - 1) & 1], std::min(kPipelineChunk, bytes - off));
+    }
+  }
+  const cudaError_t w = cudaStreamSynchronize(st);
+  return e != cudaSuccess ? e : w;
+}
+int copy_to_device(void* dst, const void* src, size_t bytes, void* stream) {
+  if (bytes == 0) return cudaSuccess;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return bytes >= kBulkCopyMin ? upload_pipelined(dst, src, bytes, st)
+                               : cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+}
+int copy_from_device(void* dst, const void* src, size_t bytes, void* stream) {
+  if (bytes == 0) return cudaSuccess;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (bytes >= kBulkCopyMin) return download_pipelined(dst, src, bytes, st);
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(st);
+}
+
 // Host<->device copy on `st`, counted in the telemetry. Copies of at most kStagedCopyMax bytes go
-// through the thread's pinned stage and have completed when the call returns (callers read the
-// host side right after their next synchronize, so nothing relies on them staying asynchronous).
+// through the context's pinned stage: the source of an upload may change as soon as the call returns,
+// and a download has arrived.
 inline cudaError_t copy_async(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, cudaStream_t st) {
   if (kind == cudaMemcpyHostToDevice) tl_telemetry.h2d += bytes;
   if (kind == cudaMemcpyDeviceToHost) tl_telemetry.d2h += bytes;
   if ((kind == cudaMemcpyHostToDevice || kind == cudaMemcpyDeviceToHost) && bytes > 0 && bytes <= kStagedCopyMax) {
-    if (void* stage = tl_pinned.get(bytes)) {
+    HostStage& hs = host_stage();
+    if (void* stage = hs.place(bytes, st)) {
       if (kind == cudaMemcpyHostToDevice) {
         std::memcpy(stage, src, bytes);
-        cudaError_t e = cudaMemcpyAsync(dst, stage, bytes, kind, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the stage is reused by the next copy
-        return e;
+        return cudaMemcpyAsync(dst, stage, bytes, kind, st);
       }
       cudaError_t e = cudaMemcpyAsync(stage, src, bytes, kind, st);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+      const cudaError_t w = hs.settle();
+      if (e == cudaSuccess) e = w;
       if (e == cudaSuccess) std::memcpy(dst, stage, bytes);
       return e;
     }
@@ -262,8 +331,27 @@ inline cudaError_t copy_async(void* dst, const void* src, size_t bytes, cudaMemc
 struct Context {
   int device = 0;
   cudaStream_t stream = nullptr;
-  double* pinned = nullptr;  // scalar readback
-  size_t pinned_count = 0;
+  HostStage stage;
+  // Device memory of the solves: kept between solves up to kPoolKept bytes (the device's default pool
+  // returns everything at each wait, and every solve then maps its memory anew), given back with the
+  // context.
+  cudaMemPool_t pool = nullptr;
+};
+constexpr uint64_t kPoolKept = uint64_t(256) << 20;
+
+// The calling thread works for context `c`: its pinned stage and memory pool.
+struct ContextScope {
+  HostStage* stage = tl_stage;
+  cudaMemPool_t pool = tl_pool;
+  explicit ContextScope(Context* c) {
+    tl_stage = &c->stage;
+    tl_pool = c->pool;
+  }
+  ~ContextScope() {
+    (void)tl_stage->settle();
+    tl_stage = stage;
+    tl_pool = pool;
+  }
 };
 
 int device_count() {
@@ -280,24 +368,34 @@ Context* context_create(int device, std::string* error) {
   c->device = device;
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMallocHost(&c->pinned, sizeof(double) * 64);
+  if (e == cudaSuccess) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    e = cudaMemPoolCreate(&c->pool, &props);
+    uint64_t kept = kPoolKept;
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &kept);
+  }
   if (e != cudaSuccess) {
     if (error) *error = cudaGetErrorString(e);
+    if (c->pool) cudaMemPoolDestroy(c->pool);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return nullptr;
   }
-  c->pinned_count = 64;
   return c;
 }
 
 int context_device(const Context* c) { return c->device; }
 void* context_stream(const Context* c) { return (void*)c->stream; }
+void* context_pool(const Context* c) { return (void*)c->pool; }
 
 void context_destroy(Context* c) {
   if (!c) return;
   cudaSetDevice(c->device);
-  if (c->pinned) cudaFreeHost(c->pinned);
+  if (c->stream) cudaStreamSynchronize(c->stream);
+  if (c->pool) cudaMemPoolDestroy(c->pool);  // memory still in use (a plan's) goes back when it is freed
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -320,7 +418,8 @@ struct DBuf {
     s = stream;
     n = count;
     if (count) {
-      CUDA_OK(cudaMallocAsync((void**)&p, sizeof(T) * count, stream));
+      CUDA_OK(tl_pool ? cudaMallocFromPoolAsync((void**)&p, sizeof(T) * count, tl_pool, stream)
+                      : cudaMallocAsync((void**)&p, sizeof(T) * count, stream));
       tl_device_bytes += sizeof(T) * count;
     }
   }
@@ -2239,6 +2338,7 @@ bool device_certify_positive_definite(Context* ctx, int n, const std::vector<int
                                       const std::vector<double>& values) {
   if (n <= 0) return true;
   CUDA_OK(cudaSetDevice(ctx->device));
+  ContextScope scope(ctx);
   cudaStream_t st = ctx->stream;
   int bwt = 0;
   for (size_t q = 0; q < rows.size(); ++q) bwt = std::max(bwt, rows[q] / kCT - cols[q] / kCT);
@@ -3442,7 +3542,7 @@ struct Solver {
       OMVGBA_LAUNCH(k_sub, grid_for(D, 256), 256, 0, st, D, b, d_q.p, d_r.p);
       check_launch();
     };
-    PcgCtl* mirror = static_cast<PcgCtl*>(tl_poll.get(2 * sizeof(PcgCtl)));
+    PcgCtl* mirror = static_cast<PcgCtl*>(host_stage().poll.get(2 * sizeof(PcgCtl)));
     if (!mirror) throw SolveFailure{8, "pinned host memory for the PCG status is not available"};
     struct Events {
       cudaEvent_t e[2] = {nullptr, nullptr};
@@ -4064,6 +4164,7 @@ void tv_basis(const double t[3], double baseline, double dir[3], double b0[3], d
 
 TwoViewReport gpu_two_view(Context* ctx, TwoViewProblem& pr, const LmOptions& opt) {
   CUDA_OK(cudaSetDevice(ctx->device));
+  ContextScope scope(ctx);
   cudaStream_t st = opt.stream ? static_cast<cudaStream_t>(opt.stream) : ctx->stream;
   const int P = (int)(pr.points.size() / 3);
   if (P < 5) throw SolveFailure{OMVGBA_NUMERICAL, "two-view bundle adjustment needs at least 5 points"};
@@ -4321,6 +4422,7 @@ NativeReport gpu_refine(Context* ctx, const NativeProblem& problem, const LmOpti
                         std::vector<double>& rotation, std::vector<double>& translation, std::vector<double>& points,
                         std::vector<double>& groups) {
   CUDA_OK(cudaSetDevice(ctx->device));
+  ContextScope scope(ctx);
   if (problem.obs_cam.size() >= (1ull << 31)) throw SolveFailure{3, "observation count exceeds 2^31"};
   Solver<double> s(ctx, problem, options);
   return s.refine(rotation, translation, points, groups);
@@ -4336,6 +4438,7 @@ struct Resident {
 
 Resident* resident_create(Context* ctx, const NativeProblem& problem, const LmOptions& options) {
   CUDA_OK(cudaSetDevice(ctx->device));
+  ContextScope scope(ctx);
   if (problem.obs_cam.size() >= (1ull << 31)) throw SolveFailure{3, "observation count exceeds 2^31"};
   Resident* r = new Resident();
   r->ctx = ctx;
@@ -4361,6 +4464,7 @@ void resident_destroy(Resident* r) {
 NativeReport resident_refine(Resident* r, std::vector<double>& rotation, std::vector<double>& translation,
                              std::vector<double>& points, std::vector<double>& groups) {
   CUDA_OK(cudaSetDevice(r->ctx->device));
+  ContextScope scope(r->ctx);
   r->linearized = false;
   r->solver->restore_initial();
   return r->solver->refine(rotation, translation, points, groups);
@@ -4395,6 +4499,7 @@ ResidentInfo resident_info(const Resident* r) {
 
 void resident_schur_product(Resident* r, double lambda, bool fp32, int stage, const double* x, double* y) {
   CUDA_OK(cudaSetDevice(r->ctx->device));
+  ContextScope scope(r->ctx);
   Solver<double>& s = *r->solver;
   if (s.direct) throw SolveFailure{2, "the plan's linear solver is direct; the tile product serves PCG plans"};
   if (fp32 && !s.mixed) throw SolveFailure{1, "FP32 products need a mixed-precision plan"};
@@ -4421,6 +4526,7 @@ void resident_schur_product(Resident* r, double lambda, bool fp32, int stage, co
 void gpu_debug_linearize(Context* ctx, const NativeProblem& problem, const LmOptions& options, double* residual,
                          double* sqrt_weight, double* point_jacobian, double* camera_jacobian) {
   CUDA_OK(cudaSetDevice(ctx->device));
+  ContextScope scope(ctx);
   Solver<double> s(ctx, problem, options);
   double scene = s.scene_scale_host();
   Gauge g = s.gauge_for(s.cur, scene);
@@ -4455,6 +4561,7 @@ void gpu_debug_linearize(Context* ctx, const NativeProblem& problem, const LmOpt
 void gpu_debug_schur_product(Context* ctx, const NativeProblem& problem, const LmOptions& options, double lambda,
                              const double* x, double* y_mv, double* y_dense, int* dimension) {
   CUDA_OK(cudaSetDevice(ctx->device));
+  ContextScope scope(ctx);
   LmOptions o = options;
   o.iterative = false;
   o.linear_solver = 1;

@@ -157,6 +157,13 @@ int device_count();
 Context* context_create(int device, std::string* error);
 int context_device(const Context* ctx);
 void* context_stream(const Context* ctx);  // the context's cudaStream_t
+void* context_pool(const Context* ctx);    // the context's cudaMemPool_t
+
+// Copies between pageable host memory and the device on a stream (a cudaStream_t), cudaSuccess or the
+// error. Large ones go through two pinned chunks, several host threads filling (emptying) one while the
+// other's DMA runs; downloads have arrived on return, uploads' sources may change.
+int copy_to_device(void* dst, const void* src, size_t bytes, void* stream);
+int copy_from_device(void* dst, const void* src, size_t bytes, void* stream);
 
 // refresh_landmark_reprojection_errors_for (openmvg-sfm ops/reconstruction/bundle.rs:510-637) on the
 // context's device, inputs and outputs in host memory (see omvgba_sfm_refresh_reprojection). The

@@ -81,13 +81,15 @@ LossDev problem_loss(const omvgba_problem& pr) {
 }
 
 // Runs body(chunk, begin, end) over `count` items cut into a fixed number of contiguous chunks, on
-// up to host_thread_limit() threads. Callers combine per-chunk results in chunk order, so every
-// result is independent of the thread count.
+// up to host_thread_limit() threads, each worth `grain` items or more (65,536 of the plain loops; fewer
+// where an item is a projection). Callers combine per-chunk results in chunk order, so every result is
+// independent of the thread count.
+constexpr size_t kProjectionGrain = 2048;
 template <typename Body>
-void for_fixed_chunks(size_t count, size_t chunks, Body body) {
+void for_fixed_chunks(size_t count, size_t chunks, Body body, size_t grain = 65536) {
   const size_t per = (count + chunks - 1) / std::max<size_t>(chunks, 1);
   const unsigned hw = host_thread_limit();
-  const size_t nthreads = std::min<size_t>(std::min<size_t>(hw, chunks), count / 65536 + 1);
+  const size_t nthreads = std::min<size_t>(std::min<size_t>(hw, chunks), count / grain + 1);
   std::atomic<size_t> next{0};
   auto worker = [&]() {
     for (size_t c; (c = next.fetch_add(1)) < chunks;) {
@@ -487,7 +489,7 @@ Lowered lower_calibrated(const omvgba_problem& pr, bool angular = false) {
           while (i < cur && !bad.compare_exchange_weak(cur, i)) {
           }
         }
-    });
+    }, kProjectionGrain);
     if (bad.load() != SIZE_MAX)
       fail(OMVGBA_NUMERICAL, "observation " + std::to_string(order[bad.load()]) +
                                  ": the measured pixel does not define a bearing of its camera model");
@@ -1042,7 +1044,7 @@ void finish_solution(const omvgba_problem& pr, Result& res, InputMetrics* cache 
     seen[c] = n_seen;
     inliers[c] = n_in;
     inlier_ss[c] = ss;
-  });
+  }, kProjectionGrain);
   if (reuse_input) {
     at_input = cache->parts;
   } else if (held_out && cache) {
@@ -1504,6 +1506,10 @@ Result solve_once(Context* ctx, const omvgba_problem& pr, const omvgba_config& c
 // bucket is selected from. Anything else takes std::nth_element over the whole vector.
 double kth_smallest(std::vector<double>& v, size_t k) {
   const size_t n = v.size();
+  if (n < (1u << 20)) {  // the histograms (16 MB) would cost more than the selection
+    std::nth_element(v.begin(), v.begin() + k, v.end());
+    return v[k];
+  }
   constexpr size_t kChunks = 64, kBins = 1 << 16;
   std::vector<uint32_t> hist(kChunks * kBins, 0);
   std::atomic<bool> plain{true};
@@ -1519,7 +1525,7 @@ double kth_smallest(std::vector<double>& v, size_t k) {
       h[bits >> 48]++;
     }
   });
-  if (!plain || n < (1u << 20)) {
+  if (!plain) {
     std::nth_element(v.begin(), v.begin() + k, v.end());
     return v[k];
   }
@@ -1925,6 +1931,7 @@ int write_error(omvgba_error* e, int code, const std::string& msg) {
 
 struct omvgba_context {
   omvgba::Context* ctx;
+  std::vector<omvgba::Context*> workers;  // of the batched solves, kept from one batch to the next
 };
 
 using namespace omvgba;
@@ -2024,11 +2031,12 @@ omvgba_context* omvgba_context_create(int32_t device, omvgba_error* error) {
     error->code = 0;
     error->message[0] = 0;
   }
-  return new omvgba_context{c};
+  return new omvgba_context{c, {}};
 }
 
 void omvgba_context_destroy(omvgba_context* context) {
   if (!context) return;
+  for (Context* w : context->workers) context_destroy(w);
   context_destroy(context->ctx);
   delete context;
 }
@@ -2153,9 +2161,14 @@ int32_t omvgba_solve_batched(omvgba_context* context, uint64_t window_count, con
   std::mutex setup_mutex;
   omvgba_config cfg = *config;
   cfg.stream = nullptr;  // every worker runs on its own context's stream
-  auto worker = [&]() {
+  // worker w's context (stream, pinned memory, device memory pool) stays for the next batch
+  if (context->workers.size() < workers) context->workers.resize(workers, nullptr);
+  const unsigned threads_each = std::max<unsigned>(1, host_thread_limit() / (unsigned)std::max<uint64_t>(workers, 1));
+  auto worker = [&](uint64_t w) {
     std::string msg;
-    Context* ctx = context_create(device, &msg);
+    set_host_thread_limit(threads_each);
+    Context*& ctx = context->workers[w];
+    if (!ctx) ctx = context_create(device, &msg);
     if (!ctx) {
       std::lock_guard<std::mutex> lock(setup_mutex);
       setup_error = "worker context creation failed: " + msg;
@@ -2177,10 +2190,9 @@ int32_t omvgba_solve_batched(omvgba_context* context, uint64_t window_count, con
         messages[i] = ex.what();
       }
     }
-    context_destroy(ctx);
   };
   std::vector<std::thread> pool;
-  for (uint64_t w = 0; w < workers; ++w) pool.emplace_back(worker);
+  for (uint64_t w = 0; w < workers; ++w) pool.emplace_back(worker, w);
   for (auto& t : pool) t.join();
   if (!setup_error.empty() && next.load() < window_count) return write_error(error, OMVGBA_CUDA_ERROR, setup_error);
   for (uint64_t i = 0; i < window_count; ++i)
@@ -2475,13 +2487,27 @@ extern "C" int32_t omvgba_sfm_refresh_reprojection(omvgba_context* context, uint
     if (N && (!tracks->track_pose || !tracks->track_intrinsic || !tracks->track_pixel || !tracks->track_support ||
               !result->track_support))
       return write_error(error, OMVGBA_INVALID_ARGUMENT, "null track array");
+    // each chunk stops at its first bad index; the first chunk with one decides the message
+    constexpr size_t kChunks = 64;
+    std::vector<std::vector<uint8_t>> chunk_used(kChunks, std::vector<uint8_t>(intrinsic_count, 0));
+    std::vector<const char*> bad(kChunks, nullptr);
+    for_fixed_chunks(N, kChunks, [&](size_t c, size_t b, size_t e) {
+      std::vector<uint8_t>& used = chunk_used[c];
+      for (uint64_t o = b; o < e; ++o) {
+        const uint32_t p = tracks->track_pose[o], i = tracks->track_intrinsic[o];
+        const bool no_pose = p != OMVGBA_NO_POSE && p >= pose_count;
+        if (no_pose || i >= intrinsic_count) {
+          bad[c] = no_pose ? "track pose index out of range" : "track intrinsic index out of range";
+          return;
+        }
+        if (p != OMVGBA_NO_POSE && tracks->track_support[o]) used[i] = 1;
+      }
+    });
+    for (const char* m : bad)
+      if (m) fail(OMVGBA_INVALID_PROBLEM, m);
     std::vector<uint8_t> used(intrinsic_count, 0);
-    for (uint64_t o = 0; o < N; ++o) {
-      const uint32_t p = tracks->track_pose[o], i = tracks->track_intrinsic[o];
-      if (p != OMVGBA_NO_POSE && p >= pose_count) fail(OMVGBA_INVALID_PROBLEM, "track pose index out of range");
-      if (i >= intrinsic_count) fail(OMVGBA_INVALID_PROBLEM, "track intrinsic index out of range");
-      if (p != OMVGBA_NO_POSE && tracks->track_support[o]) used[i] = 1;
-    }
+    for (const auto& u : chunk_used)
+      for (size_t i = 0; i < u.size(); ++i) used[i] |= u[i];
     // CameraResidualPolicy::from_pixel_limit (residual.rs:37-55) fails for a wide-angle camera
     // without a positive finite pixel-to-angle scale
     for (uint64_t i = 0; i < intrinsic_count; ++i) {

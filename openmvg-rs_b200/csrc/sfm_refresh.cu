@@ -82,7 +82,8 @@ void check(cudaError_t e, const char* what) {
 struct StreamBuf {
   void* p = nullptr;
   cudaStream_t s;
-  explicit StreamBuf(cudaStream_t stream) : s(stream) {}
+  cudaMemPool_t pool;
+  StreamBuf(cudaStream_t stream, cudaMemPool_t from) : s(stream), pool(from) {}
   StreamBuf(const StreamBuf&) = delete;
   StreamBuf& operator=(const StreamBuf&) = delete;
   ~StreamBuf() {
@@ -90,13 +91,13 @@ struct StreamBuf {
   }
   template <typename T>
   T* alloc(size_t count) {
-    check(cudaMallocAsync(&p, count ? sizeof(T) * count : 16, s), "cudaMallocAsync");
+    check(cudaMallocFromPoolAsync(&p, count ? sizeof(T) * count : 16, pool, s), "cudaMallocFromPoolAsync");
     return static_cast<T*>(p);
   }
   template <typename T>
   T* upload(const T* host, size_t count) {
     T* d = alloc<T>(count);
-    if (count) check(cudaMemcpyAsync(d, host, sizeof(T) * count, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
+    check((cudaError_t)copy_to_device(d, host, sizeof(T) * count, s), "upload");
     return d;
   }
 };
@@ -110,8 +111,10 @@ void gpu_sfm_refresh(Context* ctx, const SfmRefreshInput& in, SfmRefreshOutput& 
   std::vector<CameraDev> cams(in.intrinsic_count);
   const omvgba_intrinsic* intr = static_cast<const omvgba_intrinsic*>(in.intrinsics);
   for (uint64_t i = 0; i < in.intrinsic_count; ++i) cams[i] = make_camera_dev(intr[i]);
-  StreamBuf b_rot(st), b_cen(st), b_cam(st), b_pts(st), b_act(st), b_off(st), b_tp(st), b_ti(st), b_px(st),
-      b_sin(st), b_sout(st), b_upd(st), b_err(st), b_rem(st);
+  cudaMemPool_t pool = static_cast<cudaMemPool_t>(context_pool(ctx));
+  StreamBuf b_rot(st, pool), b_cen(st, pool), b_cam(st, pool), b_pts(st, pool), b_act(st, pool), b_off(st, pool),
+      b_tp(st, pool), b_ti(st, pool), b_px(st, pool), b_sin(st, pool), b_sout(st, pool), b_upd(st, pool),
+      b_err(st, pool), b_rem(st, pool);
   const double* rot = b_rot.upload(in.rotation, 9 * in.pose_count);
   const double* cen = b_cen.upload(in.center, 3 * in.pose_count);
   const CameraDev* dcam = b_cam.upload(cams.data(), cams.size());
@@ -132,14 +135,10 @@ void gpu_sfm_refresh(Context* ctx, const SfmRefreshInput& in, SfmRefreshOutput& 
     check(cudaGetLastError(), "k_sfm_refresh launch");
   }
   std::vector<uint32_t> removed(L);
-  if (N) check(cudaMemcpyAsync(out.track_support, sout, N, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
-  if (L) {
-    check(cudaMemcpyAsync(out.landmark_update, upd, L, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
-    check(cudaMemcpyAsync(out.reprojection_error, err, sizeof(double) * L, cudaMemcpyDeviceToHost, st),
-          "cudaMemcpyAsync");
-    check(cudaMemcpyAsync(removed.data(), rem, sizeof(uint32_t) * L, cudaMemcpyDeviceToHost, st),
-          "cudaMemcpyAsync");
-  }
+  check((cudaError_t)copy_from_device(out.track_support, sout, N, st), "download");
+  check((cudaError_t)copy_from_device(out.landmark_update, upd, L, st), "download");
+  check((cudaError_t)copy_from_device(out.reprojection_error, err, sizeof(double) * L, st), "download");
+  check((cudaError_t)copy_from_device(removed.data(), rem, sizeof(uint32_t) * L, st), "download");
   check(cudaStreamSynchronize(st), "k_sfm_refresh");
   out.rejected_landmarks = 0;
   out.removed_observations = 0;
