@@ -17,13 +17,24 @@
 //
 // Determinism: observations arrive in any order, so gradients are reduced by key with integer
 // atomics on per-output fixed-point values. A first pass records each output component's largest
-// contribution magnitude (atomicMax on the float's bits, order independent); each component then
-// gets a power-of-two scale that leaves ceil(log2 n) + 1 bits of headroom in a signed 64-bit
-// accumulator; a second pass adds the scaled, rounded contributions (integer addition is
-// associative, so the sum is the same in every run); a last pass converts and accumulates into the
-// caller's gradient arrays. Resolution: 2^-(61 - ceil(log2 n)) of the component's largest term.
+// contribution magnitude (atomicMax on the float's bits, order independent); each component's
+// power-of-two scale leaves ceil(log2 n) + 1 bits of headroom in a signed 64-bit accumulator; a second
+// pass adds the scaled, rounded contributions (integer addition is associative, so the sum is the same
+// in every run); a last pass converts and accumulates into the caller's gradient arrays. Resolution:
+// 2^-(61 - ceil(log2 n)) of the component's largest term. The rotation's left Jacobian is the same for
+// all of a camera's observations, so the passes reduce R X_p x a and the last one applies Jl^T.
+//
+// What bounds the passes is neither bytes nor flops but the number of separate lines their gathers and
+// atomics touch: a lane has its own camera and point. So a camera's constants are one 64-byte row read
+// in four 16-byte loads, the twelve contributions of an observation are handed over a warp's shared
+// memory so that one instruction's lanes cover neighbouring accumulators (about 3 observations' lines
+// instead of 32), and the first pass reads the current maximum and leaves out the atomic unless the
+// contribution is larger. Measured at 10M unordered observations of 3,000 cameras and 2M points, per
+// launch: first pass 931 -> 417 us, second 1,078 -> 521 us (a camera's 26 constants in as many scattered
+// loads, an atomic's 32 lanes on 32 lines and one atomic per contribution in both passes before).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -37,15 +48,13 @@ namespace residual {
 
 constexpr int kThreads = 256;
 
-// Per-camera constants computed once per call.
+// A camera's constants: one row of 16 values, 16-byte aligned. turn: the first radial turn (squared
+// radius), infinite when there is none.
 template <typename T>
-struct CamPre {
-  T R[9];
-  T Jl[9];  // left Jacobian of SO(3) at rotvec (VJP only)
-  T f, k1, k2, turn;
-  int has_turn;
-  int pad[3];
+struct __align__(16) CamRow {
+  T R[9], t[3], f, k1, k2, turn;
 };
+constexpr size_t kCamScratch = 104;  // bytes of workspace reserved per camera
 
 template <typename T>
 __device__ __forceinline__ void rodrigues(const T w[3], T R[9], T Jl[9]) {
@@ -76,39 +85,40 @@ __device__ __forceinline__ void rodrigues(const T w[3], T R[9], T Jl[9]) {
 }
 
 template <typename T>
-__device__ __forceinline__ CamPre<T> make_pre(const T* __restrict__ rotvec, const T* __restrict__ intr, uint64_t j) {
-  CamPre<T> c;
+__device__ __forceinline__ T radial_turn(T k1, T k2) {
+  double turn = 0.0;
+  return first_radial_turn_squared((double)k1, (double)k2, &turn) ? (T)turn : T(INFINITY);
+}
+
+// The row of camera j without its turn (infinite).
+template <typename T>
+__device__ __forceinline__ CamRow<T> make_row(const T* __restrict__ rotvec, const T* __restrict__ trans,
+                                              const T* __restrict__ intr, uint64_t j) {
+  CamRow<T> c;
   const T w[3] = {rotvec[3 * j], rotvec[3 * j + 1], rotvec[3 * j + 2]};
-  rodrigues(w, c.R, c.Jl);
+  T Jl[9];
+  rodrigues(w, c.R, Jl);
+  for (int k = 0; k < 3; ++k) c.t[k] = trans[3 * j + k];
   c.f = intr[3 * j];
   c.k1 = intr[3 * j + 1];
   c.k2 = intr[3 * j + 2];
-  double turn = 0.0;
-  c.has_turn = first_radial_turn_squared((double)c.k1, (double)c.k2, &turn) ? 1 : 0;
-  c.turn = (T)turn;
+  c.turn = T(INFINITY);
   return c;
-}
-
-template <typename T>
-__global__ void k_cam_prepare(uint64_t ncam, const T* __restrict__ rotvec, const T* __restrict__ intr,
-                              CamPre<T>* __restrict__ out) {
-  const uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (j >= ncam) return;
-  out[j] = make_pre(rotvec, intr, j);
 }
 
 // Residual, J = d residual / d X_c and the intrinsic columns (log f, k1, k2); false when the
 // observation is inadmissible.
 template <typename T>
-__device__ __forceinline__ bool radial_eval(const CamPre<T>& c, T X, T Y, T Z, T ox, T oy, T r[2], T J[2][3],
-                                            T Ji[2][3]) {
+__device__ __forceinline__ bool radial_eval(const CamRow<T>& c, T X, T Y, T Z, T ox, T oy, T r[2], T J[2][3],
+                                            T Ji[2][3], T* radius2 = nullptr) {
   const T s = fmax(fmax(fabs(X), fabs(Y)), fabs(Z));
   if (!(isfinite(X) && isfinite(Y) && isfinite(Z)) || !(Z > T(64.0 * kEps) * s)) return false;
   if (!(c.f > T(0) && isfinite(c.f) && isfinite(c.k1) && isfinite(c.k2))) return false;
   const T iz = T(1) / Z;
   const T n0 = X * iz, n1 = Y * iz;
   const T r2 = n0 * n0 + n1 * n1;
-  if (c.has_turn && r2 >= c.turn) return false;
+  if (r2 >= c.turn && c.turn < T(INFINITY)) return false;
+  if (radius2) *radius2 = r2;
   const T r4 = r2 * r2;
   const T dist = T(1) + c.k1 * r2 + c.k2 * r4;
   const T rd = c.k1 + T(2) * (c.k2 * r2);
@@ -137,17 +147,33 @@ __device__ __forceinline__ bool radial_eval(const CamPre<T>& c, T X, T Y, T Z, T
 }
 
 template <typename T>
-__device__ __forceinline__ void camera_point(const CamPre<T>& c, const T* t, const T* X, T xc[3], T rx[3]) {
+__device__ __forceinline__ void camera_point(const CamRow<T>& c, const T* X, T xc[3], T rx[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     rx[i] = c.R[3 * i] * X[0] + c.R[3 * i + 1] * X[1] + c.R[3 * i + 2] * X[2];
-    xc[i] = rx[i] + t[i];
+    xc[i] = rx[i] + c.t[i];
   }
+}
+
+// Points of a warp's lanes into `out` (96 values, lane l's at 3 l): three lanes share a point, so a load
+// instruction touches about 11 points' lines instead of 32. p must be in range (0 stands in).
+template <typename T>
+__device__ __forceinline__ void warp_points(const T* __restrict__ points, uint32_t p, T* out) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    const int at = 32 * s + lane, o = at / 3;
+    const uint32_t q = __shfl_sync(0xffffffffu, p, o);
+    out[at] = points[3 * (uint64_t)q + (at - 3 * o)];
+  }
+  __syncwarp();
 }
 
 // Forward pass: the camera constants are recomputed per observation, so the pass needs no scratch.
 // An observation whose camera or point index is out of range (a negative int32 index reads as a
-// large uint32) touches no camera or point and gets a NaN residual.
+// large uint32) touches no camera or point and gets a NaN residual. The radial turn is a handful of FP64
+// divisions and a root: it is formed only where 1 + 3 k1 s + 5 k2 s^2 could reach zero up to the
+// observation's own radius.
 template <typename T>
 __global__ void k_forward(uint64_t n, const uint32_t* __restrict__ cam, const uint32_t* __restrict__ pt,
                           const T* __restrict__ pixel, const T* __restrict__ rotvec, const T* __restrict__ intr,
@@ -156,147 +182,255 @@ __global__ void k_forward(uint64_t n, const uint32_t* __restrict__ cam, const ui
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t j = cam[i], p = pt[i];
-  if (j >= ncam || p >= npts) {
-    residual[2 * i] = T(NAN);
-    residual[2 * i + 1] = T(NAN);
-    return;
-  }
-  const CamPre<T> c = make_pre(rotvec, intr, j);
-  const T X[3] = {points[3 * (uint64_t)p], points[3 * (uint64_t)p + 1], points[3 * (uint64_t)p + 2]};
-  const T t[3] = {trans[3 * (uint64_t)j], trans[3 * (uint64_t)j + 1], trans[3 * (uint64_t)j + 2]};
-  T xc[3], rx[3], r[2], J[2][3], Ji[2][3];
-  camera_point(c, t, X, xc, rx);
-  const T nan = T(NAN);
-  if (!radial_eval(c, xc[0], xc[1], xc[2], pixel[2 * i], pixel[2 * i + 1], r, J, Ji)) {
-    residual[2 * i] = nan;
-    residual[2 * i + 1] = nan;
-    return;
+  T r[2] = {T(NAN), T(NAN)};
+  if (j < ncam && p < npts) {
+    const CamRow<T> c = make_row(rotvec, trans, intr, j);
+    const T X[3] = {points[3 * (uint64_t)p], points[3 * (uint64_t)p + 1], points[3 * (uint64_t)p + 2]};
+    T xc[3], rx[3], J[2][3], Ji[2][3], r2;
+    camera_point(c, X, xc, rx);
+    bool ok = radial_eval(c, xc[0], xc[1], xc[2], pixel[2 * i], pixel[2 * i + 1], r, J, Ji, &r2);
+    if (ok && !(T(3) * fabs(c.k1) * r2 + T(5) * fabs(c.k2) * r2 * r2 < T(0.5))) {
+      const T turn = radial_turn(c.k1, c.k2);
+      ok = !(r2 >= turn && turn < T(INFINITY));
+    }
+    if (!ok) r[0] = r[1] = T(NAN);
   }
   residual[2 * i] = r[0];
   residual[2 * i + 1] = r[1];
 }
 
+// The same with every camera's row in shared memory, formed once per CTA: a persistent grid of CTAs
+// walks the observations, pixels and residuals as 2-vectors. 16-byte chunk q of row j sits at chunk
+// q ^ swizzle(j), so that lanes with different cameras spread over the banks.
+template <typename T>
+__device__ __forceinline__ uint32_t row_chunk(uint32_t j, uint32_t q) {
+  constexpr uint32_t CH = sizeof(T);  // chunks of a row: 64 or 128 bytes
+  return j * CH + (q ^ (sizeof(T) == 4 ? (j >> 1) & 3u : j & 7u));
+}
+template <typename T>
+struct __align__(2 * sizeof(T)) Pair2 {
+  T x, y;
+};
+template <typename T>
+__global__ void __launch_bounds__(1024) k_forward_table(uint64_t n, const uint32_t* __restrict__ cam,
+                                                        const uint32_t* __restrict__ pt, const T* __restrict__ pixel,
+                                                        const T* __restrict__ rotvec, const T* __restrict__ intr,
+                                                        const T* __restrict__ trans, const T* __restrict__ points,
+                                                        uint32_t ncam, uint64_t npts, T* __restrict__ residual) {
+  extern __shared__ uint4 table[];  // ncam rows of sizeof(T) chunks
+  constexpr uint32_t CH = sizeof(T);
+  union Row {
+    CamRow<T> c;
+    uint4 q[CH];
+    __device__ Row() {}
+  };
+  for (uint32_t j = threadIdx.x; j < ncam; j += blockDim.x) {
+    Row row;
+    row.c = make_row(rotvec, trans, intr, j);
+    row.c.turn = radial_turn(row.c.k1, row.c.k2);
+#pragma unroll
+    for (uint32_t q = 0; q < CH; ++q) table[row_chunk<T>(j, q)] = row.q[q];
+  }
+  __syncthreads();
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += step) {
+    const uint32_t j = cam[i], p = pt[i];
+    const Pair2<T> px = reinterpret_cast<const Pair2<T>*>(pixel)[i];
+    T r[2] = {T(NAN), T(NAN)};
+    if (j < ncam && p < npts) {
+      const T X[3] = {points[3 * (uint64_t)p], points[3 * (uint64_t)p + 1], points[3 * (uint64_t)p + 2]};
+      Row row;
+#pragma unroll
+      for (uint32_t q = 0; q < CH; ++q) row.q[q] = table[row_chunk<T>(j, q)];
+      T xc[3], rx[3], J[2][3], Ji[2][3];
+      camera_point(row.c, X, xc, rx);
+      if (!radial_eval(row.c, xc[0], xc[1], xc[2], px.x, px.y, r, J, Ji)) r[0] = r[1] = T(NAN);
+    }
+    reinterpret_cast<Pair2<T>*>(residual)[i] = Pair2<T>{r[0], r[1]};
+  }
+}
+
 // Fixed-point accumulation tables, one entry per output component (cameras: 9 = rotvec 3,
 // translation 3, intrinsics 3; points: 3).
 struct Accum {
-  uint32_t* maxbits;  // pass 0: largest |contribution| (float bits); then the component's exponent
+  uint32_t* maxbits;  // largest |contribution| (float bits)
   unsigned long long* sum;
   uint64_t ncomp;
   uint32_t* bad_index;  // set when an observation's camera or point index is out of range
+  int headroom;
 };
 
 constexpr int kCamComps = 9;
+constexpr int kObsComps = kCamComps + 3;
 
-__device__ __forceinline__ void record_max(uint32_t* slot, float v) {
-  const float a = fabsf(v);
-  if (a != 0.0f || isnan(v)) atomicMax(slot, isnan(v) ? 0x7fc00000u : __float_as_uint(a));
+// A component's scale 2^e from its largest contribution (bits, finite): 62 - headroom - E with the
+// largest < 2^E.
+__device__ __forceinline__ int scale_exponent(uint32_t bits, int headroom) {
+  const int E = bits >= 0x00800000u ? (int)(bits >> 23) - 126 : (32 - __clz((int)bits)) - 149;
+  return 62 - headroom - E;
+}
+__device__ __forceinline__ double exp2_int(int e) {  // 2^e, e in the range of normal doubles
+  return __hiloint2double((e + 1023) << 20, 0);
 }
 
-__device__ __forceinline__ void add_fixed(const Accum& acc, uint64_t k, float v) {
-  if (v == 0.0f) return;
-  const int e = (int)acc.maxbits[k];
-  if (e == INT32_MIN) return;  // non-finite component: resolved in the finish pass
-  const long long q = llrint(ldexp((double)v, e));
-  atomicAdd(acc.sum + k, (unsigned long long)q);
+// Clears the accumulators (words of 16 bytes) and forms the camera rows.
+__global__ void k_vjp_setup(uint64_t ncam, const float* __restrict__ rotvec, const float* __restrict__ trans,
+                            const float* __restrict__ intr, CamRow<float>* __restrict__ rows, uint4* clear,
+                            uint64_t words) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x, first = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  for (uint64_t i = first; i < words; i += step) clear[i] = make_uint4(0, 0, 0, 0);
+  for (uint64_t j = first; j < ncam; j += step) {
+    CamRow<float> c = make_row(rotvec, trans, intr, j);
+    c.turn = radial_turn(c.k1, c.k2);
+    rows[j] = c;
+  }
 }
 
-// One observation's contributions; PASS 0 records maxima, PASS 1 adds fixed-point values. An
+// One observation's contributions per lane; PASS 0 records maxima, PASS 1 adds fixed-point values. An
 // observation whose camera or point index is out of range adds nothing anywhere and raises the
-// bad-index word, which makes the finish pass write NaN into every gradient output.
+// bad-index word, which makes the finish pass write NaN into every gradient output. The warp's 32 x 12
+// contributions go through shared memory: lane l of step s then takes contribution (32 s + l) % 12 of
+// observation (32 s + l) / 12.
 template <int PASS>
-__global__ void k_vjp(uint64_t n, const uint32_t* __restrict__ cam, const uint32_t* __restrict__ pt,
-                      const float* __restrict__ pixel, const CamPre<float>* __restrict__ pre,
-                      const float* __restrict__ trans, const float* __restrict__ points,
-                      const float* __restrict__ grad, uint64_t ncam, uint64_t npts, Accum acc) {
+__global__ void __launch_bounds__(kThreads) k_vjp(uint64_t n, const uint32_t* __restrict__ cam,
+                                                  const uint32_t* __restrict__ pt, const float* __restrict__ pixel,
+                                                  const CamRow<float>* __restrict__ rows,
+                                                  const float* __restrict__ points, const float* __restrict__ grad,
+                                                  uint64_t ncam, uint64_t npts, Accum acc) {
+  __shared__ float sv[kThreads / 32][kObsComps * 33];
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t j = cam[i], p = pt[i];
-  if (j >= ncam || p >= npts) {
-    if (PASS == 0) atomicOr(acc.bad_index, 1u);
-    return;
+  const int lane = threadIdx.x & 31;
+  float* mine = sv[threadIdx.x >> 5];
+  uint32_t j = 0, p = 0;
+  float v[kObsComps];
+#pragma unroll
+  for (int k = 0; k < kObsComps; ++k) v[k] = 0.0f;
+  bool live = i < n;
+  if (live) {
+    j = cam[i];
+    p = pt[i];
+    if (j >= ncam || p >= npts) {
+      if (PASS == 0) atomicOr(acc.bad_index, 1u);
+      live = false;
+      j = p = 0;
+    }
   }
-  const float g0 = grad[2 * i], g1 = grad[2 * i + 1];
-  if (g0 == 0.0f && g1 == 0.0f) return;
-  const CamPre<float> c = pre[j];
-  const float X[3] = {points[3 * (uint64_t)p], points[3 * (uint64_t)p + 1], points[3 * (uint64_t)p + 2]};
-  const float t[3] = {trans[3 * (uint64_t)j], trans[3 * (uint64_t)j + 1], trans[3 * (uint64_t)j + 2]};
-  float xc[3], rx[3], r[2], J[2][3], Ji[2][3];
-  camera_point(c, t, X, xc, rx);
-  if (!radial_eval(c, xc[0], xc[1], xc[2], pixel[2 * i], pixel[2 * i + 1], r, J, Ji)) return;
-  float v[12];
-  float a[3];
+  if (npts > 0) warp_points(points, p, mine);
+  if (live) {
+    const float g0 = grad[2 * i], g1 = grad[2 * i + 1];
+    if (!(g0 == 0.0f && g1 == 0.0f)) {
+      CamRow<float> c;
+      const float4* row = reinterpret_cast<const float4*>(rows + j);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) a[k] = J[0][k] * g0 + J[1][k] * g1;
-  // rotation: Jl^T (rx x a)
-  const float ca[3] = {rx[1] * a[2] - rx[2] * a[1], rx[2] * a[0] - rx[0] * a[2], rx[0] * a[1] - rx[1] * a[0]};
+      for (int q = 0; q < 4; ++q) reinterpret_cast<float4*>(&c)[q] = __ldg(row + q);
+      const float X[3] = {mine[3 * lane], mine[3 * lane + 1], mine[3 * lane + 2]};
+      float xc[3], rx[3], r[2], J[2][3], Ji[2][3];
+      camera_point(c, X, xc, rx);
+      if (radial_eval(c, xc[0], xc[1], xc[2], pixel[2 * i], pixel[2 * i + 1], r, J, Ji)) {
+        float a[3];
 #pragma unroll
-  for (int s = 0; s < 3; ++s) v[s] = c.Jl[s] * ca[0] + c.Jl[3 + s] * ca[1] + c.Jl[6 + s] * ca[2];
+        for (int k = 0; k < 3; ++k) a[k] = J[0][k] * g0 + J[1][k] * g1;
+        // rotation, before Jl^T: rx x a
+        v[0] = rx[1] * a[2] - rx[2] * a[1];
+        v[1] = rx[2] * a[0] - rx[0] * a[2];
+        v[2] = rx[0] * a[1] - rx[1] * a[0];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) v[3 + k] = a[k];
-  v[6] = (Ji[0][0] * g0 + Ji[1][0] * g1) / c.f;
-  v[7] = Ji[0][1] * g0 + Ji[1][1] * g1;
-  v[8] = Ji[0][2] * g0 + Ji[1][2] * g1;
-  // point: R^T a
+        for (int k = 0; k < 3; ++k) v[3 + k] = a[k];
+        v[6] = (Ji[0][0] * g0 + Ji[1][0] * g1) / c.f;
+        v[7] = Ji[0][1] * g0 + Ji[1][1] * g1;
+        v[8] = Ji[0][2] * g0 + Ji[1][2] * g1;
+        // point: R^T a
 #pragma unroll
-  for (int k = 0; k < 3; ++k) v[9 + k] = c.R[k] * a[0] + c.R[3 + k] * a[1] + c.R[6 + k] * a[2];
-  const uint64_t cbase = (uint64_t)kCamComps * j, pbase = (uint64_t)kCamComps * ncam + 3 * (uint64_t)p;
-  if (PASS == 0) {
+        for (int k = 0; k < 3; ++k) v[9 + k] = c.R[k] * a[0] + c.R[3 + k] * a[1] + c.R[6 + k] * a[2];
+      }
+    }
+  }
+  __syncwarp();  // the points are read: their place takes the contributions
 #pragma unroll
-    for (int k = 0; k < 9; ++k) record_max(acc.maxbits + cbase + k, v[k]);
+  for (int k = 0; k < kObsComps; ++k) mine[k * 33 + lane] = v[k];
+  __syncwarp();
+  // (32 s + l) / 12 and % 12 repeat every three steps, eight observations on
+  uint32_t ou[3], ku[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) record_max(acc.maxbits + pbase + k, v[9 + k]);
-  } else {
+  for (int u = 0; u < 3; ++u) {
+    ou[u] = (32 * u + lane) / kObsComps;
+    ku[u] = (32 * u + lane) % kObsComps;
+  }
+  uint32_t* const pt_max = acc.maxbits + (uint64_t)kCamComps * ncam;
+  unsigned long long* const pt_sum = acc.sum + (uint64_t)kCamComps * ncam;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) add_fixed(acc, cbase + k, v[k]);
+  for (int t = 0; t < 4; ++t) {
+    float val[3];
+    uint32_t* mx[3];
+    unsigned long long* sm[3];
+    uint32_t bits[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) add_fixed(acc, pbase + k, v[9 + k]);
+    for (int u = 0; u < 3; ++u) {
+      const uint32_t o = 8 * t + ou[u], k = ku[u];
+      const uint32_t oj = __shfl_sync(0xffffffffu, j, o), op = __shfl_sync(0xffffffffu, p, o);
+      val[u] = mine[k * 33 + o];
+      const bool cam_part = k < kCamComps;
+      const uint64_t at = cam_part ? (uint64_t)oj * kCamComps + k : (uint64_t)op * 3 + (k - kCamComps);
+      mx[u] = (cam_part ? acc.maxbits : pt_max) + at;
+      if (PASS == 1) sm[u] = (cam_part ? acc.sum : pt_sum) + at;
+      // an absent observation's values are zero: nothing to read or add
+      bits[u] = val[u] != 0.0f ? (PASS == 0 ? *mx[u] : __ldg(mx[u])) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      if (val[u] == 0.0f) continue;
+      if (PASS == 0) {
+        const uint32_t b = isnan(val[u]) ? 0x7fc00000u : __float_as_uint(fabsf(val[u]));
+        if (b > bits[u]) atomicMax(mx[u], b);  // a stale maximum only adds an atomic
+      } else if (bits[u] < 0x7f800000u) {  // else a non-finite component: resolved in the finish pass
+        const long long q = __double2ll_rn((double)val[u] * exp2_int(scale_exponent(bits[u], acc.headroom)));
+        atomicAdd(sm[u], (unsigned long long)q);
+      }
+    }
   }
 }
 
-// Converts each component's maximum into its scale exponent (in place).
-__global__ void k_vjp_scales(Accum acc, int headroom) {
-  const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (k >= acc.ncomp) return;
+// Component k's sum as a double; NaN when a contribution was not finite or an index was out of range.
+__device__ __forceinline__ double component_sum(const Accum& acc, uint64_t k, bool bad) {
   const uint32_t bits = acc.maxbits[k];
-  if (bits == 0u) {
-    acc.maxbits[k] = 0u;  // no contribution: exponent unused
-    return;
-  }
-  if (bits >= 0x7f800000u) {
-    acc.maxbits[k] = (uint32_t)INT32_MIN;
-    return;
-  }
-  int E;
-  frexp((double)__uint_as_float(bits), &E);  // max < 2^E
-  acc.maxbits[k] = (uint32_t)(62 - headroom - E);
+  if (bad || bits >= 0x7f800000u) return NAN;
+  if (bits == 0u) return 0.0;
+  return (double)(long long)acc.sum[k] * exp2_int(-scale_exponent(bits, acc.headroom));
 }
 
-__global__ void k_vjp_finish(Accum acc, uint64_t ncam, float* __restrict__ g_rot, float* __restrict__ g_t,
-                             float* __restrict__ g_int, float* __restrict__ g_pt) {
+__global__ void k_vjp_finish(Accum acc, uint64_t ncam, const float* __restrict__ rotvec, float* __restrict__ g_rot,
+                             float* __restrict__ g_t, float* __restrict__ g_int, float* __restrict__ g_pt) {
   const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (k >= acc.ncomp) return;
-  const int e = (int)acc.maxbits[k];
-  float val;
-  if (e == INT32_MIN || *acc.bad_index != 0u)
-    val = NAN;
-  else
-    val = (float)ldexp((double)(long long)acc.sum[k], -e);
-  if (k < kCamComps * ncam) {
-    const uint64_t j = k / kCamComps, c = k - kCamComps * j;
-    if (c < 3)
-      g_rot[3 * j + c] += val;
-    else if (c < 6)
+  const bool bad = *acc.bad_index != 0u;
+  if (k >= kCamComps * ncam) {
+    g_pt[k - kCamComps * ncam] += (float)component_sum(acc, k, bad);
+    return;
+  }
+  const uint64_t j = k / kCamComps, c = k - kCamComps * j;
+  if (c < 3) {  // Jl^T times the summed R X_p x a
+    const float w[3] = {rotvec[3 * j], rotvec[3 * j + 1], rotvec[3 * j + 2]};
+    float R[9], Jl[9];
+    rodrigues(w, R, Jl);
+    double val = 0.0;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const float col = c == 0 ? Jl[3 * r] : (c == 1 ? Jl[3 * r + 1] : Jl[3 * r + 2]);
+      val += (double)col * component_sum(acc, kCamComps * j + r, bad);
+    }
+    g_rot[3 * j + c] += (float)val;
+  } else {
+    const float val = (float)component_sum(acc, k, bad);
+    if (c < 6)
       g_t[3 * j + c - 3] += val;
     else
       g_int[3 * j + c - 6] += val;
-  } else {
-    g_pt[k - kCamComps * ncam] += val;
   }
 }
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Workspace: camera table, then the cleared region (maxima, sums, bad-index word).
+// Workspace: camera rows, then the cleared region (maxima, sums, bad-index word).
 struct VjpLayout {
   size_t pre, maxbits, sum, bad, total;
 };
@@ -304,7 +438,7 @@ inline VjpLayout vjp_layout(uint64_t ncam, uint64_t npts) {
   VjpLayout l;
   const uint64_t ncomp = kCamComps * ncam + 3 * npts;
   l.pre = 0;
-  l.maxbits = align256(sizeof(CamPre<float>) * ncam);
+  l.maxbits = align256(kCamScratch * ncam);
   l.sum = l.maxbits + align256(sizeof(uint32_t) * ncomp);
   l.bad = l.sum + align256(sizeof(unsigned long long) * ncomp);
   l.total = l.bad + 256;
@@ -344,11 +478,36 @@ int cuda_status(omvgba_error* e) {
   return ok(e);
 }
 
+// Which forward kernel: the shared-memory camera table pays for itself once every CTA of a persistent grid
+// has many more observations than the table has rows (kTableObservations, 32 per camera), fits beside
+// nothing else in an SM's shared memory, and needs pixels and residuals aligned for 2-vector access.
+// Everything else recomputes the row per observation. Measured, recomputed -> table: 10M observations of
+// 3,000 cameras FP32 228 -> 142 us, 1.2M of 500 cameras FP64 41 -> 29 us. At 8,000 observations the two
+// are equal (a launch's latency).
+constexpr uint64_t kTableObservations = 1u << 18;
+constexpr size_t kTableMaxBytes = 200 * 1024;
+
 template <typename T>
 int forward(void* stream, uint64_t n, const uint32_t* cam, const uint32_t* pt, const T* pixel, uint64_t ncam,
             const T* rotvec, const T* trans, const T* intr, uint64_t npts, const T* points, T* residual,
             omvgba_error* err) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const bool aligned = ((reinterpret_cast<uintptr_t>(pixel) | reinterpret_cast<uintptr_t>(residual)) % (2 * sizeof(T))) == 0;
+  if (aligned && n >= kTableObservations && n >= 32 * ncam && ncam * sizeof(CamRow<T>) <= kTableMaxBytes) {
+    const size_t smem = (size_t)ncam * sizeof(CamRow<T>);
+    const int threads = smem > kTableMaxBytes / 2 ? 1024 : 512;
+    int dev = 0, sms = 0, per = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_forward_table<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTableMaxBytes);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_forward_table<T>, threads, smem);
+    if (e != cudaSuccess) return cuda_status(err);
+    const unsigned grid = (unsigned)std::min<uint64_t>((n + threads - 1) / threads, (uint64_t)sms * std::max(per, 1));
+    k_forward_table<T><<<grid, threads, smem, st>>>(n, cam, pt, pixel, rotvec, intr, trans, points, (uint32_t)ncam, npts,
+                                                     residual);
+    return cuda_status(err);
+  }
   k_forward<T><<<grid_for(n), kThreads, 0, st>>>(n, cam, pt, pixel, rotvec, intr, trans, points, ncam, npts,
                                                   residual);
   return cuda_status(err);
@@ -416,19 +575,18 @@ int32_t omvgba_residual_vjp_f32(void* stream, uint64_t observation_count, const 
     return fail(error, OMVGBA_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
-  CamPre<float>* pre = reinterpret_cast<CamPre<float>*>(ws + l.pre);
+  CamRow<float>* rows = reinterpret_cast<CamRow<float>*>(ws + l.pre);
   Accum acc{reinterpret_cast<uint32_t*>(ws + l.maxbits), reinterpret_cast<unsigned long long*>(ws + l.sum),
-            kCamComps * camera_count + 3 * point_count, reinterpret_cast<uint32_t*>(ws + l.bad)};
-  if (cudaMemsetAsync(ws + l.maxbits, 0, l.total - l.maxbits, st) != cudaSuccess) return cuda_status(error);
-  k_cam_prepare<float><<<grid_for(camera_count), kThreads, 0, st>>>(camera_count, rotvec, intrinsics, pre);
-  k_vjp<0><<<grid_for(observation_count), kThreads, 0, st>>>(observation_count, camera_index, point_index, pixel, pre,
-                                                             translation, points, grad_residual, camera_count,
-                                                             point_count, acc);
-  k_vjp_scales<<<grid_for(acc.ncomp), kThreads, 0, st>>>(acc, ceil_log2(observation_count) + 1);
-  k_vjp<1><<<grid_for(observation_count), kThreads, 0, st>>>(observation_count, camera_index, point_index, pixel, pre,
-                                                             translation, points, grad_residual, camera_count,
-                                                             point_count, acc);
-  k_vjp_finish<<<grid_for(acc.ncomp), kThreads, 0, st>>>(acc, camera_count, grad_rotvec, grad_translation,
+            kCamComps * camera_count + 3 * point_count, reinterpret_cast<uint32_t*>(ws + l.bad),
+            ceil_log2(observation_count) + 1};
+  const uint64_t words = (l.total - l.maxbits) / 16;
+  k_vjp_setup<<<(unsigned)std::min<uint64_t>(4096, grid_for(std::max(words, camera_count))), kThreads, 0, st>>>(
+      camera_count, rotvec, translation, intrinsics, rows, reinterpret_cast<uint4*>(ws + l.maxbits), words);
+  k_vjp<0><<<grid_for(observation_count), kThreads, 0, st>>>(observation_count, camera_index, point_index, pixel, rows,
+                                                             points, grad_residual, camera_count, point_count, acc);
+  k_vjp<1><<<grid_for(observation_count), kThreads, 0, st>>>(observation_count, camera_index, point_index, pixel, rows,
+                                                             points, grad_residual, camera_count, point_count, acc);
+  k_vjp_finish<<<grid_for(acc.ncomp), kThreads, 0, st>>>(acc, camera_count, rotvec, grad_rotvec, grad_translation,
                                                          grad_intrinsics, grad_points);
   return cuda_status(error);
 }
