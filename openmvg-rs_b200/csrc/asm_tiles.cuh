@@ -152,8 +152,13 @@ __global__ void __launch_bounds__(mv_tile_obs<R>(), asm_min_blocks<R>())
 
 // Per block: the sum of its records in tile order, in the assembly record layout (kAsmRec): U lower
 // (21, packed as six rows), g (6), reduced g (6), damping diagonal (6: the diagonal of U), edge (18),
-// coupling lower (21); entries past the block's dimension are zero. One CTA per block.
-__global__ void __launch_bounds__(128) k_block_records(MvTiles mt, const int* __restrict__ blk_edge,
+// coupling lower (21); entries past the block's dimension are zero. One CTA per block, thread = (entry,
+// share of the records); a share takes every kRecordShares-th record and the shares are added in order.
+// Bound: HBM on the records at survey sizes, latency of an entry's run of loads below: one thread per entry
+// took 14.5 us for a window's 19 blocks and 36 us for 31, this 7.5 and 14 us; 77 us for 500 cameras either
+// way.
+constexpr int kRecordShares = 12;
+__global__ void __launch_bounds__(kAsmRec * kRecordShares) k_block_records(MvTiles mt, const int* __restrict__ blk_edge,
                                                        const double* __restrict__ rec_in, double* __restrict__ blk_out) {
   const int b = blockIdx.x;
   if (b >= mt.nblocks) return;
@@ -163,7 +168,9 @@ __global__ void __launch_bounds__(128) k_block_records(MvTiles mt, const int* __
   const size_t stride = (size_t)kAsmRecordScale * d;
   const double* base = rec_in + (size_t)e0 * kAsmRecordScale;
   const int di = blk_edge[b] >= 0 ? mt.blk_dim[blk_edge[b]] : 0;  // the edge's intrinsic columns
-  for (int k = threadIdx.x; k < kAsmRec; k += blockDim.x) {
+  __shared__ double sh[kRecordShares][kAsmRec];
+  {
+    const int k = threadIdx.x % kAsmRec, share = threadIdx.x / kAsmRec;
     int off = -1;
     if (k < 21) {
       int r = 0;
@@ -186,8 +193,15 @@ __global__ void __launch_bounds__(128) k_block_records(MvTiles mt, const int* __
       if (r < d) off = asm_offset(d, 3, r, idx - r * (r + 1) / 2);
     }
     double acc = 0.0;
-    if (off >= 0)
-      for (uint32_t q = 0; q < n; ++q) acc += base[q * stride + off];
+    if (off >= 0) {
+#pragma unroll 4
+      for (uint32_t q = share; q < n; q += kRecordShares) acc += base[q * stride + off];
+    }
+    sh[share][k] = acc;
+    __syncthreads();
+    if (share > 0) return;
+    acc = 0.0;
+    for (int s2 = 0; s2 < kRecordShares; ++s2) acc += sh[s2][k];
     blk_out[(size_t)kAsmRec * b + k] = acc;
   }
 }

@@ -117,11 +117,23 @@ struct FixedCameraDev {
       if (!isfinite(r2) || (has_turn && r2 >= turn_squared)) return false;
       return distortion_jacobian(x, y, &a, &b, &c, &d) && d > 1e-12;
     }
+#ifdef __CUDA_ARCH__
+    // every sample, several in flight: leaving at the first failure would chain their latencies
+    bool ok = true;
+#pragma unroll 4
+    for (int i = 0; i <= 32; ++i) {
+      double s = double(i) / 32.0;
+      const bool good = distortion_jacobian(x * s, y * s, &a, &b, &c, &d) && d > 1e-12;
+      ok = ok && good;
+    }
+    return ok;
+#else
     for (int i = 0; i <= 32; ++i) {
       double s = double(i) / 32.0;
       if (!(distortion_jacobian(x * s, y * s, &a, &b, &c, &d) && d > 1e-12)) return false;
     }
     return true;
+#endif
   }
   // validate_forward_domain (brown_conrady.rs:134-166)
   BA_HD bool forward_domain(double x, double y) const {

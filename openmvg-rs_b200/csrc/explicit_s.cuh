@@ -391,25 +391,33 @@ __host__ __device__ __forceinline__ size_t tile_at(const TileBand& b, int i, int
 
 // Scatter of the rows into the band: element (m, n) of block S_XY lands at permuted (P, Q) =
 // (perm_off[X] + m, perm_off[Y] + n) when P >= Q. With scale non-null the stored value is
-// scale_P S_PQ scale_Q; the diagonal gets + lambda diag_P, then - shift. One thread per entry.
-__global__ void k_rows_to_tiles(RowTables rt, const double* __restrict__ rows, const int* __restrict__ perm_off,
-                                const double* __restrict__ diag, double lambda, const double* __restrict__ scale,
-                                double shift, TileBand tb) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+// scale_P S_PQ scale_Q; the diagonal gets + lambda diag_P, then - shift. A warp per four blocks, eight
+// lanes a block (an element of its 36 each, in turn). The last CTA writes the identity on the padding
+// rows of the last diagonal tile and sets the factorization's status word.
+__global__ void __launch_bounds__(128) k_rows_to_tiles(RowTables rt, const double* __restrict__ rows,
+                                                       const int* __restrict__ perm_off, const double* __restrict__ diag,
+                                                       double lambda, const double* __restrict__ scale, double shift,
+                                                       TileBand tb, int* status) {
+  if (blockIdx.x == gridDim.x - 1) {
+    if (threadIdx.x == 0) status[0] = 1;
+    const int r = tb.n + threadIdx.x, i = tb.nt - 1;
+    if (r < tb.nt * kCT) tb.t[tile_at(tb, i, i) + (size_t)(r % kCT) * kCT + (r % kCT)] = 1.0;
+  }
+  const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   if (q >= rt.entries) return;
   const int X = rt.nbr_row[q], Y = rt.nbr[q];
   const int dX = rt.blk_dim[X], dY = rt.blk_dim[Y];
   const int pX = perm_off[X], pY = perm_off[Y], oX = rt.blk_off[X], oY = rt.blk_off[Y];
   const double* S = rows + rt.slot_off[q];
-  for (int m = 0; m < dX; ++m)
-    for (int n = 0; n < dY; ++n) {
-      const int P = pX + m, Q = pY + n;
-      if (P < Q) continue;
-      double v = S[m * dY + n];
-      if (scale) v *= scale[oX + m] * scale[oY + n];
-      if (P == Q) v += lambda * diag[oX + m] - shift;
-      tb.t[tile_at(tb, P / kCT, Q / kCT) + (size_t)(Q % kCT) * kCT + (P % kCT)] = v;
-    }
+  for (int e = threadIdx.x & 7; e < dX * dY; e += 8) {
+    const int m = e / dY, n = e - m * dY;
+    const int P = pX + m, Q = pY + n;
+    if (P < Q) continue;
+    double v = S[e];
+    if (scale) v *= scale[oX + m] * scale[oY + n];
+    if (P == Q) v += lambda * diag[oX + m] - shift;
+    tb.t[tile_at(tb, P / kCT, Q / kCT) + (size_t)(Q % kCT) * kCT + (P % kCT)] = v;
+  }
 }
 
 // Scatter of lower-triangle entries (row >= col) given as triplets into the band.
@@ -509,28 +517,25 @@ __device__ __forceinline__ void mma8(int depth, FA a, FB b, double& c0, double& 
 // POTRF of diagonal tile k and the inverse W_k = L_kk^-1 of its factor, one CTA of 8 warps, blocked by
 // 8 columns. A panel (all rows, 8 columns) is factored by warp 0 in registers, two rows per lane: a
 // step is one reciprocal root, one scaling and the shuffles that hand the pivot row's entries to the
-// columns right of it, with no barrier; then every warp subtracts the panel's rank-8 product from
-// its 8 x 8 blocks of the trailing triangle on the FP64 tensor pipe. The inverse of the factor starts
+// columns right of it, with no barrier (the pivots' roots and reciprocals, which only the output and the
+// inverse need, come after the panel, a lane each); then every warp subtracts the panel's rank-8 product
+// from its 8 x 8 blocks of the trailing triangle on the FP64 tensor pipe. The inverse of the factor starts
 // from the 8 x 8 diagonal blocks (a warp each) and doubles the block size three times with
 // W_21 = -W_22 (L_21 W_11), the products on the tensor pipe, their middle factor in the unused upper
 // triangle. Bound: the 64 dependent pivot steps. A right-looking factor with one barrier per column and
-// a second sweep of 64 barriers for the inverse took 64 us per tile; this takes 23.5.
+// a second sweep of 64 barriers for the inverse took 64 us per tile; this takes 18.5.
 // status[0] = 0 when a pivot is not finite and positive; later launches of the factorization then
 // return at once.
 constexpr size_t kPotrfSmem = 2 * kStagedTile;
-__global__ void __launch_bounds__(256) k_tile_potrf(TileBand tb, int k, int* status) {
-  extern __shared__ __align__(16) double sh[];
+// A: the tile in shared memory (visible to the CTA), then L, its strict upper triangle scratch; W: a
+// second staged tile.
+__device__ void potrf_tile(const TileBand& tb, int k, double* A, double* W, int* status) {
   __shared__ double rdiag[kCT];
   __shared__ int s_bad;
-  if (status[0] == 0) return;
-  double* A = sh;               // the tile, then L; the strict upper triangle is scratch
-  double* W = sh + kCT * kTS;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
   double* gt = tb.t + tile_at(tb, k, k);
-  stage_tile(gt, A);
   for (int i = tid; i < kCT * kTS; i += 256) W[i] = 0.0;
   if (tid == 0) s_bad = 0;
-  stage_wait();
   __syncthreads();
   for (int j0 = 0; j0 < kCT; j0 += 8) {
     if (w == 0) {
@@ -542,22 +547,16 @@ __global__ void __launch_bounds__(256) k_tile_potrf(TileBand tb, int k, int* sta
       }
       const bool upper_half = j0 >= 32;  // the panel's diagonal rows lie in hi
       bool bad = false;
+      double pivot = 1.0;  // lane c < 8: column c's
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         const int pl = (j0 + c) & 31;
         const double d = __shfl_sync(0xffffffffu, upper_half ? hi[c] : lo[c], pl);
         bad = bad || !(isfinite(d) && d > 0.0);
+        if (lane == c) pivot = d;
         const double rs = rsqrt(d);
         lo[c] *= rs;
         hi[c] *= rs;
-        if (lane == pl) {
-          const double sd = sqrt(d);
-          if (upper_half)
-            hi[c] = sd;
-          else
-            lo[c] = sd;
-          rdiag[j0 + c] = 1.0 / sd;
-        }
 #pragma unroll
         for (int c2 = c + 1; c2 < 8; ++c2) {
           const double l = __shfl_sync(0xffffffffu, upper_half ? hi[c] : lo[c], (j0 + c2) & 31);
@@ -567,8 +566,13 @@ __global__ void __launch_bounds__(256) k_tile_potrf(TileBand tb, int k, int* sta
       }
 #pragma unroll
       for (int c = 0; c < 8; ++c) {  // rows above the panel's diagonal are scratch
-        if (lane >= j0 + c) A[(j0 + c) * kTS + lane] = lo[c];
-        if (lane + 32 >= j0 + c) A[(j0 + c) * kTS + lane + 32] = hi[c];
+        if (lane > j0 + c) A[(j0 + c) * kTS + lane] = lo[c];
+        if (lane + 32 > j0 + c) A[(j0 + c) * kTS + lane + 32] = hi[c];
+      }
+      if (lane < 8) {
+        const double sd = sqrt(pivot);
+        A[(j0 + lane) * kTS + j0 + lane] = sd;
+        rdiag[j0 + lane] = 1.0 / sd;
       }
       if (bad && lane == 0) s_bad = 1;
     }
@@ -638,6 +642,15 @@ __global__ void __launch_bounds__(256) k_tile_potrf(TileBand tb, int k, int* sta
   for (int i = tid; i < kCTT; i += 256) wk[i] = W[(i >> 6) * kTS + (i & 63)];
 }
 
+__global__ void __launch_bounds__(256) k_tile_potrf(TileBand tb, int k, int* status) {
+  extern __shared__ __align__(16) double sh[];
+  if (status[0] == 0) return;
+  stage_tile(tb.t + tile_at(tb, k, k), sh);
+  stage_wait();
+  __syncthreads();
+  potrf_tile(tb, k, sh, sh + kCT * kTS, status);
+}
+
 // TRSM as a product: the tiles below diagonal tile k, L_ik = A_ik W_k^T (CTA per tile). Dynamic shared
 // memory: two staged operands.
 constexpr size_t kTrsmSmem = 2 * kStagedTile;
@@ -659,9 +672,12 @@ __global__ void __launch_bounds__(256) k_tile_trsm(TileBand tb, int k, const int
 }
 
 // Trailing update of step k: A_ij -= L_ik L_jk^T for k < j <= i <= min(k + bwt, nt - 1), one CTA per
-// tile; the sum over the tile's 64 columns runs in order.
+// tile; the sum over the tile's 64 columns runs in order. CTA 0 has the next diagonal tile: it goes on to
+// factor it (potrf_tile) while the other CTAs update theirs, so a column costs its factorization and its
+// trsm, and the update runs in the factorization's shadow (500-camera survey, per column: 18.5 us of potrf,
+// 6.1 of trsm and 7.0 of update become 6.1 + 22.7).
 constexpr size_t kUpdateSmem = 2 * kStagedTile;
-__global__ void __launch_bounds__(256) k_tile_update(TileBand tb, int k, const int* status) {
+__global__ void __launch_bounds__(256) k_tile_update(TileBand tb, int k, int* status) {
   extern __shared__ __align__(16) double sh[];
   if (status[0] == 0) return;
   double* Ta = sh;
@@ -696,7 +712,14 @@ __global__ void __launch_bounds__(256) k_tile_update(TileBand tb, int k, const i
     for (int b = 0; b < 4; ++b)
 #pragma unroll
       for (int e = 0; e < 2; ++e) acc.v[a][b][e] = old.v[a][b][e] - acc.v[a][b][e];
-  acc_store(acc, cij);
+  if (idx > 0) {
+    acc_store(acc, cij);
+    return;
+  }
+  __syncthreads();  // the operands are read: their place takes the diagonal tile
+  acc_each(acc, [&](int r, int c, double v) { Ta[c * kTS + r] = v; });
+  __syncthreads();
+  potrf_tile(tb, k + 1, Ta, Tb, status);
 }
 
 // Forward (L y = b) and backward (L^T x = y) substitution with the banded tiled factor, in place on the
@@ -937,44 +960,91 @@ __global__ void k_z_marginals(TileBand Z, int ngroups, const int* __restrict__ p
 // normalized iterate): out[0] = lambda, out[1] = 1 when it settled (|rq - lambda| <= 1e-10 |rq| after
 // the 8th iteration) or ran its 200 iterations with finite values, 0 otherwise. n <= kPowerMax.
 //
-// One cluster of kPowerCtas CTAs runs every iteration, so the host waits once. Each CTA keeps the whole
-// iterate in shared memory and takes every kPowerCtas-th block row, several warps a row when it has few; a
-// row's results go to all CTAs' shared memory, one cluster barrier ends the product, and every CTA forms the same
-// norm and quotient in the same order, so all leave the loop together. Bound: 200 dependent iterations of
-// a row's L1/L2 latency and a cluster barrier. One CTA that kept the iterate in global memory took 1.80 ms
-// at n = 113; this takes 1.04.
+// One cluster of kPowerCtas CTAs runs every iteration, so the host waits once. CTA r owns the block rows
+// X = r mod kPowerCtas; a task is 32 blocks of one row, a block per lane. Every CTA keeps the whole
+// iterate in shared memory, not normalized (the products are scaled by the last norm); a row's results go
+// to all CTAs' shared memory, one cluster barrier ends the product, and every CTA forms the same norm
+// and quotient in the same order, so all leave the loop together. While the CTA's tasks fit (kPowerTasks)
+// their blocks stay in shared memory too, element by element with the lanes side by side: the cluster
+// barrier drops L1, so each iteration would otherwise wait for L2 three times over.
+// Bound: 200 dependent iterations of a barrier and a reduction. One CTA that kept the iterate in global
+// memory took 1.80 ms at n = 113, the cluster without the blocks in shared memory 1.04 ms, this 0.56 ms.
 constexpr int kPowerCtas = 8;
 constexpr int kPowerMax = 2048;
-constexpr size_t power_smem(int n) { return 3 * sizeof(double) * (size_t)n; }
-__global__ void __launch_bounds__(1024) k_power_iteration(RowTables rt, const double* __restrict__ rows,
-                                                          const double* __restrict__ scale, int n, double* out) {
+constexpr int kPowerThreads = 512;
+constexpr int kPowerWarps = kPowerThreads / 32;
+constexpr int kPowerTasks = 16;                             // cached tasks of a CTA
+constexpr size_t kPowerTaskDoubles = 36 * 32;
+constexpr size_t power_smem(int n) { return sizeof(double) * (3 * (size_t)n + kPowerTasks * kPowerTaskDoubles); }
+__global__ void __launch_bounds__(kPowerThreads) k_power_iteration(RowTables rt, const double* __restrict__ rows,
+                                                                   const double* __restrict__ scale, int n, double* out) {
   namespace cg = cooperative_groups;
-  extern __shared__ __align__(16) double sh[];  // the iterate, and the product in two alternating buffers
-  __shared__ double red[32][2], s_part[32][6];
-  __shared__ double s_sum[2];
+  extern __shared__ __align__(16) double sh[];  // three iterates in turn, then the cached tasks
+  __shared__ double red[kPowerWarps][2], s_part[kPowerWarps][6];
+  __shared__ int t_row[kPowerTasks], t_off[kPowerTasks][32];  // cached tasks: row; per lane offset << 3 | dim
+  __shared__ int s_tasks;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // warps per row: as many as keep the CTA's rows in one round
-  const int mine = (rt.nblocks + kPowerCtas - 1 - rank) / kPowerCtas;
-  int split = 8;
-  while (split > 1 && mine * split > 32) split /= 2;
-  const int per = 32 / split;
-  double* v = sh;
+  double* cache = sh + 3 * (size_t)n;
+  if (tid == 0) {  // the CTA's tasks, row after row
+    int nt = 0;
+    for (int X = rank; X < rt.nblocks && nt <= kPowerTasks; X += kPowerCtas) {
+      const int m = (int)(rt.nbr_begin[X + 1] - rt.nbr_begin[X] + 31) / 32;
+      for (int q = 0; q < m && nt < kPowerTasks; ++q) t_row[nt + q] = X;
+      nt += m;
+      if (nt > kPowerTasks) break;
+    }
+    s_tasks = nt;
+  }
   const double v0 = 1.0 / sqrt((double)n);
-  for (int i = tid; i < n; i += 1024) v[i] = v0;
+  for (int i = tid; i < n; i += kPowerThreads) sh[i] = v0;
   __syncthreads();
-  cluster.sync();  // every CTA runs before any of them is written to
-  double lam = 0.0;
+  const bool cached = s_tasks <= kPowerTasks;
+  const int tasks = s_tasks;
+  if (cached)
+    for (int t = warp; t < tasks; t += kPowerWarps) {
+      const int X = t_row[t], dX = rt.blk_dim[X];
+      int first = t;
+      while (first > 0 && t_row[first - 1] == X) --first;
+      const uint32_t q = rt.nbr_begin[X] + 32 * (t - first) + lane;
+      const bool have = q < rt.nbr_begin[X + 1];
+      const int Y = have ? rt.nbr[q] : 0, dY = have ? rt.blk_dim[Y] : 0, oY = have ? rt.blk_off[Y] : 0;
+      t_off[t][lane] = oY << 3 | dY;
+      const double* S = rows + (have ? rt.slot_off[q] : 0);
+#pragma unroll
+      for (int m = 0; m < 6; ++m)
+#pragma unroll
+        for (int c = 0; c < 6; ++c)
+          cache[t * kPowerTaskDoubles + (6 * m + c) * 32 + lane] = m < dX && c < dY ? S[m * dY + c] * scale[oY + c] : 0.0;
+    }
+  cluster.sync();  // every CTA runs before any of them is written to; the cache is in place
+  double lam = 0.0, inv = 1.0;
   int ok = 0;
   for (int it = 0; it < 200; ++it) {
-    double* w = sh + (1 + (it & 1)) * (size_t)n;
-    for (int x0 = 0; x0 * kPowerCtas + rank < rt.nblocks; x0 += per) {  // this CTA's rows, `per` at a time
-      const int X = (x0 + warp / split) * kPowerCtas + rank;
-      const bool have = X < rt.nblocks;
-      const int dX = have ? rt.blk_dim[X] : 0;
-      if (have) {
-        double acc[6] = {0, 0, 0, 0, 0, 0};
-        row_times(rt, rows, X, dX, 32u * (warp % split) + lane, 32u * split, [&](int i) { return scale[i] * v[i]; }, acc);
+    const double* v = sh + (it % 3) * (size_t)n;  // times inv: the normalized iterate
+    double* w = sh + ((it + 1) % 3) * (size_t)n;
+    auto publish = [&](int X, int first, int count) {  // rows of s_part [first, first + count) to every CTA
+      const int dX = rt.blk_dim[X], oX = rt.blk_off[X];
+      for (int e = lane; e < dX * kPowerCtas; e += 32) {
+        const int m = e / kPowerCtas;
+        double r = 0.0;
+        for (int q = 0; q < count; ++q) r += s_part[first + q][m];
+        *cluster.map_shared_rank(w + oX + m, e % kPowerCtas) = r * inv * scale[oX + m];
+      }
+    };
+    if (cached) {
+      if (warp < tasks) {
+        const double* C = cache + warp * kPowerTaskDoubles + lane;
+        const int at = t_off[warp][lane], dY = at & 7;
+        double xv[6], acc[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) xv[c] = c < dY ? v[(at >> 3) + c] : 0.0;
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+          acc[m] = 0.0;
+#pragma unroll
+          for (int c = 0; c < 6; ++c) acc[m] += C[(6 * m + c) * 32] * xv[c];
+        }
 #pragma unroll
         for (int m = 0; m < 6; ++m) {
           acc[m] = warp_sum(acc[m]);
@@ -982,18 +1052,32 @@ __global__ void __launch_bounds__(1024) k_power_iteration(RowTables rt, const do
         }
       }
       __syncthreads();
-      if (warp % split == 0)  // element lane / kPowerCtas of the row to CTA lane % kPowerCtas
-        for (int e = lane; e < dX * kPowerCtas; e += 32) {
-          const int m = e / kPowerCtas, o = rt.blk_off[X] + m;
-          double r = 0.0;
-          for (int q = 0; q < split; ++q) r += s_part[warp + q][m];
-          *cluster.map_shared_rank(w + o, e % kPowerCtas) = r * scale[o];
+      if (warp < tasks && (warp == 0 || t_row[warp - 1] != t_row[warp])) {
+        int count = 1;
+        while (warp + count < tasks && t_row[warp + count] == t_row[warp]) ++count;
+        publish(t_row[warp], warp, count);
+      }
+    } else {
+      for (int x0 = 0; x0 * kPowerCtas + rank < rt.nblocks; x0 += kPowerWarps / 2) {  // two warps a row
+        const int X = (x0 + warp / 2) * kPowerCtas + rank;
+        const bool have = X < rt.nblocks;
+        if (have) {
+          double acc[6] = {0, 0, 0, 0, 0, 0};
+          row_times(rt, rows, X, rt.blk_dim[X], 32u * (warp % 2) + lane, 64u, [&](int i) { return scale[i] * v[i]; }, acc);
+#pragma unroll
+          for (int m = 0; m < 6; ++m) {
+            acc[m] = warp_sum(acc[m]);
+            if (lane == 0) s_part[warp][m] = acc[m];
+          }
         }
-      __syncthreads();
+        __syncthreads();
+        if (have && warp % 2 == 0) publish(X, warp, 2);
+        __syncthreads();
+      }
     }
     cluster.sync();
     double nn = 0.0, rq = 0.0;
-    for (int i = tid; i < n; i += 1024) {
+    for (int i = tid; i < n; i += kPowerThreads) {
       nn += w[i] * w[i];
       rq += v[i] * w[i];
     }
@@ -1004,23 +1088,20 @@ __global__ void __launch_bounds__(1024) k_power_iteration(RowTables rt, const do
       red[warp][1] = rq;
     }
     __syncthreads();
-    if (warp == 0) {
-      const double a = warp_sum(red[lane][0]), b = warp_sum(red[lane][1]);
-      if (lane == 0) {
-        s_sum[0] = sqrt(a);
-        s_sum[1] = b;
-      }
+    nn = rq = 0.0;
+#pragma unroll
+    for (int q = 0; q < kPowerWarps; ++q) {  // the same sums in every thread of every CTA
+      nn += red[q][0];
+      rq += red[q][1];
     }
-    __syncthreads();
-    const double nrm = s_sum[0], q = s_sum[1];
+    const double nrm = sqrt(nn), quot = rq * inv;
     if (!(isfinite(nrm) && nrm > 0.0)) {
       ok = 0;
       break;
     }
-    const bool settled = it > 8 && fabs(q - lam) <= 1e-10 * fabs(q);
-    lam = q;
-    for (int i = tid; i < n; i += 1024) v[i] = w[i] / nrm;
-    __syncthreads();
+    const bool settled = it > 8 && fabs(quot - lam) <= 1e-10 * fabs(quot);
+    lam = quot;
+    inv = 1.0 / nrm;
     ok = 1;
     if (settled) break;
   }

@@ -2363,13 +2363,11 @@ bool device_certify_positive_definite(Context* ctx, int n, const std::vector<int
     OMVGBA_LAUNCH(k_triplets_to_tiles, grid_for(rows.size(), 256), 256, 0, st, (uint32_t)rows.size(), d_rows.p,
                   d_cols.p, vals.p, tb);
   OMVGBA_LAUNCH(k_tiles_pad, 1, kCT, 0, st, tb);
-  for (int k = 0; k < nt; ++k) {
-    OMVGBA_LAUNCH(k_tile_potrf, 1, 256, kPotrfSmem, st, tb, k, status.p);
+  OMVGBA_LAUNCH(k_tile_potrf, 1, 256, kPotrfSmem, st, tb, 0, status.p);
+  for (int k = 0; k < nt - 1; ++k) {
     const int m = std::min(bwt, nt - 1 - k);
-    if (m > 0) {
-      OMVGBA_LAUNCH(k_tile_trsm, m, 256, kTrsmSmem, st, tb, k, status.p);
-      OMVGBA_LAUNCH(k_tile_update, m * (m + 1) / 2, 256, kUpdateSmem, st, tb, k, status.p);
-    }
+    OMVGBA_LAUNCH(k_tile_trsm, m, 256, kTrsmSmem, st, tb, k, status.p);
+    OMVGBA_LAUNCH(k_tile_update, m * (m + 1) / 2, 256, kUpdateSmem, st, tb, k, status.p);
   }
   CUDA_OK(cudaGetLastError());
   int ok = 0;
@@ -2913,7 +2911,7 @@ struct Solver {
         OMVGBA_LAUNCH(k_block_tiles<T>, mt.ntiles, mv_tile_obs<T>(),
                       asm_smem_bytes<T>(), st, mt, lin(), pt_off, d_asm_rec.p);
     }
-    OMVGBA_LAUNCH(k_block_records, nb, 128, 0, st, mt, bt.blk_edge, d_asm_rec.p, d_blk_out.p);
+    OMVGBA_LAUNCH(k_block_records, nb, kAsmRec * kRecordShares, 0, st, mt, bt.blk_edge, d_asm_rec.p, d_blk_out.p);
   }
 
   // The camera-pair tables, once per solver; false when the pairs do not serve this problem: more
@@ -3210,19 +3208,15 @@ struct Solver {
     if (d_winv.n != (size_t)S.nt * kCTT) d_winv.alloc((size_t)S.nt * kCTT, st);
     tile_factor_attributes();  // per device and cheap: set on every factorization
     CUDA_OK(cudaMemsetAsync(d_tiles.p, 0, sizeof(double) * count, st));
-    OMVGBA_LAUNCH(k_set_int, 1, 1, 0, st, d_status.p, 1);
     const TileBand tb = tile_band();
-    OMVGBA_LAUNCH(k_rows_to_tiles, grid_for(S.nbr.size(), 128), 128, 0, st, row_tables(), d_rows.p, d_perm_off.p,
-                  d_diag.p, lambda, scale, shift, tb);
-    OMVGBA_LAUNCH(k_tiles_pad, 1, kCT, 0, st, tb);
+    OMVGBA_LAUNCH(k_rows_to_tiles, grid_for(8 * S.nbr.size(), 128), 128, 0, st, row_tables(), d_rows.p, d_perm_off.p,
+                  d_diag.p, lambda, scale, shift, tb, d_status.p);
     run_as_graph([&] {
-      for (int k = 0; k < S.nt; ++k) {
-        OMVGBA_LAUNCH(k_tile_potrf, 1, 256, kPotrfSmem, st, tb, k, d_status.p);
+      OMVGBA_LAUNCH(k_tile_potrf, 1, 256, kPotrfSmem, st, tb, 0, d_status.p);
+      for (int k = 0; k < S.nt - 1; ++k) {  // each update factors the next diagonal tile
         const int m = std::min(S.bwt, S.nt - 1 - k);
-        if (m > 0) {
-          OMVGBA_LAUNCH(k_tile_trsm, m, 256, kTrsmSmem, st, tb, k, d_status.p);
-          OMVGBA_LAUNCH(k_tile_update, m * (m + 1) / 2, 256, kUpdateSmem, st, tb, k, d_status.p);
-        }
+        OMVGBA_LAUNCH(k_tile_trsm, m, 256, kTrsmSmem, st, tb, k, d_status.p);
+        OMVGBA_LAUNCH(k_tile_update, m * (m + 1) / 2, 256, kUpdateSmem, st, tb, k, d_status.p);
       }
     });
     check_launch();
@@ -3266,7 +3260,7 @@ struct Solver {
     CUDA_OK(copy_async(d_e.p, sc.data(), sizeof(double) * D, cudaMemcpyHostToDevice, st));
     CUDA_OK(cudaFuncSetAttribute(k_power_iteration, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)power_smem(kPowerMax)));
-    launch_cluster(k_power_iteration, kPowerCtas, 1024, power_smem(D), st, row_tables(), (const double*)d_rows.p,
+    launch_cluster(k_power_iteration, kPowerCtas, kPowerThreads, power_smem(D), st, row_tables(), (const double*)d_rows.p,
                    (const double*)d_e.p, D, d_power.p);
     check_launch();
     double out[2];
@@ -3361,7 +3355,7 @@ struct Solver {
 
   // y = S_lambda x (implicit, matrix-free); ctl: optional PCG control for graph-launched iterations
   // fp32: use the FP32 record copy (mixed precision inner solves)
-  int mv_finalize_ctas() const { return std::max(1, grid_for((size_t)nb * 32, 256)); }
+  int mv_finalize_ctas() const { return std::max(1, grid_for((size_t)nb * finalize_split(nb), kFinalizeWarps)); }
   // CTAs of the product's last kernel, each of which leaves one curvature term
   int product_ctas() const { return explicit_op ? rows_product_ctas() : mv_finalize_ctas(); }
   // xy: optional per-finalize-CTA sums of x_b . y_b over the CTA's blocks (the PCG curvature terms)
@@ -3376,8 +3370,10 @@ struct Solver {
     matvec_tiles(x, ctl, fp32, pdl_tiles);
     const TileSetDev& ts = mixed ? dT32 : dT64;
     MvTiles mt = ts.view(d_blk_dim.p, d_blk_off.p, nb);
-    launch_pdl(pdl, k_mv_tiles_finalize, mv_finalize_ctas(), 256, st, mt, ts.partial.p, d_diag.p, lambda, x, y, xy,
-               ctl);
+    const int split = finalize_split(nb);
+    // a dependent launch of the tile pass, inside a graph or not: it orders itself with pdl_wait
+    launch_pdl(true, split == 8 ? k_mv_tiles_finalize<8> : (split == 4 ? k_mv_tiles_finalize<4> : k_mv_tiles_finalize<1>),
+               mv_finalize_ctas(), 32 * kFinalizeWarps, st, mt, ts.partial.p, d_diag.p, lambda, x, y, xy, ctl);
     check_launch();
   }
   // The tile pass of the product alone: the per-(segment, parameter) partials.

@@ -257,61 +257,75 @@ __global__ void __launch_bounds__(mv_tile_obs<R>(), sizeof(T) == sizeof(R) ? 4 :
   }
 }
 
-// y_b = sum of block b's partials (its segments in tile order) + lambda diag_b x_b: one warp per
-// block; lane l sums segments l, l + 32, ... of the block's contiguous region in order, then a
-// fixed shuffle tree. A block no observation touches has an empty region: y_b = lambda diag_b x_b.
-// With xy non-null, xy[CTA] = sum over the CTA's blocks, in block order, of x_b . y_b (the PCG
-// curvature terms). With ctl the damping is the control block's.
-__global__ void __launch_bounds__(256) k_mv_tiles_finalize(MvTiles mt, const double* __restrict__ partial,
-                                                           const double* __restrict__ diag, double lambda,
-                                                           const double* __restrict__ x, double* __restrict__ y,
-                                                           double* __restrict__ xy, const PcgCtl* ctl) {
-  __shared__ double s_dot[8];
+// y_b = sum of block b's partials (its segments in tile order) + lambda diag_b x_b: SPLIT warps per
+// block; lane l of warp w sums segments 32 w + l, 32 (SPLIT + w) + l, ... of the block's contiguous region
+// in order, then a fixed shuffle tree and the warps in order. A block no observation touches has an
+// empty region: y_b = lambda diag_b x_b. With xy non-null, xy[CTA] = sum over the CTA's blocks, in block
+// order, of x_b . y_b (the PCG curvature terms). With ctl the damping is the control block's.
+// Bound: latency of a block's own run of loads. SPLIT: few blocks mean long regions and idle SMs, many
+// blocks fill the chip with a warp each: at 31 blocks one warp each took 7.8 us, eight take 4.9; above
+// 1,184 blocks (eight warps an SM) there is nothing left to fill.
+constexpr int kFinalizeWarps = 8;
+inline int finalize_split(int nblocks) { return nblocks <= 296 ? 8 : (nblocks <= 1184 ? 4 : 1); }
+template <int SPLIT>
+__global__ void __launch_bounds__(32 * kFinalizeWarps) k_mv_tiles_finalize(MvTiles mt, const double* __restrict__ partial,
+                                                                           const double* __restrict__ diag,
+                                                                           double lambda, const double* __restrict__ x,
+                                                                           double* __restrict__ y,
+                                                                           double* __restrict__ xy, const PcgCtl* ctl) {
+  constexpr int BLOCKS = kFinalizeWarps / SPLIT;
+  __shared__ double s_part[kFinalizeWarps][6];
+  __shared__ double s_dot[BLOCKS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.x * 8 + warp;
+  const int b = blockIdx.x * BLOCKS + warp / SPLIT;
   // the block's layout and diagonal are constant during the PCG loop: loaded before the wait
   const bool have = b < mt.nblocks;
   const int o = have ? mt.blk_off[b] : 0, d = have ? mt.blk_dim[b] : 0;
   const uint32_t a0 = have ? mt.blk_part[b] : 0u, a1 = have ? mt.blk_part[b + 1] : 0u;
-  double dg[6];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) dg[c] = lane == 0 && c < d ? diag[o + c] : 0.0;
+  const double dg = lane < d ? diag[o + lane] : 0.0;
   pdl_trigger();
   pdl_wait();
   if (pcg_stopped(ctl)) return;
   if (ctl) lambda = ctl->lambda;
-  double dot = 0.0;
+  const double xv = lane < d ? x[o + lane] : 0.0;
   if (have) {
-    double xv[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) xv[c] = lane == 0 && c < d ? x[o + c] : 0.0;
     const uint32_t nseg = d > 0 ? (a1 - a0) / (uint32_t)d : 0u;
     double acc[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll 4
-    for (uint32_t j = lane; j < nseg; j += 32) {
+    for (uint32_t j = 32u * (warp % SPLIT) + lane; j < nseg; j += 32u * SPLIT) {
       const double* pp = partial + a0 + (size_t)j * d;
 #pragma unroll
       for (int c = 0; c < 6; ++c)
         if (c < d) acc[c] += pp[c];
     }
 #pragma unroll
-    for (int c = 0; c < 6; ++c) acc[c] = warp_sum(acc[c]);  // full sums land in lane 0
-    if (lane == 0) {
-#pragma unroll
-      for (int c = 0; c < 6; ++c)
-        if (c < d) {
-          const double v = acc[c] + lambda * dg[c] * xv[c];
-          y[o + c] = v;
-          dot += xv[c] * v;
-        }
+    for (int c = 0; c < 6; ++c) {
+      acc[c] = warp_sum(acc[c]);  // full sums land in lane 0
+      if (lane == 0) s_part[warp][c] = acc[c];
     }
   }
+  if (SPLIT > 1)
+    __syncthreads();
+  else
+    __syncwarp();
+  if (warp % SPLIT == 0) {
+    double dot = 0.0;
+    if (lane < d) {
+      double v = 0.0;
+#pragma unroll
+      for (int s = 0; s < SPLIT; ++s) v += s_part[warp + s][lane];
+      v += lambda * dg * xv;
+      y[o + lane] = v;
+      dot = xv * v;
+    }
+    dot = warp_sum(dot);
+    if (lane == 0) s_dot[warp / SPLIT] = dot;
+  }
   if (xy) {
-    if (lane == 0) s_dot[warp] = dot;
     __syncthreads();
     if (threadIdx.x == 0) {
       double t = 0.0;
-      for (int w = 0; w < 8; ++w) t += s_dot[w];
+      for (int w = 0; w < BLOCKS; ++w) t += s_dot[w];
       xy[blockIdx.x] = t;
     }
   }
