@@ -1484,46 +1484,16 @@ __global__ void k_retract(DevView v, int ng, const double* step, Gauge g, const 
   }
 }
 
-// Admitted track cost (schur/point.rs:705-728): returns false when a projection fails or the
-// geometry is not admitted.
-__device__ __noinline__ bool admitted_cost(const DevView& v, const double* pose, const double* groups, const double X[3], int p,
-                              const LossDev& loss, double scene, int admission, double* cost) {
-  TrackGeometryDev geo;
-  geo.init(scene);
-  double total = 0.0;
-  for (uint32_t o = v.pt_off[p]; o < v.pt_off[p + 1]; ++o) {
-    int cam = v.obs_cam[o];
-    const double* P = pose + 12 * cam;
-    double xc[3];
-    for (int i = 0; i < 3; ++i) xc[i] = P[3 * i] * X[0] + P[3 * i + 1] * X[1] + P[3 * i + 2] * X[2] + P[9 + i];
-    double r[2], J[2][3], Ji[2][3];
-    if (!project_obs(v, groups, o, xc, r, J, Ji)) return false;
-    // rotate_transposed(R, camera point)
-    double off[3];
-    for (int j = 0; j < 3; ++j) off[j] = P[j] * xc[0] + P[3 + j] * xc[1] + P[6 + j] * xc[2];
-    geo.push(off[0], off[1], off[2]);
-    total += loss.cost(sqrt(r[0] * r[0] + r[1] * r[1]));
-  }
-  bool ok = admission == 0 ? true : (admission == 1 ? !geo.collapsed() : !geo.degenerate());
-  if (!ok) return false;
-  *cost = total;
-  return true;
-}
-
-struct CandidateOut {
-  double cost, step_sq, damping, failed;
-};
-
 // Back-substitution, the candidate points and their cost, one CTA per record tile (whole points), one
 // thread per observation: the observation's share of the back-substitution from the coalesced record;
 // then a thread per point sums its track in order, forms the step and the moved point; then every
 // observation projects its moved point with the candidate cameras, and the point's thread admits the
-// track and sums its cost in track order. A point whose move is not admitted (rare) tries the unmoved
-// point by itself, observation after observation.
+// track and sums its cost in track order. A tile with points whose move is not admitted goes through
+// the remaining tries of the candidate rule the same way.
 // Bound: HBM on the records at survey sizes, latency below. A thread per point that walked its track for
 // both passes read the records in separate lines and left the projections of a track (33 distortion
-// samples each with k3) in one chain: 78 -> 39 us for 8,000 observations in 20 cameras, 206 -> 149 us for
-// 1.2M, 1.49 -> 1.52 ms for 12M (FP32 records).
+// samples each with k3) in one chain: 78 -> 28 us for 8,000 observations in 20 cameras, 206 -> 158 us for
+// 1.2M, 1.49 -> 1.53 ms for 12M (FP32 records).
 template <typename T>
 __global__ void __launch_bounds__(mv_tile_obs<T>(), sizeof(T) == 4 ? 3 : 6)
     k_candidate_tiles(const __grid_constant__ DevView v, LinOut<T> lin, const double* __restrict__ step, DevState cur,
@@ -1597,42 +1567,67 @@ __global__ void __launch_bounds__(mv_tile_obs<T>(), sizeof(T) == 4 ? 3 : 6)
     }
     for (int c = 0; c < 3; ++c) moved_x[c][tid] = st[c];
   }
-  __syncthreads();
-  if (obs) {
-    const uint32_t lp = lpt[tid];
+  // candidate_rule (point_geometry.rs:110-130), admitting tracks as schur/point.rs:705-728: the moved point
+  // off degenerate geometry (a fixed point: any), else the unmoved point if it does not collapse; where it
+  // does under the current cameras too, the unmoved point in any geometry. A try is a pass over the tile:
+  // its observations project their points in parallel, then each point that is still undecided
+  // walks its track's rays and costs in order. Tries after the first run only in tiles that need them.
+  enum { kMoved, kUnmoved, kCurrent, kAny, kDone };
+  const uint32_t lp = obs ? lpt[tid] : 0;
+  auto project = [&](const DevState& at) {  // this observation of its point's current try
     const double x[3] = {moved_x[0][lp], moved_x[1][lp], moved_x[2][lp]};
-    const double* P = cand.pose + 12 * cam;
+    const double* P = at.pose + 12 * cam;
     double xc[3], r[2], J[2][3], Ji[2][3];
     for (int i = 0; i < 3; ++i) xc[i] = P[3 * i] * x[0] + P[3 * i + 1] * x[1] + P[3 * i + 2] * x[2] + P[9 + i];
-    const bool ok = project_obs(v, cand.groups, o, xc, r, J, Ji);
+    const bool ok = project_obs(v, at.groups, o, xc, r, J, Ji);
     okf[tid] = ok ? 1 : 0;
     if (ok) {
       for (int j = 0; j < 3; ++j) term[j][tid] = P[j] * xc[0] + P[3 + j] * xc[1] + P[6 + j] * xc[2];
       term[3][tid] = loss.cost(sqrt(r[0] * r[0] + r[1] * r[1]));
     }
-  }
+  };
+  auto walk = [&](int admission, double* total) {  // 0: any geometry, 1: not collapsed, 2: not degenerate
+    TrackGeometryDev geo;
+    geo.init(fixed ? 0.0 : g.scene);
+    double sum = 0.0;
+    for (uint32_t i = a; i < b; ++i) {
+      if (!okf[i]) return false;
+      geo.push(term[0][i], term[1][i], term[2][i]);
+      sum += term[3][i];
+    }
+    *total = sum;
+    return admission == 0 ? true : (admission == 1 ? !geo.collapsed() : !geo.degenerate());
+  };
   __syncthreads();
-  if (!point) return;
-  // admitted_cost of the first attempt: a free point must stay off degenerate geometry
-  TrackGeometryDev geo;
-  geo.init(fixed ? 0.0 : g.scene);
+  if (obs) project(cand);
+  __syncthreads();
   double c = 0.0;
-  bool have = true;
-  for (uint32_t i = a; i < b && have; ++i) {
-    have = okf[i] != 0;
-    if (!have) break;
-    geo.push(term[0][i], term[1][i], term[2][i]);
-    c += term[3][i];
+  bool have = point && walk(fixed ? 0 : 2, &c);
+  const bool moved = have && !fixed;
+  int stage = point && !have && !fixed ? kUnmoved : kDone;
+  if (__syncthreads_or(stage != kDone)) {
+    if (stage != kDone)
+      for (int k = 0; k < 3; ++k) moved_x[k][tid] = X[k];
+    for (int t0 = kUnmoved; t0 < kDone; ++t0) {
+      if (point) okf[tid] = stage == t0 ? 1 : 0;  // the points that take this try
+      if (!__syncthreads_or(stage == t0)) continue;
+      const bool want = obs && okf[lp] != 0;
+      __syncthreads();
+      if (want) project(t0 == kCurrent ? cur : cand);
+      __syncthreads();
+      if (stage == t0) {
+        const bool ok = walk(t0 == kAny ? 0 : 1, &c);
+        if (t0 == kCurrent) {
+          stage = ok ? kDone : kAny;  // collapsed only under the candidate cameras: the candidate fails
+        } else {
+          have = ok;
+          stage = ok || t0 == kAny ? kDone : kCurrent;
+        }
+      }
+      __syncthreads();  // the try's flags and terms are read
+    }
   }
-  have = have && (fixed || !geo.degenerate());
-  bool moved = have && !fixed;
-  if (!have && !fixed) {  // candidate_rule (point_geometry.rs:110-130): the unmoved point
-    double c2;
-    if (admitted_cost(v, cand.pose, cand.groups, X, p, loss, g.scene, 1, &c))
-      have = true;
-    else if (!admitted_cost(v, cur.pose, cur.groups, X, p, loss, g.scene, 1, &c2))
-      have = admitted_cost(v, cand.pose, cand.groups, X, p, loss, g.scene, 0, &c);
-  }
+  if (!point) return;
   RedVec<4> res;
   res.v[0] = res.v[1] = res.v[2] = res.v[3] = 0.0;
   if (fixed || have)
