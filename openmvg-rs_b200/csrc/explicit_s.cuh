@@ -956,145 +956,169 @@ __global__ void k_z_marginals(TileBand Z, int ngroups, const int* __restrict__ p
     }
 }
 
+// ---- loops over S inside one cluster -------------------------------------------------------------
+// One cluster of kLoopCtas CTAs runs a whole iteration (power iteration, PCG), so the host waits once and
+// no launch lies between two products. CTA r owns the block rows X = r mod kLoopCtas; a task is 32 blocks
+// of one row, a block per lane. Every CTA keeps the whole iterate in shared memory; a row's results go to
+// all CTAs' shared memory and one cluster barrier ends the product. While a CTA's tasks fit (kLoopTasks,
+// a warp each) their blocks stay in shared memory too, element by element with the lanes side by side: the
+// cluster barrier drops L1, so each iteration would otherwise wait for L2 three times over.
+constexpr int kLoopCtas = 8;
+constexpr int kLoopThreads = 512;
+constexpr int kLoopWarps = kLoopThreads / 32;
+constexpr int kLoopTasks = kLoopWarps;
+constexpr size_t kLoopTaskDoubles = 36 * 32;
+
+struct LoopTasks {
+  int row[kLoopTasks], off[kLoopTasks][32];  // row; per lane first parameter << 3 | dimension
+  int count;                                 // above kLoopTasks: not cached
+  double part[kLoopWarps][6];
+};
+inline int loop_row_tasks(uint32_t blocks) { return (int)((blocks + 31) / 32); }
+
+// The CTA's tasks in row order (thread 0, before a barrier).
+__device__ __forceinline__ void loop_list(const RowTables& rt, int rank, LoopTasks& t) {
+  int nt = 0;
+  for (int X = rank; X < rt.nblocks; X += kLoopCtas) {
+    const int m = (int)(rt.nbr_begin[X + 1] - rt.nbr_begin[X] + 31) / 32;
+    for (int q = 0; q < m && nt + q < kLoopTasks; ++q) t.row[nt + q] = X;
+    nt += m;
+    if (nt > kLoopTasks) break;
+  }
+  t.count = nt;
+}
+// Their blocks into `cache`, columns times scale when it is given (all warps).
+__device__ __forceinline__ void loop_load(const RowTables& rt, const double* __restrict__ rows,
+                                          const double* __restrict__ scale, LoopTasks& t, double* cache) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w >= t.count) return;
+  const int X = t.row[w], dX = rt.blk_dim[X];
+  int first = w;
+  while (first > 0 && t.row[first - 1] == X) --first;
+  const uint32_t q = rt.nbr_begin[X] + 32 * (w - first) + lane;
+  const bool have = q < rt.nbr_begin[X + 1];
+  const int Y = have ? rt.nbr[q] : 0, dY = have ? rt.blk_dim[Y] : 0, oY = have ? rt.blk_off[Y] : 0;
+  t.off[w][lane] = oY << 3 | dY;
+  const double* S = rows + (have ? rt.slot_off[q] : 0);
+#pragma unroll
+  for (int m = 0; m < 6; ++m)
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+      cache[w * kLoopTaskDoubles + (6 * m + c) * 32 + lane] =
+          m < dX && c < dY ? S[m * dY + c] * (scale ? scale[oY + c] : 1.0) : 0.0;
+}
+// The cached tasks' products with v (shared memory) into t.part, a barrier, then put(X, m, sum) by the
+// warp of a row's first task: element e = lane, lane + 32, ... of dX x kLoopCtas, m = e / kLoopCtas, for
+// CTA e % kLoopCtas.
+template <typename F>
+__device__ __forceinline__ void loop_product(const RowTables& rt, LoopTasks& t, const double* cache, const double* v,
+                                             F put) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w < t.count) {
+    const double* C = cache + w * kLoopTaskDoubles + lane;
+    const int at = t.off[w][lane], dY = at & 7;
+    double xv[6], acc[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) xv[c] = c < dY ? v[(at >> 3) + c] : 0.0;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      acc[m] = 0.0;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) acc[m] += C[(6 * m + c) * 32] * xv[c];
+    }
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      acc[m] = warp_sum(acc[m]);
+      if (lane == 0) t.part[w][m] = acc[m];
+    }
+  }
+  __syncthreads();
+  if (w < t.count && (w == 0 || t.row[w - 1] != t.row[w])) {
+    const int X = t.row[w], dX = rt.blk_dim[X];
+    int count = 1;
+    while (w + count < t.count && t.row[w + count] == X) ++count;
+    for (int e = lane; e < dX * kLoopCtas; e += 32) {
+      const int m = e / kLoopCtas;
+      double r = 0.0;
+      for (int q = 0; q < count; ++q) r += t.part[w + q][m];
+      put(rt.blk_off[X] + m, e % kLoopCtas, r);
+    }
+  }
+}
+// The CTA-wide sum of v in a fixed order, the same value in every thread; red: kLoopWarps doubles that no
+// thread still reads.
+__device__ __forceinline__ double loop_sum(double v, double* red) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = 0.0;
+#pragma unroll
+  for (int q = 0; q < kLoopWarps; ++q) s += red[q];
+  return s;
+}
+
 // Largest |eigenvalue| of the equilibrated D S D by power iteration (Rayleigh quotient of the
 // normalized iterate): out[0] = lambda, out[1] = 1 when it settled (|rq - lambda| <= 1e-10 |rq| after
-// the 8th iteration) or ran its 200 iterations with finite values, 0 otherwise. n <= kPowerMax.
-//
-// One cluster of kPowerCtas CTAs runs every iteration, so the host waits once. CTA r owns the block rows
-// X = r mod kPowerCtas; a task is 32 blocks of one row, a block per lane. Every CTA keeps the whole
-// iterate in shared memory, not normalized (the products are scaled by the last norm); a row's results go
-// to all CTAs' shared memory, one cluster barrier ends the product, and every CTA forms the same norm
-// and quotient in the same order, so all leave the loop together. While the CTA's tasks fit (kPowerTasks)
-// their blocks stay in shared memory too, element by element with the lanes side by side: the cluster
-// barrier drops L1, so each iteration would otherwise wait for L2 three times over.
+// the 8th iteration) or ran its 200 iterations with finite values, 0 otherwise. n <= kPowerMax. The iterate
+// is not normalized (the products are scaled by the last norm); every CTA forms the same norm and
+// quotient in the same order, so all leave the loop together.
 // Bound: 200 dependent iterations of a barrier and a reduction. One CTA that kept the iterate in global
 // memory took 1.80 ms at n = 113, the cluster without the blocks in shared memory 1.04 ms, this 0.56 ms.
-constexpr int kPowerCtas = 8;
 constexpr int kPowerMax = 2048;
-constexpr int kPowerThreads = 512;
-constexpr int kPowerWarps = kPowerThreads / 32;
-constexpr int kPowerTasks = 16;                             // cached tasks of a CTA
-constexpr size_t kPowerTaskDoubles = 36 * 32;
-constexpr size_t power_smem(int n) { return sizeof(double) * (3 * (size_t)n + kPowerTasks * kPowerTaskDoubles); }
-__global__ void __launch_bounds__(kPowerThreads) k_power_iteration(RowTables rt, const double* __restrict__ rows,
-                                                                   const double* __restrict__ scale, int n, double* out) {
+constexpr size_t power_smem(int n) { return sizeof(double) * (3 * (size_t)n + kLoopTasks * kLoopTaskDoubles); }
+__global__ void __launch_bounds__(kLoopThreads) k_power_iteration(RowTables rt, const double* __restrict__ rows,
+                                                                  const double* __restrict__ scale, int n, double* out) {
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) double sh[];  // three iterates in turn, then the cached tasks
-  __shared__ double red[kPowerWarps][2], s_part[kPowerWarps][6];
-  __shared__ int t_row[kPowerTasks], t_off[kPowerTasks][32];  // cached tasks: row; per lane offset << 3 | dim
-  __shared__ int s_tasks;
+  __shared__ double red[2][kLoopWarps];
+  __shared__ LoopTasks t;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* cache = sh + 3 * (size_t)n;
-  if (tid == 0) {  // the CTA's tasks, row after row
-    int nt = 0;
-    for (int X = rank; X < rt.nblocks && nt <= kPowerTasks; X += kPowerCtas) {
-      const int m = (int)(rt.nbr_begin[X + 1] - rt.nbr_begin[X] + 31) / 32;
-      for (int q = 0; q < m && nt < kPowerTasks; ++q) t_row[nt + q] = X;
-      nt += m;
-      if (nt > kPowerTasks) break;
-    }
-    s_tasks = nt;
-  }
+  if (tid == 0) loop_list(rt, rank, t);
   const double v0 = 1.0 / sqrt((double)n);
-  for (int i = tid; i < n; i += kPowerThreads) sh[i] = v0;
+  for (int i = tid; i < n; i += kLoopThreads) sh[i] = v0;
   __syncthreads();
-  const bool cached = s_tasks <= kPowerTasks;
-  const int tasks = s_tasks;
-  if (cached)
-    for (int t = warp; t < tasks; t += kPowerWarps) {
-      const int X = t_row[t], dX = rt.blk_dim[X];
-      int first = t;
-      while (first > 0 && t_row[first - 1] == X) --first;
-      const uint32_t q = rt.nbr_begin[X] + 32 * (t - first) + lane;
-      const bool have = q < rt.nbr_begin[X + 1];
-      const int Y = have ? rt.nbr[q] : 0, dY = have ? rt.blk_dim[Y] : 0, oY = have ? rt.blk_off[Y] : 0;
-      t_off[t][lane] = oY << 3 | dY;
-      const double* S = rows + (have ? rt.slot_off[q] : 0);
-#pragma unroll
-      for (int m = 0; m < 6; ++m)
-#pragma unroll
-        for (int c = 0; c < 6; ++c)
-          cache[t * kPowerTaskDoubles + (6 * m + c) * 32 + lane] = m < dX && c < dY ? S[m * dY + c] * scale[oY + c] : 0.0;
-    }
+  const bool cached = t.count <= kLoopTasks;
+  if (cached) loop_load(rt, rows, scale, t, cache);
   cluster.sync();  // every CTA runs before any of them is written to; the cache is in place
   double lam = 0.0, inv = 1.0;
   int ok = 0;
   for (int it = 0; it < 200; ++it) {
     const double* v = sh + (it % 3) * (size_t)n;  // times inv: the normalized iterate
     double* w = sh + ((it + 1) % 3) * (size_t)n;
-    auto publish = [&](int X, int first, int count) {  // rows of s_part [first, first + count) to every CTA
-      const int dX = rt.blk_dim[X], oX = rt.blk_off[X];
-      for (int e = lane; e < dX * kPowerCtas; e += 32) {
-        const int m = e / kPowerCtas;
-        double r = 0.0;
-        for (int q = 0; q < count; ++q) r += s_part[first + q][m];
-        *cluster.map_shared_rank(w + oX + m, e % kPowerCtas) = r * inv * scale[oX + m];
-      }
-    };
     if (cached) {
-      if (warp < tasks) {
-        const double* C = cache + warp * kPowerTaskDoubles + lane;
-        const int at = t_off[warp][lane], dY = at & 7;
-        double xv[6], acc[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) xv[c] = c < dY ? v[(at >> 3) + c] : 0.0;
-#pragma unroll
-        for (int m = 0; m < 6; ++m) {
-          acc[m] = 0.0;
-#pragma unroll
-          for (int c = 0; c < 6; ++c) acc[m] += C[(6 * m + c) * 32] * xv[c];
-        }
-#pragma unroll
-        for (int m = 0; m < 6; ++m) {
-          acc[m] = warp_sum(acc[m]);
-          if (lane == 0) s_part[warp][m] = acc[m];
-        }
-      }
-      __syncthreads();
-      if (warp < tasks && (warp == 0 || t_row[warp - 1] != t_row[warp])) {
-        int count = 1;
-        while (warp + count < tasks && t_row[warp + count] == t_row[warp]) ++count;
-        publish(t_row[warp], warp, count);
-      }
+      loop_product(rt, t, cache, v, [&](int i, int cta, double r) { *cluster.map_shared_rank(w + i, cta) = r * inv * scale[i]; });
     } else {
-      for (int x0 = 0; x0 * kPowerCtas + rank < rt.nblocks; x0 += kPowerWarps / 2) {  // two warps a row
-        const int X = (x0 + warp / 2) * kPowerCtas + rank;
+      for (int x0 = 0; x0 * kLoopCtas + rank < rt.nblocks; x0 += kLoopWarps / 2) {  // two warps a row
+        const int X = (x0 + warp / 2) * kLoopCtas + rank;
         const bool have = X < rt.nblocks;
+        const int dX = have ? rt.blk_dim[X] : 0;
         if (have) {
           double acc[6] = {0, 0, 0, 0, 0, 0};
-          row_times(rt, rows, X, rt.blk_dim[X], 32u * (warp % 2) + lane, 64u, [&](int i) { return scale[i] * v[i]; }, acc);
+          row_times(rt, rows, X, dX, 32u * (warp % 2) + lane, 64u, [&](int i) { return scale[i] * v[i]; }, acc);
 #pragma unroll
           for (int m = 0; m < 6; ++m) {
             acc[m] = warp_sum(acc[m]);
-            if (lane == 0) s_part[warp][m] = acc[m];
+            if (lane == 0) t.part[warp][m] = acc[m];
           }
         }
         __syncthreads();
-        if (have && warp % 2 == 0) publish(X, warp, 2);
+        if (have && warp % 2 == 0)
+          for (int e = lane; e < dX * kLoopCtas; e += 32) {
+            const int m = e / kLoopCtas, o = rt.blk_off[X] + m;
+            *cluster.map_shared_rank(w + o, e % kLoopCtas) = (t.part[warp][m] + t.part[warp + 1][m]) * inv * scale[o];
+          }
         __syncthreads();
       }
     }
     cluster.sync();
     double nn = 0.0, rq = 0.0;
-    for (int i = tid; i < n; i += kPowerThreads) {
+    for (int i = tid; i < n; i += kLoopThreads) {
       nn += w[i] * w[i];
       rq += v[i] * w[i];
     }
-    nn = warp_sum(nn);
-    rq = warp_sum(rq);
-    if (lane == 0) {
-      red[warp][0] = nn;
-      red[warp][1] = rq;
-    }
-    __syncthreads();
-    nn = rq = 0.0;
-#pragma unroll
-    for (int q = 0; q < kPowerWarps; ++q) {  // the same sums in every thread of every CTA
-      nn += red[q][0];
-      rq += red[q][1];
-    }
-    const double nrm = sqrt(nn), quot = rq * inv;
+    const double nrm = sqrt(loop_sum(nn, red[0])), quot = loop_sum(rq, red[1]) * inv;
     if (!(isfinite(nrm) && nrm > 0.0)) {
       ok = 0;
       break;
@@ -1109,6 +1133,163 @@ __global__ void __launch_bounds__(kPowerThreads) k_power_iteration(RowTables rt,
   if (rank == 0 && tid == 0) {
     out[0] = lam;
     out[1] = ok;
+  }
+}
+
+// The whole PCG run of a small system (sparse/pcg.rs:23-119) for (S + lambda diag) x = -g with x0 = 0: n
+// at most kLoopThreads and every CTA's tasks cached, so thread i of every CTA keeps x_i, r_i and row i of
+// the inverse of its preconditioner block, the products go over the cluster, and every CTA forms the same
+// scalars in the same order. When the recursive residual meets the tolerance it is confirmed by the true
+// residual g + S x, and the iteration starts over from it where it is not. fail: the preconditioner's
+// per-block flags; any of them ends the run without a step.
+// Bound: a cluster barrier, six CTA barriers and their reductions per iteration. A solve of 12 runs of about
+// 27 iterations each at n = 185 (32 spherical cameras) went from 15.2 to 10.1 ms; the four kernels of a
+// graph iteration take 19 us.
+struct LoopPcgResult {
+  int accepted, exhausted, terms, pad;
+  double rel;
+};
+constexpr size_t pcg_loop_smem(int n) { return sizeof(double) * (4 * (size_t)n + kLoopTasks * kLoopTaskDoubles); }
+__global__ void __launch_bounds__(kLoopThreads) k_pcg_loop(RowTables rt, const double* __restrict__ rows,
+                                                           const double* __restrict__ diag, double lambda,
+                                                           const double* __restrict__ factor, const int* __restrict__ fail,
+                                                           const double* __restrict__ g, int n, int max_it, double tol,
+                                                           double* __restrict__ x_out, LoopPcgResult* out) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) double sh[];  // the product's vector, r, the product in two buffers, the tasks
+  __shared__ double red[4][kLoopWarps];
+  __shared__ LoopTasks t;
+  __shared__ int s_block[kLoopThreads];  // element's block
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), tid = threadIdx.x;
+  double *vec = sh, *rs = sh + n, *qbuf = sh + 2 * (size_t)n, *cache = sh + 4 * (size_t)n;
+  if (tid == 0) loop_list(rt, rank, t);
+  int bad = 0;
+  for (int b = tid; b < rt.nblocks; b += kLoopThreads) {
+    bad |= fail[b];
+    for (int k = 0; k < rt.blk_dim[b]; ++k) s_block[rt.blk_off[b] + k] = b;
+  }
+  bad = __syncthreads_or(bad);
+  loop_load(rt, rows, nullptr, t, cache);
+  const bool live = tid < n;
+  const int blk = live ? s_block[tid] : 0, base = live ? rt.blk_off[blk] : 0, dim = live ? rt.blk_dim[blk] : 0;
+  const double dg = live ? lambda * diag[tid] : 0.0, b = live ? -g[tid] : 0.0;
+  double inv[6] = {0, 0, 0, 0, 0, 0};  // row of the inverse of the block (factor F and scales): F F^T scaled
+  if (live && !bad) {
+    const double* F = factor + 42 * (size_t)blk;
+    const int me = tid - base;
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+      if (i < dim) {
+        double v = i == me ? 1.0 / F[36 + i] : 0.0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+          if (k < i) v -= F[6 * i + k] * inv[k];
+        inv[i] = v / F[6 * i + i];
+      }
+#pragma unroll
+    for (int i = 5; i >= 0; --i)
+      if (i < dim) {
+        double v = inv[i];
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+          if (k > i && k < dim) v -= F[6 * k + i] * inv[k];
+        inv[i] = v / F[6 * i + i];
+      }
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+      if (i < dim) inv[i] /= F[36 + i];
+  }
+  int parity = 0;
+  auto product = [&](double mine) {  // (S + lambda diag) vec, this thread's element; mine = vec[tid]
+    double* q = qbuf + parity * (size_t)n;
+    parity ^= 1;
+    loop_product(rt, t, cache, vec, [&](int i, int cta, double r) { *cluster.map_shared_rank(q + i, cta) = r; });
+    cluster.sync();
+    return live ? q[tid] + dg * mine : 0.0;
+  };
+  auto precond = [&]() {  // row tid of the preconditioner times rs (visible to the CTA)
+    double z = 0.0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      if (k < dim) z += inv[k] * rs[base + k];
+    return z;
+  };
+  cluster.sync();  // every CTA runs before any of them is written to; the cache is in place
+  LoopPcgResult res{0, 0, 0, 0, NAN};
+  double x = 0.0, r = b;
+  if (live) rs[tid] = r;
+  const double n0 = sqrt(loop_sum(r * r, red[0]));  // its barrier makes rs visible
+  double z = precond();
+  double rho = loop_sum(r * z, red[1]);
+  if (bad || !isfinite(n0)) {
+    // no step
+  } else if (n0 == 0.0) {
+    res.accepted = 1;
+    res.rel = 0.0;
+  } else if (isfinite(rho) && rho > 0.0 && max_it > 0) {
+    double d = z;
+    for (;;) {  // one iteration, all threads of all CTAs together
+      if (live) vec[tid] = d;
+      __syncthreads();
+      const double q = product(d);
+      const double curv = loop_sum(d * q, red[0]);
+      if (!(isfinite(curv) && curv > 0.0)) break;
+      const double alpha = rho / curv;
+      if (!isfinite(alpha)) break;
+      x += alpha * d;
+      r -= alpha * q;
+      if (live) rs[tid] = r;
+      const double rr = loop_sum(r * r, red[1]);
+      z = precond();
+      const double rz = loop_sum(r * z, red[2]);
+      ++res.terms;
+      const double ratio = sqrt(rr) / n0;
+      if (!isfinite(ratio)) break;
+      bool over = res.terms >= max_it;
+      if (ratio <= tol) {  // confirm with the true residual
+        if (live) vec[tid] = x;
+        __syncthreads();
+        const double sx = product(x);  // every thread: the product holds barriers
+        r = live ? b - sx : 0.0;
+        if (live) rs[tid] = r;
+        const double tr = sqrt(loop_sum(r * r, red[3])) / n0;
+        if (!isfinite(tr)) break;
+        if (tr <= tol) {
+          res.accepted = 1;
+          res.rel = tr;
+          break;
+        }
+        z = precond();
+        rho = loop_sum(r * z, red[0]);
+        if (!(isfinite(rho) && rho > 0.0)) {
+          res.rel = tr;
+          break;
+        }
+        d = z;
+      } else {
+        if (!(isfinite(rz) && rz > 0.0)) break;
+        const double beta = rz / rho;
+        if (!isfinite(beta)) break;
+        d = z + beta * d;
+        rho = rz;
+      }
+      if (over) {  // the iteration limit: the residual the step is left with
+        if (live) vec[tid] = x;
+        __syncthreads();
+        const double sx = product(x);  // every thread: the product holds barriers
+        r = live ? b - sx : 0.0;
+        res.rel = sqrt(loop_sum(r * r, red[3])) / n0;
+        res.terms = max_it;
+        res.exhausted = 1;
+        break;
+      }
+    }
+  }
+  cluster.sync();  // no CTA leaves while another may still write to it
+  if (rank == 0) {
+    if (live) x_out[tid] = x;
+    if (tid == 0) *out = res;
   }
 }
 

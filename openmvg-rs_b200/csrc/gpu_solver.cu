@@ -2501,7 +2501,9 @@ struct Solver {
     direct = !opt.iterative;
     // the PCG operator: the explicit S by block rows (rebuilt every assembly, a block-sparse product
     // that stays in L2) or the matrix-free tile product over the Jacobian records
-    explicit_op = !direct && opt.matvec == 1;  // Auto starts matrix-free (see kExplicitSwitchTerms)
+    // (Auto starts matrix-free, see kExplicitSwitchTerms, except where a whole FP64 PCG run fits one cluster)
+    pcg_loop = fits_pcg_loop();
+    explicit_op = !direct && (opt.matvec == 1 || (opt.matvec == 0 && opt.precision == 0 && pcg_loop));
     const uint64_t bytes_before = tl_device_bytes;
     const double t1 = now();
     // mixed precision keeps only FP32 Jacobian records (and their tiles); FP64 mode only FP64 ones
@@ -2909,6 +2911,20 @@ struct Solver {
     OMVGBA_LAUNCH(k_block_records, nb, kAsmRec * kRecordShares, 0, st, mt, bt.blk_edge, d_asm_rec.p, d_blk_out.p);
   }
 
+  // Whether a PCG run on the explicit S fits one cluster (k_pcg_loop): a thread per parameter, a warp per
+  // cached task. 36 us for the rows and 2 us an iteration against 19 us an iteration of the graph's kernels.
+  bool pcg_loop = false;
+  bool fits_pcg_loop() const {
+    if (D == 0 || D > kLoopThreads) return false;
+    const int nblocks = (int)S.blk_off.size();
+    for (int r = 0; r < kLoopCtas; ++r) {
+      int tasks = 0;
+      for (int X = r; X < nblocks; X += kLoopCtas) tasks += loop_row_tasks(S.nbr_begin[X + 1] - S.nbr_begin[X]);
+      if (tasks > kLoopTasks) return false;
+    }
+    return true;
+  }
+
   // The camera-pair tables, once per solver; false when the pairs do not serve this problem: more
   // cameras than a neighbour bitmap holds, operands and lists past kPairMaxBytes, or past what the
   // caller's workspace budget leaves. Those build by block rows (k_block_rows), which needs no storage
@@ -3255,7 +3271,7 @@ struct Solver {
     CUDA_OK(copy_async(d_e.p, sc.data(), sizeof(double) * D, cudaMemcpyHostToDevice, st));
     CUDA_OK(cudaFuncSetAttribute(k_power_iteration, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)power_smem(kPowerMax)));
-    launch_cluster(k_power_iteration, kPowerCtas, kPowerThreads, power_smem(D), st, row_tables(), (const double*)d_rows.p,
+    launch_cluster(k_power_iteration, kLoopCtas, kLoopThreads, power_smem(D), st, row_tables(), (const double*)d_rows.p,
                    (const double*)d_e.p, D, d_power.p);
     check_launch();
     double out[2];
@@ -3388,7 +3404,8 @@ struct Solver {
     }
   }
 
-  bool factor_preconditioner(double lambda) {
+  // With check false the blocks' flags stay on the device (k_pcg_loop reads them).
+  bool factor_preconditioner(double lambda, bool check = true) {
     BlockTables bt = tables();
     PairTables xt = pairs();
     if (explicit_op) {
@@ -3404,6 +3421,7 @@ struct Solver {
       OMVGBA_LAUNCH(k_block_factor, grid_for(nb, 64), 64, 0, st, bt, d_blk_out.p, d_diag.p, lambda, d_xpair_out.p,
                     d_blk_cross_begin.p, d_blk_cross_end.p, d_factor.p, d_fail.p);
     check_launch();
+    if (!check) return true;
     std::vector<int> fail(std::max(nb, 1));
     if (nb > 0) CUDA_OK(copy_async(fail.data(), d_fail.p, sizeof(int) * nb, cudaMemcpyDeviceToHost, st));
     sync();
@@ -3616,6 +3634,26 @@ struct Solver {
   }
 
   PcgResult pcg(double lambda, uint64_t max_it, double tol) {
+    if (explicit_op && pcg_loop) {
+      CUDA_OK(cudaFuncSetAttribute(k_pcg_loop, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)pcg_loop_smem(kLoopThreads)));
+      static_assert(sizeof(LoopPcgResult) <= 16 * sizeof(double), "the result lies in d_scalars");
+      LoopPcgResult* dres = reinterpret_cast<LoopPcgResult*>(d_scalars.p);
+      launch_cluster(k_pcg_loop, kLoopCtas, kLoopThreads, pcg_loop_smem(D), st, row_tables(), (const double*)d_rows.p,
+                     (const double*)d_diag.p, lambda, (const double*)d_factor.p, (const int*)d_fail.p,
+                     (const double*)d_gred.p, D, (int)std::min<uint64_t>(max_it, (uint64_t)INT32_MAX), tol, d_step.p,
+                     dres);
+      check_launch();
+      LoopPcgResult r{};
+      CUDA_OK(copy_async(&r, dres, sizeof(r), cudaMemcpyDeviceToHost, st));
+      sync();
+      PcgResult res;
+      res.accepted = r.accepted != 0;
+      res.exhausted = r.exhausted != 0;
+      res.terms = (uint64_t)r.terms;
+      res.rel = r.rel;
+      return res;
+    }
     OMVGBA_LAUNCH(k_neg_copy, grid_for(D, 256), 256, 0, st, D, d_gred.p, d_rhs.p);
     check_launch();
     return pcg_run(d_rhs.p, d_step.p, lambda, max_it, tol, false, true);
@@ -3836,7 +3874,7 @@ struct Solver {
         if (direct) {
           if (D > 0) direct_step(lambda);  // its status comes with the candidate's results
         } else {
-          solved = factor_preconditioner(lambda);
+          solved = factor_preconditioner(lambda, !(explicit_op && pcg_loop));
           if (solved) {
             double tol = confirm ? std::min(opt.pcg_tolerance, iter_tol) : opt.pcg_tolerance;
             uint64_t limit = confirm ? opt.pcg_max_iterations : std::min<uint64_t>(opt.pcg_max_iterations, (uint64_t)D);
@@ -4498,7 +4536,7 @@ void resident_schur_product(Resident* r, double lambda, bool fp32, int stage, co
     s.restore_initial();
     double scene = s.scene_scale_host();
     Gauge g = s.gauge_for(s.cur, scene);
-    auto a = s.assemble(s.cur, g, s.opt.loss, lambda, false);
+    auto a = s.assemble(s.cur, g, s.opt.loss, lambda, s.explicit_op);  // the operator's rows, where it uses them
     if (!a.valid) throw SolveFailure{4, "linearization is not valid"};
     r->linearized = true;
     r->lambda = lambda;
