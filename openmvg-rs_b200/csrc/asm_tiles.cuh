@@ -153,13 +153,15 @@ __global__ void __launch_bounds__(mv_tile_obs<R>(), asm_min_blocks<R>())
 // Per block: the sum of its records in tile order, in the assembly record layout (kAsmRec): U lower
 // (21, packed as six rows), g (6), reduced g (6), damping diagonal (6: the diagonal of U), edge (18),
 // coupling lower (21); entries past the block's dimension are zero. One CTA per block, thread = (entry,
-// share of the records); a share takes every kRecordShares-th record and the shares are added in order.
+// share of the records); a share takes every kRecordShares-th record and the shares are added in order. The
+// block's vectors (g, reduced g, damping diagonal) go out with it.
 // Bound: HBM on the records at survey sizes, latency of an entry's run of loads below: one thread per entry
 // took 14.5 us for a window's 19 blocks and 36 us for 31, this 7.5 and 14 us; 77 us for 500 cameras either
 // way.
 constexpr int kRecordShares = 12;
 __global__ void __launch_bounds__(kAsmRec * kRecordShares) k_block_records(MvTiles mt, const int* __restrict__ blk_edge,
-                                                       const double* __restrict__ rec_in, double* __restrict__ blk_out) {
+                                                       const double* __restrict__ rec_in, double* __restrict__ blk_out,
+                                                       BlockVectors bv) {
   const int b = blockIdx.x;
   if (b >= mt.nblocks) return;
   const int d = mt.blk_dim[b];
@@ -199,11 +201,15 @@ __global__ void __launch_bounds__(kAsmRec * kRecordShares) k_block_records(MvTil
     }
     sh[share][k] = acc;
     __syncthreads();
-    if (share > 0) return;
-    acc = 0.0;
-    for (int s2 = 0; s2 < kRecordShares; ++s2) acc += sh[s2][k];
-    blk_out[(size_t)kAsmRec * b + k] = acc;
+    if (share == 0) {
+      acc = 0.0;
+      for (int s2 = 0; s2 < kRecordShares; ++s2) acc += sh[s2][k];
+      sh[0][k] = acc;  // the thread's own place: no other reads it before the barrier
+      blk_out[(size_t)kAsmRec * b + k] = acc;
+    }
   }
+  __syncthreads();
+  if (threadIdx.x == 0) block_vectors(bv, b, d, sh[0]);
 }
 
 }  // namespace omvgba

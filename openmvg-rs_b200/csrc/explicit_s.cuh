@@ -722,8 +722,9 @@ __global__ void __launch_bounds__(256) k_tile_update(TileBand tb, int k, int* st
   potrf_tile(tb, k + 1, Ta, Tb, status);
 }
 
-// Forward (L y = b) and backward (L^T x = y) substitution with the banded tiled factor, in place on the
-// permuted vector v (n entries; the padding is not touched), one cluster of up to kSolveCtas CTAs.
+// Forward (L y = -g) and backward (L^T x = y) substitution with the banded tiled factor, on the vector v in
+// the factor's order (n entries; the padding is not touched), gathered from g and scattered to step_out in
+// the parameters' order; one cluster of up to kSolveCtas CTAs.
 // Right-looking: CTA i mod size owns rows of tile i. In step k the owner of tile k multiplies its
 // finished part by the inverse of the diagonal tile (W_k, from the factorization), hands the 64
 // results to every CTA's shared memory, and after one cluster barrier each CTA subtracts the products
@@ -761,19 +762,25 @@ __device__ __forceinline__ void tile_times_t(const double* __restrict__ M, const
   }
   __syncthreads();
 }
-__global__ void __launch_bounds__(256) k_tile_solve(TileBand tb, double* v, const int* status) {
+__global__ void __launch_bounds__(256) k_tile_solve(TileBand tb, double* v, const int* status,
+                                                    const int* __restrict__ perm_to_orig, const double* __restrict__ g,
+                                                    double* __restrict__ step_out) {
   namespace cg = cooperative_groups;
   __shared__ double part[4 * kCT], u[kCT], y[kCT];
   __shared__ double step[2][kCT];  // the finished part of the step, from its owner
-  if (status[0] == 0) return;      // the same value in every CTA of the cluster
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), size = (int)cluster.num_blocks(), tid = threadIdx.x;
+  const bool factored = status[0] != 0;  // the same value in every CTA of the cluster
   auto load = [&](int tile) {
     if (tid < kCT) u[tid] = tile * kCT + tid < tb.n ? v[tile * kCT + tid] : 0.0;
     __syncthreads();
   };
-  auto publish = [&](int tile, int buf) {  // y: store it and hand it to every CTA
-    if (tid < kCT && tile * kCT + tid < tb.n) v[tile * kCT + tid] = y[tid];
+  auto publish = [&](int tile, int buf, bool last) {  // y: store it and hand it to every CTA
+    const int P = tile * kCT + tid;
+    if (tid < kCT && P < tb.n) {
+      v[P] = y[tid];
+      if (last) step_out[perm_to_orig[P]] = y[tid];
+    }
     for (int i = tid; i < size * kCT; i += 256) {
       double* dst = cluster.map_shared_rank(&step[buf][0], i / kCT);
       dst[i % kCT] = y[i % kCT];
@@ -783,13 +790,21 @@ __global__ void __launch_bounds__(256) k_tile_solve(TileBand tb, double* v, cons
     if (tid < kCT && tile * kCT + tid < tb.n) v[tile * kCT + tid] -= y[tid];
     __syncthreads();
   };
+  // the right-hand side -g in the factor's order, each CTA its own tiles
+  for (int tile = rank; tile < tb.nt; tile += size)
+    if (tid < kCT && tile * kCT + tid < tb.n) {
+      const int o = perm_to_orig[tile * kCT + tid];
+      v[tile * kCT + tid] = -g[o];
+      if (!factored) step_out[o] = -g[o];  // a step that the host refuses, but one of defined values
+    }
+  if (!factored) return;
   cluster.sync();  // every CTA runs before any of them is written to
   for (int k = 0; k < tb.nt; ++k) {
     const int buf = k & 1;
     if (k % size == rank) {
       load(k);
       tile_times(tb.w + (size_t)k * kCTT, u, part, y);
-      publish(k, buf);
+      publish(k, buf, false);
     }
     cluster.sync();
     const int last = min(tb.nt - 1, k + tb.bwt);
@@ -803,7 +818,7 @@ __global__ void __launch_bounds__(256) k_tile_solve(TileBand tb, double* v, cons
     if (k % size == rank) {
       load(k);
       tile_times_t(tb.w + (size_t)k * kCTT, u, y);
-      publish(k, buf);
+      publish(k, buf, true);
     }
     cluster.sync();
     const int first = max(0, k - tb.bwt);
@@ -813,18 +828,6 @@ __global__ void __launch_bounds__(256) k_tile_solve(TileBand tb, double* v, cons
     }
   }
   cluster.sync();  // no CTA leaves while another may still write to it
-}
-
-// Gather / scatter between the original and the permuted parameter order.
-__global__ void k_perm_gather(int n, const int* __restrict__ perm_to_orig, const double* __restrict__ src,
-                              double sign, double* __restrict__ dst) {
-  const int P = blockIdx.x * blockDim.x + threadIdx.x;
-  if (P < n) dst[P] = sign * src[perm_to_orig[P]];
-}
-__global__ void k_perm_scatter(int n, const int* __restrict__ perm_to_orig, const double* __restrict__ src,
-                               double* __restrict__ dst) {
-  const int P = blockIdx.x * blockDim.x + threadIdx.x;
-  if (P < n) dst[perm_to_orig[P]] = src[P];
 }
 
 // ---- selected inverse within the band (intrinsic marginal covariances) -----------------------

@@ -542,72 +542,98 @@ __device__ __forceinline__ double warp_min(double x) {
   return x;
 }
 
-// Reduce an array of PointSummary (one per point) into per-block partials; fixed order.
-__global__ void k_reduce_summary(const PointSummary* in, int n, PointSummary* out) {
-  __shared__ PointSummary sh[kReduceThreads / 32];
-  int tid = threadIdx.x;
-  PointSummary acc{0, 0, 0, 0, 1.0, 0, 0, 0};
-  for (int i = blockIdx.x * blockDim.x + tid; i < n; i += gridDim.x * blockDim.x) {
-    PointSummary s = in[i];
-    acc.cost += s.cost;
-    acc.sq += s.sq;
-    acc.point_red += s.point_red;
-    acc.grad_norm = fmax(acc.grad_norm, s.grad_norm);
-    acc.min_rcond = fmin(acc.min_rcond, s.min_rcond);
-    acc.invalid += s.invalid;
-    acc.weak += s.weak;
-  }
-  acc.cost = warp_sum(acc.cost);
-  acc.sq = warp_sum(acc.sq);
-  acc.point_red = warp_sum(acc.point_red);
-  acc.grad_norm = warp_max(acc.grad_norm);
-  acc.min_rcond = warp_min(acc.min_rcond);
-  acc.invalid = warp_sum(acc.invalid);
-  acc.weak = warp_sum(acc.weak);
-  if ((tid & 31) == 0) sh[tid >> 5] = acc;
+// Whether the calling CTA is the last of its grid to get here, all threads alike; its writes before the
+// call are visible to the last CTA. The counter starts at zero and is left there.
+__device__ __forceinline__ bool last_cta(unsigned* counter) {
+  __threadfence();
   __syncthreads();
-  if (tid == 0) {
-    PointSummary t = sh[0];
-    for (int w = 1; w < (int)(blockDim.x / 32); ++w) {
-      t.cost += sh[w].cost;
-      t.sq += sh[w].sq;
-      t.point_red += sh[w].point_red;
-      t.grad_norm = fmax(t.grad_norm, sh[w].grad_norm);
-      t.min_rcond = fmin(t.min_rcond, sh[w].min_rcond);
-      t.invalid += sh[w].invalid;
-      t.weak += sh[w].weak;
-    }
-    out[blockIdx.x] = t;
+  bool last = false;
+  if (threadIdx.x == 0) {
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    if (last) *counter = 0;
   }
+  last = __syncthreads_or(last);
+  if (last) __threadfence();
+  return last;
 }
 
-// Sum of NV-component records (e.g. dot products) with a fixed grid: per block partial, then the
-// final pass over partials in index order.
+__device__ __forceinline__ PointSummary combine(const PointSummary& a, const PointSummary& b) {
+  return {a.cost + b.cost, a.sq + b.sq, a.point_red + b.point_red, fmax(a.grad_norm, b.grad_norm),
+          fmin(a.min_rcond, b.min_rcond), a.invalid + b.invalid, a.weak + b.weak, 0.0};
+}
+__device__ __forceinline__ PointSummary warp_combine(PointSummary a) {
+  a.cost = warp_sum(a.cost);
+  a.sq = warp_sum(a.sq);
+  a.point_red = warp_sum(a.point_red);
+  a.grad_norm = warp_max(a.grad_norm);
+  a.min_rcond = warp_min(a.min_rcond);
+  a.invalid = warp_sum(a.invalid);
+  a.weak = warp_sum(a.weak);
+  return a;
+}
+// Reduction of an array of PointSummary (one per point) in a fixed order: per-CTA partials, which the
+// last CTA combines in index order.
+__global__ void __launch_bounds__(kReduceThreads) k_reduce_summary(const PointSummary* in, int n, PointSummary* part,
+                                                                   PointSummary* out, unsigned* counter) {
+  __shared__ PointSummary sh[kReduceThreads / 32];
+  const int tid = threadIdx.x;
+  auto cta = [&](PointSummary acc) {  // the CTA's total, valid in thread 0
+    acc = warp_combine(acc);
+    if ((tid & 31) == 0) sh[tid >> 5] = acc;
+    __syncthreads();
+    PointSummary t = sh[0];
+    for (int w = 1; w < kReduceThreads / 32; ++w) t = combine(t, sh[w]);
+    return t;
+  };
+  PointSummary acc{0, 0, 0, 0, 1.0, 0, 0, 0};
+  for (int i = blockIdx.x * blockDim.x + tid; i < n; i += gridDim.x * blockDim.x) acc = combine(acc, in[i]);
+  acc = cta(acc);
+  if (tid == 0) part[blockIdx.x] = acc;
+  if (!last_cta(counter)) return;
+  acc = {0, 0, 0, 0, 1.0, 0, 0, 0};
+  for (int i = tid; i < (int)gridDim.x; i += blockDim.x) {
+    PointSummary p;
+    for (int k = 0; k < 8; ++k) reinterpret_cast<double*>(&p)[k] = __ldcg(reinterpret_cast<const double*>(part + i) + k);
+    acc = combine(acc, p);
+  }
+  acc = cta(acc);
+  if (tid == 0) *out = acc;
+}
+
+// Sum of NV-component records with a fixed grid: per-CTA partials, which the last CTA adds in index order.
 template <int NV>
-__global__ void k_reduce_vec(const RedVec<NV>* in, int n, RedVec<NV>* out) {
+__global__ void __launch_bounds__(kReduceThreads) k_reduce_vec(const RedVec<NV>* in, int n, RedVec<NV>* part,
+                                                               RedVec<NV>* out, unsigned* counter) {
   __shared__ double sh[kReduceThreads / 32][NV];
-  int tid = threadIdx.x;
+  const int tid = threadIdx.x;
+  auto cta = [&](double acc[NV], RedVec<NV>* to) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) acc[k] = warp_sum(acc[k]);
+    if ((tid & 31) == 0)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) sh[tid >> 5][k] = acc[k];
+    __syncthreads();
+    if (tid == 0)
+      for (int k = 0; k < NV; ++k) {
+        double s = 0.0;
+        for (int w = 0; w < kReduceThreads / 32; ++w) s += sh[w][k];
+        to->v[k] = s;
+      }
+  };
   double acc[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) acc[k] = 0.0;
   for (int i = blockIdx.x * blockDim.x + tid; i < n; i += gridDim.x * blockDim.x)
 #pragma unroll
     for (int k = 0; k < NV; ++k) acc[k] += in[i].v[k];
+  cta(acc, part + blockIdx.x);
+  if (!last_cta(counter)) return;
 #pragma unroll
-  for (int k = 0; k < NV; ++k) acc[k] = warp_sum(acc[k]);
-  if ((tid & 31) == 0)
+  for (int k = 0; k < NV; ++k) acc[k] = 0.0;
+  for (int i = tid; i < (int)gridDim.x; i += blockDim.x)
 #pragma unroll
-    for (int k = 0; k < NV; ++k) sh[tid >> 5][k] = acc[k];
-  __syncthreads();
-  if (tid == 0) {
-    RedVec<NV> t;
-    for (int k = 0; k < NV; ++k) {
-      double s = 0.0;
-      for (int w = 0; w < (int)(blockDim.x / 32); ++w) s += sh[w][k];
-      t.v[k] = s;
-    }
-    out[blockIdx.x] = t;
-  }
+    for (int k = 0; k < NV; ++k) acc[k] += __ldcg(&part[i].v[k]);
+  cta(acc, out);
 }
 
 // Dot products of D-vectors: out[k] = sum_i a_k[i] * b_k[i], fixed order.
@@ -809,17 +835,19 @@ struct BlockTables {
 // Assembly record per block: U lower (21), g (6), reduced g (6), diag (6), edge (18), coupling lower (21)
 constexpr int kAsmRec = 21 + 6 + 6 + 6 + 18 + 21;
 
-// Scatter block records into the D-vectors (g, reduced g, diag) — one thread per block.
-__global__ void k_block_vectors(BlockTables bt, const double* blk_out, double* gfull, double* gred, double* diag,
-                                int* clamp_count, double* diag_minmax) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= bt.nblocks) return;
-  const double* rec = blk_out + (size_t)kAsmRec * b;
-  int o = bt.blk_off[b], d = bt.blk_dim[b];
+// A block's assembly record (in shared memory) scattered into the D-vectors (g, reduced g, diag), with its
+// damping clamp: one thread.
+struct BlockVectors {
+  const int* blk_off;
+  double *gfull, *gred, *diag, *minmax;
+  int* clamp;
+};
+__device__ __forceinline__ void block_vectors(const BlockVectors& bv, int b, int d, const double* rec) {
+  const int o = bv.blk_off[b];
   double s = 0.0;
   for (int k = 0; k < d; ++k) {
-    gfull[o + k] = rec[21 + k];
-    gred[o + k] = rec[27 + k];
+    bv.gfull[o + k] = rec[21 + k];
+    bv.gred[o + k] = rec[27 + k];
     s = fmax(s, rec[33 + k]);
   }
   // raw diagonal extrema before clamping (finalize_assembly, schur/assembly.rs:701-712)
@@ -828,10 +856,10 @@ __global__ void k_block_vectors(BlockTables bt, const double* blk_out, double* g
     mn = fmin(mn, rec[33 + k]);
     mx = fmax(mx, rec[33 + k]);
   }
-  diag_minmax[2 * b] = mn;
-  diag_minmax[2 * b + 1] = mx;
+  bv.minmax[2 * b] = mn;
+  bv.minmax[2 * b + 1] = mx;
   // clamp_damping_block (schur/assembly.rs:744-766)
-  double fl = s > 0.0 ? 64.0 * kEps * s : 1.0;
+  const double fl = s > 0.0 ? 64.0 * kEps * s : 1.0;
   int cl = 0;
   for (int k = 0; k < d; ++k) {
     double v = rec[33 + k];
@@ -839,9 +867,9 @@ __global__ void k_block_vectors(BlockTables bt, const double* blk_out, double* g
       v = fl;
       ++cl;
     }
-    diag[o + k] = v;
+    bv.diag[o + k] = v;
   }
-  clamp_count[b] = cl;
+  bv.clamp[b] = cl;
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -2438,13 +2466,50 @@ struct Solver {
   DBuf<uint32_t> d_ent, d_ent_point, d_chunk_begin, d_chunk_end;
   DBuf<int> d_seg_col;
   DBuf<double> d_blk_out;
-  DBuf<double> d_gfull, d_gred, d_diag, d_diag_minmax;
-  DBuf<int> d_clamp;
+  // What the host reads of an assembly and of a candidate, in one buffer so that each is one copy:
+  // summary | diag_minmax | clamp | gfull | gred | diag for the assembly, diag | step | scalars | cand_out |
+  // status for the candidate.
+  template <typename V>
+  struct Slice {
+    V* p = nullptr;
+    size_t n = 0;
+  };
+  DBuf<double> d_results;
+  Slice<PointSummary> d_summary_out;
+  Slice<double> d_diag_minmax, d_gfull, d_gred, d_diag, d_step, d_scalars;
+  Slice<int> d_clamp, d_status;
+  Slice<RedVec<4>> d_cand_out;
+  DBuf<unsigned> d_counter;
+  void place_results() {
+    size_t at = 0;
+    auto bytes_to_doubles = [](size_t b) { return (b + sizeof(double) - 1) / sizeof(double); };
+    size_t offsets[10];
+    const size_t counts[10] = {bytes_to_doubles(sizeof(PointSummary)), 2 * (size_t)std::max(1, nb),
+                               bytes_to_doubles(sizeof(int) * std::max(1, nb)), (size_t)std::max(1, D),
+                               (size_t)std::max(1, D), (size_t)std::max(1, D), (size_t)std::max(1, D), 16, 4, 2};
+    for (int k = 0; k < 10; ++k) {
+      offsets[k] = at;
+      at += counts[k];
+    }
+    d_results.alloc(at, st);
+    double* base = d_results.p;
+    d_summary_out = {reinterpret_cast<PointSummary*>(base + offsets[0]), 1};
+    d_diag_minmax = {base + offsets[1], counts[1]};
+    d_clamp = {reinterpret_cast<int*>(base + offsets[2]), (size_t)std::max(1, nb)};
+    d_gfull = {base + offsets[3], counts[3]};
+    d_gred = {base + offsets[4], counts[4]};
+    d_diag = {base + offsets[5], counts[5]};
+    d_step = {base + offsets[6], counts[6]};
+    d_scalars = {base + offsets[7], counts[7]};
+    d_cand_out = {reinterpret_cast<RedVec<4>*>(base + offsets[8]), 1};
+    d_status = {reinterpret_cast<int*>(base + offsets[9]), 4};
+    d_counter.alloc(1, st);
+    d_counter.zero();
+  }
   // pairs
   DBuf<int> d_xgrp_row, d_xgrp_col, d_blk_cross_begin, d_blk_cross_end;
   DBuf<uint32_t> d_xgrp_begin, d_xgrp_end, d_xpair_a, d_xpair_b, d_xpair_p;
   DBuf<double> d_xpair_out;
-  DBuf<int> d_status;
   // explicit S: block rows, permutation and the banded tiled factor
   DBuf<uint32_t> d_blk_ent, d_nbr_begin;
   DBuf<int> d_ent_block, d_nbr, d_nbr_row, d_perm_off, d_perm_to_orig;
@@ -2466,11 +2531,11 @@ struct Solver {
   bool asm_attr = false;    // k_block_tiles stages kAsmComp (TILE + 1) doubles in dynamic shared memory
   DBuf<double> d_asm_rec;   // per (block, segment) assembly records, kAsmRecordScale per partial element
   // PCG vectors
-  DBuf<double> d_step, d_r, d_z, d_dir, d_q, d_factor, d_tmp, d_rhs, d_r64, d_e, d_dq, d_rr_part, d_rz_part;
+  DBuf<double> d_r, d_z, d_dir, d_q, d_factor, d_tmp, d_rhs, d_r64, d_e, d_dq, d_rr_part, d_rz_part;
   DBuf<int> d_fail;
 
 
-  DBuf<double> d_scalars, d_ctl;
+  DBuf<double> d_ctl;
   DBuf<RedVec<4>> d_cand, d_cand_part;
   DBuf<RedVec<3>> d_met, d_met_part;
   DBuf<RedVec<1>> d_one, d_one_part;
@@ -2694,13 +2759,8 @@ struct Solver {
     up_i(d_blk_cross_begin, S.blk_cross_begin);
     up_i(d_blk_cross_end, S.blk_cross_end);
     d_blk_out.alloc((size_t)kAsmRec * std::max(1, nb), st);
-    d_gfull.alloc(std::max(1, D), st);
-    d_gred.alloc(std::max(1, D), st);
-    d_diag.alloc(std::max(1, D), st);
-    d_diag_minmax.alloc(2 * std::max(1, nb), st);
-    d_clamp.alloc(std::max(1, nb), st);
+    place_results();
     d_xpair_out.alloc((size_t)36 * std::max<size_t>(1, S.xgrp_row.size()), st);
-    d_status.alloc(4, st);
     up_u(d_blk_ent, S.blk_ent);
     up_i(d_ent_block, S.ent_block);
     up_u(d_nbr_begin, S.nbr_begin);
@@ -2712,7 +2772,7 @@ struct Solver {
     d_rows.alloc(std::max<uint64_t>(1, S.slot_off.empty() ? 1 : S.slot_off.back()), st);
     d_perm_vec.alloc(std::max(1, D), st);
     d_power.alloc(2, st);
-    for (DBuf<double>* b : {&d_step, &d_r, &d_z, &d_dir, &d_q, &d_tmp, &d_rhs, &d_r64, &d_e}) b->alloc(std::max(1, D), st);
+    for (DBuf<double>* b : {&d_r, &d_z, &d_dir, &d_q, &d_tmp, &d_rhs, &d_r64, &d_e}) b->alloc(std::max(1, D), st);
     d_factor.alloc((size_t)42 * std::max(1, nb), st);
     d_dq.alloc(std::max(1, nb), st);
     d_rr_part.alloc(std::max(1, grid_for(nb, kUpdThreads)), st);
@@ -2727,7 +2787,6 @@ struct Solver {
       dT64.prefetch_ahead = per64 * sms;
       dT32.prefetch_ahead = per32 * sms;
     }
-    d_scalars.alloc(16, st);
     d_ctl.alloc((sizeof(PcgCtl) + sizeof(double) - 1) / sizeof(double), st);
     d_cand.alloc(P, st);
     d_cand_part.alloc(red_blocks, st);
@@ -2742,11 +2801,12 @@ struct Solver {
 
   template <int NV>
   RedVec<NV> reduce(const RedVec<NV>* in, int count, DBuf<RedVec<NV>>& part) {
-    OMVGBA_LAUNCH(k_reduce_vec<NV>, red_blocks, kReduceThreads, 0, st, in, count, part.p);
-    OMVGBA_LAUNCH(k_reduce_vec<NV>, 1, kReduceThreads, 0, st, part.p, red_blocks, part.p + 0);
+    static_assert(sizeof(RedVec<NV>) <= 16 * sizeof(double), "the result lies in d_scalars");
+    RedVec<NV>* out = reinterpret_cast<RedVec<NV>*>(d_scalars.p);
+    OMVGBA_LAUNCH(k_reduce_vec<NV>, red_blocks, kReduceThreads, 0, st, in, count, part.p, out, d_counter.p);
     check_launch();
     RedVec<NV> h;
-    CUDA_OK(copy_async(&h, part.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(copy_async(&h, out, sizeof(h), cudaMemcpyDeviceToHost, st));
     sync();
     return h;
   }
@@ -2814,26 +2874,30 @@ struct Solver {
       }
     }
     check_launch();
-    OMVGBA_LAUNCH(k_reduce_summary, red_blocks, kReduceThreads, 0, st, d_summary.p, P, d_summary_part.p);
-    OMVGBA_LAUNCH(k_reduce_summary, 1, kReduceThreads, 0, st, d_summary_part.p, red_blocks, d_summary_part.p);
+    OMVGBA_LAUNCH(k_reduce_summary, red_blocks, kReduceThreads, 0, st, d_summary.p, P, d_summary_part.p,
+                  d_summary_out.p, d_counter.p);
     check_launch();
     BlockTables bt = tables();
     if (bt.nchunks > 0) {
       camera_sums();
-      OMVGBA_LAUNCH(k_block_vectors, grid_for(nb, 64), 64, 0, st, bt, d_blk_out.p, d_gfull.p, d_gred.p, d_diag.p, d_clamp.p,
-                                                     d_diag_minmax.p);
       check_launch();
     }
     rows_valid = false;
     if (build_rows && D > 0) this->build_rows();
-    // every result of the assembly with one wait
-    Readback rb(st, Readback::room(sizeof(PointSummary)) + Readback::room(sizeof(double) * 2 * nb) +
-                        Readback::room(sizeof(int) * nb) + 3 * Readback::room(sizeof(double) * D));
-    const PointSummary* psp = rb.add(d_summary_part.p, 1);
-    const double* mm = rb.add(d_diag_minmax.p, 2 * (size_t)nb);
-    const int* cl = rb.add(d_clamp.p, nb);
-    const double *gvals = rb.add(d_gfull.p, D), *dvals = rb.add(d_diag.p, D), *gr = rb.add(d_gred.p, D);
+    // every result of the assembly with one copy and one wait
+    const double* dev = d_results.p;
+    Readback rb(st, Readback::room(sizeof(double) * (size_t)(d_step.p - dev)));
+    const double* host = rb.add(dev, (size_t)(d_step.p - dev));
+    auto at = [&](const void* device) {  // the host copy of a result
+      return reinterpret_cast<const char*>(host) + (static_cast<const char*>(device) - reinterpret_cast<const char*>(dev));
+    };
     rb.wait();
+    const PointSummary* psp = reinterpret_cast<const PointSummary*>(at(d_summary_out.p));
+    const double* mm = reinterpret_cast<const double*>(at(d_diag_minmax.p));
+    const int* cl = reinterpret_cast<const int*>(at(d_clamp.p));
+    const double *gvals = reinterpret_cast<const double*>(at(d_gfull.p)),
+                 *dvals = reinterpret_cast<const double*>(at(d_diag.p)),
+                 *gr = reinterpret_cast<const double*>(at(d_gred.p));
     const PointSummary ps = *psp;
     Assembly a;
     a.valid = ps.invalid == 0.0;
@@ -2870,13 +2934,12 @@ struct Solver {
   // Whether the factorization succeeded is in d_status when the stream gets there.
   void direct_step(double lambda) {
     factor_band(lambda, nullptr, 0.0, false);
-    OMVGBA_LAUNCH(k_perm_gather, grid_for(D, 256), 256, 0, st, D, d_perm_to_orig.p, d_gred.p, -1.0, d_perm_vec.p);
     {  // one cluster: a CTA per tile of the band, up to kSolveCtas
       int ctas = 1;
       while (ctas < kSolveCtas && ctas < S.bwt) ctas *= 2;
-      launch_cluster(k_tile_solve, ctas, 256, 0, st, tile_band(), d_perm_vec.p, (const int*)d_status.p);
+      launch_cluster(k_tile_solve, ctas, 256, 0, st, tile_band(), d_perm_vec.p, (const int*)d_status.p,
+                     (const int*)d_perm_to_orig.p, (const double*)d_gred.p, d_step.p);
     }
-    OMVGBA_LAUNCH(k_perm_scatter, grid_for(D, 256), 256, 0, st, D, d_perm_to_orig.p, d_perm_vec.p, d_step.p);
     check_launch();
   }
 
@@ -2908,7 +2971,8 @@ struct Solver {
         OMVGBA_LAUNCH(k_block_tiles<T>, mt.ntiles, mv_tile_obs<T>(),
                       asm_smem_bytes<T>(), st, mt, lin(), pt_off, d_asm_rec.p);
     }
-    OMVGBA_LAUNCH(k_block_records, nb, kAsmRec * kRecordShares, 0, st, mt, bt.blk_edge, d_asm_rec.p, d_blk_out.p);
+    OMVGBA_LAUNCH(k_block_records, nb, kAsmRec * kRecordShares, 0, st, mt, bt.blk_edge, d_asm_rec.p, d_blk_out.p,
+                  BlockVectors{d_blk_off.p, d_gfull.p, d_gred.p, d_diag.p, d_diag_minmax.p, d_clamp.p});
   }
 
   // Whether a PCG run on the explicit S fits one cluster (k_pcg_loop): a thread per parameter, a warp per
@@ -3918,8 +3982,8 @@ struct Solver {
         check_launch();
         // the candidate's sums and the model reduction (camera_step.rs:44-81, optimizer.rs:590-618,
         // retained/mod.rs:742-800): everything queued, then one wait
-        OMVGBA_LAUNCH(k_reduce_vec<4>, red_blocks, kReduceThreads, 0, st, d_cand.p, P, d_cand_part.p);
-        OMVGBA_LAUNCH(k_reduce_vec<4>, 1, kReduceThreads, 0, st, d_cand_part.p, red_blocks, d_cand_part.p);
+        OMVGBA_LAUNCH(k_reduce_vec<4>, red_blocks, kReduceThreads, 0, st, d_cand.p, P, d_cand_part.p, d_cand_out.p,
+                      d_counter.p);
         check_launch();
         if (D > 0) {
           if (!iterative_step)
@@ -3932,13 +3996,14 @@ struct Solver {
         double cd[1] = {0.0};
         RedVec<4> cr;
         {
-          Readback rb(st, Readback::room(sizeof(cr)) + Readback::room(sizeof(double) * 2) + Readback::room(sizeof(int)) +
-                              2 * Readback::room(sizeof(double) * D));
-          const RedVec<4>* crp = rb.add(d_cand_part.p, 1);
-          const double* dp = rb.add(d_scalars.p, 2);
-          const int* okp = rb.add(d_status.p, 1);
-          const double *hs = rb.add(d_step.p, D), *hd = rb.add(d_diag.p, D);
+          const size_t first = (size_t)(d_diag.p - d_results.p), count = d_results.n - first;
+          Readback rb(st, Readback::room(sizeof(double) * count));
+          const double* host = rb.add(d_diag.p, count);
           rb.wait();
+          const double *hd = host, *hs = host + (d_step.p - d_diag.p), *dp = host + (d_scalars.p - d_diag.p);
+          const RedVec<4>* crp = reinterpret_cast<const RedVec<4>*>(
+              host + (reinterpret_cast<const double*>(d_cand_out.p) - d_diag.p));
+          const int* okp = reinterpret_cast<const int*>(host + (reinterpret_cast<const double*>(d_status.p) - d_diag.p));
           cr = *crp;
           if (direct && D > 0) solved = *okp != 0;
           if (D > 0) {
