@@ -515,131 +515,146 @@ __device__ __forceinline__ void mma8(int depth, FA a, FB b, double& c0, double& 
 }
 
 // POTRF of diagonal tile k and the inverse W_k = L_kk^-1 of its factor, one CTA of 8 warps, blocked by
-// 8 columns. A panel (all rows, 8 columns) is factored by warp 0 in registers, two rows per lane: a
-// step is one reciprocal root, one scaling and the shuffles that hand the pivot row's entries to the
-// columns right of it, with no barrier (the pivots' roots and reciprocals, which only the output and the
-// inverse need, come after the panel, a lane each); then every warp subtracts the panel's rank-8 product
-// from its 8 x 8 blocks of the trailing triangle on the FP64 tensor pipe. The inverse of the factor starts
-// from the 8 x 8 diagonal blocks (a warp each) and doubles the block size three times with
-// W_21 = -W_22 (L_21 W_11), the products on the tensor pipe, their middle factor in the unused upper
-// triangle. Bound: the 64 dependent pivot steps. A right-looking factor with one barrier per column and
-// a second sweep of 64 barriers for the inverse took 64 us per tile; this takes 18.5.
+// 8 columns. Warp 0 factors a panel (all rows, 8 columns) in registers, two rows per lane. Each lane also
+// holds the panel's 8 x 8 diagonal block, so a pivot step is a reciprocal root, a product and a fused
+// multiply-add, with no shuffle and no barrier in the chain. Then every warp subtracts the panel's rank-8
+// product from one 8 x 8 block of the next panel's columns on the FP64 tensor pipe; the rest of the
+// trailing triangle, the panel's columns of the factor and its row of the inverse,
+// W_q. = -W_qq (L_q. W), are done by warps 1 to 7 while warp 0 factors the next panel (the pivots' roots
+// and reciprocals, which only these need, among them). Bound: the 64 dependent pivot steps. A right-looking
+// factor with one barrier per column and a second sweep of 64 barriers for the inverse took 64 us per tile;
+// with shuffled pivots, every block of the triangle between two panels and the inverse afterwards it took
+// 18.5; this takes 13.6.
 // status[0] = 0 when a pivot is not finite and positive; later launches of the factorization then
 // return at once.
 constexpr size_t kPotrfSmem = 2 * kStagedTile;
-// A: the tile in shared memory (visible to the CTA), then L, its strict upper triangle scratch; W: a
-// second staged tile.
+// A: the tile in shared memory (visible to the CTA), then L below its diagonal; W: a second staged tile,
+// the inverse on and below its diagonal, the products L_q. W above it.
 __device__ void potrf_tile(const TileBand& tb, int k, double* A, double* W, int* status) {
-  __shared__ double rdiag[kCT];
+  __shared__ double pivots[kCT];
   __shared__ int s_bad;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
   double* gt = tb.t + tile_at(tb, k, k);
-  for (int i = tid; i < kCT * kTS; i += 256) W[i] = 0.0;
+  // C(bi, bj) -= panel p's product, one warp
+  auto trailing = [&](int p, int bi, int bj) {
+    double* C = A + (8 * bj + 2 * t) * kTS + 8 * bi + g;
+    double c0 = C[0], c1 = C[kTS];
+    mma8(8, [&](int r, int kk) { return -A[(8 * p + kk) * kTS + 8 * bi + r]; },
+         [&](int kk, int c) { return A[(8 * p + kk) * kTS + 8 * bj + c]; }, c0, c1);
+    C[0] = c0;
+    C[kTS] = c1;
+  };
+  // Columns of the factor and row of the inverse of panel q, warps 1 to 7.
+  auto finish = [&](int q) {
+    for (int i = tid - 32; i < 8 * kCT; i += 224) {  // the factor (zero above the diagonal)
+      const int c = 8 * q + (i >> 6), r = i & 63;
+      if (r != c) gt[c * kCT + r] = r > c ? A[c * kTS + r] : 0.0;
+    }
+    if (w == 7) {  // W_qq, lane c its column c
+      const int col = lane & 7;
+      const double sd = sqrt(pivots[8 * q + col]), rd = 1.0 / sd;
+      if (lane < 8) gt[(8 * q + lane) * (kCT + 1)] = sd;
+      double x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        double v = i == col ? 1.0 : 0.0;
+#pragma unroll
+        for (int z = 0; z < i; ++z) v -= A[(8 * q + z) * kTS + 8 * q + i] * x[z];
+        const double r = __shfl_sync(0xffffffffu, rd, i);
+        x[i] = i >= col ? v * r : 0.0;
+        if (lane < 8) W[(8 * q + lane) * kTS + 8 * q + i] = x[i];
+      }
+    }
+    // block column j: warp j + 1, warp 7 those left after W_qq
+    const int j = w - 1;
+    double* T = W + (8 * q + 2 * t) * kTS + 8 * j + g;
+    if (j < q) {
+      double c0 = 0.0, c1 = 0.0;
+      mma8(8 * (q - j), [&](int r, int kk) { return A[(8 * j + kk) * kTS + 8 * q + r]; },
+           [&](int kk, int c) { return W[(8 * j + c) * kTS + 8 * j + kk]; }, c0, c1);
+      T[0] = c0;
+      T[kTS] = c1;
+    }
+    asm volatile("bar.sync 1, 224;" ::: "memory");  // warps 1 to 7: W_qq and the products are there
+    if (j < q) {
+      double c0 = 0.0, c1 = 0.0;
+      mma8(8, [&](int r, int kk) { return -W[(8 * q + kk) * kTS + 8 * q + r]; },
+           [&](int kk, int c) { return W[(8 * q + c) * kTS + 8 * j + kk]; }, c0, c1);
+      double* O = W + (8 * j + 2 * t) * kTS + 8 * q + g;
+      O[0] = c0;
+      O[kTS] = c1;
+    }
+  };
   if (tid == 0) s_bad = 0;
   __syncthreads();
-  for (int j0 = 0; j0 < kCT; j0 += 8) {
+  for (int p = 0; p < 8; ++p) {
+    const int j0 = 8 * p;
     if (w == 0) {
       double lo[8], hi[8];  // rows lane and lane + 32 of the panel
+      double d[8][8];       // its diagonal block, d[c][r]
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
+#pragma unroll
+        for (int r = c & ~1; r < 8; r += 2) {
+          const double2 v = *reinterpret_cast<const double2*>(A + (j0 + c) * kTS + j0 + r);
+          d[c][r] = v.x;
+          d[c][r + 1] = v.y;
+        }
         lo[c] = A[(j0 + c) * kTS + lane];
         hi[c] = A[(j0 + c) * kTS + lane + 32];
       }
-      const bool upper_half = j0 >= 32;  // the panel's diagonal rows lie in hi
       bool bad = false;
       double pivot = 1.0;  // lane c < 8: column c's
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        const int pl = (j0 + c) & 31;
-        const double d = __shfl_sync(0xffffffffu, upper_half ? hi[c] : lo[c], pl);
-        bad = bad || !(isfinite(d) && d > 0.0);
-        if (lane == c) pivot = d;
-        const double rs = rsqrt(d);
+        bad = bad || !(isfinite(d[c][c]) && d[c][c] > 0.0);
+        if (lane == c) pivot = d[c][c];
+        const double rs = rsqrt(d[c][c]);
         lo[c] *= rs;
         hi[c] *= rs;
 #pragma unroll
+        for (int r = c + 1; r < 8; ++r) d[c][r] *= rs;
+#pragma unroll
         for (int c2 = c + 1; c2 < 8; ++c2) {
-          const double l = __shfl_sync(0xffffffffu, upper_half ? hi[c] : lo[c], (j0 + c2) & 31);
-          lo[c2] -= lo[c] * l;
-          hi[c2] -= hi[c] * l;
+#pragma unroll
+          for (int r = c2; r < 8; ++r) d[c2][r] -= d[c][r] * d[c][c2];
+          lo[c2] -= lo[c] * d[c][c2];
+          hi[c2] -= hi[c] * d[c][c2];
         }
       }
+      __syncwarp();  // every lane has read the panel
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {  // rows above the panel's diagonal are scratch
+      for (int c = 0; c < 8; ++c) {
         if (lane > j0 + c) A[(j0 + c) * kTS + lane] = lo[c];
         if (lane + 32 > j0 + c) A[(j0 + c) * kTS + lane + 32] = hi[c];
       }
-      if (lane < 8) {
-        const double sd = sqrt(pivot);
-        A[(j0 + lane) * kTS + j0 + lane] = sd;
-        rdiag[j0 + lane] = 1.0 / sd;
-      }
+      if (lane < 8) pivots[j0 + lane] = pivot;
       if (bad && lane == 0) s_bad = 1;
+    } else if (p > 0) {
+      // blocks (bi >= bj > p) of the panel before, column by column of blocks
+      const int m = 7 - p;
+      for (int q = w - 1; q < m * (m + 1) / 2; q += 7) {
+        int col = 0, at = q;
+        while (at >= m - col) at -= m - col++;
+        trailing(p - 1, p + 1 + col + at, p + 1 + col);
+      }
+      finish(p - 1);
     }
     __syncthreads();
     if (s_bad) {
       if (tid == 0) status[0] = 0;
       return;
     }
-    // trailing blocks (bi >= bj > j0 / 8), column by column of blocks
-    const int p = j0 >> 3, m = 7 - p;
-    for (int q = w; q < m * (m + 1) / 2; q += 8) {
-      int col = 0, at = q;
-      while (at >= m - col) at -= m - col++;
-      const int bj = p + 1 + col, bi = bj + at;
-      double* C = A + (8 * bj + 2 * t) * kTS + 8 * bi + g;
-      double c0 = C[0], c1 = C[kTS];
-      mma8(8, [&](int r, int kk) { return -A[(j0 + kk) * kTS + 8 * bi + r]; },
-           [&](int kk, int c) { return A[(j0 + kk) * kTS + 8 * bj + c]; }, c0, c1);
-      C[0] = c0;
-      C[kTS] = c1;
-    }
+    if (p + 1 + w < 8) trailing(p, p + 1 + w, p + 1);
     __syncthreads();
   }
-  // the factor out (zero above the diagonal)
+  if (w > 0) finish(7);
+  __syncthreads();
+  double* wk = tb.w + (size_t)k * kCTT;
   for (int i = tid; i < kCTT; i += 256) {
     const int c = i >> 6, r = i & 63;
-    gt[i] = r >= c ? A[c * kTS + r] : 0.0;
+    wk[i] = r >= c ? W[c * kTS + r] : 0.0;
   }
-  // W: diagonal blocks, warp w block w, lane c its column c
-  if (lane < 8) {
-    double x[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      double v = i == lane ? 1.0 : 0.0;
-#pragma unroll
-      for (int q = 0; q < i; ++q) v -= A[(8 * w + q) * kTS + 8 * w + i] * x[q];
-      x[i] = i >= lane ? v * rdiag[8 * w + i] : 0.0;
-      W[(8 * w + lane) * kTS + 8 * w + i] = x[i];
-    }
-  }
-  __syncthreads();  // the factor has been read out: the upper triangle is scratch from here on
-  for (int h = 8; h < kCT; h *= 2) {
-    const int nbk = h / 8, per = nbk * nbk, pairs = kCT / (2 * h);
-    // T = L_21 W_11 (h x h) of every pair, into rows [b, b + h), columns [b + h, b + 2 h)
-    for (int q = w; q < pairs * per; q += 8) {
-      const int b = 2 * h * (q / per), bi = (q % per) % nbk, bj = (q % per) / nbk;
-      double c0 = 0.0, c1 = 0.0;
-      mma8(h, [&](int r, int kk) { return A[(b + kk) * kTS + b + h + 8 * bi + r]; },
-           [&](int kk, int c) { return W[(b + 8 * bj + c) * kTS + b + kk]; }, c0, c1);
-      double* T = A + (b + h + 8 * bj + 2 * t) * kTS + b + 8 * bi + g;
-      T[0] = c0;
-      T[kTS] = c1;
-    }
-    __syncthreads();
-    for (int q = w; q < pairs * per; q += 8) {
-      const int b = 2 * h * (q / per), bi = (q % per) % nbk, bj = (q % per) / nbk;
-      double c0 = 0.0, c1 = 0.0;
-      mma8(h, [&](int r, int kk) { return -W[(b + h + kk) * kTS + b + h + 8 * bi + r]; },
-           [&](int kk, int c) { return A[(b + h + 8 * bj + c) * kTS + b + kk]; }, c0, c1);
-      double* O = W + (b + 8 * bj + 2 * t) * kTS + b + h + 8 * bi + g;
-      O[0] = c0;
-      O[kTS] = c1;
-    }
-    __syncthreads();
-  }
-  double* wk = tb.w + (size_t)k * kCTT;
-  for (int i = tid; i < kCTT; i += 256) wk[i] = W[(i >> 6) * kTS + (i & 63)];
 }
 
 __global__ void __launch_bounds__(256) k_tile_potrf(TileBand tb, int k, int* status) {
@@ -674,8 +689,8 @@ __global__ void __launch_bounds__(256) k_tile_trsm(TileBand tb, int k, const int
 // Trailing update of step k: A_ij -= L_ik L_jk^T for k < j <= i <= min(k + bwt, nt - 1), one CTA per
 // tile; the sum over the tile's 64 columns runs in order. CTA 0 has the next diagonal tile: it goes on to
 // factor it (potrf_tile) while the other CTAs update theirs, so a column costs its factorization and its
-// trsm, and the update runs in the factorization's shadow (500-camera survey, per column: 18.5 us of potrf,
-// 6.1 of trsm and 7.0 of update become 6.1 + 22.7).
+// trsm, and the update runs in the factorization's shadow (500-camera survey, per column: 13.6 us of potrf,
+// 6.1 of trsm and 7.0 of update become 6.1 + 17.2).
 constexpr size_t kUpdateSmem = 2 * kStagedTile;
 __global__ void __launch_bounds__(256) k_tile_update(TileBand tb, int k, int* status) {
   extern __shared__ __align__(16) double sh[];
