@@ -740,71 +740,151 @@ __global__ void __launch_bounds__(256) k_tile_update(TileBand tb, int k, int* st
 // Forward (L y = -g) and backward (L^T x = y) substitution with the banded tiled factor, on the vector v in
 // the factor's order (n entries; the padding is not touched), gathered from g and scattered to step_out in
 // the parameters' order; one cluster of up to kSolveCtas CTAs.
-// Right-looking: CTA i mod size owns rows of tile i. In step k the owner of tile k multiplies its
-// finished part by the inverse of the diagonal tile (W_k, from the factorization), hands the 64
-// results to every CTA's shared memory, and after one cluster barrier each CTA subtracts the products
-// of its own tiles of the column (forward) or row (backward). Each entry of v is only ever touched
-// by its owner, in step order. Bound: 2 nt steps of one L2 latency, one cluster barrier and one more
-// L2 latency. One CTA that walked each row of the band with an in-tile triangular solve by one warp took
-// 12.8 ms for 71 tiles in a band of 14; this takes 0.79 ms (two tiles: 184 us before).
+// Right-looking: CTA i mod size owns rows of tile i. In step k every CTA has the 64 finished results of
+// tile k in its shared memory. The owner of tile k + 1 subtracts their product with T(k + 1, k), multiplies
+// by the inverse of the diagonal tile (W, from the factorization) and hands the results to every CTA; then
+// it signals the cluster barrier of step k + 1, and only then does each CTA subtract the products of its
+// other tiles of the column (forward) or row (backward), which no later step but k + 2 and on waits for.
+// Both tiles of a CTA's next turn are loaded into registers a turn ahead and the next of its other tiles one
+// product ahead, so no load lies in the chain. A CTA may thus still read the results of tile k while those
+// of tile k + 2 are being written: three buffers. Each entry of v is only ever touched by one thread, in
+// step order. Bound: 2 nt steps of two products, their CTA barriers and a cluster barrier, or the band's
+// tiles from L2 through 8 SMs where the band is wide. One CTA that walked each row of the band with an
+// in-tile triangular solve by one warp took 12.8 ms for 71 tiles in a band of 14; with every load and every
+// product of a step between two cluster barriers it took 0.93 ms; this takes 0.31.
 constexpr int kSolveCtas = 8;
-// y[0..64) = M u (or M^T u) for the column-major 64 x 64 tile M; 256 threads, u in shared memory.
-__device__ __forceinline__ void tile_times(const double* __restrict__ M, const double* u, double* part, double* y) {
-  const int r = threadIdx.x & (kCT - 1), qtr = threadIdx.x >> 6;
-  double m[16];
+constexpr int kSolveBuffers = 3;
+struct SolveShared {
+  double part[2][4 * kCT], u[kCT];
+  double step[kSolveBuffers][kCT];  // finished parts of the vector, from their owners
+};
+// One sweep over the tiles: k-th tile is tile k of the factor (FORWARD) or tile nt - 1 - k.
+template <bool FORWARD>
+__device__ __forceinline__ void solve_sweep(const TileBand& tb, double* v, const int* __restrict__ perm_to_orig,
+                                            double* __restrict__ step_out, SolveShared& sh) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int size = (int)cluster.num_blocks(), tid = threadIdx.x, r = tid & (kCT - 1), qtr = tid >> 6;
+  const int nt = tb.nt;
+  auto actual = [&](int k) { return FORWARD ? k : nt - 1 - k; };
+  // the CTA's tiles are first, first + size, ...
+  const int rank = (int)cluster.block_rank(), first = FORWARD ? rank : ((nt - 1 - rank) % size + size) % size;
+  const int base = FORWARD ? 0 : nt;  // results are numbered on from the forward sweep's
+  auto step = [&](int k) { return sh.step[(base + k) % kSolveBuffers]; };
+  // A thread's 16 entries of a tile: of row r (columns 16 qtr ...), or of column tid / 4 (every fourth row).
+  auto load = [&](const double* __restrict__ M, double m[16]) {
+    if (FORWARD) {
 #pragma unroll
-  for (int c = 0; c < 16; ++c) m[c] = M[(size_t)(16 * qtr + c) * kCT + r];
-  double s = 0.0;
+      for (int c = 0; c < 16; ++c) m[c] = M[(size_t)(16 * qtr + c) * kCT + r];
+    } else {
 #pragma unroll
-  for (int c = 0; c < 16; ++c) s += m[c] * u[16 * qtr + c];
-  part[qtr * kCT + r] = s;
-  __syncthreads();
-  if (threadIdx.x < kCT) y[r] = ((part[r] + part[kCT + r]) + part[2 * kCT + r]) + part[3 * kCT + r];
-  __syncthreads();
-}
-__device__ __forceinline__ void tile_times_t(const double* __restrict__ M, const double* u, double* y) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  double m0[8], m1[8];
+      for (int j = 0; j < 16; ++j) m[j] = M[(size_t)(tid >> 2) * kCT + 4 * j + (tid & 3)];
+    }
+  };
+  auto load_t = [&](int i, int k, double m[16]) {  // T of the i-th and the k-th tile, i > k
+    load(tb.t + (FORWARD ? tile_at(tb, actual(i), actual(k)) : tile_at(tb, actual(k), actual(i))), m);
+  };
+  auto load_w = [&](int k, double m[16]) { load(tb.w + (size_t)actual(k) * kCTT, m); };
+  auto partial = [&](const double m[16], const double* x) {
+    if (FORWARD) {
+      double s = 0.0;
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    m0[c] = M[(size_t)(8 * w + c) * kCT + lane];
-    m1[c] = M[(size_t)(8 * w + c) * kCT + lane + 32];
+      for (int c = 0; c < 16; ++c) s += m[c] * x[16 * qtr + c];
+      return s;
+    }
+    double s[8];  // rows i and i + 32, then a balanced sum
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] = m[j] * x[4 * j + (tid & 3)] + m[j + 8] * x[4 * j + (tid & 3) + 32];
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+      for (int j = 0; j < h; ++j) s[j] += s[j + h];
+    return s[0];
+  };
+  int used = 0;
+  auto total = [&](double s) {  // entry r of the product, in every thread
+    double* part = sh.part[used];
+    used ^= 1;  // the buffer's next use lies after the next barrier
+    if (FORWARD) {
+      part[tid] = s;
+      __syncthreads();
+      return ((part[r] + part[kCT + r]) + part[2 * kCT + r]) + part[3 * kCT + r];
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    if ((tid & 3) == 0) part[tid >> 2] = s;
+    __syncthreads();
+    return part[r];
+  };
+  // The entry of the i-th tile that this thread keeps (threads 0 to 63).
+  auto own = [&](int i) { return tid < kCT && actual(i) * kCT + tid < tb.n; };
+  auto entry = [&](int i) { return own(i) ? v[actual(i) * kCT + tid] : 0.0; };
+  // Tile k's results from u = its right-hand side less all products, and to every CTA.
+  auto finish = [&](int k, double u, const double w[16]) {
+    if (tid < kCT) sh.u[tid] = u;
+    __syncthreads();
+    const double y = total(partial(w, sh.u));
+    double* to = step(k) + r;
+    for (int c = qtr; c < size; c += 4) *cluster.map_shared_rank(to, c) = y;
+    if (own(k)) {
+      const int P = actual(k) * kCT + tid;
+      v[P] = y;
+      if (!FORWARD) step_out[perm_to_orig[P]] = y;
+    }
+  };
+  double mt[16], mw[16], mn[16];
+  if (first == 0) {
+    load_w(0, mw);
+    finish(0, entry(0), mw);
   }
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    const double s = warp_sum(m0[c] * u[lane] + m1[c] * u[lane + 32]);
-    if (lane == 0) y[8 * w + c] = s;
+  cluster.barrier_arrive();
+  int turn = first == 0 ? size : first;  // the CTA's next tile to finish
+  auto load_turn = [&] {
+    if (turn >= nt) return;
+    if (tb.bwt > 0) load_t(turn, turn - 1, mt);
+    load_w(turn, mw);
+  };
+  load_turn();
+  int ik = -1, i = nt;  // the next of the CTA's other products, tile i in step ik
+  auto next = [&] {
+    i += size;
+    while (ik < nt && i > min(nt - 1, ik + tb.bwt)) {
+      ++ik;
+      i = first + (max(0, ik + 2 - first) + size - 1) / size * size;
+    }
+    if (ik < nt) load_t(i, ik, mn);
+  };
+  next();
+  for (int k = 0; k < nt; ++k) {
+    const bool mine = turn == k + 1 && turn < nt;
+    const double rhs = mine ? entry(turn) : 0.0;
+    cluster.barrier_wait();
+    if (mine) {
+      const double x = tb.bwt > 0 ? total(partial(mt, step(k))) : 0.0;
+      finish(turn, own(turn) ? rhs - x : 0.0, mw);
+    }
+    if (k + 1 < nt) cluster.barrier_arrive();
+    if (mine) {
+      turn += size;
+      load_turn();
+    }
+    while (ik == k) {
+      const int at = i;
+      const double before = entry(at), s = partial(mn, step(k));
+      next();
+      const double x = total(s);
+      if (own(at)) v[actual(at) * kCT + tid] = before - x;
+    }
   }
-  __syncthreads();
 }
 __global__ void __launch_bounds__(256) k_tile_solve(TileBand tb, double* v, const int* status,
                                                     const int* __restrict__ perm_to_orig, const double* __restrict__ g,
                                                     double* __restrict__ step_out) {
   namespace cg = cooperative_groups;
-  __shared__ double part[4 * kCT], u[kCT], y[kCT];
-  __shared__ double step[2][kCT];  // the finished part of the step, from its owner
+  __shared__ __align__(16) SolveShared sh;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), size = (int)cluster.num_blocks(), tid = threadIdx.x;
   const bool factored = status[0] != 0;  // the same value in every CTA of the cluster
-  auto load = [&](int tile) {
-    if (tid < kCT) u[tid] = tile * kCT + tid < tb.n ? v[tile * kCT + tid] : 0.0;
-    __syncthreads();
-  };
-  auto publish = [&](int tile, int buf, bool last) {  // y: store it and hand it to every CTA
-    const int P = tile * kCT + tid;
-    if (tid < kCT && P < tb.n) {
-      v[P] = y[tid];
-      if (last) step_out[perm_to_orig[P]] = y[tid];
-    }
-    for (int i = tid; i < size * kCT; i += 256) {
-      double* dst = cluster.map_shared_rank(&step[buf][0], i / kCT);
-      dst[i % kCT] = y[i % kCT];
-    }
-  };
-  auto subtract = [&](int tile) {
-    if (tid < kCT && tile * kCT + tid < tb.n) v[tile * kCT + tid] -= y[tid];
-    __syncthreads();
-  };
   // the right-hand side -g in the factor's order, each CTA its own tiles
   for (int tile = rank; tile < tb.nt; tile += size)
     if (tid < kCT && tile * kCT + tid < tb.n) {
@@ -814,34 +894,8 @@ __global__ void __launch_bounds__(256) k_tile_solve(TileBand tb, double* v, cons
     }
   if (!factored) return;
   cluster.sync();  // every CTA runs before any of them is written to
-  for (int k = 0; k < tb.nt; ++k) {
-    const int buf = k & 1;
-    if (k % size == rank) {
-      load(k);
-      tile_times(tb.w + (size_t)k * kCTT, u, part, y);
-      publish(k, buf, false);
-    }
-    cluster.sync();
-    const int last = min(tb.nt - 1, k + tb.bwt);
-    for (int i = k + 1 + (rank - (k + 1) % size + size) % size; i <= last; i += size) {
-      tile_times(tb.t + tile_at(tb, i, k), step[buf], part, y);
-      subtract(i);
-    }
-  }
-  for (int k = tb.nt - 1; k >= 0; --k) {
-    const int buf = (tb.nt + tb.nt - 1 - k) & 1;  // alternates on from the forward sweep's last step
-    if (k % size == rank) {
-      load(k);
-      tile_times_t(tb.w + (size_t)k * kCTT, u, y);
-      publish(k, buf, true);
-    }
-    cluster.sync();
-    const int first = max(0, k - tb.bwt);
-    for (int j = first + (rank - first % size + size) % size; j < k; j += size) {
-      tile_times_t(tb.t + tile_at(tb, k, j), step[buf], y);
-      subtract(j);
-    }
-  }
+  solve_sweep<true>(tb, v, perm_to_orig, step_out, sh);
+  solve_sweep<false>(tb, v, perm_to_orig, step_out, sh);
   cluster.sync();  // no CTA leaves while another may still write to it
 }
 
