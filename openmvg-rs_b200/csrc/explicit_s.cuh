@@ -659,6 +659,7 @@ __device__ void potrf_tile(const TileBand& tb, int k, double* A, double* W, int*
 
 __global__ void __launch_bounds__(256) k_tile_potrf(TileBand tb, int k, int* status) {
   extern __shared__ __align__(16) double sh[];
+  pdl_trigger();
   if (status[0] == 0) return;
   stage_tile(tb.t + tile_at(tb, k, k), sh);
   stage_wait();
@@ -671,6 +672,8 @@ __global__ void __launch_bounds__(256) k_tile_potrf(TileBand tb, int k, int* sta
 constexpr size_t kTrsmSmem = 2 * kStagedTile;
 __global__ void __launch_bounds__(256) k_tile_trsm(TileBand tb, int k, const int* status) {
   extern __shared__ __align__(16) double shm[];
+  pdl_trigger();
+  pdl_wait();
   if (status[0] == 0) return;
   double* Ta = shm;
   double* Tb = shm + kCT * kTS;
@@ -694,6 +697,8 @@ __global__ void __launch_bounds__(256) k_tile_trsm(TileBand tb, int k, const int
 constexpr size_t kUpdateSmem = 2 * kStagedTile;
 __global__ void __launch_bounds__(256) k_tile_update(TileBand tb, int k, int* status) {
   extern __shared__ __align__(16) double sh[];
+  pdl_trigger();
+  pdl_wait();
   if (status[0] == 0) return;
   double* Ta = sh;
   double* Tb = sh + kCT * kTS;
@@ -923,6 +928,8 @@ constexpr int kTakahashiDiagCtas = 8;
 __global__ void __launch_bounds__(256) k_takahashi_partial(TileBand L, TileBand Z, int j, double* part,
                                                            const int* status) {
   extern __shared__ __align__(16) double sh[];
+  pdl_trigger();
+  pdl_wait();
   if (status[0] == 0) return;
   double* Ta = sh;
   double* Tb = sh + kCT * kTS;
@@ -949,6 +956,8 @@ __global__ void __launch_bounds__(256) k_takahashi_offdiag(TileBand L, TileBand 
                                                            const double* __restrict__ part, double* q,
                                                            const int* status) {
   extern __shared__ __align__(16) double sh[];
+  pdl_trigger();
+  pdl_wait();
   if (status[0] == 0) return;
   double* Ta = sh;
   double* Tb = sh + kCT * kTS;
@@ -983,6 +992,8 @@ __global__ void __launch_bounds__(256) k_takahashi_offdiag(TileBand L, TileBand 
 __global__ void __launch_bounds__(256) k_takahashi_diag(TileBand L, TileBand Z, int j, int m,
                                                         const double* __restrict__ q, const int* status) {
   extern __shared__ __align__(16) double sh[];
+  pdl_trigger();
+  pdl_wait();
   if (status[0] == 0) return;
   double* Ta = sh;             // 8 rows x 64: element (r, c) at c * 12 + r
   double* Tb = sh + kCT * 12;

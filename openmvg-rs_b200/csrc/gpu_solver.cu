@@ -72,11 +72,12 @@ void telemetry_read(uint64_t* launches, uint64_t* h2d, uint64_t* d2h) {
 // (programmatic stream serialization; the kernel orders itself with pdl_wait). A failed launch is
 // reported by the next launch check, like the <<<>>> launches.
 template <typename... KArgs, typename... Args>
-void launch_pdl(bool pdl, void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t st, Args... args) {
+void launch_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
+                Args... args) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -3230,7 +3231,7 @@ struct Solver {
   void rows_product(bool pdl, const double* x, double* y, double lambda, double* xy, const PcgCtl* ctl) {
     const int split = row_split(nb);
     launch_pdl(pdl, split == 4 ? k_rows_matvec<4> : (split == 2 ? k_rows_matvec<2> : k_rows_matvec<1>),
-               rows_product_ctas(), 32 * kRowProductWarps, st, row_tables(), (const double*)d_rows.p,
+               rows_product_ctas(), 32 * kRowProductWarps, 0, st, row_tables(), (const double*)d_rows.p,
                (const double*)d_diag.p, lambda, x, y, xy, ctl);
     check_launch();
   }
@@ -3242,35 +3243,6 @@ struct Solver {
   // Cholesky of (S + lambda diag) -- equilibrated as scale S scale and shifted by -shift I when scale
   // is given -- into the banded tiles; true when every pivot is finite and positive.
   static constexpr size_t kMaxTileBytes = size_t(16) << 30;
-  static constexpr int kGraphColumns = 64;  // tile columns from which a column loop runs as a graph
-  // Runs a long fixed sequence of launches (a tile-column loop) as one CUDA graph: captured on the
-  // solver's stream, instantiated, launched and waited for, so the device runs the columns back to
-  // back whatever the host is doing meanwhile.
-  template <typename Body>
-  void run_as_graph(Body body) {
-    if (S.nt < kGraphColumns) {  // short loops: capture and instantiation would cost more than they save
-      body();
-      return;
-    }
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    CUDA_OK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    body();
-    const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-    if (ce != cudaSuccess) {
-      if (graph) cudaGraphDestroy(graph);
-      CUDA_OK(ce);
-    }
-    const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
-    CUDA_OK(ie);
-    const cudaError_t le = cudaGraphLaunch(exec, st);
-    const cudaError_t se = cudaStreamSynchronize(st);
-    cudaGraphExecDestroy(exec);
-    CUDA_OK(le);
-    CUDA_OK(se);
-  }
-
   // With check false the status stays on the device: the kernels after a failed factorization return at
   // once, and the caller reads d_status with its next results.
   bool factor_band(double lambda, const double* scale, double shift, bool check = true) {
@@ -3286,14 +3258,14 @@ struct Solver {
     const TileBand tb = tile_band();
     OMVGBA_LAUNCH(k_rows_to_tiles, grid_for(8 * S.nbr.size(), 128), 128, 0, st, row_tables(), d_rows.p, d_perm_off.p,
                   d_diag.p, lambda, scale, shift, tb, d_status.p);
-    run_as_graph([&] {
-      OMVGBA_LAUNCH(k_tile_potrf, 1, 256, kPotrfSmem, st, tb, 0, d_status.p);
-      for (int k = 0; k < S.nt - 1; ++k) {  // each update factors the next diagonal tile
-        const int m = std::min(S.bwt, S.nt - 1 - k);
-        OMVGBA_LAUNCH(k_tile_trsm, m, 256, kTrsmSmem, st, tb, k, d_status.p);
-        OMVGBA_LAUNCH(k_tile_update, m * (m + 1) / 2, 256, kUpdateSmem, st, tb, k, d_status.p);
-      }
-    });
+    // Each update factors the next diagonal tile. The launches overlap: a graph of the loop cost its capture
+    // and instantiation on every factorization.
+    OMVGBA_LAUNCH(k_tile_potrf, 1, 256, kPotrfSmem, st, tb, 0, d_status.p);
+    for (int k = 0; k < S.nt - 1; ++k) {
+      const int m = std::min(S.bwt, S.nt - 1 - k);
+      launch_pdl(true, k_tile_trsm, m, 256, kTrsmSmem, st, tb, k, (const int*)d_status.p);
+      launch_pdl(true, k_tile_update, m * (m + 1) / 2, 256, kUpdateSmem, st, tb, k, d_status.p);
+    }
     check_launch();
     if (!check) return true;
     int ok = 0;
@@ -3377,19 +3349,18 @@ struct Solver {
     const size_t npart = (size_t)std::max(S.bwt, 1) * std::max(max_split, 1) * kCTT;
     if (d_zpart.n != npart) d_zpart.alloc(npart, st);
     if (d_zq.n != (size_t)std::max(S.bwt, 1) * kCTT) d_zq.alloc((size_t)std::max(S.bwt, 1) * kCTT, st);
-    run_as_graph([&] {
-      for (int j = S.nt - 1; j >= 0; --j) {
-        const int m = std::min(S.bwt, S.nt - 1 - j);
-        if (m > 0) {
-          const int nsplit = (m + kTakahashiChunk - 1) / kTakahashiChunk;
-          OMVGBA_LAUNCH(k_takahashi_partial, dim3(m, nsplit), 256, kTakahashiSmem, st, tl, tz, j, d_zpart.p,
-                        d_status.p);
-          OMVGBA_LAUNCH(k_takahashi_offdiag, m, 256, kTakahashiSmem, st, tl, tz, j, nsplit, d_zpart.p, d_zq.p,
-                        d_status.p);
-        }
-        OMVGBA_LAUNCH(k_takahashi_diag, kTakahashiDiagCtas, 256, kTakahashiSmem, st, tl, tz, j, m, d_zq.p, d_status.p);
+    for (int j = S.nt - 1; j >= 0; --j) {
+      const int m = std::min(S.bwt, S.nt - 1 - j);
+      const int* status = d_status.p;
+      if (m > 0) {
+        const int nsplit = (m + kTakahashiChunk - 1) / kTakahashiChunk;
+        launch_pdl(true, k_takahashi_partial, dim3(m, nsplit), 256, kTakahashiSmem, st, tl, tz, j, d_zpart.p, status);
+        launch_pdl(true, k_takahashi_offdiag, m, 256, kTakahashiSmem, st, tl, tz, j, nsplit,
+                   (const double*)d_zpart.p, d_zq.p, status);
       }
-    });
+      launch_pdl(j < S.nt - 1, k_takahashi_diag, kTakahashiDiagCtas, 256, kTakahashiSmem, st, tl, tz, j, m,
+                 (const double*)d_zq.p, status);
+    }
     DBuf<int> d_pos, d_dims;
     d_pos.upload(pos.data(), pos.size(), st);
     d_dims.upload(dims.data(), dims.size(), st);
@@ -3448,7 +3419,7 @@ struct Solver {
     const int split = finalize_split(nb);
     // a dependent launch of the tile pass, inside a graph or not: it orders itself with pdl_wait
     launch_pdl(true, split == 8 ? k_mv_tiles_finalize<8> : (split == 4 ? k_mv_tiles_finalize<4> : k_mv_tiles_finalize<1>),
-               mv_finalize_ctas(), 32 * kFinalizeWarps, st, mt, ts.partial.p, d_diag.p, lambda, x, y, xy, ctl);
+               mv_finalize_ctas(), 32 * kFinalizeWarps, 0, st, mt, ts.partial.p, d_diag.p, lambda, x, y, xy, ctl);
     check_launch();
   }
   // The tile pass of the product alone: the per-(segment, parameter) partials.
@@ -3457,13 +3428,13 @@ struct Solver {
     MvTiles mt = ts.view(d_blk_dim.p, d_blk_off.p, nb);
     if (mt.ntiles > 0) {
       if (fp32)
-        launch_pdl(pdl, k_mv_tiles<float, float>, mt.ntiles, mv_tile_obs<float>(), st, mt, d_rec32.p, d_vfac.p, x,
+        launch_pdl(pdl, k_mv_tiles<float, float>, mt.ntiles, mv_tile_obs<float>(), 0, st, mt, d_rec32.p, d_vfac.p, x,
                    ts.partial.p, ctl);
       else if (mixed)  // FP64 arithmetic on the FP32 records: the refinement's residual product
-        launch_pdl(pdl, k_mv_tiles<float, double>, mt.ntiles, mv_tile_obs<float>(), st, mt, d_rec32.p, d_vfac.p, x,
+        launch_pdl(pdl, k_mv_tiles<float, double>, mt.ntiles, mv_tile_obs<float>(), 0, st, mt, d_rec32.p, d_vfac.p, x,
                    ts.partial.p, ctl);
       else
-        launch_pdl(pdl, k_mv_tiles<T, T>, mt.ntiles, mv_tile_obs<T>(), st, mt, d_rec.p, d_vfac.p, x, ts.partial.p,
+        launch_pdl(pdl, k_mv_tiles<T, T>, mt.ntiles, mv_tile_obs<T>(), 0, st, mt, d_rec.p, d_vfac.p, x, ts.partial.p,
                    ctl);
     }
   }
@@ -3536,9 +3507,9 @@ struct Solver {
       const int slot = it & 1;
       matvec(d_dir.p, d_q.p, 0.0, dctl, fp32, d_dq.p, it > 0, true);
       const int nupd = grid_for(nb, kUpdThreads);
-      launch_pdl(true, k_pcg_update_precond, nupd, kUpdThreads, st, tables(), d_factor.p, d_dq.p, product_ctas(),
+      launch_pdl(true, k_pcg_update_precond, nupd, kUpdThreads, 0, st, tables(), d_factor.p, d_dq.p, product_ctas(),
                  d_dir.p, d_q.p, x, d_r.p, d_z.p, d_rr_part.p, d_rz_part.p, slot, dctl);
-      launch_pdl(true, k_pcg_direction, grid_for(D, 256), 256, st, D, d_rr_part.p, d_rz_part.p, nupd, d_z.p, d_dir.p,
+      launch_pdl(true, k_pcg_direction, grid_for(D, 256), 256, 0, st, D, d_rr_part.p, d_rz_part.p, nupd, d_z.p, d_dir.p,
                  slot, dctl);
     }
     const cudaError_t ce = cudaStreamEndCapture(st, &graph);
