@@ -791,35 +791,37 @@ __device__ __forceinline__ void solve_sweep(const TileBand& tb, double* v, const
   };
   auto load_w = [&](int k, double m[16]) { load(tb.w + (size_t)actual(k) * kCTT, m); };
   auto partial = [&](const double m[16], const double* x) {
-    if (FORWARD) {
+    if constexpr (FORWARD) {
       double s = 0.0;
 #pragma unroll
       for (int c = 0; c < 16; ++c) s += m[c] * x[16 * qtr + c];
       return s;
+    } else {
+      double s[8];  // rows i and i + 32, then a balanced sum
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s[j] = m[j] * x[4 * j + (tid & 3)] + m[j + 8] * x[4 * j + (tid & 3) + 32];
+#pragma unroll
+      for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+        for (int j = 0; j < h; ++j) s[j] += s[j + h];
+      return s[0];
     }
-    double s[8];  // rows i and i + 32, then a balanced sum
-#pragma unroll
-    for (int j = 0; j < 8; ++j) s[j] = m[j] * x[4 * j + (tid & 3)] + m[j + 8] * x[4 * j + (tid & 3) + 32];
-#pragma unroll
-    for (int h = 4; h > 0; h >>= 1)
-#pragma unroll
-      for (int j = 0; j < h; ++j) s[j] += s[j + h];
-    return s[0];
   };
   int used = 0;
   auto total = [&](double s) {  // entry r of the product, in every thread
     double* part = sh.part[used];
     used ^= 1;  // the buffer's next use lies after the next barrier
-    if (FORWARD) {
+    if constexpr (FORWARD) {
       part[tid] = s;
       __syncthreads();
       return ((part[r] + part[kCT + r]) + part[2 * kCT + r]) + part[3 * kCT + r];
+    } else {
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      if ((tid & 3) == 0) part[tid >> 2] = s;
+      __syncthreads();
+      return part[r];
     }
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    if ((tid & 3) == 0) part[tid >> 2] = s;
-    __syncthreads();
-    return part[r];
   };
   // The entry of the i-th tile that this thread keeps (threads 0 to 63).
   auto own = [&](int i) { return tid < kCT && actual(i) * kCT + tid < tb.n; };
@@ -906,31 +908,55 @@ __global__ void __launch_bounds__(256) k_tile_solve(TileBand tb, double* v, cons
 
 // ---- selected inverse within the band (intrinsic marginal covariances) -----------------------
 // Z = S^-1 restricted to the band of the factor, by the Takahashi recurrence on tiles, from the last
-// tile column to the first: with Z L = L^-T,
-//   Z_ij = -(sum_{k=j+1}^{j+bwt} Z_ik L_kj) L_jj^-1                      (i > j)
-//   Z_jj = (L_jj^-T - sum_{k=j+1}^{j+bwt} Z_kj^T L_kj) L_jj^-1
+// tile column to the first: with Z L = L^-T, W_j = L_jj^-1 and M_kj = L_kj W_j,
+//   Z_ij = -sum_{k=j+1}^{j+bwt} Z_ik M_kj                      (i > j)
+//   Z_jj = W_j^T W_j - sum_{k=j+1}^{j+bwt} Z_kj^T M_kj
 // where Z_ik for i < k is Z_ki^T; every Z_ik needed lies in the band. The marginal covariance of a
 // group is the block of Z at its parameters' positions (sparse/covariance.rs:564-587 gets the same
 // block by solving S x = e_p column by column).
 //
-// Column j runs as three launches, so that the column's 64 x 64 products spread over the GPU:
-//  k_takahashi_partial  CTA (b, s): part(b, s) = sum over k in chunk s of Z_ik L_kj, i = j + 1 + b,
+// The products with W_j lie outside the chain of columns, in one launch over all tiles; column j then runs
+// as three launches, each in place when the one before ends, so that the column's 64 x 64 products spread
+// over the GPU:
+//  k_takahashi_scale    CTA per tile of the band, in place of the factor: M_kj, and W_j^T W_j on the diagonal
+//  k_takahashi_partial  CTA (b, s): part(b, s) = sum over k in chunk s of Z_ik M_kj, i = j + 1 + b,
 //                       chunks of kTakahashiChunk consecutive k in order
-//  k_takahashi_offdiag  CTA b: Z_ij = -(sum_s part(b, s)) W_j, and its share of the diagonal sum,
-//                       q(b) = Z_ij^T L_ij
-//  k_takahashi_diag     CTA r: rows 8 r .. 8 r + 7 of Z_jj = (W_j^T - sum_b q(b)) W_j
+//  k_takahashi_offdiag  CTA b: Z_ij = -sum_s part(b, s), and its share of the diagonal sum,
+//                       q(b) = Z_ij^T M_ij
+//  k_takahashi_diag     Z_jj = W_j^T W_j - sum_b q(b), an element per thread
 // Every sum runs in a fixed order, so Z does not depend on scheduling. Dynamic shared memory:
-// kTakahashiSmem (two staged operands).
+// kTakahashiSmem (two staged operands). Bound: the chain of columns, each the latency of three launches and
+// two tile products (at a band of 35 tiles the partial sums' products on the tensor pipe). With the products
+// with W_j inside the columns these took, at a band of 14 tiles, 16 + 21 + 9 us a column, and 35 + 29 + 14 at
+// a band of 35; now 16 + 11 + 6.5 and 34 + 18 + 7.5.
 constexpr size_t kTakahashiSmem = 2 * kStagedTile;
 constexpr int kTakahashiChunk = 4;
-constexpr int kTakahashiDiagCtas = 8;
+constexpr int kTakahashiDiagThreads = 64;
 
+__global__ void __launch_bounds__(256) k_takahashi_scale(TileBand L, const int* status) {
+  extern __shared__ __align__(16) double sh[];
+  if (status[0] == 0) return;
+  const int j = blockIdx.x, i = j + blockIdx.y;
+  if (i >= L.nt) return;
+  double* Ta = sh;
+  double* Tb = sh + kCT * kTS;
+  double* out = L.t + tile_at(L, i, j);
+  stage_tile(L.w + (size_t)j * kCTT, Tb);
+  if (i > j) stage_tile(out, Ta);
+  stage_wait();
+  __syncthreads();
+  TileAcc acc;
+  zero_acc(acc);
+  if (i > j)
+    tile_mma_acc<false, false>(Ta, Tb, acc);
+  else
+    tile_mma_acc<true, false>(Tb, Tb, acc);
+  acc_store(acc, out);
+}
 __global__ void __launch_bounds__(256) k_takahashi_partial(TileBand L, TileBand Z, int j, double* part,
                                                            const int* status) {
   extern __shared__ __align__(16) double sh[];
   pdl_trigger();
-  pdl_wait();
-  if (status[0] == 0) return;
   double* Ta = sh;
   double* Tb = sh + kCT * kTS;
   const int i = j + 1 + blockIdx.x;
@@ -938,10 +964,16 @@ __global__ void __launch_bounds__(256) k_takahashi_partial(TileBand L, TileBand 
   const int k0 = j + 1 + kTakahashiChunk * blockIdx.y, k1 = min(kmax, k0 + kTakahashiChunk - 1);
   TileAcc acc;
   zero_acc(acc);
+  stage_tile(L.t + tile_at(L, k0, j), Tb);  // M is there before the column loop begins
+  pdl_wait();
+  if (status[0] == 0) {
+    stage_wait();
+    return;
+  }
   for (int k = k0; k <= k1; ++k) {
     __syncthreads();
     stage_tile(Z.t + (i >= k ? tile_at(Z, i, k) : tile_at(Z, k, i)), Ta);  // Z_ik, or Z_ki for its transpose
-    stage_tile(L.t + tile_at(L, k, j), Tb);
+    if (k > k0) stage_tile(L.t + tile_at(L, k, j), Tb);
     stage_wait();
     __syncthreads();
     if (i >= k)
@@ -957,64 +989,48 @@ __global__ void __launch_bounds__(256) k_takahashi_offdiag(TileBand L, TileBand 
                                                            const int* status) {
   extern __shared__ __align__(16) double sh[];
   pdl_trigger();
-  pdl_wait();
-  if (status[0] == 0) return;
   double* Ta = sh;
   double* Tb = sh + kCT * kTS;
   const int i = j + 1 + blockIdx.x;
-  stage_tile(L.w + (size_t)j * kCTT, Tb);  // W_j
-  // -(sum of the partial tiles, in order) into the A operand
+  stage_tile(L.t + tile_at(L, i, j), Tb);  // M_ij, there before the column loop begins
+  pdl_wait();
+  if (status[0] == 0) {
+    stage_wait();
+    return;
+  }
+  // Z_ij = -(sum of the partial tiles, in order)
   const double* pb = part + (size_t)blockIdx.x * nsplit * kCTT;
-#pragma unroll 4
-  for (int w = threadIdx.x; w < kCTT; w += 256) {
-    double v = 0.0;
-    for (int s = 0; s < nsplit; ++s) v += pb[(size_t)s * kCTT + w];
-    Ta[(w >> 6) * kTS + (w & 63)] = -v;
+  double* z = Z.t + tile_at(Z, i, j);
+  double v[kCTT / 256];
+#pragma unroll
+  for (int e = 0; e < kCTT / 256; ++e) v[e] = 0.0;
+  for (int s = 0; s < nsplit; ++s)
+#pragma unroll
+    for (int e = 0; e < kCTT / 256; ++e) v[e] += pb[(size_t)s * kCTT + 256 * e + threadIdx.x];
+#pragma unroll
+  for (int e = 0; e < kCTT / 256; ++e) {
+    const int w = 256 * e + threadIdx.x;
+    Ta[(w >> 6) * kTS + (w & 63)] = -v[e];
+    z[w] = -v[e];
   }
   stage_wait();
   __syncthreads();
   TileAcc acc;
   zero_acc(acc);
-  tile_mma_acc<false, false>(Ta, Tb, acc);
-  acc_store(acc, Z.t + tile_at(Z, i, j));
-  __syncthreads();
-  stage_tile(L.t + tile_at(L, i, j), Tb);  // L_ij
-  acc_each(acc, [&](int r, int c, double v) { Ta[c * kTS + r] = v; });
-  stage_wait();
-  __syncthreads();
-  zero_acc(acc);
-  tile_mma_acc<true, false>(Ta, Tb, acc);  // Z_ij^T L_ij
+  tile_mma_acc<true, false>(Ta, Tb, acc);  // Z_ij^T M_ij
   acc_store(acc, q + (size_t)blockIdx.x * kCTT);
 }
-
-// The diagonal tile's sum over the column's m shares reads m tiles: split by rows over eight CTAs (at
-// m = 14 one CTA took 45.5 us, the eight take 9.1).
-__global__ void __launch_bounds__(256) k_takahashi_diag(TileBand L, TileBand Z, int j, int m,
-                                                        const double* __restrict__ q, const int* status) {
-  extern __shared__ __align__(16) double sh[];
+__global__ void __launch_bounds__(kTakahashiDiagThreads) k_takahashi_diag(TileBand L, TileBand Z, int j, int m,
+                                                                          const double* __restrict__ q,
+                                                                          const int* status) {
   pdl_trigger();
   pdl_wait();
   if (status[0] == 0) return;
-  double* Ta = sh;             // 8 rows x 64: element (r, c) at c * 12 + r
-  double* Tb = sh + kCT * 12;
-  const int r0 = 8 * blockIdx.x, tid = threadIdx.x;
-  const double* wj = L.w + (size_t)j * kCTT;
-  stage_tile(wj, Tb);
-  for (int w = tid; w < 8 * kCT; w += 256) {
-    const int c = w >> 3, r = w & 7;
-    double v = 0.0;
-    for (int b = 0; b < m; ++b) v += q[(size_t)b * kCTT + c * kCT + r0 + r];
-    Ta[c * 12 + r] = wj[(size_t)(r0 + r) * kCT + c] - v;  // W_j^T(r, c) = W_j(c, r)
-  }
-  stage_wait();
-  __syncthreads();
-  const int lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
-  double c0 = 0.0, c1 = 0.0;
-  mma8(kCT, [&](int r, int kk) { return Ta[kk * 12 + r]; },
-       [&](int kk, int c) { return Tb[(8 * w + c) * kTS + kk]; }, c0, c1);
-  double* out = Z.t + tile_at(Z, j, j) + (size_t)(8 * w + 2 * t) * kCT + r0 + g;
-  out[0] = c0;
-  out[kCT] = c1;
+  const int w = blockIdx.x * kTakahashiDiagThreads + threadIdx.x;
+  double v = 0.0;
+#pragma unroll 8
+  for (int b = 0; b < m; ++b) v += q[(size_t)b * kCTT + w];
+  Z.t[tile_at(Z, j, j) + w] = L.t[tile_at(L, j, j) + w] - v;
 }
 
 // (S^-1)_gg of each free group from Z: 9 values per group (row-major), thread per group.

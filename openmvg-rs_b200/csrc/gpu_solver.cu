@@ -3341,7 +3341,7 @@ struct Solver {
     if (d_ztiles.n != count) d_ztiles.alloc(count, st);
     CUDA_OK(cudaFuncSetAttribute(k_takahashi_partial, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakahashiSmem));
     CUDA_OK(cudaFuncSetAttribute(k_takahashi_offdiag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakahashiSmem));
-    CUDA_OK(cudaFuncSetAttribute(k_takahashi_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakahashiSmem));
+    CUDA_OK(cudaFuncSetAttribute(k_takahashi_scale, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakahashiSmem));
     const TileBand tl = tile_band();
     const TileBand tz{D, S.nt, S.bwt, d_ztiles.p, nullptr};
     // scratch: the split partial sums of one column and the diagonal shares of its tiles
@@ -3349,17 +3349,19 @@ struct Solver {
     const size_t npart = (size_t)std::max(S.bwt, 1) * std::max(max_split, 1) * kCTT;
     if (d_zpart.n != npart) d_zpart.alloc(npart, st);
     if (d_zq.n != (size_t)std::max(S.bwt, 1) * kCTT) d_zq.alloc((size_t)std::max(S.bwt, 1) * kCTT, st);
+    const int* status = d_status.p;
+    OMVGBA_LAUNCH(k_takahashi_scale, dim3(S.nt, S.bwt + 1), 256, kTakahashiSmem, st, tl, status);
     for (int j = S.nt - 1; j >= 0; --j) {
       const int m = std::min(S.bwt, S.nt - 1 - j);
-      const int* status = d_status.p;
       if (m > 0) {
         const int nsplit = (m + kTakahashiChunk - 1) / kTakahashiChunk;
         launch_pdl(true, k_takahashi_partial, dim3(m, nsplit), 256, kTakahashiSmem, st, tl, tz, j, d_zpart.p, status);
         launch_pdl(true, k_takahashi_offdiag, m, 256, kTakahashiSmem, st, tl, tz, j, nsplit,
                    (const double*)d_zpart.p, d_zq.p, status);
       }
-      launch_pdl(j < S.nt - 1, k_takahashi_diag, kTakahashiDiagCtas, 256, kTakahashiSmem, st, tl, tz, j, m,
-                 (const double*)d_zq.p, status);
+      // the first waits for the scaled factor, which the kernels of later columns read before their wait
+      launch_pdl(j < S.nt - 1, k_takahashi_diag, kCTT / kTakahashiDiagThreads, kTakahashiDiagThreads, 0, st, tl, tz, j,
+                 m, (const double*)d_zq.p, status);
     }
     DBuf<int> d_pos, d_dims;
     d_pos.upload(pos.data(), pos.size(), st);

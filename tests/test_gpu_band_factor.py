@@ -21,7 +21,7 @@ def _ring(cameras, dims):
     return synthetic.ring_problem(seed=8, cameras=cameras, points=400, pose_variables=masks)
 
 
-@pytest.mark.parametrize("cameras,dims", [(8, 6), (8, 9), (13, 63), (13, 66), (23, 129), (36, 192), (60, 351)])
+@pytest.mark.parametrize("cameras,dims", [(8, 6), (8, 9), (13, 63), (13, 66), (23, 129), (36, 192), (60, 351), (122, 723)])
 def test_direct_step_matches_oracle(adjuster, cameras, dims):
     p = _ring(cameras, dims)
     cfg = SolveConfig(linear_solver=abi.SOLVER_DIRECT, max_iterations=2)
