@@ -6,8 +6,8 @@
 // one CTA per parameter block X computes every block S_XY of its row (all co-visible blocks Y, both
 // triangles), walking X's entities in a fixed order and the entities of each entity's point, so the
 // row is the same bits run to run, needs no atomics and no storage beyond the rows. The rows serve as
-// a block-sparse (BSR) operator directly (the PCG product and the model reduction) and are scattered into a banded tiled
-// matrix for the factorization.
+// a block-sparse (BSR) operator directly (the PCG product and the model reduction) and are scattered
+// into a banded tiled matrix for the factorization.
 //
 // Factorization. The parameter blocks are permuted so that each camera's pose block is followed by
 // the intrinsic blocks it introduces; with cameras in their native order the co-visibility graph of

@@ -8,9 +8,11 @@
 //   K2  k_block_tiles ...... camera-side deterministic segmented sums over the record tiles: U blocks,
 //       k_block_records      g, reduced g, damping diagonal, pose/intrinsic edges, diagonal point
 //                            coupling (asm_tiles.cuh)
-//       k_pairs ............ explicit Schur blocks S_bb' -= W V^-1 W^T (schur/assembly.rs:999-1038)
-//   K3  k_block_rows ....... explicit S by block rows (BSR), banded tiled FP64 Cholesky and solves
-//                            (explicit_s.cuh; stands in for faer's sparse LLT)
+//   K3  k_pair_operands, ... explicit S (BSR) from camera pairs, S_XY -= W V^-1 W^T (pair_rows.cuh;
+//       k_pair_products,     schur/assembly.rs:999-1038); k_block_rows where the pair tables do not fit
+//       k_pair_gather
+//       k_tile_* ........... banded tiled FP64 Cholesky and solves (explicit_s.cuh; stands in for faer's
+//                            sparse LLT)
 //       k_mv_tiles ......... matrix-free reduced-camera-system product S x (retained/operator.rs:137-227)
 //       block-Jacobi PCG ... sparse/pcg.rs:23-119, retained/mod.rs:682-934, retained/block.rs:148-246
 //   K4  k_retract, k_candidate_tiles: step cap, retraction, back-substitution and candidate rule
@@ -2432,8 +2434,9 @@ struct TileSetDev {
 };
 
 // Auto operator switch: a PCG run of at least this many products moves the rest of the solve to the
-// explicit S. One build of the rows costs about as much as this many tile products on the survey
-// grids (plane500: ~2 ms of rows against ~60 us per product, the explicit product ~25 us).
+// explicit S. On the survey grids a build costs as much as the tile products of a shorter run save
+// (plane500: 0.7 ms a build, 38 us against 16 us a product: 32; plane3000: 6.6 ms, 315 against 39 us: 24), and
+// the runs of a solve differ by about a factor of two, so the line lies where the next runs still gain.
 constexpr uint64_t kExplicitSwitchTerms = 64;
 
 template <typename T>
@@ -2565,7 +2568,7 @@ struct Solver {
       if (!n.self_cal && !n.angular && n.translation_only) opt.iterative = false;
     }
     direct = !opt.iterative;
-    // the PCG operator: the explicit S by block rows (rebuilt every assembly, a block-sparse product
+    // the PCG operator: the explicit S (rebuilt every assembly, a block-sparse product
     // that stays in L2) or the matrix-free tile product over the Jacobian records
     // (Auto starts matrix-free, see kExplicitSwitchTerms, except where a whole FP64 PCG run fits one cluster)
     pcg_loop = fits_pcg_loop();
