@@ -67,3 +67,40 @@ def test_plan_product_of_an_explicit_operator(adjuster):
             out.append(y)
     for y in out[:2]:
         assert float((y - out[2]).abs().max()) <= 1e-9 * float(out[2].abs().max())
+
+
+def _unobserved_pose():
+    p = _ring(20)
+    return _without(p, p.observation_pose == 5)
+
+
+def _unobserved_group():
+    p = _ring(20, self_calibrating=True)
+    p.intrinsics = p.intrinsics + [p.intrinsics[0]]  # free, and no observation names it
+    return p
+
+
+def _without(p, drop):
+    for k in ("observation_pose", "observation_intrinsic", "observation_point", "observation_pixel"):
+        setattr(p, k, getattr(p, k)[~drop])
+    return p
+
+
+@pytest.mark.parametrize("case", [_unobserved_pose, _unobserved_group])
+@pytest.mark.parametrize("limit", [0, 3])
+def test_a_free_block_without_observations(adjuster, case, limit):
+    """Its row of S is empty: the product there is lambda diag x and its step is zero, in the cluster kernel
+    as in the matrix-free product; the rank test sees a zero row whichever operator took the steps."""
+    p = case()
+    cfg = SolveConfig(linear_solver=abi.SOLVER_ITERATIVE, max_iterations=6, pcg_relative_tolerance=1e-10,
+                      pcg_max_iterations=limit)
+    a = adjuster.solve(p, cfg)
+    b = adjuster.solve(p, cfg.with_(matvec=abi.MATVEC_IMPLICIT))
+    for k in ("iteration_count", "accepted_step_count", "rejected_step_count", "rejected_step_solve", "status",
+              "pcg_iteration_count", "observability", "unconstrained_intrinsic_count"):
+        assert a.report[k] == b.report[k], (k, a.report[k], b.report[k])
+    assert abs(a.report["final_objective"] - b.report["final_objective"]) <= 1e-9 * b.report["final_objective"]
+    assert np.max(np.abs(a.rotations - b.rotations)) < 1e-7 and np.max(np.abs(a.centers - b.centers)) < 1e-7
+    assert np.max(np.abs(a.points - b.points)) < 1e-7
+    again = adjuster.solve(p, cfg)
+    assert np.array_equal(a.points, again.points) and np.array_equal(a.centers, again.centers)
