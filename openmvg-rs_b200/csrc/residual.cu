@@ -416,7 +416,9 @@ __global__ void k_vjp_finish(Accum acc, uint64_t ncam, const float* __restrict__
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
       const float col = c == 0 ? Jl[3 * r] : (c == 1 ? Jl[3 * r + 1] : Jl[3 * r + 2]);
-      val += (double)col * component_sum(acc, kCamComps * j + r, bad);
+      const double s = component_sum(acc, kCamComps * j + r, bad);
+      // a camera without contributions may have no finite Jl (its rotation vector is not finite)
+      if (s != 0.0) val += (double)col * s;
     }
     g_rot[3 * j + c] += (float)val;
   } else {

@@ -85,3 +85,21 @@ def test_adjoint_of_crowded_accumulators(observations, cameras, points):
     want = torch.autograd.grad(res, leaves, f32(g).double())
     for a, b in zip(got, want):
         assert float(torch.linalg.vector_norm(a.double() - b)) <= 2e-4 * float(torch.linalg.vector_norm(b)) + 1e-12
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), 1e30])
+def test_adjoint_of_a_camera_without_a_finite_rotation(bad):
+    """Its observations are inadmissible, so it contributes nothing anywhere: its gradients are zero, and the
+    other cameras' are those of the call without its observations."""
+    from openmvg_ba_cuda.autograd import vjp
+    d = synthetic.residual_inputs(seed=3, observations=5000, cameras=7, points=500, dtype=np.float64)
+    cam, pt, px, rv, tr, it, X = _dev(d, torch.float32)
+    rv[2, 1] = bad
+    g = torch.ones_like(px)
+    got = vjp(cam, pt, px, rv, tr, it, X, g)
+    g[cam == 2] = 0.0
+    want = vjp(cam, pt, px, torch.nan_to_num(rv, nan=0.0, posinf=0.0).clamp(max=10.0), tr, it, X, g)
+    for a, b in zip(got[:3], want[:3]):
+        assert float(a[2].abs().max()) == 0.0
+        assert torch.equal(a, b)
+    assert torch.equal(got[3], want[3])
