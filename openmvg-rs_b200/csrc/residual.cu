@@ -495,7 +495,8 @@ int forward(void* stream, uint64_t n, const uint32_t* cam, const uint32_t* pt, c
             omvgba_error* err) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool aligned = ((reinterpret_cast<uintptr_t>(pixel) | reinterpret_cast<uintptr_t>(residual)) % (2 * sizeof(T))) == 0;
-  if (aligned && n >= kTableObservations && n >= 32 * ncam && ncam * sizeof(CamRow<T>) <= kTableMaxBytes) {
+  // (the rows first: a caller that does not know its camera count may pass any bound, also one whose products wrap)
+  if (aligned && ncam <= kTableMaxBytes / sizeof(CamRow<T>) && n >= kTableObservations && n >= 32 * ncam) {
     const size_t smem = (size_t)ncam * sizeof(CamRow<T>);
     const int threads = smem > kTableMaxBytes / 2 ? 1024 : 512;
     int dev = 0, sms = 0, per = 0;

@@ -103,3 +103,25 @@ def test_adjoint_of_a_camera_without_a_finite_rotation(bad):
         assert float(a[2].abs().max()) == 0.0
         assert torch.equal(a, b)
     assert torch.equal(got[3], want[3])
+
+
+@pytest.mark.parametrize("count", [1 << 32, 1 << 58, 1 << 59, (1 << 64) - 1])
+def test_a_camera_count_whose_products_wrap_takes_the_per_observation_forward(count):
+    """The count only bounds the indices: the arrays hold the cameras that the observations name. The same
+    bits as that kernel's, which calls of fewer observations take."""
+    import ctypes as C
+    from openmvg_ba_cuda import abi
+    from openmvg_ba_cuda._lib import lib
+    from openmvg_ba_cuda.autograd import residual_f64
+    d = synthetic.residual_inputs(seed=4, observations=EDGE, cameras=40, points=20_000, dtype=np.float64)
+    cam, pt, px, rv, tr, it, X = _dev(d, torch.float64)
+    half = EDGE // 2
+    want = torch.cat([residual_f64(cam[s].contiguous(), pt[s].contiguous(), px[s].contiguous(), rv, tr, it, X)
+                      for s in (slice(0, half), slice(half, EDGE))])
+    got, err = torch.empty_like(want), abi.Error()
+    assert lib().omvgba_residual_forward_f64(torch.cuda.current_stream().cuda_stream, EDGE, cam.data_ptr(),
+                                             pt.data_ptr(), px.data_ptr(), count, rv.data_ptr(), tr.data_ptr(),
+                                             it.data_ptr(), X.shape[0], X.data_ptr(), got.data_ptr(),
+                                             C.byref(err)) == 0
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(torch.nan_to_num(got), torch.nan_to_num(want))
