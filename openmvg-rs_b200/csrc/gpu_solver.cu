@@ -3000,15 +3000,19 @@ struct Solver {
   // caller's workspace budget leaves. Those build by block rows (k_block_rows), which needs no storage
   // of its own.
   static constexpr uint64_t kPairMaxBytes = uint64_t(48) << 30;
-  static constexpr int kPairMaxCameras = 8 * 48 * 1024;
   bool ensure_pairs() {
     if (pair_state != kPairsUnknown) return pair_state == kPairsReady;
     pair_state = kPairsUnusable;
     int widest = 0;
     for (int c = 0; c < n.ncam; ++c)
       widest = std::max(widest, L.pose_dim[c] + (n.self_cal ? L.intr_dim[n.cam_group[c]] : 0));
-    if (N == 0 || nb == 0 || widest == 0 || n.ncam > kPairMaxCameras) return false;
+    if (N == 0 || nb == 0 || widest == 0) return false;
     const int ncam = n.ncam, gw = 3 * widest;
+    // a neighbour bitmap, a bit per camera, in the shared memory that the kernel's own variables leave
+    const size_t bits = sizeof(uint32_t) * (size_t)((ncam + 31) / 32);
+    cudaFuncAttributes neighbours{};
+    CUDA_OK(cudaFuncGetAttributes(&neighbours, k_pair_neighbours));
+    if (bits > (size_t)neighbours.maxDynamicSharedSizeBytes) return false;
     uint64_t bytes = 2 * sizeof(double) * (uint64_t)N * gw + 2 * sizeof(uint32_t) * (uint64_t)N;
     auto fits = [&](uint64_t b) {
       return b <= kPairMaxBytes && (!opt.workspace_budget || workspace_bytes + b <= opt.workspace_budget);
@@ -3045,7 +3049,6 @@ struct Solver {
     t.cam_begin = d_pr_cam_begin.p;
     t.cam_obs = d_pr_cam_obs.p;
     // neighbours
-    const size_t bits = sizeof(uint32_t) * (size_t)((ncam + 31) / 32);
     full.alloc(ncam, st);
     upper.alloc(ncam, st);
     d_pr_adj_begin.alloc(ncam + 1, st);

@@ -110,3 +110,22 @@ def test_a_budget_without_room_for_the_pairs_builds_by_block_rows(adjuster):
     assert rel <= 1e-9
     assert np.max(np.abs(tight.points - free.points)) <= 1e-7
     assert np.max(np.abs(tight.centers - free.centers)) <= 1e-7
+
+
+@pytest.mark.parametrize("cameras", [393_152, 393_153, 393_216, 393_217])
+def test_camera_counts_at_the_limit_of_the_neighbour_bitmap(adjuster, cameras):
+    """A neighbour bitmap, a bit per camera, has the 48 KB of a CTA's shared memory less the kernel's own
+    variables (two words, and what the compiler aligns); S is built by block rows above that. Fixed cameras
+    that see nothing change no result."""
+    p = _ring(points=200)
+    cfg = SolveConfig(linear_solver=abi.SOLVER_DIRECT, max_iterations=3)
+    few = adjuster.solve(p, cfg)
+    more = cameras - len(p.centers)
+    p.rotations = np.concatenate([p.rotations, np.broadcast_to(np.eye(3), (more, 3, 3))])
+    p.centers = np.concatenate([p.centers, np.zeros((more, 3))])
+    p.pose_variables = np.concatenate([p.pose_variables, np.zeros(more, dtype=np.uint32)])
+    many = adjuster.solve(p, cfg)
+    assert many.report["iteration_count"] == few.report["iteration_count"]
+    assert abs(many.report["final_objective"] - few.report["final_objective"]) <= 1e-9 * few.report["final_objective"]
+    assert np.max(np.abs(many.points - few.points)) <= 1e-7
+    assert np.max(np.abs(many.centers[:len(few.centers)] - few.centers)) <= 1e-7
