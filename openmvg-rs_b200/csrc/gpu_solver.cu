@@ -418,15 +418,16 @@ struct DBuf {
   DBuf() = default;
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
-  void alloc(size_t count, cudaStream_t stream) {
-    release();
-    s = stream;
-    n = count;
-    if (count) {
-      CUDA_OK(tl_pool ? cudaMallocFromPoolAsync((void**)&p, sizeof(T) * count, tl_pool, stream)
-                      : cudaMallocAsync((void**)&p, sizeof(T) * count, stream));
-      tl_device_bytes += sizeof(T) * count;
+  void alloc(size_t count, cudaStream_t stream) { CUDA_OK(allocate(count, stream)); }
+  // false, with nothing held, when the device has no memory for it
+  bool try_alloc(size_t count, cudaStream_t stream) {
+    const cudaError_t e = allocate(count, stream);
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      return false;
     }
+    CUDA_OK(e);
+    return true;
   }
   void upload(const T* host, size_t count, cudaStream_t stream) {
     alloc(count, stream);
@@ -444,6 +445,23 @@ struct DBuf {
     n = 0;
   }
   ~DBuf() { release(); }
+
+ private:
+  cudaError_t allocate(size_t count, cudaStream_t stream) {
+    release();
+    s = stream;
+    if (count) {
+      const cudaError_t e = tl_pool ? cudaMallocFromPoolAsync((void**)&p, sizeof(T) * count, tl_pool, stream)
+                                    : cudaMallocAsync((void**)&p, sizeof(T) * count, stream);
+      if (e != cudaSuccess) {
+        p = nullptr;
+        return e;
+      }
+      tl_device_bytes += sizeof(T) * count;
+    }
+    n = count;
+    return cudaSuccess;
+  }
 };
 
 // Uploads v, or, when v holds fewer than min_count elements, a zero-padded copy of it (device
@@ -2996,13 +3014,42 @@ struct Solver {
   }
 
   // The camera-pair tables, once per solver; false when the pairs do not serve this problem: more
-  // cameras than a neighbour bitmap holds, operands and lists past kPairMaxBytes, or past what the
-  // caller's workspace budget leaves. Those build by block rows (k_block_rows), which needs no storage
-  // of its own.
+  // cameras than a neighbour bitmap holds, operands and lists past kPairMaxBytes, past what the
+  // caller's workspace budget leaves, or past the memory that the device has free. Those build by block rows
+  // (k_block_rows), which needs no storage of its own.
   static constexpr uint64_t kPairMaxBytes = uint64_t(48) << 30;
   bool ensure_pairs() {
-    if (pair_state != kPairsUnknown) return pair_state == kPairsReady;
+    if (pair_state == kPairsUnknown) {
+      pair_state = kPairsUnusable;
+      if (make_pairs())
+        pair_state = kPairsReady;
+      else
+        release_pairs();
+    }
+    return pair_state == kPairsReady;
+  }
+  // S is built by block rows from here on.
+  void release_pairs() {
     pair_state = kPairsUnusable;
+    for (DBuf<uint32_t>* d : {&d_pr_point, &d_pr_cam_begin, &d_pr_cam_obs, &d_pr_adj_begin, &d_pr_adj, &d_pr_up_begin,
+                              &d_pr_item_begin, &d_pr_item_pair, &d_pr_cont_begin, &d_pr_heavy})
+      d->release();
+    for (DBuf<uint2>* d : {&d_pr_entries, &d_pr_cont}) d->release();
+    for (DBuf<double>* d : {&d_pr_operands, &d_pr_part}) d->release();
+    d_pr_unit.release();
+    d_pr_list_begin.release();
+  }
+  // Memory that a later stage needs; the pair tables, which only save time, make room for it.
+  template <typename V>
+  void alloc_later(DBuf<V>& buffer, size_t count) {
+    if (pair_state == kPairsReady) {
+      if (buffer.try_alloc(count, st)) return;
+      release_pairs();
+      sync();
+    }
+    buffer.alloc(count, st);
+  }
+  bool make_pairs() {
     int widest = 0;
     for (int c = 0; c < n.ncam; ++c)
       widest = std::max(widest, L.pose_dim[c] + (n.self_cal ? L.intr_dim[n.cam_group[c]] : 0));
@@ -3018,6 +3065,7 @@ struct Solver {
       return b <= kPairMaxBytes && (!opt.workspace_budget || workspace_bytes + b <= opt.workspace_budget);
     };
     if (!fits(bytes)) return false;
+    auto take = [&](auto& buffer, size_t count) { return buffer.try_alloc(std::max<size_t>(count, 1), st); };
     CamPairs t{};
     t.ncam = ncam;
     t.gw = gw;
@@ -3025,21 +3073,19 @@ struct Solver {
     t.obs_cam = d_obs_cam.p;
     t.fixed_points = d_fixed_points.p;
     // cameras' observations
-    d_pr_point.alloc(N, st);
+    if (!take(d_pr_operands, (size_t)2 * N * gw) || !take(d_pr_point, N) || !take(d_pr_unit, ncam)) return false;
     OMVGBA_LAUNCH(k_pair_obs_point, grid_for(P, 256), 256, 0, st, P, d_pt_off.p, d_pr_point.p);
     t.obs_point = d_pr_point.p;
-    d_pr_unit.alloc(ncam, st);
     OMVGBA_LAUNCH(k_pair_units, grid_for(ncam, 256), 256, 0, st, ncam, d_pose_dim.p, d_cam_group.p, d_intr_dim.p,
                   n.self_cal ? 1 : 0, d_pr_unit.p);
     t.unit_dim = d_pr_unit.p;
     const int nchunks = (int)std::min<size_t>(512, ((size_t)N + 1023) / 1024);
     const uint32_t per = (uint32_t)(((size_t)N + nchunks - 1) / nchunks);
     DBuf<uint32_t> counts, total, full, upper;
-    counts.alloc((size_t)nchunks * ncam, st);
+    if (!take(counts, (size_t)nchunks * ncam) || !take(total, ncam) || !take(d_pr_cam_begin, ncam + 1) ||
+        !take(d_pr_cam_obs, N))
+      return false;
     counts.zero();
-    total.alloc(ncam, st);
-    d_pr_cam_begin.alloc(ncam + 1, st);
-    d_pr_cam_obs.alloc(N, st);
     OMVGBA_LAUNCH(k_pair_cam_sort, nchunks, 32, 0, st, (uint32_t)N, per, ncam, d_obs_cam.p, counts.p,
                   (const uint32_t*)nullptr, (uint32_t*)nullptr);
     OMVGBA_LAUNCH(k_pair_cam_prefix, grid_for(ncam, 128), 128, 0, st, ncam, nchunks, counts.p, total.p);
@@ -3049,10 +3095,8 @@ struct Solver {
     t.cam_begin = d_pr_cam_begin.p;
     t.cam_obs = d_pr_cam_obs.p;
     // neighbours
-    full.alloc(ncam, st);
-    upper.alloc(ncam, st);
-    d_pr_adj_begin.alloc(ncam + 1, st);
-    d_pr_up_begin.alloc(ncam + 1, st);
+    if (!take(full, ncam) || !take(upper, ncam) || !take(d_pr_adj_begin, ncam + 1) || !take(d_pr_up_begin, ncam + 1))
+      return false;
     OMVGBA_LAUNCH(k_pair_neighbours, ncam, 256, bits, st, t, full.p, upper.p, (uint32_t*)nullptr);
     OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, full.p, (size_t)ncam, d_pr_adj_begin.p);
     OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, upper.p, (size_t)ncam, d_pr_up_begin.p);
@@ -3063,7 +3107,7 @@ struct Solver {
     sync();
     t.adj_begin = d_pr_adj_begin.p;
     t.up_begin = d_pr_up_begin.p;
-    d_pr_adj.alloc(std::max<uint32_t>(nadj, 1), st);
+    if (!take(d_pr_adj, nadj)) return false;
     OMVGBA_LAUNCH(k_pair_neighbours, ncam, 256, bits, st, t, (uint32_t*)nullptr, (uint32_t*)nullptr, d_pr_adj.p);
     t.adj = d_pr_adj.p;
     // lists: a warp per (camera, segment of about 256 observations)
@@ -3072,10 +3116,8 @@ struct Solver {
     const size_t cells = (size_t)t.npairs * t.segs;
     DBuf<uint32_t> cell_count;
     DBuf<uint64_t> cursor;
-    cell_count.alloc(std::max<size_t>(cells, 1), st);
+    if (!take(cell_count, cells) || !take(cursor, cells + 1) || !take(d_pr_list_begin, cells + 1)) return false;
     cell_count.zero();
-    cursor.alloc(cells + 1, st);
-    d_pr_list_begin.alloc(cells + 1, st);
     OMVGBA_LAUNCH(k_pair_lists<uint32_t>, dim3(ncam, t.segs), 32, 0, st, t, cell_count.p, (uint2*)nullptr);
     OMVGBA_LAUNCH(k_pair_scan<uint64_t>, 1, 1024, 0, st, cell_count.p, cells, d_pr_list_begin.p);
     t.list_begin = d_pr_list_begin.p;
@@ -3088,20 +3130,12 @@ struct Solver {
     t.chunk = (uint32_t)std::min<uint64_t>(256, std::max<uint64_t>(32, entries / (148 * 32) / 32 * 32));
     bytes += sizeof(uint2) * entries + sizeof(double) * kPairPart * (entries / t.chunk + t.npairs) +
              sizeof(uint64_t) * cells + sizeof(uint2) * S.nbr.size();
-    if (!fits(bytes) || t.npairs >= (1u << 31)) {
-      for (DBuf<uint32_t>* d : {&d_pr_point, &d_pr_cam_begin, &d_pr_cam_obs, &d_pr_adj_begin, &d_pr_adj, &d_pr_up_begin})
-        d->release();
-      d_pr_list_begin.release();
-      d_pr_unit.release();
-      return false;
-    }
+    if (!fits(bytes) || t.npairs >= (1u << 31) || !take(d_pr_entries, entries)) return false;
     CUDA_OK(cudaMemcpyAsync(cursor.p, d_pr_list_begin.p, sizeof(uint64_t) * (cells + 1), cudaMemcpyDeviceToDevice, st));
-    d_pr_entries.alloc(std::max<uint64_t>(entries, 1), st);
     OMVGBA_LAUNCH(k_pair_lists<uint64_t>, dim3(ncam, t.segs), 32, 0, st, t, cursor.p, d_pr_entries.p);
     t.entries = d_pr_entries.p;
     DBuf<uint32_t> item_count, cont_count;
-    item_count.alloc(std::max<uint32_t>(t.npairs, 1), st);
-    d_pr_item_begin.alloc(t.npairs + 1, st);
+    if (!take(item_count, t.npairs) || !take(d_pr_item_begin, (size_t)t.npairs + 1)) return false;
     if (t.npairs > 0)
       OMVGBA_LAUNCH(k_pair_item_count, grid_for(t.npairs, 256), 256, 0, st, t, item_count.p);
     OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, item_count.p, (size_t)t.npairs, d_pr_item_begin.p);
@@ -3126,15 +3160,18 @@ struct Solver {
     }
     DBuf<uint32_t> d_bc_begin, d_bc_cams, heavy_n;
     DBuf<int> d_blk_pose, d_blk_group;
-    d_bc_begin.upload(bc_begin.data(), bc_begin.size(), st);
-    d_bc_cams.upload(bc_cams.data(), bc_cams.size(), st);
-    d_blk_pose.upload(blk_pose.data(), blk_pose.size(), st);
-    d_blk_group.upload(blk_group.data(), blk_group.size(), st);
+    auto up = [&](auto& buffer, const auto& host) {
+      if (!take(buffer, host.size())) return false;
+      CUDA_OK(copy_async(buffer.p, host.data(), sizeof(host[0]) * host.size(), cudaMemcpyHostToDevice, st));
+      return true;
+    };
+    if (!up(d_bc_begin, bc_begin) || !up(d_bc_cams, bc_cams) || !up(d_blk_pose, blk_pose) || !up(d_blk_group, blk_group))
+      return false;
     const BlockCams bc{d_bc_begin.p, d_bc_cams.p, d_blk_pose.p, d_blk_group.p, d_cam_group.p, d_pose_dim.p};
     const uint32_t slots = (uint32_t)S.nbr.size();
-    cont_count.alloc(std::max<uint32_t>(slots, 1), st);
-    d_pr_cont_begin.alloc(slots + 1, st);
-    d_pr_heavy.alloc(slots + 1, st);  // the number of heavy blocks, then the blocks
+    if (!take(cont_count, slots) || !take(d_pr_cont_begin, (size_t)slots + 1) ||
+        !take(d_pr_heavy, (size_t)slots + 1))  // the number of heavy blocks, then the blocks
+      return false;
     CUDA_OK(cudaMemsetAsync(d_pr_heavy.p, 0, sizeof(uint32_t), st));
     OMVGBA_LAUNCH(k_pair_slots, grid_for(slots, 8), 256, 0, st, t, bc, slots, d_nbr.p, d_nbr_row.p, cont_count.p,
                   (const uint32_t*)nullptr, (uint2*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr);
@@ -3145,8 +3182,8 @@ struct Solver {
     CUDA_OK(copy_async(&ncont, d_pr_cont_begin.p + slots, sizeof(ncont), cudaMemcpyDeviceToHost, st));
     sync();
     t.nitems = nitems;
-    d_pr_item_pair.alloc(std::max<uint32_t>(nitems, 1), st);
-    d_pr_cont.alloc(std::max<uint32_t>(ncont, 1), st);
+    if (!take(d_pr_item_pair, nitems) || !take(d_pr_cont, ncont) || !take(d_pr_part, (size_t)kPairPart * nitems))
+      return false;
     if (t.npairs > 0) OMVGBA_LAUNCH(k_pair_item_fill, grid_for(t.npairs, 256), 256, 0, st, t, d_pr_item_pair.p);
     t.item_pair = d_pr_item_pair.p;
     OMVGBA_LAUNCH(k_pair_slots, grid_for(slots, 8), 256, 0, st, t, bc, slots, d_nbr.p, d_nbr_row.p,
@@ -3154,8 +3191,6 @@ struct Solver {
     check_launch();
     uint32_t heavy = 0;
     CUDA_OK(copy_async(&heavy, d_pr_heavy.p, sizeof(heavy), cudaMemcpyDeviceToHost, st));
-    d_pr_operands.alloc((size_t)2 * N * gw, st);
-    d_pr_part.alloc((size_t)kPairPart * std::max<uint32_t>(nitems, 1), st);
     sync();
     heavy_ctas = heavy;
     // the tables the build does not read again
@@ -3163,7 +3198,6 @@ struct Solver {
     d_pr_cam_begin.release();
     d_pr_cam_obs.release();
     cam_pairs = t;
-    pair_state = kPairsReady;
     return true;
   }
 
@@ -3259,8 +3293,8 @@ struct Solver {
     const size_t count = (size_t)S.nt * (S.bwt + 1) * kCTT;
     if (sizeof(double) * count > kMaxTileBytes)
       throw SolveFailure{3, "the banded factor of the reduced camera system exceeds 16 GiB"};
-    if (d_tiles.n != count) d_tiles.alloc(count, st);
-    if (d_winv.n != (size_t)S.nt * kCTT) d_winv.alloc((size_t)S.nt * kCTT, st);
+    if (d_tiles.n != count) alloc_later(d_tiles, count);
+    if (d_winv.n != (size_t)S.nt * kCTT) alloc_later(d_winv, (size_t)S.nt * kCTT);
     tile_factor_attributes();  // per device and cheap: set on every factorization
     CUDA_OK(cudaMemsetAsync(d_tiles.p, 0, sizeof(double) * count, st));
     const TileBand tb = tile_band();
@@ -3346,7 +3380,7 @@ struct Solver {
     if (!factored_s && !factor_band(0.0, nullptr, 0.0)) return false;
     // selected inverse of S inside the band (Takahashi recurrence), last tile column first
     const size_t count = (size_t)S.nt * (S.bwt + 1) * kCTT;
-    if (d_ztiles.n != count) d_ztiles.alloc(count, st);
+    if (d_ztiles.n != count) alloc_later(d_ztiles, count);
     CUDA_OK(cudaFuncSetAttribute(k_takahashi_partial, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakahashiSmem));
     CUDA_OK(cudaFuncSetAttribute(k_takahashi_offdiag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakahashiSmem));
     CUDA_OK(cudaFuncSetAttribute(k_takahashi_scale, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakahashiSmem));
@@ -3355,8 +3389,8 @@ struct Solver {
     // scratch: the split partial sums of one column and the diagonal shares of its tiles
     const int max_split = (S.bwt + kTakahashiChunk - 1) / kTakahashiChunk;
     const size_t npart = (size_t)std::max(S.bwt, 1) * std::max(max_split, 1) * kCTT;
-    if (d_zpart.n != npart) d_zpart.alloc(npart, st);
-    if (d_zq.n != (size_t)std::max(S.bwt, 1) * kCTT) d_zq.alloc((size_t)std::max(S.bwt, 1) * kCTT, st);
+    if (d_zpart.n != npart) alloc_later(d_zpart, npart);
+    if (d_zq.n != (size_t)std::max(S.bwt, 1) * kCTT) alloc_later(d_zq, (size_t)std::max(S.bwt, 1) * kCTT);
     const int* status = d_status.p;
     OMVGBA_LAUNCH(k_takahashi_scale, dim3(S.nt, S.bwt + 1), 256, kTakahashiSmem, st, tl, status);
     for (int j = S.nt - 1; j >= 0; --j) {

@@ -129,3 +129,50 @@ def test_camera_counts_at_the_limit_of_the_neighbour_bitmap(adjuster, cameras):
     assert abs(many.report["final_objective"] - few.report["final_objective"]) <= 1e-9 * few.report["final_objective"]
     assert np.max(np.abs(many.points - few.points)) <= 1e-7
     assert np.max(np.abs(many.centers[:len(few.centers)] - few.centers)) <= 1e-7
+
+
+def _three_views(p):
+    keep = (np.bincount(p.observation_point, minlength=len(p.points)) >= 3)[p.observation_point]
+    points, index = np.unique(p.observation_point[keep], return_inverse=True)
+    p.points, p.point_fixed, p.observation_point = p.points[points], p.point_fixed[points], index.astype(np.uint32)
+    p.observation_pose, p.observation_intrinsic = p.observation_pose[keep], p.observation_intrinsic[keep]
+    p.observation_pixel = p.observation_pixel[keep]
+    return p
+
+
+def test_device_memory_that_others_hold_leaves_the_solve_with_block_rows(adjuster):
+    """Whatever of the pair tables the device has no room for, the solve goes on: by block rows, and with the
+    tables given back where the factor or the selected inverse needs their memory. The rest of a solve with
+    its tables was measured, the memory left to it runs from what block rows need to all of it."""
+    torch = pytest.importorskip("torch")
+    from openmvg_ba_cuda.adjuster import CudaBundleAdjuster
+    p = _three_views(synthetic.plane_problem(seed=13, cameras=250, points=60_000, mean_track=7.0, extent=70.0))
+    cfg = SolveConfig(linear_solver=abi.SOLVER_DIRECT, max_iterations=2)
+
+    def solve(room):
+        """A plan's solve with `room` bytes of device memory free at its start (None: all of it), and what it took."""
+        with CudaBundleAdjuster(0) as own, own.plan(p, cfg) as plan:
+            torch.cuda.empty_cache()
+            torch.cuda.synchronize()
+            before = torch.cuda.mem_get_info()[0]
+            filler = torch.empty(before - room, dtype=torch.uint8, device="cuda") if room else None
+            try:
+                s = plan.solve()
+                return s, before - torch.cuda.mem_get_info()[0]
+            finally:
+                del filler
+                torch.cuda.empty_cache()
+
+    want, grown = solve(None)
+    launches = set()
+    n = p.observation_count
+    assert grown > 2 * 27 * 8 * n  # the operands alone
+    for share in (0.35, 0.5, 0.6, 0.7, 0.8, 0.9, 0.95, 1.0):
+        got, _ = solve(int(share * grown) + (16 << 20))
+        launches.add(got.report["kernel_launches"])
+        for k in ("iteration_count", "accepted_step_count", "status", "observability"):
+            assert got.report[k] == want.report[k], (share, k)
+        assert abs(got.report["final_objective"] - want.report["final_objective"]) <= 1e-9 * want.report["final_objective"]
+        assert np.max(np.abs(got.points - want.points)) <= 1e-7
+    # the tightest took block rows from the start: one kernel a build and no tables
+    assert min(launches) < want.report["kernel_launches"] and len(launches) > 1
