@@ -3060,12 +3060,17 @@ struct Solver {
     cudaFuncAttributes neighbours{};
     CUDA_OK(cudaFuncGetAttributes(&neighbours, k_pair_neighbours));
     if (bits > (size_t)neighbours.maxDynamicSharedSizeBytes) return false;
-    uint64_t bytes = 2 * sizeof(double) * (uint64_t)N * gw + 2 * sizeof(uint32_t) * (uint64_t)N;
-    auto fits = [&](uint64_t b) {
-      return b <= kPairMaxBytes && (!opt.workspace_budget || workspace_bytes + b <= opt.workspace_budget);
+    // every table and temporary counts, as long as it is held; the operands, the largest, come first
+    const uint64_t before = tl_device_bytes;
+    auto take = [&](auto& buffer, size_t count) {
+      count = std::max<size_t>(count, 1);
+      const uint64_t held = tl_device_bytes - before + sizeof(*buffer.p) * (uint64_t)count;
+      if (held > kPairMaxBytes || (opt.workspace_budget && workspace_bytes + held > opt.workspace_budget)) return false;
+      return buffer.try_alloc(count, st);
     };
-    if (!fits(bytes)) return false;
-    auto take = [&](auto& buffer, size_t count) { return buffer.try_alloc(std::max<size_t>(count, 1), st); };
+    enum { kNeighbours, kUpper, kItems, kContributions, kTotals };  // sums of 32-bit counts
+    DBuf<unsigned long long> totals;
+    if (!take(totals, kTotals)) return false;
     CamPairs t{};
     t.ncam = ncam;
     t.gw = gw;
@@ -3089,27 +3094,35 @@ struct Solver {
     OMVGBA_LAUNCH(k_pair_cam_sort, nchunks, 32, 0, st, (uint32_t)N, per, ncam, d_obs_cam.p, counts.p,
                   (const uint32_t*)nullptr, (uint32_t*)nullptr);
     OMVGBA_LAUNCH(k_pair_cam_prefix, grid_for(ncam, 128), 128, 0, st, ncam, nchunks, counts.p, total.p);
-    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, total.p, (size_t)ncam, d_pr_cam_begin.p);
+    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, total.p, (size_t)ncam, d_pr_cam_begin.p,
+                  (unsigned long long*)nullptr);
     OMVGBA_LAUNCH(k_pair_cam_sort, nchunks, 32, 0, st, (uint32_t)N, per, ncam, d_obs_cam.p, counts.p,
                   (const uint32_t*)d_pr_cam_begin.p, d_pr_cam_obs.p);
     t.cam_begin = d_pr_cam_begin.p;
     t.cam_obs = d_pr_cam_obs.p;
+    counts.release();
+    total.release();
     // neighbours
     if (!take(full, ncam) || !take(upper, ncam) || !take(d_pr_adj_begin, ncam + 1) || !take(d_pr_up_begin, ncam + 1))
       return false;
     OMVGBA_LAUNCH(k_pair_neighbours, ncam, 256, bits, st, t, full.p, upper.p, (uint32_t*)nullptr);
-    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, full.p, (size_t)ncam, d_pr_adj_begin.p);
-    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, upper.p, (size_t)ncam, d_pr_up_begin.p);
+    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, full.p, (size_t)ncam, d_pr_adj_begin.p, totals.p + kNeighbours);
+    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, upper.p, (size_t)ncam, d_pr_up_begin.p, totals.p + kUpper);
     check_launch();
-    uint32_t nadj = 0;
-    CUDA_OK(copy_async(&nadj, d_pr_adj_begin.p + ncam, sizeof(nadj), cudaMemcpyDeviceToHost, st));
-    CUDA_OK(copy_async(&t.npairs, d_pr_up_begin.p + ncam, sizeof(t.npairs), cudaMemcpyDeviceToHost, st));
+    unsigned long long sums[kTotals];
+    CUDA_OK(copy_async(sums, totals.p, sizeof(sums), cudaMemcpyDeviceToHost, st));
     sync();
+    // a pair's top bit marks the transposed contribution
+    if (sums[kNeighbours] > UINT32_MAX || sums[kUpper] >= (1u << 31)) return false;
+    const uint32_t nadj = (uint32_t)sums[kNeighbours];
+    t.npairs = (uint32_t)sums[kUpper];
     t.adj_begin = d_pr_adj_begin.p;
     t.up_begin = d_pr_up_begin.p;
     if (!take(d_pr_adj, nadj)) return false;
     OMVGBA_LAUNCH(k_pair_neighbours, ncam, 256, bits, st, t, (uint32_t*)nullptr, (uint32_t*)nullptr, d_pr_adj.p);
     t.adj = d_pr_adj.p;
+    full.release();
+    upper.release();
     // lists: a warp per (camera, segment of about 256 observations)
     t.segs = (int)std::min<size_t>(256, std::max<size_t>(1, (size_t)N / ncam / 256));
     while (t.segs > 1 && (uint64_t)t.npairs * t.segs > (uint64_t(1) << 26)) t.segs /= 2;
@@ -3119,8 +3132,10 @@ struct Solver {
     if (!take(cell_count, cells) || !take(cursor, cells + 1) || !take(d_pr_list_begin, cells + 1)) return false;
     cell_count.zero();
     OMVGBA_LAUNCH(k_pair_lists<uint32_t>, dim3(ncam, t.segs), 32, 0, st, t, cell_count.p, (uint2*)nullptr);
-    OMVGBA_LAUNCH(k_pair_scan<uint64_t>, 1, 1024, 0, st, cell_count.p, cells, d_pr_list_begin.p);
+    OMVGBA_LAUNCH(k_pair_scan<uint64_t>, 1, 1024, 0, st, cell_count.p, cells, d_pr_list_begin.p,
+                  (unsigned long long*)nullptr);
     t.list_begin = d_pr_list_begin.p;
+    cell_count.release();
     check_launch();
     uint64_t entries = 0;
     CUDA_OK(copy_async(&entries, d_pr_list_begin.p + cells, sizeof(entries), cudaMemcpyDeviceToHost, st));
@@ -3128,9 +3143,7 @@ struct Solver {
     // items of at most 256 entries, fewer when that would leave less than two items per resident warp slot
     // of the chip's SMs
     t.chunk = (uint32_t)std::min<uint64_t>(256, std::max<uint64_t>(32, entries / (148 * 32) / 32 * 32));
-    bytes += sizeof(uint2) * entries + sizeof(double) * kPairPart * (entries / t.chunk + t.npairs) +
-             sizeof(uint64_t) * cells + sizeof(uint2) * S.nbr.size();
-    if (!fits(bytes) || t.npairs >= (1u << 31) || !take(d_pr_entries, entries)) return false;
+    if (!take(d_pr_entries, entries)) return false;
     CUDA_OK(cudaMemcpyAsync(cursor.p, d_pr_list_begin.p, sizeof(uint64_t) * (cells + 1), cudaMemcpyDeviceToDevice, st));
     OMVGBA_LAUNCH(k_pair_lists<uint64_t>, dim3(ncam, t.segs), 32, 0, st, t, cursor.p, d_pr_entries.p);
     t.entries = d_pr_entries.p;
@@ -3138,7 +3151,8 @@ struct Solver {
     if (!take(item_count, t.npairs) || !take(d_pr_item_begin, (size_t)t.npairs + 1)) return false;
     if (t.npairs > 0)
       OMVGBA_LAUNCH(k_pair_item_count, grid_for(t.npairs, 256), 256, 0, st, t, item_count.p);
-    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, item_count.p, (size_t)t.npairs, d_pr_item_begin.p);
+    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, item_count.p, (size_t)t.npairs, d_pr_item_begin.p,
+                  totals.p + kItems);
     t.item_begin = d_pr_item_begin.p;
     // contributions of the pairs to the blocks of S
     std::vector<uint32_t> bc_begin(nb + 1, 0), bc_cams;
@@ -3175,12 +3189,13 @@ struct Solver {
     CUDA_OK(cudaMemsetAsync(d_pr_heavy.p, 0, sizeof(uint32_t), st));
     OMVGBA_LAUNCH(k_pair_slots, grid_for(slots, 8), 256, 0, st, t, bc, slots, d_nbr.p, d_nbr_row.p, cont_count.p,
                   (const uint32_t*)nullptr, (uint2*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr);
-    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, cont_count.p, (size_t)slots, d_pr_cont_begin.p);
+    OMVGBA_LAUNCH(k_pair_scan<uint32_t>, 1, 1024, 0, st, cont_count.p, (size_t)slots, d_pr_cont_begin.p,
+                  totals.p + kContributions);
     check_launch();
-    uint32_t nitems = 0, ncont = 0;
-    CUDA_OK(copy_async(&nitems, d_pr_item_begin.p + t.npairs, sizeof(nitems), cudaMemcpyDeviceToHost, st));
-    CUDA_OK(copy_async(&ncont, d_pr_cont_begin.p + slots, sizeof(ncont), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(copy_async(sums, totals.p, sizeof(sums), cudaMemcpyDeviceToHost, st));
     sync();
+    if (sums[kItems] > UINT32_MAX || sums[kContributions] > UINT32_MAX) return false;
+    const uint32_t nitems = (uint32_t)sums[kItems], ncont = (uint32_t)sums[kContributions];
     t.nitems = nitems;
     if (!take(d_pr_item_pair, nitems) || !take(d_pr_cont, ncont) || !take(d_pr_part, (size_t)kPairPart * nitems))
       return false;

@@ -122,9 +122,11 @@ __global__ void k_pair_cam_prefix(int ncam, int nchunks, uint32_t* counts, uint3
   total[c] = run;
 }
 
-// out[0..n] = exclusive prefix sums of in[0..n), one CTA: each thread its contiguous share.
+// out[0..n] = exclusive prefix sums of in[0..n), one CTA: each thread its contiguous share. total: the sum
+// itself, where it may be past TOut.
 template <typename TOut>
-__global__ void __launch_bounds__(1024) k_pair_scan(const uint32_t* __restrict__ in, size_t n, TOut* __restrict__ out) {
+__global__ void __launch_bounds__(1024) k_pair_scan(const uint32_t* __restrict__ in, size_t n, TOut* __restrict__ out,
+                                                    unsigned long long* total) {
   __shared__ unsigned long long warp_tot[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const size_t per = (n + blockDim.x - 1) / blockDim.x, b = min(n, per * tid), e = min(n, b + per);
@@ -143,7 +145,10 @@ __global__ void __launch_bounds__(1024) k_pair_scan(const uint32_t* __restrict__
     out[i] = (TOut)run;
     run += in[i];
   }
-  if (tid == (int)blockDim.x - 1) out[n] = (TOut)run;
+  if (tid == (int)blockDim.x - 1) {
+    out[n] = (TOut)run;
+    if (total) *total = run;
+  }
 }
 
 // Neighbours of each camera: one CTA per camera marks them in a bitmap (dynamic shared memory, a bit

@@ -176,3 +176,61 @@ def test_device_memory_that_others_hold_leaves_the_solve_with_block_rows(adjuste
         assert np.max(np.abs(got.points - want.points)) <= 1e-7
     # the tightest took block rows from the start: one kernel a build and no tables
     assert min(launches) < want.report["kernel_launches"] and len(launches) > 1
+
+
+def _long_tracks_of_one_group():
+    """1,000 cameras that share one free intrinsic group and meet in most pairs: the group's blocks collect
+    every pair again."""
+    cameras, points, track = 1000, 400, 60
+    p = synthetic.ring_problem(seed=14, cameras=cameras, points=points, self_calibrating=True, radius=3.0)
+    rng = np.random.default_rng(14)
+    p.observation_pose = np.concatenate([rng.choice(cameras, track, replace=False) for _ in range(points)]).astype(np.uint32)
+    p.observation_point = np.repeat(np.arange(points), track).astype(np.uint32)
+    p.observation_intrinsic = np.zeros(points * track, dtype=np.uint32)
+    px, _ = synthetic._project(p.rotations[p.observation_pose], p.centers[p.observation_pose],
+                               p.points[p.observation_point], 500.0, 320.0, 240.0, -0.1, 0.01, 0.0)
+    p.observation_pixel = px + rng.normal(size=px.shape)
+    return p
+
+
+def _pair_table_bytes(p):
+    """The tables of the pair build that a solver keeps, for cameras of 9 parameters in one group: operands,
+    list entries, at least one partial product per pair, the neighbours, and the contributions of a pair
+    to the blocks of its poses, its poses with the group (twice) and the group itself."""
+    cameras = len(p.centers)
+    seen = np.zeros((cameras, len(p.points)), dtype=np.int64)
+    np.add.at(seen, (p.observation_pose, p.observation_point), 1)
+    meet = seen @ seen.T
+    neighbours, entries = np.count_nonzero(meet), int(np.triu(meet).sum())
+    pairs = (neighbours + cameras) // 2
+    return 2 * 27 * 8 * p.observation_count + 8 * entries + 8 * 81 * pairs + 4 * neighbours + 8 * 4 * neighbours
+
+
+@pytest.mark.parametrize("case", [_long_tracks_of_one_group, lambda: _ring(points=600)])
+def test_a_budget_holds_the_pair_tables_or_the_solve_takes_block_rows(adjuster, case):
+    """The build that a budget leaves is read from the number of launches: the smallest budget that the
+    solve is accepted with takes block rows, a large one the pairs, and the smallest one that takes the
+    pairs has room for their tables."""
+    p = case()
+    cfg = SolveConfig(linear_solver=abi.SOLVER_DIRECT, max_iterations=1)
+
+    def launches(budget):
+        try:
+            return adjuster.solve(p, cfg.with_(workspace_budget_bytes=budget)).report["kernel_launches"]
+        except Exception as e:
+            assert "budget" in str(e)
+            return 0
+
+    def smallest(low, high, good):  # to a quarter megabyte
+        while high - low > 1 << 18:
+            mid = (low + high) // 2
+            low, high = (low, mid) if good(launches(mid)) else (mid, high)
+        return high
+
+    pairs = adjuster.solve(p, cfg).report["kernel_launches"]
+    assert launches(1 << 36) == pairs
+    accepted = smallest(0, 1 << 36, lambda n: n > 0)
+    assert 0 < launches(accepted) < pairs
+    with_pairs = smallest(accepted, 1 << 36, lambda n: n == pairs)
+    if len(p.centers) == 1000:
+        assert with_pairs - (accepted - (1 << 18)) >= _pair_table_bytes(p)
