@@ -28,6 +28,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -136,9 +138,10 @@ struct PinnedStage {
 constexpr size_t kStagedCopyMax = 1u << 20;
 constexpr size_t kStagedRoom = 4u << 20;
 
-// Pinned host memory of one solver at a time: the staged copies' room, the PCG loop's status mirrors
-// (read while the next batch runs) and the results of a group of kernels (Readback). It belongs to a
-// context, so that it is pinned once and not for every solve or worker thread.
+// Pinned host memory of one call at a time: the staged copies' room, the PCG loop's status mirrors
+// (read while the next batch runs) and the results of a group of kernels (Readback). A context keeps one
+// for each of the calls that have run on it at the same time, so that it is pinned once and not for every
+// solve or worker thread.
 // Staged host->device copies take successive places in the room; the stream is waited for only when the
 // room is used up (or belongs to another stream), so a set-up's many small tables queue up behind each
 // other. A device->host copy waits anyway and starts the room over.
@@ -164,7 +167,7 @@ struct HostStage {
   }
 };
 thread_local HostStage tl_own_stage;           // callers without a context
-thread_local HostStage* tl_stage = nullptr;    // the stage of the context in use (ContextScope)
+thread_local HostStage* tl_stage = nullptr;    // the stage of the call in progress (ContextScope)
 thread_local cudaMemPool_t tl_pool = nullptr;  // its device memory pool
 inline HostStage& host_stage() { return tl_stage ? *tl_stage : tl_own_stage; }
 
@@ -336,7 +339,8 @@ inline cudaError_t copy_async(void* dst, const void* src, size_t bytes, cudaMemc
 struct Context {
   int device = 0;
   cudaStream_t stream = nullptr;
-  HostStage stage;
+  std::mutex mutex;
+  std::vector<std::unique_ptr<HostStage>> stages;  // those no call holds
   // Device memory of the solves: kept between solves up to kPoolKept bytes (the device's default pool
   // returns everything at each wait, and every solve then maps its memory anew), given back with the
   // context.
@@ -344,18 +348,34 @@ struct Context {
 };
 constexpr uint64_t kPoolKept = uint64_t(256) << 20;
 
-// The calling thread works for context `c`: its pinned stage and memory pool.
+// The calling thread works for context `c`: its memory pool, and a pinned stage of its own until the scope
+// ends (plans of one context may be solved from several threads at a time).
 struct ContextScope {
+  Context* context;
+  std::unique_ptr<HostStage> own;
   HostStage* stage = tl_stage;
   cudaMemPool_t pool = tl_pool;
-  explicit ContextScope(Context* c) {
-    tl_stage = &c->stage;
+  explicit ContextScope(Context* c) : context(c) {
+    {
+      std::lock_guard<std::mutex> lock(c->mutex);
+      if (!c->stages.empty()) {
+        own = std::move(c->stages.back());
+        c->stages.pop_back();
+      }
+    }
+    if (!own) own = std::make_unique<HostStage>();
+    tl_stage = own.get();
     tl_pool = c->pool;
   }
   ~ContextScope() {
-    (void)tl_stage->settle();
+    (void)own->settle();
     tl_stage = stage;
     tl_pool = pool;
+    std::lock_guard<std::mutex> lock(context->mutex);
+    try {
+      context->stages.push_back(std::move(own));
+    } catch (const std::bad_alloc&) {  // the stage goes instead
+    }
   }
 };
 
