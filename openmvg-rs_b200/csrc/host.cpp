@@ -1931,7 +1931,9 @@ int write_error(omvgba_error* e, int code, const std::string& msg) {
 
 struct omvgba_context {
   omvgba::Context* ctx;
-  std::vector<omvgba::Context*> workers;  // of the batched solves, kept from one batch to the next
+  std::mutex mutex;
+  std::vector<omvgba::Context*> workers;  // of the batched solves, kept from one batch to the next; a batch in
+                                          // progress has taken them out
 };
 
 using namespace omvgba;
@@ -2031,7 +2033,7 @@ omvgba_context* omvgba_context_create(int32_t device, omvgba_error* error) {
     error->code = 0;
     error->message[0] = 0;
   }
-  return new omvgba_context{c, {}};
+  return new omvgba_context{c, {}, {}};
 }
 
 void omvgba_context_destroy(omvgba_context* context) {
@@ -2161,13 +2163,19 @@ int32_t omvgba_solve_batched(omvgba_context* context, uint64_t window_count, con
   std::mutex setup_mutex;
   omvgba_config cfg = *config;
   cfg.stream = nullptr;  // every worker runs on its own context's stream
-  // worker w's context (stream, pinned memory, device memory pool) stays for the next batch
-  if (context->workers.size() < workers) context->workers.resize(workers, nullptr);
+  // worker w's context (stream, pinned memory, device memory pool) stays for the next batch; batches that run
+  // at the same time have workers of their own, and those of the first to end are kept
+  std::vector<Context*> contexts;
+  {
+    std::lock_guard<std::mutex> lock(context->mutex);
+    contexts.swap(context->workers);
+  }
+  if (contexts.size() < workers) contexts.resize(workers, nullptr);
   const unsigned threads_each = std::max<unsigned>(1, host_thread_limit() / (unsigned)std::max<uint64_t>(workers, 1));
   auto worker = [&](uint64_t w) {
     std::string msg;
     set_host_thread_limit(threads_each);
-    Context*& ctx = context->workers[w];
+    Context*& ctx = contexts[w];
     if (!ctx) ctx = context_create(device, &msg);
     if (!ctx) {
       std::lock_guard<std::mutex> lock(setup_mutex);
@@ -2194,6 +2202,11 @@ int32_t omvgba_solve_batched(omvgba_context* context, uint64_t window_count, con
   std::vector<std::thread> pool;
   for (uint64_t w = 0; w < workers; ++w) pool.emplace_back(worker, w);
   for (auto& t : pool) t.join();
+  {
+    std::lock_guard<std::mutex> lock(context->mutex);
+    if (context->workers.empty()) contexts.swap(context->workers);
+  }
+  for (Context* c : contexts) context_destroy(c);
   if (!setup_error.empty() && next.load() < window_count) return write_error(error, OMVGBA_CUDA_ERROR, setup_error);
   for (uint64_t i = 0; i < window_count; ++i)
     if (codes[i] != OMVGBA_OK) {

@@ -57,3 +57,16 @@ def test_plans_of_one_context_on_their_own_streams(adjuster, solver):
     finally:
         for plan in plans:
             plan.close()
+
+
+def test_batches_on_one_context(adjuster):
+    """More batches at a time than one, of different sizes, twice over: each has workers of its own."""
+    windows = synthetic.window_problems(seed=32, windows=10, total_observations=30_000, min_points=200, max_points=2000,
+                                        max_cameras=16)
+    cfg = SolveConfig(max_iterations=10)
+    alone = [adjuster.solve(w, cfg) for w in windows]
+    for _ in range(2):
+        together = _in_threads([lambda n=n: adjuster.solve_batched(windows[:n], cfg) for n in (10, 3, 7)])
+        for batch in together:
+            for a, b in zip(alone, batch):
+                _same(a, b)
