@@ -226,7 +226,13 @@ typedef struct omvgba_solution {
   omvgba_report report;
 } omvgba_solution;
 
-/* One solver context per thread or stream: device workspaces, streams, no global state. */
+/*
+ * One solver context per thread or stream: device workspaces, streams, no global state. Between calls a
+ * context keeps up to 256 MiB of device memory and about 4 MiB of pinned host memory (for each of the calls
+ * that have run on it at the same time); after a batched solve its workers (16, or OMVGBA_BATCH_WORKERS) keep
+ * as much pinned memory each and 256 MiB of device memory between them. omvgba_context_destroy gives all of
+ * it back.
+ */
 typedef struct omvgba_context omvgba_context;
 
 /* Number of CUDA devices visible to this process (0 when none or when the driver is missing). */

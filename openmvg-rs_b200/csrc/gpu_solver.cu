@@ -416,6 +416,12 @@ int context_device(const Context* c) { return c->device; }
 void* context_stream(const Context* c) { return (void*)c->stream; }
 void* context_pool(const Context* c) { return (void*)c->pool; }
 
+void context_trim(Context* c, unsigned contexts) {
+  if (!c) return;
+  (void)cudaStreamSynchronize(c->stream);  // memory counts as free once the stream has passed its release
+  (void)cudaMemPoolTrimTo(c->pool, kPoolKept / std::max(contexts, 1u));
+}
+
 void context_destroy(Context* c) {
   if (!c) return;
   cudaSetDevice(c->device);

@@ -2202,6 +2202,7 @@ int32_t omvgba_solve_batched(omvgba_context* context, uint64_t window_count, con
   std::vector<std::thread> pool;
   for (uint64_t w = 0; w < workers; ++w) pool.emplace_back(worker, w);
   for (auto& t : pool) t.join();
+  for (Context* c : contexts) context_trim(c, (unsigned)contexts.size());
   {
     std::lock_guard<std::mutex> lock(context->mutex);
     if (context->workers.empty()) contexts.swap(context->workers);
