@@ -2502,9 +2502,10 @@ extern "C" int32_t omvgba_sfm_refresh_reprojection(omvgba_context* context, uint
               !result->track_support))
       return write_error(error, OMVGBA_INVALID_ARGUMENT, "null track array");
     // each chunk stops at its first bad index; the first chunk with one decides the message
-    // (a quarter million entries, about 0.2 ms, before another thread is worth its start)
+    // (a quarter million entries, about 0.2 ms, before another thread is worth its start; each chunk clears
+    // and merges a flag per intrinsic, so no more chunks than their entries outweigh)
     constexpr size_t kGrain = 262144;
-    const size_t chunks = N <= kGrain ? 1 : 64;
+    const size_t chunks = N <= kGrain ? 1 : (size_t)std::clamp<uint64_t>(N / std::max<uint64_t>(intrinsic_count, 1), 1, 64);
     std::vector<std::vector<uint8_t>> chunk_used(chunks, std::vector<uint8_t>(intrinsic_count, 0));
     std::vector<const char*> bad(chunks, nullptr);
     for_fixed_chunks(
