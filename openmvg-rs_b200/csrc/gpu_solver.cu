@@ -1406,17 +1406,6 @@ __global__ void k_block_precond(BlockTables bt, const double* factor, const doub
   for (int i = 0; i < d; ++i) z[o + i] = s[i] / F[36 + i];
 }
 
-__global__ void k_axpy2(int n, double alpha, const double* d, const double* q, double* x, double* r) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    x[i] += alpha * d[i];
-    r[i] -= alpha * q[i];
-  }
-}
-__global__ void k_xpby(int n, const double* z, double beta, double* d) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) d[i] = z[i] + beta * d[i];
-}
 __global__ void k_neg_copy(int n, const double* a, double* b) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = -a[i];
@@ -1428,10 +1417,6 @@ __global__ void k_sub(int n, const double* b, const double* q, double* r) {
 __global__ void k_axpy(int n, double a, const double* x, double* y) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] += a * x[i];
-}
-__global__ void k_residual_update(int n, const double* g, const double* q, double* r) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) r[i] = -g[i] - q[i];
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -2589,7 +2574,6 @@ struct Solver {
   DBuf<RedVec<4>> d_cand, d_cand_part;
   DBuf<RedVec<3>> d_met, d_met_part;
   DBuf<RedVec<1>> d_one, d_one_part;
-  DBuf<RedVec<1>> d_norm_part;
   int red_blocks;
   uint64_t workspace_bytes = 0;
   bool explicit_op = false;
@@ -3168,7 +3152,9 @@ struct Solver {
     sync();
     // items of at most 256 entries, fewer when that would leave less than two items per resident warp slot
     // of the chip's SMs
-    t.chunk = (uint32_t)std::min<uint64_t>(256, std::max<uint64_t>(32, entries / (148 * 32) / 32 * 32));
+    int sms = 0;
+    CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    t.chunk = (uint32_t)std::min<uint64_t>(256, std::max<uint64_t>(32, entries / (32 * (uint64_t)sms) / 32 * 32));
     if (!take(d_pr_entries, entries)) return false;
     CUDA_OK(cudaMemcpyAsync(cursor.p, d_pr_list_begin.p, sizeof(uint64_t) * (cells + 1), cudaMemcpyDeviceToDevice, st));
     OMVGBA_LAUNCH(k_pair_lists<uint64_t>, dim3(ncam, t.segs), 32, 0, st, t, cursor.p, d_pr_entries.p);
@@ -3198,7 +3184,7 @@ struct Solver {
       if (n.self_cal)
         if (const int b = S.grp_block[n.cam_group[c]]; b >= 0) bc_cams[at[b]++] = (uint32_t)c;
     }
-    DBuf<uint32_t> d_bc_begin, d_bc_cams, heavy_n;
+    DBuf<uint32_t> d_bc_begin, d_bc_cams;
     DBuf<int> d_blk_pose, d_blk_group;
     auto up = [&](auto& buffer, const auto& host) {
       if (!take(buffer, host.size())) return false;

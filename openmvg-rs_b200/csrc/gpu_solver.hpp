@@ -161,9 +161,9 @@ void* context_pool(const Context* ctx);    // the context's cudaMemPool_t
 // Gives back the device memory that the context keeps beyond its share of one context's allowance.
 void context_trim(Context* ctx, unsigned contexts);
 
-// Copies between pageable host memory and the device on a stream (a cudaStream_t), cudaSuccess or the
-// error. Large ones go through two pinned chunks, several host threads filling (emptying) one while the
-// other's DMA runs; downloads have arrived on return, uploads' sources may change.
+// Copies between host memory and the device on a stream (a cudaStream_t), cudaSuccess or the error. Large ones
+// go through two pinned chunks, several host threads filling (emptying) one while the other's DMA runs. In
+// both directions the host memory must stay valid, and untouched, until the stream has been waited for.
 int copy_to_device(void* dst, const void* src, size_t bytes, void* stream);
 int copy_from_device(void* dst, const void* src, size_t bytes, void* stream);
 
