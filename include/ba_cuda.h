@@ -230,8 +230,8 @@ typedef struct omvgba_solution {
  * One solver context per thread or stream: device workspaces, streams, no global state. Between calls a
  * context keeps up to 256 MiB of device memory and about 4 MiB of pinned host memory (for each of the calls
  * that have run on it at the same time); after a batched solve its workers (16, or OMVGBA_BATCH_WORKERS) keep
- * as much pinned memory each and 256 MiB of device memory between them. omvgba_context_destroy gives all of
- * it back.
+ * as much pinned memory each, and 256 MiB of device memory each up to 2 GiB between them.
+ * omvgba_context_destroy gives all of it back.
  */
 typedef struct omvgba_context omvgba_context;
 

@@ -158,7 +158,7 @@ Context* context_create(int device, std::string* error);
 int context_device(const Context* ctx);
 void* context_stream(const Context* ctx);  // the context's cudaStream_t
 void* context_pool(const Context* ctx);    // the context's cudaMemPool_t
-// Gives back the device memory that the context keeps beyond its share of one context's allowance.
+// Gives back the device memory that a batch's worker context keeps beyond its share of the batch's allowance.
 void context_trim(Context* ctx, unsigned contexts);
 
 // Copies between host memory and the device on a stream (a cudaStream_t), cudaSuccess or the error. Large ones

@@ -45,11 +45,11 @@ def test_a_failing_window_is_reported_by_index(adjuster, windows):
 
 def test_workers_share_one_allowance_of_device_memory():
     """What the workers of a batch keep afterwards does not grow with their number or with the windows: with
-    the context's own allowance at most 512 MiB, plus the pools' granularity (a few MiB each). A window here
-    takes about 0.1 GB, 16 of them six times what may stay."""
+    the context's own allowance at most 2.25 GiB, plus the pools' granularity (a few MiB each). A window here
+    takes more than 0.25 GB, 16 of them twice what may stay."""
     torch = pytest.importorskip("torch")
     from openmvg_ba_cuda.adjuster import CudaBundleAdjuster
-    w = synthetic.plane_problem(seed=33, cameras=40, points=30_000, mean_track=6.0, extent=30.0,
+    w = synthetic.plane_problem(seed=33, cameras=40, points=60_000, mean_track=6.0, extent=30.0,
                                 per_camera_intrinsics=False, free_intrinsics=False)
     cfg = SolveConfig(max_iterations=2)
     with CudaBundleAdjuster(0) as warm:  # modules and other lasting memory of the process
@@ -62,5 +62,5 @@ def test_workers_share_one_allowance_of_device_memory():
         kept = before - torch.cuda.mem_get_info()[0]
         own.solve_batched([w] * 2, cfg)
     torch.cuda.synchronize()
-    assert kept <= (512 << 20) + 17 * (8 << 20)
+    assert kept <= (2304 << 20) + 17 * (8 << 20)
     assert before - torch.cuda.mem_get_info()[0] <= 64 << 20  # given back with the context
