@@ -255,9 +255,11 @@ const char* omvgba_adjuster_name(void);
  * device memory happen in omvgba_plan_create; every omvgba_plan_solve then starts from the
  * problem's initial state with everything already in device memory, and returns what omvgba_solve
  * would return for the same problem and config. The problem's arrays must stay alive and unchanged
- * until omvgba_plan_destroy. A plan runs on config->stream (or the context's stream) and, like its
- * context, is used by one thread at a time. No reference counterpart: the reference lowers and
- * solves in one call (native/mod.rs:117-367).
+ * until omvgba_plan_destroy. A plan runs on config->stream (or the context's stream) and is used by one
+ * thread at a time; plans of one context on streams of their own may run at the same time. Its first solve
+ * adds, and the plan keeps, the factor's band, the selected inverse's (self-calibration) and, where the
+ * budget and the device have room, the camera-pair tables (up to 48 GiB); omvgba_plan_info leaves them out.
+ * No reference counterpart: the reference lowers and solves in one call (native/mod.rs:117-367).
  */
 typedef struct omvgba_plan omvgba_plan;
 
@@ -287,7 +289,8 @@ int32_t omvgba_plan_info_get(const omvgba_plan* plan, omvgba_plan_info* info, om
  * explicit S of the linearization (x and y untouched), for timing that build; stage 3
  * runs only the camera-side sums of the linearization's assembly (U blocks, gradients, damping
  * diagonal, pose/intrinsic edges and point coupling per block; x and y untouched). Runs on
- * the plan's stream without synchronizing. Operator: retained/operator.rs:137-227.
+ * the plan's stream without synchronizing, but for the first call and each that re-linearizes, and the
+ * first build of the explicit S, which makes its tables. Operator: retained/operator.rs:137-227.
  */
 int32_t omvgba_plan_schur_product(omvgba_plan* plan, double lambda, int32_t fp32, int32_t stage, const double* x,
                                   double* y, omvgba_error* error);
