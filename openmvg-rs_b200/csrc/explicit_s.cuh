@@ -1059,11 +1059,10 @@ __global__ void k_z_marginals(TileBand Z, int ngroups, const int* __restrict__ p
 // One cluster of kLoopCtas CTAs runs a whole iteration (power iteration, PCG), so the host waits once and
 // no launch lies between two products. CTA r owns the block rows X = r mod kLoopCtas; a task is 32 blocks
 // of one row, a block per lane. Every CTA keeps the whole iterate in shared memory; a row's results go to
-// all CTAs' shared memory and one cluster barrier ends the product. A row without blocks (a free parameter
-// block that no observation touches) has one empty task, so that its results, zeros, are written like every
-// row's. While a CTA's tasks fit (kLoopTasks,
-// a warp each) their blocks stay in shared memory too, element by element with the lanes side by side: the
-// cluster barrier drops L1, so each iteration would otherwise wait for L2 three times over.
+// all CTAs' shared memory and one cluster barrier ends the product. Every row has a block, its own at least,
+// and so a task that writes its results. While a CTA's tasks fit (kLoopTasks, a warp each) their blocks
+// stay in shared memory too, element by element with the lanes side by side: the cluster barrier drops L1, so
+// each iteration would otherwise wait for L2 three times over.
 constexpr int kLoopCtas = 8;
 constexpr int kLoopThreads = 512;
 constexpr int kLoopWarps = kLoopThreads / 32;
@@ -1075,9 +1074,7 @@ struct LoopTasks {
   int count;                                 // above kLoopTasks: not cached
   double part[kLoopWarps][6];
 };
-__host__ __device__ __forceinline__ int loop_row_tasks(uint32_t blocks) {
-  return blocks > 0 ? (int)((blocks + 31) / 32) : 1;
-}
+__host__ __device__ __forceinline__ int loop_row_tasks(uint32_t blocks) { return (int)((blocks + 31) / 32); }
 
 // The CTA's tasks in row order (thread 0, before a barrier).
 __device__ __forceinline__ void loop_list(const RowTables& rt, int rank, LoopTasks& t) {

@@ -2174,8 +2174,8 @@ static void build_tables(const NativeProblem& n, const Layout& L, Setup& S) {
   S.ent_block = std::move(ent_block);
 }
 
-// Neighbour lists of the explicit S (every block Y that shares a point with block X, X included,
-// ascending), the offsets of the row blocks, and the factorization order: each camera's pose block,
+// Neighbour lists of the explicit S (every block Y that shares a point with block X, and X itself, also
+// where no observation touches it: the damping lies on its diagonal; ascending), the offsets of the row blocks, and the factorization order: each camera's pose block,
 // then the intrinsic blocks whose first camera it is (cameras in native order), which makes the
 // reduced system of a survey banded. bwt is the band of the factor in tiles.
 static void build_explicit(const NativeProblem& n, const Layout& L, Setup& S) {
@@ -2193,6 +2193,8 @@ static void build_explicit(const NativeProblem& n, const Layout& L, Setup& S) {
     std::vector<int> stamp(nb, -1);
     for (size_t X = b0; X < b1; ++X) {
       std::vector<int>& out = nbrs[X];
+      stamp[X] = (int)X;
+      out.push_back((int)X);
       for (uint32_t i = S.blk_ent[X]; i < S.blk_ent[X + 1]; ++i) {
         const uint32_t p = S.ent_point[i];
         for (uint64_t o = n.pt_off[p]; o < n.pt_off[p + 1]; ++o)
@@ -2283,7 +2285,7 @@ static void pattern_counts(const NativeProblem& n, const Layout& L, const Setup&
     for (uint32_t q = S.nbr_begin[X]; q < S.nbr_begin[X + 1]; ++q) {
       const int Y = S.nbr[q];
       if (Y < X) nnz += dX * (uint64_t)S.blk_dim[Y];
-      if (Y == X) nnz += dX * (dX + 1) / 2;
+      if (Y == X && S.blk_ent[X + 1] > S.blk_ent[X]) nnz += dX * (dX + 1) / 2;  // a block some point touches
     }
   }
   uint64_t rows = 0;

@@ -50,3 +50,22 @@ def test_wide_band_step_matches_oracle(adjuster):
         assert g.report[k] == o.report[k], k
     assert np.array_equal(g.unconstrained_intrinsics, o.unconstrained_intrinsics)
     assert abs(g.report["final_objective"] - o.report["final_objective"]) <= 1e-9 * o.report["final_objective"]
+
+
+@pytest.mark.parametrize("cameras,unobserved", [(13, 3), (13, 12), (60, 20)])
+@pytest.mark.parametrize("solver", [abi.SOLVER_DIRECT, abi.SOLVER_AUTO])
+def test_a_free_camera_without_observations_takes_a_zero_step(adjuster, cameras, unobserved, solver):
+    """S is zero there and the damping its only diagonal: the factor succeeds, the camera stays, and the rank
+    test of the undamped system finds the zero row, as in the oracle."""
+    p = synthetic.ring_problem(seed=8, cameras=cameras, points=400)
+    keep = p.observation_pose != unobserved
+    for k in ("observation_pose", "observation_intrinsic", "observation_point", "observation_pixel"):
+        setattr(p, k, getattr(p, k)[keep])
+    cfg = SolveConfig(linear_solver=solver, max_iterations=2)
+    g, o = adjuster.solve(p, cfg), O.solve(p, cfg)
+    for k in ("iteration_count", "accepted_step_count", "rejected_step_count", "status", "observability"):
+        assert g.report[k] == o.report[k], k
+    assert g.report["accepted_step_count"] > 0
+    assert abs(g.report["final_objective"] - o.report["final_objective"]) <= 1e-9 * o.report["final_objective"]
+    assert np.max(np.abs(g.rotations - o.rotations)) < 1e-7
+    assert np.max(np.abs(g.centers - o.centers)) < 1e-7
