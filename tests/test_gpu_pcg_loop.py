@@ -89,7 +89,7 @@ def _without(p, drop):
 @pytest.mark.parametrize("case", [_unobserved_pose, _unobserved_group])
 @pytest.mark.parametrize("limit", [0, 3])
 def test_a_free_block_without_observations(adjuster, case, limit):
-    """Its row of S is empty: the product there is lambda diag x and its step is zero, in the cluster kernel
+    """Its row of S is zero: the product there is lambda diag x and its step is zero, in the cluster kernel
     as in the matrix-free product; the rank test sees a zero row whichever operator took the steps."""
     p = case()
     cfg = SolveConfig(linear_solver=abi.SOLVER_ITERATIVE, max_iterations=6, pcg_relative_tolerance=1e-10,
